@@ -140,6 +140,19 @@ def test_linear_cross_entropy(chunk, monkeypatch):
     torch.testing.assert_close(w.main_grad, w2.grad, rtol=1e-5, atol=1e-6)
 
 
+def test_linear_cross_entropy_without_grad_leaves_gradients_alone():
+    from train_large_model_from_scratch_b200.ops import functional as Fo
+    torch.manual_seed(2)
+    w = torch.nn.Parameter(torch.randn(24, 16))
+    w.main_grad = torch.full((24, 16), 3.0)
+    h, t = torch.randn(10, 16, requires_grad=True), torch.randint(0, 24, (10,))
+    with torch.no_grad():
+        s = Fo.linear_cross_entropy(h, w, t, torch.tensor(0.1))
+    assert abs(s.item() - torch.nn.functional.cross_entropy(h @ w.t(), t, reduction="sum").item()) < 1e-3
+    assert torch.equal(w.main_grad, torch.full((24, 16), 3.0)) and not s.requires_grad
+
+
+
 def test_moe_local_matches_oracle_and_grads():
     torch.manual_seed(1)
     M, D, I, E, k = 24, 16, 12, 4, 2

@@ -391,9 +391,8 @@ class _LinearCrossEntropy(torch.autograd.Function):
     CHUNK_ROWS_CPU = 8192      # the fp32 path keeps its transient logits small
 
     @staticmethod
-    def forward(ctx, h, weight, targets, grad_scale, ignore_index):
+    def forward(ctx, h, weight, targets, grad_scale, ignore_index, need_grad):
         M = h.shape[0]
-        need_grad = bool(ctx.needs_input_grad[0] or ctx.needs_input_grad[1])
         if not need_grad and _use_native(h, weight) and weight.shape[0] % 8 == 0:
             # evaluation: the loss needs no logits at all (statistics in the GEMM epilogue, see native)
             ctx.dh = None
@@ -465,7 +464,7 @@ class _LinearCrossEntropy(torch.autograd.Function):
                                     rtol=1e-3, atol=0.0):
                 raise RuntimeError("linear_cross_entropy: the upstream gradient differs from grad_scale; multiply "
                                    "the returned sum by exactly the grad_scale that was passed in")
-        return dh, None, None, None, None
+        return dh, None, None, None, None, None
 
 
 def _lm_head_recompute() -> bool:
@@ -476,7 +475,11 @@ def _lm_head_recompute() -> bool:
 
 
 def linear_cross_entropy(h, weight, targets, grad_scale, ignore_index: int = -100) -> torch.Tensor:
-    return _LinearCrossEntropy.apply(h, weight, targets.reshape(-1), grad_scale, ignore_index)
+    # `needs_input_grad` only says that an input requires a gradient, not that gradients are being recorded: under
+    # no_grad the forward would still run the dgrad and wgrad GEMMs and add into the parameters' gradient buffer.
+    # Evaluation of the 16-layer, hidden-1024 model at 8 x 4096 tokens: 33.95 ms with them, 27.0 ms without.
+    need_grad = torch.is_grad_enabled() and (h.requires_grad or weight.requires_grad)
+    return _LinearCrossEntropy.apply(h, weight, targets.reshape(-1), grad_scale, ignore_index, need_grad)
 
 
 def cross_entropy_from_logits(logits: torch.Tensor, targets: torch.Tensor, ignore_index: int = -100):
