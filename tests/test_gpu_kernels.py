@@ -303,6 +303,29 @@ def test_grouped_gemms(nat, gemm_mode, counts, N, K):
         r += c
 
 
+@pytest.mark.parametrize("E", [255, 256, 257, 300])
+def test_row_grouped_gemms_around_the_group_limit_of_a_launch(nat, gemm_mode, E):
+    """256 groups fit one launch's tile list, more run as several launches: ragged groups (empty ones, one of more than
+    two row tiles), gate|up + SwiGLU and the plain grouped product; rows behind the last group keep their content."""
+    counts = [(37 * i) % 61 if i % 7 else 0 for i in range(E)]
+    counts[E // 2], counts[-1] = 530, 45
+    I, D, R = 128, 64, sum(counts)
+    x, w_pair = _rand(R + 40, D, seed=70), _rand(2 * E, I, D, seed=71, scale=0.2)
+    rs = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32, device="cuda")
+    gu, act = nat.grouped_gemm_swiglu(x, w_pair, nat.DeviceCounts(rs, R))
+    out = torch.full((R + 40, I), 7.0, device="cuda").bfloat16()
+    nat._check(nat.lib().tlm_gemm_grouped_rows(x.data_ptr(), w_pair.data_ptr(), out.data_ptr(), rs.data_ptr(), E, R + 40, I, D,
+                                               D, D, I * D, I, 0, nat.EPI_BF16, R, nat._stream()), "grouped")
+    nat.raise_on_device_status()
+    grp = torch.repeat_interleave(torch.arange(E, device="cuda"), torch.tensor(counts, device="cuda"))
+    g = torch.einsum("rd,rid->ri", x[:R].float(), w_pair[:E].float()[grp])
+    u = torch.einsum("rd,rid->ri", x[:R].float(), w_pair[E:].float()[grp])
+    assert _rel_err(out[:R], g) < 6e-3 and bool((out[R:] == 7.0).all())
+    assert _rel_err(gu[:R, :I], g) < 6e-3 and _rel_err(gu[:R, I:], u) < 6e-3
+    gb, ub = gu[:R, :I].float(), gu[:R, I:].float()
+    assert _rel_err(act[:R], torch.nn.functional.silu(gb) * ub) < 6e-3
+
+
 @pytest.mark.parametrize("M,E,k", [(300, 8, 2), (129, 128, 8), (64, 4, 1), (1000, 40, 3)])
 def test_moe_route_and_row_movement(nat, M, E, k):
     """Device routing (top-k, softmax of the winners, stable expert-major order) and the gather / combine /

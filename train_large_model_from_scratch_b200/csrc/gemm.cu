@@ -36,12 +36,14 @@ constexpr int GEMM_THREADS = 192;
 constexpr int GEMM_THREADS_WIDE = 320;               // 8 epilogue warps (two per TMEM lane quarter) for the heavy epilogue
 constexpr int EPI_BUF_BYTES = 32 * 128;              // one warp's 32 rows x 64 bf16 staging tile
 constexpr int EPI_BYTES = 4 * 2 * EPI_BUF_BYTES;     // 4 epilogue warps x 2 buffers = 32 KB
-constexpr int GEMM_SMEM = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
+constexpr int MAX_GROUPS = 256;                       // groups of one row-grouped launch (more run as several launches)
+constexpr int TAIL_BYTES = 256 /*barriers*/ + (MAX_GROUPS + 1) * 4 + 12 /*row tiles before each group*/;
+constexpr int GEMM_SMEM = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align slack*/ + TAIL_BYTES;
 // CTA pairs (see gemm_body, PAIR): each CTA stages its own 128 rows of A and HALF of the tile's B rows, so a stage is
 // 32 KB per CTA and the ring is six stages deep.
 constexpr int PAIR_STAGES = 6;
 constexpr int PAIR_STAGE_BYTES = A_BYTES + B_BYTES / 2;
-constexpr int GEMM_SMEM_PAIR = PAIR_STAGES * PAIR_STAGE_BYTES + EPI_BYTES + 1024 + 256;
+constexpr int GEMM_SMEM_PAIR = PAIR_STAGES * PAIR_STAGE_BYTES + EPI_BYTES + 1024 + TAIL_BYTES;
 
 enum Epilogue { EPI_BF16 = 0, EPI_F32_ACC = 1, EPI_F32 = 2, EPI_HEADS = 3, EPI_SWIGLU = 4, EPI_SWIGLU_BWD = 5, EPI_LSE = 6,
                 EPI_ROWS = 7 /* bf16 rows stored at looked-up (buffer, row): the expert-parallel combine */ };
@@ -57,12 +59,13 @@ struct GemmParams {
   long long ldc;            // elements
   unsigned int* status;
   // grouped mode (MoE): problem g covers rows [row_start[g], row_start[g+1]) of a
-  // row-grouped operand; see grouped launchers. groups == 0 -> plain GEMM.
+  // row-grouped operand; see grouped launchers. groups == 0 -> plain GEMM. The kernels' GROUP parameter says which
+  // operand is grouped: 1: rows of A/C, B per group (3-D map); 2: K (wgrad), C per group.
   int groups;
   const int* row_start;     // device, groups + 1 entries
-  int group_mode;           // 1: rows of A/C grouped, B per group (3-D map); 2: K grouped (wgrad), C per group
-  long long c_group_stride; // elements between per-group C matrices (mode 2)
-  int max_tiles_m;          // upper bound of m-tiles per group (mode 1)
+  int grp0;                 // rows grouped: index of the launch's first group among the B matrices
+  int up_off;               // rows grouped, paired matrices: distance (in matrices) from a group's first to its second
+  long long c_group_stride; // elements between per-group C matrices (K grouped)
   int split_k;              // plain GEMM with fp32 accumulate: reduction split into this many tiles (>= 1);
                             // with split_k > 1 the epilogue adds with red.global (order not deterministic)
   int k_chunk;              // reduction length per split (multiple of BK)
@@ -85,7 +88,7 @@ struct GemmParams {
   //   columns from `aux` ([M, 2 I], row pitch 2 N) and writes d(gate), d(up) into C = d(gate_up) [M, 2 I].
   // Both round their GEMM result to bf16 first, so the numbers equal the separate GEMM + SwiGLU kernels'.
   const __nv_bfloat16* aux;
-  // Grouped SwiGLU (MoE experts): rows grouped like group_mode 1, B holds 2 * groups matrices (gate of group g at g,
+  // Grouped SwiGLU (MoE experts): rows grouped (GROUP 1), B holds 2 * groups matrices (gate of group g at g,
   // up at groups + g). A tile's rows past its group's end belong to the next group, so warps whose 32 rows cross
   // that end store row by row with a mask instead of with TMA tile stores; `act` / `ld_act` locate the act tensor
   // for those stores.
@@ -184,7 +187,14 @@ __device__ __forceinline__ TileCoord plain_tile(const GemmParams& p, int tile_in
 // 48 KB. Barriers: `full` lives in rank 0 (both producers' loads complete on it), `empty` and `accumulator full` are
 // signalled in both CTAs by the leader's commits, `accumulator empty` lives in rank 0 and collects both CTAs'
 // epilogue warps.
-template <bool A_MN, bool B_MN, int EPI, bool GATED = false, bool PAIR = false>
+//
+// GROUP 1 (rows grouped): the row tiles of all groups form one dense list. A warp turns row_start into the number of row
+// tiles before each group (shared memory) when the kernel starts, and every role walks its share of the list, finding
+// the group by moving forward from the previous tile's. The host only knows an upper bound of a group's rows (all of
+// them): enumerating that many tiles per group and skipping the missing ones took most of the time. Gate|up + SwiGLU of
+// 65536 rows: 128 groups x 512 rows, 2 x 256 columns, K 1024: 317 -> 77 us; 8 groups, 32768 rows, 2 x 2048 columns: 255
+// -> 202 us.
+template <bool A_MN, bool B_MN, int EPI, bool GATED = false, bool PAIR = false, int GROUP = 0>
 __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC,
                                           const GemmParams& p, const CUtensorMap* dst_maps) {
   static_assert(!(PAIR && GATED), "the gated instantiations run as single CTAs");
@@ -207,7 +217,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
   auto acce_bar = [&](int a) { return bar0 + 8u * (2 * STAGES + 2 + a); };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int* tiles_before = reinterpret_cast<int*>(smem_al + STAGES * STAGE_BYTES + EPI_BYTES + 256);    // [groups + 1], GROUP 1
 
+  constexpr int TILE_N = EPI == EPI_SWIGLU ? 128 : BN;      // output columns per tile (SwiGLU: 128 gate + 128 up)
+  constexpr int TILE_M = PAIR ? 2 * BM : BM;                // rows per tile walker
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // The SwiGLU-backward epilogue reads gate / up from global memory and is as long as the main loop of its
   // K = hidden-size tiles, so it runs on 8 warps: warps 2-5 take the left 128 columns, warps 6-9 the right.
@@ -225,35 +238,60 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     if (PAIR) { tmem_alloc_pair(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish_pair(); }
     else { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
   }
+  if (GROUP == 1 && warp == 2) {
+    // exclusive prefix sum of the groups' row-tile counts: lane l owns groups [8 l, 8 l + 8)
+    constexpr int PER = MAX_GROUPS / 32;
+    int n[PER], run = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int g = lane * PER + i;
+      n[i] = g < p.groups ? (p.row_start[g + 1] - p.row_start[g] + TILE_M - 1) / TILE_M : 0;
+      run += n[i];
+    }
+    int before = run;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, before, o);
+      if (lane >= o) before += v;
+    }
+    before -= run;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int g = lane * PER + i;
+      if (g <= p.groups) tiles_before[g] = before;
+      before += n[i];
+    }
+    if (lane == 31 && p.groups == MAX_GROUPS) tiles_before[MAX_GROUPS] = before;
+  }
   tc_fence_before();
   if (PAIR) cluster_sync_all();          // the peer's barriers are initialised before anything signals them
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  constexpr int TILE_N = EPI == EPI_SWIGLU ? 128 : BN;      // output columns per tile (SwiGLU: 128 gate + 128 up)
-  constexpr int TILE_M = PAIR ? 2 * BM : BM;                // rows per tile walker
   const int tiles_n = (p.N + TILE_N - 1) / TILE_N;
-  int tiles_m, total_tiles;
-  if (p.groups == 0) { tiles_m = (p.M + TILE_M - 1) / TILE_M; total_tiles = tiles_m * tiles_n * p.split_k; }
-  else if (p.group_mode == 1) { tiles_m = p.max_tiles_m; total_tiles = p.groups * tiles_m * tiles_n; }
-  else { tiles_m = (p.M + BM - 1) / BM; total_tiles = p.groups * tiles_m * tiles_n; }
+  const int tiles_m = (p.M + TILE_M - 1) / TILE_M;          // GROUP 1: per group instead, see get_tile
+  const int total_tiles = GROUP == 1 ? tiles_before[p.groups] * tiles_n
+                                     : tiles_m * tiles_n * (GROUP == 2 ? p.groups : p.split_k);
 
-  auto get_tile = [&](int tile) -> TileCoord {
-    if (p.groups == 0) return plain_tile(p, tile, tiles_m, tiles_n, TILE_N, TILE_M, (int)cta_rank * BM);
+  // `grp`: the caller's group cursor (GROUP 1), 0 before its first tile; tiles are asked for in ascending order
+  auto get_tile = [&](int tile, int& grp) -> TileCoord {
+    if (GROUP == 0) return plain_tile(p, tile, tiles_m, tiles_n, TILE_N, TILE_M, (int)cta_rank * BM);
     TileCoord t;
-    int per = tiles_m * tiles_n;
-    int g = tile / per, r = tile - g * per;
-    int tm = r % tiles_m, tn = r / tiles_m;
-    int lo = p.row_start[g], hi = p.row_start[g + 1];
-    if (p.group_mode == 1) {            // rows grouped: A rows [lo,hi), B = weight[g]
-      // PAIR: both CTAs of a pair must agree on whether the tile exists, so that is decided on the pair's first row;
-      // a second half that starts past the group's end runs with every row masked
-      const int m_first = lo + tm * TILE_M;
-      t.m0 = m_first + (int)cta_rank * BM; t.a_row0 = t.m0; t.n0 = tn * TILE_N; t.b_grp = g; t.b_n0 = t.n0;
-      if (p.pair_n > 0 && t.n0 >= p.pair_n) { t.b_grp = g + p.groups; t.b_n0 = t.n0 - p.pair_n; }
-      t.k_lo = 0; t.k_hi = p.K; t.m_end = hi; t.c_off = 0; t.valid = m_first < hi;
+    if (GROUP == 1) {                   // rows grouped: A rows [lo,hi), B = weight[g]
+      while (tile >= tiles_before[grp + 1] * tiles_n) ++grp;
+      const int g = grp, first = tiles_before[g], g_tiles = tiles_before[g + 1] - first;
+      const int r = tile - first * tiles_n, tn = r / g_tiles, tm = r - tn * g_tiles;
+      const int lo = p.row_start[g], hi = p.row_start[g + 1];
+      // PAIR: a second half that starts past the group's end runs with every row masked
+      t.m0 = lo + tm * TILE_M + (int)cta_rank * BM; t.a_row0 = t.m0; t.n0 = tn * TILE_N; t.b_grp = g + p.grp0; t.b_n0 = t.n0;
+      if (p.pair_n > 0 && t.n0 >= p.pair_n) { t.b_grp += p.up_off; t.b_n0 = t.n0 - p.pair_n; }
+      t.k_lo = 0; t.k_hi = p.K; t.m_end = hi; t.c_off = 0; t.valid = true;
     } else {                            // reduction grouped: K range [lo,hi), C = C_base + g * stride
+      const int per = tiles_m * tiles_n;
+      const int g = tile / per, r = tile - g * per;
+      const int tm = r % tiles_m, tn = r / tiles_m;
+      const int lo = p.row_start[g], hi = p.row_start[g + 1];
       t.m0 = tm * BM; t.a_row0 = t.m0; t.n0 = tn * BN; t.b_grp = 0; t.b_n0 = t.n0;
       t.k_lo = lo; t.k_hi = hi; t.m_end = p.M; t.c_off = (long long)g * p.c_group_stride; t.valid = hi > lo;
     }
@@ -273,10 +311,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       asm volatile("fence.proxy.async;" ::: "memory");      // the peers' (generic-proxy) stores before this warp's TMA reads
     }
     if (lane == 0 && (!GATED || gate_ok)) {
-      int stage = 0; uint32_t phase = 0;
+      int stage = 0, grp = 0; uint32_t phase = 0;
       bool ok = true;
       for (int tile = worker; tile < total_tiles && ok; tile += n_workers) {
-        TileCoord t = get_tile(tile);
+        TileCoord t = get_tile(tile, grp);
         if (!t.valid) continue;
         for (int k0 = t.k_lo; k0 < t.k_hi; k0 += BK) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, 1, abort_flag, p.status)) { ok = false; break; }
@@ -293,12 +331,12 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             }
             const int half_n0 = (int)cta_rank * (BN / 2);       // this CTA's half of the tile's B rows
             int pbk = k0, pbg = t.b_grp;
-            if (p.pair_k > 0 && k0 >= p.pair_k) { pbk = k0 - p.pair_k; pbg += p.groups; }
+            if (p.pair_k > 0 && k0 >= p.pair_k) { pbk = k0 - p.pair_k; pbg += p.up_off; }
             if (B_MN) {
 #pragma unroll
               for (int j = 0; j < BN / 128; ++j) tma_load_3d_pair(sb + j * BOX_MN_BYTES, &tmB, fb, t.b_n0 + half_n0 + 64 * j, pbk, pbg);
             } else if (EPI == EPI_SWIGLU) {                     // rank 0: 128 gate rows, rank 1: the matching up rows
-              if (p.groups > 0) tma_load_3d_pair(sb, &tmB, fb, k0, t.n0, t.b_grp + (leader ? 0 : p.groups));
+              if (GROUP == 1) tma_load_3d_pair(sb, &tmB, fb, k0, t.n0, t.b_grp + (leader ? 0 : p.up_off));
               else tma_load_3d_pair(sb, &tmB, fb, k0, (leader ? 0 : p.N) + t.n0, 0);
             } else {
               tma_load_3d_pair(sb, &tmB, fb, pbk, t.b_n0 + half_n0, pbg);
@@ -314,14 +352,14 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             tma_load_2d(sa, &tmA, full_bar(stage), k0, t.a_row0);
           }
           int bk = k0, bg = t.b_grp;
-          if (p.pair_k > 0 && k0 >= p.pair_k) { bk = k0 - p.pair_k; bg += p.groups; }
+          if (p.pair_k > 0 && k0 >= p.pair_k) { bk = k0 - p.pair_k; bg += p.up_off; }
           if (B_MN) {
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j) tma_load_3d(sb + j * BOX_MN_BYTES, &tmB, full_bar(stage), t.b_n0 + 64 * j, bk, bg);
           } else if (EPI == EPI_SWIGLU) {       // 128 gate rows, then the matching 128 up rows
-            if (p.groups > 0) {                 // experts: gate matrix of the group, then its up matrix
+            if (GROUP == 1) {                   // experts: gate matrix of the group, then its up matrix
               tma_load_3d(sb, &tmB, full_bar(stage), k0, t.n0, t.b_grp);
-              tma_load_3d(sb + B_BYTES / 2, &tmB, full_bar(stage), k0, t.n0, t.b_grp + p.groups);
+              tma_load_3d(sb + B_BYTES / 2, &tmB, full_bar(stage), k0, t.n0, t.b_grp + p.up_off);
             } else {
               tma_load_3d(sb, &tmB, full_bar(stage), k0, t.n0, 0);
               tma_load_3d(sb + B_BYTES / 2, &tmB, full_bar(stage), k0, p.N + t.n0, 0);
@@ -339,10 +377,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     // shared memory); lane 0 alone issues the MMAs and commits.
     constexpr uint32_t idesc = umma_idesc_bf16(TILE_M, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
     int stage = 0; uint32_t phase = 0;
-    int acc = 0; uint32_t acc_phase = 0;
+    int acc = 0, grp = 0; uint32_t acc_phase = 0;
     bool ok = !PAIR || leader;                      // the follower's MMA warp only allocates and frees tensor memory
     for (int tile = worker; tile < total_tiles && ok; tile += n_workers) {
-      TileCoord t = get_tile(tile);
+      TileCoord t = get_tile(tile, grp);
       if (!t.valid) continue;
       if (!mbar_wait(acce_bar(acc), acc_phase ^ 1u, 2, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
@@ -352,7 +390,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         if (!mbar_wait(full_bar(stage), phase, 3, abort_flag, p.status)) { ok = false; break; }
         tc_fence_after();
         const uint32_t sa = smem_base + stage * STAGE_BYTES, sb = sa + A_BYTES;
-        if (A_MN && B_MN && p.group_mode == 2 && t.k_hi - k0 < BK) {
+        if (GROUP == 2 && t.k_hi - k0 < BK) {
           // grouped reduction: rows past this group's end belong to the next group.
           // Zero them in the A tile (each k index is one 128-byte row per 64-wide box,
           // so whole-row zeroing is independent of the swizzle).
@@ -398,10 +436,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)
     const int q = warp & 3;                        // TMEM lane quarter this warp may read
-    int acc = 0; uint32_t acc_phase = 0;
+    int acc = 0, grp = 0; uint32_t acc_phase = 0;
     bool ok = true;
     for (int tile = worker; tile < total_tiles && ok; tile += n_workers) {
-      TileCoord t = get_tile(tile);
+      TileCoord t = get_tile(tile, grp);
       if (!t.valid) continue;
       if (EPI == EPI_SWIGLU_BWD) {
         // gate / up of the NEXT tile start moving into L2 now, a whole tile time before they are read
@@ -418,7 +456,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         };
         if (tile == worker) prefetch_aux(t);
         const int nxt = tile + n_workers;
-        if (nxt < total_tiles) { const TileCoord tn = get_tile(nxt); if (tn.valid) prefetch_aux(tn); }
+        int ngrp = grp;
+        if (nxt < total_tiles) { const TileCoord tn = get_tile(nxt, ngrp); if (tn.valid) prefetch_aux(tn); }
       }
       if (!mbar_wait(accf_bar(acc), acc_phase, 4, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
@@ -737,7 +776,9 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         }
         if (row_ok) p.lse_part[(long long)row * p.lse_tiles + t.n0 / BN] = make_float2(m_run, s_run);
       } else if (EPI == EPI_BF16 && p.tma_store) {
-        // 64-column slabs: TMEM -> bf16 -> swizzled staging tile -> TMA store (clips at the matrix edge).
+        // 64-column slabs: TMEM -> bf16 -> swizzled staging tile -> TMA store (clips at the matrix edge). GROUP 1: a warp
+        // whose 32 rows cross the end of the tile's group stores its own rows one by one.
+        const bool whole = GROUP != 1 || t.m0 + q * 32 + 32 <= t.m_end;
         uint8_t* ebuf = smem_al + STAGES * STAGE_BYTES + (warp - 2) * 2 * EPI_BUF_BYTES;
         const uint32_t ebuf_s = smem_base + STAGES * STAGE_BYTES + (warp - 2) * 2 * EPI_BUF_BYTES;
 #pragma unroll 1
@@ -770,6 +811,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             }
           }
           uint8_t* rowp = ebuf + bsel * EPI_BUF_BYTES + lane * 128;
+          __nv_bfloat16* grow = reinterpret_cast<__nv_bfloat16*>(p.C) + (long long)row * p.ldc + t.n0 + slab * 64;
 #pragma unroll
           for (int ch = 0; ch < 8; ++ch) {
             const uint32_t* r = ch < 4 ? r0 : r1;
@@ -779,13 +821,14 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             v.y = pack_bf16(__uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
             v.z = pack_bf16(__uint_as_float(r[j + 4]), __uint_as_float(r[j + 5]));
             v.w = pack_bf16(__uint_as_float(r[j + 6]), __uint_as_float(r[j + 7]));
-            *reinterpret_cast<uint4*>(rowp + ((ch ^ (lane & 7)) << 4)) = v;
+            if (GROUP != 1 || whole) *reinterpret_cast<uint4*>(rowp + ((ch ^ (lane & 7)) << 4)) = v;
+            else if (row_ok && t.n0 + slab * 64 + ch * 8 < p.N) *reinterpret_cast<uint4*>(grow + ch * 8) = v;
           }
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
             const int c0 = t.n0 + slab * 64, c1 = t.m0 + q * 32;
-            if (c0 < p.N && c1 < p.M)
+            if (whole && c0 < p.N && c1 < p.M)
               asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
                            ::"l"((uint64_t)&tmC), "r"(ebuf_s + bsel * EPI_BUF_BYTES), "r"(c0), "r"(c1) : "memory");
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
@@ -934,11 +977,11 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
   }
 }
 
-template <bool A_MN, bool B_MN, int EPI, bool GATED = false>
+template <bool A_MN, bool B_MN, int EPI, bool GATED = false, int GROUP = 0>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ CUtensorMap tmC, const GemmParams p) {
-  gemm_body<A_MN, B_MN, EPI, GATED>(tmA, tmB, tmC, p, nullptr);
+  gemm_body<A_MN, B_MN, EPI, GATED, false, GROUP>(tmA, tmB, tmC, p, nullptr);
 }
 
 // Same main loop, head-scatter epilogue: the output maps (one per destination rank) replace the C map.
@@ -951,23 +994,25 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 
 // MLP forward / backward with the SwiGLU math in the epilogue: `tmC` is the [M, 2 I] tensor the epilogue
 // stores gate|up (forward) or d(gate)|d(up) (backward) into, `tmD` the forward's act [M, I].
+template <int GROUP>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_swiglu_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmD, const GemmParams p) {
-  gemm_body<false, false, EPI_SWIGLU>(tmA, tmB, tmC, p, &tmD);
+  gemm_body<false, false, EPI_SWIGLU, false, false, GROUP>(tmA, tmB, tmC, p, &tmD);
 }
+template <int GROUP>
 __global__ void __launch_bounds__(GEMM_THREADS_WIDE, 1)
 gemm_swiglu_bwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                        const __grid_constant__ CUtensorMap tmC, const GemmParams p) {
-  gemm_body<false, true, EPI_SWIGLU_BWD>(tmA, tmB, tmC, p, nullptr);
+  gemm_body<false, true, EPI_SWIGLU_BWD, false, false, GROUP>(tmA, tmB, tmC, p, nullptr);
 }
 
 // CTA-pair instantiations (clusters of two CTAs, see gemm_body): plain GEMMs and the dense fused epilogues.
-template <bool A_MN, bool B_MN, int EPI>
+template <bool A_MN, bool B_MN, int EPI, int GROUP = 0>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const GemmParams p) {
-  gemm_body<A_MN, B_MN, EPI, false, true>(tmA, tmB, tmC, p, nullptr);
+  gemm_body<A_MN, B_MN, EPI, false, true, GROUP>(tmA, tmB, tmC, p, nullptr);
 }
 template <bool B_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
@@ -975,16 +1020,18 @@ gemm_heads_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
                        const __grid_constant__ HeadDstMaps dst, const GemmParams p) {
   gemm_body<false, B_MN, EPI_HEADS, false, true>(tmA, tmB, tmA, p, dst.m);
 }
+template <int GROUP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_swiglu_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                         const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmD,
                         const GemmParams p) {
-  gemm_body<false, false, EPI_SWIGLU, false, true>(tmA, tmB, tmC, p, &tmD);
+  gemm_body<false, false, EPI_SWIGLU, false, true, GROUP>(tmA, tmB, tmC, p, &tmD);
 }
+template <int GROUP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS_WIDE, 1)
 gemm_swiglu_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                             const __grid_constant__ CUtensorMap tmC, const GemmParams p) {
-  gemm_body<false, true, EPI_SWIGLU_BWD, false, true>(tmA, tmB, tmC, p, nullptr);
+  gemm_body<false, true, EPI_SWIGLU_BWD, false, true, GROUP>(tmA, tmB, tmC, p, nullptr);
 }
 
 // ---- host side ---------------------------------------------------------------------------------
@@ -1006,6 +1053,22 @@ static bool use_pair_grouped(int M, int groups) { return use_pair(M) && (g_pair_
 static int pair_grid(long long tiles) {
   const int walkers = num_sms() / 2;
   return 2 * (int)(tiles < walkers ? tiles : walkers);
+}
+// Row-grouped launch: `launch(params, tiles)` for every MAX_GROUPS groups (one launch up to 256 groups); `tiles` bounds
+// the tiles of the chunk: no group has more than `max_rows` rows, all of them together at most `rows`.
+template <typename F>
+static int for_group_chunks(GemmParams p, int groups, const int* row_start, int rows, int max_rows, int tiles_n, bool pair, F launch) {
+  const int tm = pair ? 2 * BM : BM;
+  for (int g0 = 0; g0 < groups; g0 += MAX_GROUPS) {
+    p.groups = groups - g0 < MAX_GROUPS ? groups - g0 : MAX_GROUPS;
+    p.row_start = row_start + g0;
+    p.grp0 = g0;
+    long long tiles = (long long)p.groups * ((max_rows + tm - 1) / tm);
+    if (tiles > rows / tm + p.groups) tiles = rows / tm + p.groups;
+    const int e = launch(p, (int)(tiles * tiles_n));
+    if (e) return e;
+  }
+  return 0;
 }
 // Operand description: `ptr` points at element (0,0); K-major operands are
 // [rows, K] with leading dimension `ld`; MN-major operands are [K, rows] with
@@ -1035,11 +1098,11 @@ static int build_map(CUtensorMap* map, const Operand& o, int box_rows) {
   return make_tmap_bf16(map, o.ptr, rank, dims, strides, box);
 }
 
-template <bool A_MN, bool B_MN, int EPI, bool GATED = false>
+template <bool A_MN, bool B_MN, int EPI, bool GATED = false, int GROUP = 0>
 static int launch_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const GemmParams& p, int tiles,
                     cudaStream_t st) {
   static bool configured = false;
-  auto kern = gemm_kernel<A_MN, B_MN, EPI, GATED>;
+  auto kern = gemm_kernel<A_MN, B_MN, EPI, GATED, GROUP>;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
     if (e != cudaSuccess) return (int)e;
@@ -1052,11 +1115,11 @@ static int launch_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensor
   return launch_status();
 }
 
-template <bool A_MN, bool B_MN, int EPI>
+template <bool A_MN, bool B_MN, int EPI, int GROUP = 0>
 static int launch_pair_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const GemmParams& p,
                          int tiles, cudaStream_t st) {
   static bool configured = false;
-  auto kern = gemm_pair_kernel<A_MN, B_MN, EPI>;
+  auto kern = gemm_pair_kernel<A_MN, B_MN, EPI, GROUP>;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_PAIR);
     if (e != cudaSuccess) return (int)e;
@@ -1071,17 +1134,17 @@ static int launch_pair_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUt
 
 // `pair`: `tiles` counts 256-row tiles and the B map was built with 128-row boxes (see pair_maps)
 static int dispatch(bool a_mn, bool b_mn, int epi, const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p,
-                    int tiles, cudaStream_t st, bool pair = false) {
+                    int tiles, cudaStream_t st, bool pair = false, int group = 0) {
   CUtensorMap mc = ma;                      // placeholder when the TMA-store epilogue is off
   if (p.split_k < 1) { p.split_k = 1; p.k_chunk = p.K; }
-  if (epi == EPI_BF16 && p.groups == 0 && p.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0) {
+  if (epi == EPI_BF16 && group <= 1 && p.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0) {
     uint64_t dims[2] = {(uint64_t)p.N, (uint64_t)p.M}, strides[1] = {(uint64_t)p.ldc * 2};
     uint32_t box[2] = {64, 32};
     if (make_tmap_bf16(&mc, p.C, 2, dims, strides, box) == 0) p.tma_store = 1;
   }
   static int f32_reduce = -1;                 // TLM_GEMM_TMA_REDUCE=0: fp32 accumulation with loads and stores / red.global
   if (f32_reduce < 0) { const char* v = getenv("TLM_GEMM_TMA_REDUCE"); f32_reduce = (v != nullptr && v[0] == '0') ? 0 : 1; }
-  if (epi == EPI_F32_ACC && f32_reduce && p.groups == 0 && p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0) {
+  if (epi == EPI_F32_ACC && f32_reduce && group == 0 && p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0) {
     uint64_t dims[2] = {(uint64_t)p.N, (uint64_t)p.M}, strides[1] = {(uint64_t)p.ldc * 4};
     uint32_t box[2] = {32, 32};
     if (make_tmap_f32(&mc, p.C, 2, dims, strides, box) == 0) p.tma_store = 1;
@@ -1090,15 +1153,17 @@ static int dispatch(bool a_mn, bool b_mn, int epi, const CUtensorMap& ma, const 
   // x W^T with a pending "parameters ready" gate: the gated instantiation (see gemm_body)
   if (!a_mn && !b_mn && epi == EPI_BF16 && p.wait_flags[0] != nullptr)
     return launch_t<false, false, EPI_BF16, true>(ma, mb, mc, p, tiles, st);
-  if (pair && ((p.groups != 0 && p.group_mode != 1) || p.wait_flags[0] != nullptr)) return -8;
-#define TLM_CASE(A, B, E)                                                          \
-  if (a_mn == A && b_mn == B && epi == E)                                          \
-    return pair ? launch_pair_t<A, B, E>(ma, mb, mc, p, tiles, st) : launch_t<A, B, E>(ma, mb, mc, p, tiles, st);
-  TLM_CASE(false, false, EPI_BF16) TLM_CASE(false, true, EPI_BF16) TLM_CASE(true, true, EPI_F32_ACC)
-  TLM_CASE(false, false, EPI_F32) TLM_CASE(true, true, EPI_F32) TLM_CASE(false, false, EPI_F32_ACC)
-  TLM_CASE(true, true, EPI_BF16) TLM_CASE(false, true, EPI_F32) TLM_CASE(false, false, EPI_LSE)
-  TLM_CASE(false, false, EPI_ROWS) TLM_CASE(false, true, EPI_ROWS)
+  if (pair && (group == 2 || p.wait_flags[0] != nullptr)) return -8;
+#define TLM_CASE(A, B, E, G)                                                          \
+  if (a_mn == A && b_mn == B && epi == E && group == G)                               \
+    return pair ? launch_pair_t<A, B, E, G>(ma, mb, mc, p, tiles, st) : launch_t<A, B, E, false, G>(ma, mb, mc, p, tiles, st);
+  TLM_CASE(false, false, EPI_BF16, 0) TLM_CASE(false, true, EPI_BF16, 0) TLM_CASE(true, true, EPI_F32_ACC, 0)
+  TLM_CASE(false, false, EPI_F32, 0) TLM_CASE(true, true, EPI_F32, 0) TLM_CASE(false, false, EPI_F32_ACC, 0)
+  TLM_CASE(true, true, EPI_BF16, 0) TLM_CASE(false, true, EPI_F32, 0) TLM_CASE(false, false, EPI_LSE, 0)
+  TLM_CASE(false, false, EPI_BF16, 1) TLM_CASE(false, true, EPI_BF16, 1)
+  TLM_CASE(false, false, EPI_ROWS, 1) TLM_CASE(false, true, EPI_ROWS, 1)
 #undef TLM_CASE
+  if (a_mn && b_mn && epi == EPI_F32_ACC && group == 2) return launch_t<true, true, EPI_F32_ACC, false, 2>(ma, mb, mc, p, tiles, st);
   return -2;
 }
 
@@ -1227,24 +1292,24 @@ TLM_API int tlm_gemm_swiglu(const void* x, const void* w_gu, void* gate_up, void
   if (use_pair(M)) {               // the B map's 128-row boxes serve both forms: rank 0 loads gate rows, rank 1 up rows
     static bool pconfigured = false;
     if (!pconfigured) {
-      cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_PAIR);
+      cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_pair_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_PAIR);
       if (ce != cudaSuccess) return (int)ce;
       pconfigured = true;
     }
     const int pgrid = pair_grid((long long)((M + 2 * BM - 1) / (2 * BM)) * (I / 128));
-    gemm_swiglu_pair_kernel<<<pgrid, GEMM_THREADS, GEMM_SMEM_PAIR, stream>>>(ma, mb, mc, md, p);
+    gemm_swiglu_pair_kernel<0><<<pgrid, GEMM_THREADS, GEMM_SMEM_PAIR, stream>>>(ma, mb, mc, md, p);
     count_launch();
     return launch_status();
   }
   static bool configured = false;
   if (!configured) {
-    cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
+    cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
     if (ce != cudaSuccess) return (int)ce;
     configured = true;
   }
   const int tiles = ((M + BM - 1) / BM) * (I / 128);
   const int grid = tiles < num_sms() ? tiles : num_sms();
-  gemm_swiglu_kernel<<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ma, mb, mc, md, p);
+  gemm_swiglu_kernel<0><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ma, mb, mc, md, p);
   count_launch();
   return launch_status();
 }
@@ -1269,24 +1334,24 @@ TLM_API int tlm_gemm_swiglu_bwd(const void* dy, const void* w_down, const void* 
   if (use_pair(M)) {               // MN-major B: 64-wide boxes in both forms
     static bool pconfigured = false;
     if (!pconfigured) {
-      cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_bwd_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_PAIR);
+      cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_bwd_pair_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_PAIR);
       if (ce != cudaSuccess) return (int)ce;
       pconfigured = true;
     }
     const int pgrid = pair_grid((long long)((M + 2 * BM - 1) / (2 * BM)) * ((I + BN - 1) / BN));
-    gemm_swiglu_bwd_pair_kernel<<<pgrid, GEMM_THREADS_WIDE, GEMM_SMEM_PAIR, stream>>>(ma, mb, mc, p);
+    gemm_swiglu_bwd_pair_kernel<0><<<pgrid, GEMM_THREADS_WIDE, GEMM_SMEM_PAIR, stream>>>(ma, mb, mc, p);
     count_launch();
     return launch_status();
   }
   static bool configured = false;
   if (!configured) {
-    cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
+    cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_bwd_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
     if (ce != cudaSuccess) return (int)ce;
     configured = true;
   }
   const int tiles = ((M + BM - 1) / BM) * ((I + BN - 1) / BN);
   const int grid = tiles < num_sms() ? tiles : num_sms();
-  gemm_swiglu_bwd_kernel<<<grid, GEMM_THREADS_WIDE, GEMM_SMEM, stream>>>(ma, mb, mc, p);
+  gemm_swiglu_bwd_kernel<0><<<grid, GEMM_THREADS_WIDE, GEMM_SMEM, stream>>>(ma, mb, mc, p);
   count_launch();
   return launch_status();
 }
@@ -1337,33 +1402,21 @@ TLM_API int tlm_gemm_swiglu_grouped(const void* x, const void* w_pair, void* gat
   if (e) return e;
   GemmParams p{};
   p.M = R; p.N = I; p.K = K; p.C = gate_up; p.ldc = 2LL * I; p.status = status_word(); p.split_k = 1; p.k_chunk = K;
-  p.act = (__nv_bfloat16*)act; p.ld_act = I;
-  p.groups = groups; p.row_start = row_start; p.group_mode = 1;
-  if (use_pair_grouped(R, groups)) {
-    p.max_tiles_m = (max_rows_per_group + 2 * BM - 1) / (2 * BM);
-    static bool pconfigured = false;
-    if (!pconfigured) {
-      cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_PAIR);
-      if (ce != cudaSuccess) return (int)ce;
-      pconfigured = true;
-    }
-    const int pgrid = pair_grid((long long)groups * p.max_tiles_m * (I / 128));
-    gemm_swiglu_pair_kernel<<<pgrid, GEMM_THREADS, GEMM_SMEM_PAIR, stream>>>(ma, mb, mc, md, p);
-    count_launch();
-    return launch_status();
-  }
-  p.max_tiles_m = (max_rows_per_group + BM - 1) / BM;
+  p.act = (__nv_bfloat16*)act; p.ld_act = I; p.up_off = groups;
+  const bool pair = use_pair_grouped(R, groups);
   static bool configured = false;
   if (!configured) {
-    cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
+    cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_pair_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_PAIR);
+    if (ce == cudaSuccess) ce = cudaFuncSetAttribute(gemm_swiglu_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
     if (ce != cudaSuccess) return (int)ce;
     configured = true;
   }
-  const int tiles = groups * p.max_tiles_m * (I / 128);
-  const int grid = tiles < num_sms() ? tiles : num_sms();
-  gemm_swiglu_kernel<<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ma, mb, mc, md, p);
-  count_launch();
-  return launch_status();
+  return for_group_chunks(p, groups, row_start, R, max_rows_per_group, I / 128, pair, [&](const GemmParams& q, int tiles) {
+    if (pair) gemm_swiglu_pair_kernel<1><<<pair_grid(tiles), GEMM_THREADS, GEMM_SMEM_PAIR, stream>>>(ma, mb, mc, md, q);
+    else gemm_swiglu_kernel<1><<<tiles < num_sms() ? tiles : num_sms(), GEMM_THREADS, GEMM_SMEM, stream>>>(ma, mb, mc, md, q);
+    count_launch();
+    return launch_status();
+  });
 }
 
 // MoE experts, backward of the down projection + SwiGLU: for the rows of each group g
@@ -1385,32 +1438,20 @@ TLM_API int tlm_gemm_swiglu_bwd_grouped(const void* dy, const void* w_down, cons
   GemmParams p{};
   p.M = R; p.N = I; p.K = D; p.C = d_gate_up; p.ldc = 2LL * I; p.status = status_word(); p.split_k = 1; p.k_chunk = D;
   p.aux = (const __nv_bfloat16*)gate_up;
-  p.groups = groups; p.row_start = row_start; p.group_mode = 1;
-  if (use_pair_grouped(R, groups)) {
-    p.max_tiles_m = (max_rows_per_group + 2 * BM - 1) / (2 * BM);
-    static bool pconfigured = false;
-    if (!pconfigured) {
-      cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_bwd_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_PAIR);
-      if (ce != cudaSuccess) return (int)ce;
-      pconfigured = true;
-    }
-    const int pgrid = pair_grid((long long)groups * p.max_tiles_m * ((I + BN - 1) / BN));
-    gemm_swiglu_bwd_pair_kernel<<<pgrid, GEMM_THREADS_WIDE, GEMM_SMEM_PAIR, stream>>>(ma, mb, mc, p);
-    count_launch();
-    return launch_status();
-  }
-  p.max_tiles_m = (max_rows_per_group + BM - 1) / BM;
+  const bool pair = use_pair_grouped(R, groups);
   static bool configured = false;
   if (!configured) {
-    cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
+    cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_bwd_pair_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_PAIR);
+    if (ce == cudaSuccess) ce = cudaFuncSetAttribute(gemm_swiglu_bwd_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
     if (ce != cudaSuccess) return (int)ce;
     configured = true;
   }
-  const int tiles = groups * p.max_tiles_m * ((I + BN - 1) / BN);
-  const int grid = tiles < num_sms() ? tiles : num_sms();
-  gemm_swiglu_bwd_kernel<<<grid, GEMM_THREADS_WIDE, GEMM_SMEM, stream>>>(ma, mb, mc, p);
-  count_launch();
-  return launch_status();
+  return for_group_chunks(p, groups, row_start, R, max_rows_per_group, (I + BN - 1) / BN, pair, [&](const GemmParams& q, int tiles) {
+    if (pair) gemm_swiglu_bwd_pair_kernel<1><<<pair_grid(tiles), GEMM_THREADS_WIDE, GEMM_SMEM_PAIR, stream>>>(ma, mb, mc, q);
+    else gemm_swiglu_bwd_kernel<1><<<tiles < num_sms() ? tiles : num_sms(), GEMM_THREADS_WIDE, GEMM_SMEM, stream>>>(ma, mb, mc, q);
+    count_launch();
+    return launch_status();
+  });
 }
 
 // Log-sum-exp statistics of logits = x [M, K] * w [N, K]^T without storing the logits (see GemmParams, EPI_LSE):
@@ -1529,10 +1570,9 @@ TLM_API int tlm_gemm_grouped_rows(const void* A, const void* B, void* C, const i
   if (e) return e;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.status = status_word();
-  p.groups = groups; p.row_start = row_start; p.group_mode = 1;
-  p.max_tiles_m = (max_rows_per_group + (pair ? 2 : 1) * BM - 1) / ((pair ? 2 : 1) * BM);
-  int tiles = groups * p.max_tiles_m * ((N + BN - 1) / BN);
-  return dispatch(false, b_mn != 0, epi, ma, mb, p, tiles, stream, pair);
+  return for_group_chunks(p, groups, row_start, M, max_rows_per_group, (N + BN - 1) / BN, pair, [&](const GemmParams& q, int tiles) {
+    return dispatch(false, b_mn != 0, epi, ma, mb, q, tiles, stream, pair, 1);
+  });
 }
 
 // Paired grouped GEMMs for the MoE gate / up projections. `W` holds 2 * groups matrices [I, D] (gate of
@@ -1556,11 +1596,11 @@ TLM_API int tlm_gemm_grouped_pair(const void* A, const void* W, void* C, const i
   if (e) return e;
   GemmParams p{};
   p.M = R; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.status = status_word();
-  p.groups = groups; p.row_start = row_start; p.group_mode = 1;
-  p.max_tiles_m = (max_rows_per_group + (pair ? 2 : 1) * BM - 1) / ((pair ? 2 : 1) * BM);
   if (dgrad) p.pair_k = I; else p.pair_n = I;
-  int tiles = groups * p.max_tiles_m * ((N + BN - 1) / BN);
-  return dispatch(false, dgrad != 0, EPI_BF16, ma, mb, p, tiles, stream, pair);
+  p.up_off = groups;
+  return for_group_chunks(p, groups, row_start, R, max_rows_per_group, (N + BN - 1) / BN, pair, [&](const GemmParams& q, int tiles) {
+    return dispatch(false, dgrad != 0, EPI_BF16, ma, mb, q, tiles, stream, pair, 1);
+  });
 }
 
 // Same as tlm_gemm_grouped_rows with a bf16 store, but output row r goes to dst_ptrs[dest_rank[r]] row dest_row[r]
@@ -1581,12 +1621,11 @@ TLM_API int tlm_gemm_grouped_rows_scatter(const void* A, const void* B, const in
   if (e) return e;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.C = nullptr; p.ldc = ldc; p.status = status_word();
-  p.groups = groups; p.row_start = row_start; p.group_mode = 1;
-  p.max_tiles_m = (max_rows_per_group + (pair ? 2 : 1) * BM - 1) / ((pair ? 2 : 1) * BM);
   p.rs_rank = dest_rank; p.rs_row = dest_row; p.rs_rows = dst_rows;
   for (int i = 0; i < n_dst; ++i) p.rs_dst[i] = dst_ptrs[i];
-  int tiles = groups * p.max_tiles_m * ((N + BN - 1) / BN);
-  return dispatch(false, b_mn != 0, EPI_ROWS, ma, mb, p, tiles, stream, pair);
+  return for_group_chunks(p, groups, row_start, M, max_rows_per_group, (N + BN - 1) / BN, pair, [&](const GemmParams& q, int tiles) {
+    return dispatch(false, b_mn != 0, EPI_ROWS, ma, mb, q, tiles, stream, pair, 1);
+  });
 }
 
 // Grouped wgrad: C[g] ([M,N] fp32, `c_group_stride` apart) += A[rows_g, M]^T * B[rows_g, N]
@@ -1604,7 +1643,7 @@ TLM_API int tlm_gemm_grouped_k(const void* A, const void* B, void* C, const int*
   if (e) return e;
   GemmParams p{};
   p.M = M; p.N = N; p.K = R; p.C = C; p.ldc = ldc; p.status = status_word();
-  p.groups = groups; p.row_start = row_start; p.group_mode = 2; p.c_group_stride = c_group_stride;
+  p.groups = groups; p.row_start = row_start; p.c_group_stride = c_group_stride;
   int tiles = groups * ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  return dispatch(true, true, epi, ma, mb, p, tiles, stream);
+  return dispatch(true, true, epi, ma, mb, p, tiles, stream, false, 2);
 }
