@@ -326,6 +326,25 @@ def test_row_grouped_gemms_around_the_group_limit_of_a_launch(nat, gemm_mode, E)
     assert _rel_err(act[:R], torch.nn.functional.silu(gb) * ub) < 6e-3
 
 
+@pytest.mark.parametrize("counts", [[130, 0, 64, 257], [1, 63, 65, 700, 7], [0, 0, 5], [64, 128, 64]])
+@pytest.mark.parametrize("I,D", [(256, 264), (512, 72), (384, 256)])
+def test_grouped_pair_weight_gradients(nat, gemm_mode, counts, I, D):
+    """gate and up weight gradients in one launch (I % 256 == 0) and in two, reduction ranges that end inside a 64-row
+    block, one-row and empty groups; the rows behind the last group are not finite and must not be seen."""
+    E, R = len(counts), sum(counts)
+    dgu, x = _rand(R + 70, 2 * I, seed=80), _rand(R + 70, D, seed=81)
+    dgu[R:], x[R:] = float("nan"), float("inf")
+    rs = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32, device="cuda")
+    acc = torch.ones(2 * E, I, D, device="cuda")
+    nat.grouped_gemm_pair_wgrad(dgu, x, acc, nat.DeviceCounts(rs, R))
+    nat.raise_on_device_status()
+    r = 0
+    for e, c in enumerate(counts):
+        ref = 1.0 + dgu[r:r + c].float().t() @ x[r:r + c].float()
+        assert _rel_err(acc[e], ref[:I]) < 1e-4 and _rel_err(acc[E + e], ref[I:]) < 1e-4, e
+        r += c
+
+
 @pytest.mark.parametrize("M,E,k", [(300, 8, 2), (129, 128, 8), (64, 4, 1), (1000, 40, 3)])
 def test_moe_route_and_row_movement(nat, M, E, k):
     """Device routing (top-k, softmax of the winners, stable expert-major order) and the gather / combine /

@@ -113,6 +113,9 @@ struct GemmParams {
   // gate|up [R, 2 I]). pair_k > 0: reduction indices >= pair_k come from the second matrix (dgrad of both
   // projections in one GEMM with K = 2 I, so their sum needs no extra pass).
   int pair_n, pair_k;
+  // Paired groups, K grouped (weight gradients of gate and up in one launch): rows of the product at and past pair_m
+  // (> 0) belong to C matrix g + up_off, rows before it to matrix g. pair_m is a multiple of the tile height.
+  int pair_m;
   // Row-scatter epilogue (bf16 store, grouped rows): output row r is not written to C but to
   //   rs_dst[rs_rank[r]] + rs_row[r] * ldc   (rows with rs_rank[r] < 0 are dropped).
   // This is the expert-parallel combine: the down-projection's accumulator goes straight to the
@@ -150,7 +153,7 @@ struct TileCoord {
   int b_n0;         // row (K-major) / column (MN-major) coordinate of the tile in the B matrix; n0 unless pair_n
   int k_lo, k_hi;   // reduction range
   int m_end;        // exclusive row bound for stores
-  long long c_off;  // element offset added to C
+  int c_grp;        // C matrix (K grouped)
   bool valid;
 };
 
@@ -170,7 +173,7 @@ __device__ __forceinline__ TileCoord plain_tile(const GemmParams& p, int tile_in
   int tm = first_m + r % gm, tn = r / gm;
   TileCoord t;
   t.m0 = tm * tile_m + m_shift; t.n0 = tn * tile_n; t.a_row0 = t.m0; t.b_grp = 0; t.b_n0 = t.n0;
-  t.k_lo = ks * p.k_chunk; t.k_hi = min(p.K, t.k_lo + p.k_chunk); t.m_end = p.M; t.c_off = 0; t.valid = t.k_hi > t.k_lo;
+  t.k_lo = ks * p.k_chunk; t.k_hi = min(p.K, t.k_lo + p.k_chunk); t.m_end = p.M; t.c_grp = 0; t.valid = t.k_hi > t.k_lo;
   return t;
 }
 
@@ -198,6 +201,10 @@ template <bool A_MN, bool B_MN, int EPI, bool GATED = false, bool PAIR = false, 
 __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC,
                                           const GemmParams& p, const CUtensorMap* dst_maps) {
   static_assert(!(PAIR && GATED), "the gated instantiations run as single CTAs");
+  // K grouped on CTA pairs: the last k-block of a group holds rows of the next group, which each CTA's MMA warp clears in
+  // its own shared memory. Such a block's loads complete on the loading CTA's own `tail` barrier, and the arrival on the
+  // leader's `full` barrier, otherwise its producer's, comes from the follower's MMA warp when it has cleared its rows.
+  constexpr bool TAIL_PAIR = PAIR && GROUP == 2;
   constexpr int STAGES = PAIR ? PAIR_STAGES : tlm::STAGES;
   constexpr int B_TILE_BYTES = PAIR ? B_BYTES / 2 : B_BYTES;
   constexpr int STAGE_BYTES = A_BYTES + B_TILE_BYTES;
@@ -215,7 +222,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
   auto empty_bar = [&](int s) { return bar0 + 8u * (STAGES + s); };
   auto accf_bar = [&](int a) { return bar0 + 8u * (2 * STAGES + a); };
   auto acce_bar = [&](int a) { return bar0 + 8u * (2 * STAGES + 2 + a); };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+  auto tail_bar = [&](int s) { return bar0 + 8u * (2 * STAGES + 4 + s); };       // TAIL_PAIR only
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* tiles_before = reinterpret_cast<int*>(smem_al + STAGES * STAGE_BYTES + EPI_BYTES + 256);    // [groups + 1], GROUP 1
 
@@ -227,7 +235,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
   constexpr int EPI_WARPS = EPI == EPI_SWIGLU_BWD ? 8 : 4;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+    for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); mbar_init(tail_bar(s), 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(accf_bar(a), 1); mbar_init(acce_bar(a), EPI_WARPS * (PAIR ? 2 : 1)); }
     *abort_flag = 0;
     fence_mbar_init();
@@ -286,14 +294,19 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       // PAIR: a second half that starts past the group's end runs with every row masked
       t.m0 = lo + tm * TILE_M + (int)cta_rank * BM; t.a_row0 = t.m0; t.n0 = tn * TILE_N; t.b_grp = g + p.grp0; t.b_n0 = t.n0;
       if (p.pair_n > 0 && t.n0 >= p.pair_n) { t.b_grp += p.up_off; t.b_n0 = t.n0 - p.pair_n; }
-      t.k_lo = 0; t.k_hi = p.K; t.m_end = hi; t.c_off = 0; t.valid = true;
+      t.k_lo = 0; t.k_hi = p.K; t.m_end = hi; t.c_grp = 0; t.valid = true;
     } else {                            // reduction grouped: K range [lo,hi), C = C_base + g * stride
       const int per = tiles_m * tiles_n;
       const int g = tile / per, r = tile - g * per;
       const int tm = r % tiles_m, tn = r / tiles_m;
       const int lo = p.row_start[g], hi = p.row_start[g + 1];
-      t.m0 = tm * BM; t.a_row0 = t.m0; t.n0 = tn * BN; t.b_grp = 0; t.b_n0 = t.n0;
-      t.k_lo = lo; t.k_hi = hi; t.m_end = p.M; t.c_off = (long long)g * p.c_group_stride; t.valid = hi > lo;
+      t.a_row0 = tm * TILE_M + (int)cta_rank * BM; t.m0 = t.a_row0; t.n0 = tn * BN; t.b_grp = 0; t.b_n0 = t.n0;
+      t.m_end = p.M; t.c_grp = g;
+      if (p.pair_m > 0) {
+        t.m_end = p.pair_m;
+        if (t.m0 >= p.pair_m) { t.m0 -= p.pair_m; t.c_grp += p.up_off; }
+      }
+      t.k_lo = lo; t.k_hi = hi; t.valid = hi > lo;
     }
     return t;
   };
@@ -321,8 +334,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
           const uint32_t sa = smem_base + stage * STAGE_BYTES, sb = sa + A_BYTES;
           if (PAIR) {
             // both CTAs' loads of this stage complete on the leader's barrier
-            const uint32_t fb = mapa_shared(full_bar(stage), 0);
-            if (leader) mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);
+            const bool tail = TAIL_PAIR && t.k_hi - k0 < BK;
+            const uint32_t fb = mapa_shared(tail ? tail_bar(stage) : full_bar(stage), tail ? cta_rank : 0u);
+            if (tail) mbar_expect_tx(tail_bar(stage), STAGE_BYTES);
+            else if (leader) mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);
             if (A_MN) {
 #pragma unroll
               for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * BOX_MN_BYTES, &tmA, fb, t.a_row0 + 64 * j, k0);
@@ -379,6 +394,36 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     int stage = 0; uint32_t phase = 0;
     int acc = 0, grp = 0; uint32_t acc_phase = 0;
     bool ok = !PAIR || leader;                      // the follower's MMA warp only allocates and frees tensor memory
+    // GROUP 2, last k-block of a group: rows past this group's end belong to the next group. Clear them in the A and B
+    // tiles (each k index is one 128-byte row per 64-wide box, so whole-row clearing is independent of the swizzle; the
+    // boxes of A and B are contiguous in the stage; B as well, so that a non-finite value in a foreign row cannot meet a zero).
+    auto clear_tail = [&](int st, int valid) {
+      uint8_t* a_ptr = smem_al + st * STAGE_BYTES;
+      const int n16 = (BK - valid) * 8;                        // 16-byte pieces per box
+      for (int box = 0; box < STAGE_BYTES / BOX_MN_BYTES; ++box)
+        for (int i = lane; i < n16; i += 32)
+          *reinterpret_cast<uint4*>(a_ptr + box * BOX_MN_BYTES + valid * 128 + i * 16) = make_uint4(0, 0, 0, 0);
+      fence_proxy_async_smem();
+      __syncwarp();
+    };
+    uint32_t tail_phase = 0;                        // bit s: parity of tail_bar(s)'s current phase
+    if (TAIL_PAIR && !leader) {                     // ... except that it clears the tail of its own operand tiles
+      bool alive = true;
+      for (int tile = worker; tile < total_tiles && alive; tile += n_workers) {
+        const TileCoord t = get_tile(tile, grp);
+        if (!t.valid) continue;
+        const int blocks = (t.k_hi - t.k_lo + BK - 1) / BK;
+        stage = (stage + blocks - 1) % STAGES;
+        const int valid = t.k_hi - t.k_lo - (blocks - 1) * BK;
+        if (valid < BK) {
+          if (!mbar_wait(tail_bar(stage), (tail_phase >> stage) & 1u, 5, abort_flag, p.status)) { alive = false; break; }
+          tail_phase ^= 1u << stage;
+          clear_tail(stage, valid);
+          if (lane == 0) mbar_arrive_cluster(mapa_shared(full_bar(stage), 0));
+        }
+        stage = (stage + 1) % STAGES;
+      }
+    }
     for (int tile = worker; tile < total_tiles && ok; tile += n_workers) {
       TileCoord t = get_tile(tile, grp);
       if (!t.valid) continue;
@@ -387,23 +432,15 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
       uint32_t accumulate = 0;
       for (int k0 = t.k_lo; k0 < t.k_hi; k0 += BK) {
-        if (!mbar_wait(full_bar(stage), phase, 3, abort_flag, p.status)) { ok = false; break; }
+        if (TAIL_PAIR && t.k_hi - k0 < BK) {
+          if (!mbar_wait(tail_bar(stage), (tail_phase >> stage) & 1u, 5, abort_flag, p.status)) { ok = false; break; }
+          tail_phase ^= 1u << stage;
+          clear_tail(stage, t.k_hi - k0);
+          if (!mbar_wait<true>(full_bar(stage), phase, 3, abort_flag, p.status)) { ok = false; break; }
+        } else if (!mbar_wait(full_bar(stage), phase, 3, abort_flag, p.status)) { ok = false; break; }
         tc_fence_after();
         const uint32_t sa = smem_base + stage * STAGE_BYTES, sb = sa + A_BYTES;
-        if (GROUP == 2 && t.k_hi - k0 < BK) {
-          // grouped reduction: rows past this group's end belong to the next group.
-          // Zero them in the A tile (each k index is one 128-byte row per 64-wide box,
-          // so whole-row zeroing is independent of the swizzle).
-          const int valid = t.k_hi - k0;
-          uint8_t* a_ptr = smem_al + stage * STAGE_BYTES;
-          const int n16 = (BK - valid) * 8;                      // 16-byte pieces per box
-          // A and B boxes are contiguous in the stage (2 + 4 boxes of 8 KB); B is cleared as well so that
-          // a non-finite value in a foreign row cannot meet a zero
-          for (int box = 0; box < (BM + BN) / 64; ++box)
-            for (int i = lane; i < n16; i += 32)
-              *reinterpret_cast<uint4*>(a_ptr + box * BOX_MN_BYTES + valid * 128 + i * 16) = make_uint4(0, 0, 0, 0);
-          fence_proxy_async_smem();
-        }
+        if (GROUP == 2 && !PAIR && t.k_hi - k0 < BK) clear_tail(stage, t.k_hi - k0);
         __syncwarp();
         if (lane == 0) {
           // K-major: 16 bf16 = 32 B further along the 128 B row;
@@ -857,9 +894,14 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            if (t.n0 + c < p.N && row0 < p.M)
-              asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
-                           ::"l"((uint64_t)&tmC), "r"(ebuf_s + bsel * EPI_BUF_BYTES), "r"(t.n0 + c), "r"(row0) : "memory");
+            if (t.n0 + c < p.N && row0 < t.m_end) {
+              if (GROUP == 2)
+                asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+                             ::"l"((uint64_t)&tmC), "r"(ebuf_s + bsel * EPI_BUF_BYTES), "r"(t.n0 + c), "r"(row0), "r"(t.c_grp) : "memory");
+              else
+                asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
+                             ::"l"((uint64_t)&tmC), "r"(ebuf_s + bsel * EPI_BUF_BYTES), "r"(t.n0 + c), "r"(row0) : "memory");
+            }
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         }
@@ -921,7 +963,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         const int col = t.n0 + c;
         if (row_live && col < p.N) {
           if (EPI == EPI_BF16) {
-            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + t.c_off + (long long)row * p.ldc + col;
+            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + t.c_grp * p.c_group_stride + (long long)row * p.ldc + col;
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
               if (col + j < p.N) {
@@ -934,7 +976,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
               }
             }
           } else {
-            float* out = reinterpret_cast<float*>(p.C) + t.c_off + (long long)row * p.ldc + col;
+            float* out = reinterpret_cast<float*>(p.C) + t.c_grp * p.c_group_stride + (long long)row * p.ldc + col;
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
               if (col + j < p.N) {
@@ -1144,16 +1186,18 @@ static int dispatch(bool a_mn, bool b_mn, int epi, const CUtensorMap& ma, const 
   }
   static int f32_reduce = -1;                 // TLM_GEMM_TMA_REDUCE=0: fp32 accumulation with loads and stores / red.global
   if (f32_reduce < 0) { const char* v = getenv("TLM_GEMM_TMA_REDUCE"); f32_reduce = (v != nullptr && v[0] == '0') ? 0 : 1; }
-  if (epi == EPI_F32_ACC && f32_reduce && group == 0 && p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0) {
-    uint64_t dims[2] = {(uint64_t)p.N, (uint64_t)p.M}, strides[1] = {(uint64_t)p.ldc * 4};
-    uint32_t box[2] = {32, 32};
-    if (make_tmap_f32(&mc, p.C, 2, dims, strides, box) == 0) p.tma_store = 1;
+  if (epi == EPI_F32_ACC && f32_reduce && group != 1 && p.ldc % 4 == 0 && p.c_group_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0) {
+    // K grouped: all groups' C matrices as one 3-D tensor, so that a tile past a matrix's last row is clipped there
+    uint64_t dims[3] = {(uint64_t)p.N, (uint64_t)(p.pair_m > 0 ? p.pair_m : p.M), (uint64_t)p.groups * (p.pair_m > 0 ? 2 : 1)};
+    uint64_t strides[2] = {(uint64_t)p.ldc * 4, (uint64_t)p.c_group_stride * 4};
+    uint32_t box[3] = {32, 32, 1};
+    if (make_tmap_f32(&mc, p.C, group == 2 ? 3 : 2, dims, strides, box) == 0) p.tma_store = 1;
   }
   if (p.dl_lse != nullptr && !p.tma_store) return -6;       // the gradient transform lives in the TMA-store epilogue
   // x W^T with a pending "parameters ready" gate: the gated instantiation (see gemm_body)
   if (!a_mn && !b_mn && epi == EPI_BF16 && p.wait_flags[0] != nullptr)
     return launch_t<false, false, EPI_BF16, true>(ma, mb, mc, p, tiles, st);
-  if (pair && (group == 2 || p.wait_flags[0] != nullptr)) return -8;
+  if (pair && p.wait_flags[0] != nullptr) return -8;
 #define TLM_CASE(A, B, E, G)                                                          \
   if (a_mn == A && b_mn == B && epi == E && group == G)                               \
     return pair ? launch_pair_t<A, B, E, G>(ma, mb, mc, p, tiles, st) : launch_t<A, B, E, false, G>(ma, mb, mc, p, tiles, st);
@@ -1162,8 +1206,8 @@ static int dispatch(bool a_mn, bool b_mn, int epi, const CUtensorMap& ma, const 
   TLM_CASE(true, true, EPI_BF16, 0) TLM_CASE(false, true, EPI_F32, 0) TLM_CASE(false, false, EPI_LSE, 0)
   TLM_CASE(false, false, EPI_BF16, 1) TLM_CASE(false, true, EPI_BF16, 1)
   TLM_CASE(false, false, EPI_ROWS, 1) TLM_CASE(false, true, EPI_ROWS, 1)
+  TLM_CASE(true, true, EPI_F32_ACC, 2)
 #undef TLM_CASE
-  if (a_mn && b_mn && epi == EPI_F32_ACC && group == 2) return launch_t<true, true, EPI_F32_ACC, false, 2>(ma, mb, mc, p, tiles, st);
   return -2;
 }
 
@@ -1628,12 +1672,9 @@ TLM_API int tlm_gemm_grouped_rows_scatter(const void* A, const void* B, const in
   });
 }
 
-// Grouped wgrad: C[g] ([M,N] fp32, `c_group_stride` apart) += A[rows_g, M]^T * B[rows_g, N]
-// where rows_g = [row_start[g], row_start[g+1]) is the reduction range.
-// A is stored [R, M] and B [R, N] (both MN-major with respect to the product).
-TLM_API int tlm_gemm_grouped_k(const void* A, const void* B, void* C, const int* row_start, int groups, int R,
-                               int M, int N, long long lda, long long ldb, long long ldc, long long c_group_stride,
-                               int epi, cudaStream_t stream) {
+static int grouped_k(const void* A, const void* B, void* C, const int* row_start, int groups, int R, int M, int N,
+                     long long lda, long long ldb, long long ldc, long long c_group_stride, int pair_m, int epi,
+                     cudaStream_t stream) {
   if (M <= 0 || N <= 0 || R <= 0 || groups <= 0) return 0;
   Operand oa{A, M, R, lda, true, 0, 0}, ob{B, N, R, ldb, true, 1, (long long)R * N};
   CUtensorMap ma, mb;
@@ -1643,7 +1684,36 @@ TLM_API int tlm_gemm_grouped_k(const void* A, const void* B, void* C, const int*
   if (e) return e;
   GemmParams p{};
   p.M = M; p.N = N; p.K = R; p.C = C; p.ldc = ldc; p.status = status_word();
-  p.groups = groups; p.row_start = row_start; p.c_group_stride = c_group_stride;
-  int tiles = groups * ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  return dispatch(true, true, epi, ma, mb, p, tiles, stream, false, 2);
+  p.groups = groups; p.row_start = row_start; p.c_group_stride = c_group_stride; p.pair_m = pair_m; p.up_off = groups;
+  // CTA pairs on 256-row tiles for matrices of at least that height, gate and up in one launch, results through TMA
+  // reduce-add. The three weight gradients of an expert MLP, against single CTAs with loads and stores of C: 128 groups
+  // of 512 rows, 256 x 1024 matrices 542 -> 190 us; 8 groups of 4096 rows, 2048 x 1024 452 -> 321 us.
+  const bool pair = use_pair(M);
+  const int tile_m = pair ? 2 * BM : BM;
+  int tiles = groups * ((M + tile_m - 1) / tile_m) * ((N + BN - 1) / BN);
+  return dispatch(true, true, epi, ma, mb, p, tiles, stream, pair, 2);
+}
+
+// Grouped wgrad: C[g] ([M,N] fp32, `c_group_stride` apart) += A[rows_g, M]^T * B[rows_g, N]
+// where rows_g = [row_start[g], row_start[g+1]) is the reduction range.
+// A is stored [R, M] and B [R, N] (both MN-major with respect to the product).
+TLM_API int tlm_gemm_grouped_k(const void* A, const void* B, void* C, const int* row_start, int groups, int R,
+                               int M, int N, long long lda, long long ldb, long long ldc, long long c_group_stride,
+                               int epi, cudaStream_t stream) {
+  return grouped_k(A, B, C, row_start, groups, R, M, N, lda, ldb, ldc, c_group_stride, 0, epi, stream);
+}
+
+// Same for a pair of projections whose gradients lie side by side: A = [R, 2 I] (gate | up), C = [2 * groups, I, N] fp32
+// contiguous, C[g] += A[rows_g, :I]^T B[rows_g], C[groups + g] += A[rows_g, I:]^T B[rows_g].
+TLM_API int tlm_gemm_grouped_k_pair(const void* A, const void* B, void* C, const int* row_start, int groups, int R, int I,
+                                    int N, long long lda, long long ldb, cudaStream_t stream) {
+  const long long stride = (long long)I * N;
+  if (I % (2 * BM) == 0)                 // no tile spans the two matrices
+    return grouped_k(A, B, C, row_start, groups, R, 2 * I, N, lda, ldb, N, stride, I, EPI_F32_ACC, stream);
+  for (int h = 0; h < 2; ++h) {
+    const int e = grouped_k((const __nv_bfloat16*)A + h * I, B, (float*)C + h * groups * stride, row_start, groups, R, I, N, lda,
+                            ldb, N, stride, 0, EPI_F32_ACC, stream);
+    if (e) return e;
+  }
+  return 0;
 }

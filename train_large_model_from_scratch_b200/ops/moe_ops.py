@@ -85,11 +85,8 @@ class _GroupedGateUp(torch.autograd.Function):
     def backward(ctx, dgu):
         (x,) = ctx.saved_tensors
         w, counts = ctx.w_pair, ctx.counts
-        E, I = w.shape[0] // 2, w.shape[1]
-        mg = F_ops._main_grad(w)
         dgu = dgu.contiguous()
-        native.grouped_gemm_tn_accum(dgu[:, :I], x, mg[:E], counts)
-        native.grouped_gemm_tn_accum(dgu[:, I:], x, mg[E:], counts)
+        native.grouped_gemm_pair_wgrad(dgu, x, F_ops._main_grad(w), counts)
         return native.grouped_gemm_pair_dgrad(dgu, w, counts), None, None
 
 
@@ -116,12 +113,9 @@ class _ExpertMLP(torch.autograd.Function):
 def expert_mlp_backward(dy, x, gu, act, w_pair, w_down, counts):
     """Shared by `_ExpertMLP` and the expert-parallel variant (`parallel.expert_parallel.peer`): accumulates the
     three weight gradients into their `main_grad` buffers and returns the gradient of the grouped input rows."""
-    E, I = w_pair.shape[0] // 2, w_pair.shape[1]
     native.grouped_gemm_tn_accum(dy, act, F_ops._main_grad(w_down), counts)
     dgu = native.grouped_gemm_swiglu_bwd(dy, w_down, gu, counts)
-    mg = F_ops._main_grad(w_pair)
-    native.grouped_gemm_tn_accum(dgu[:, :I], x, mg[:E], counts)
-    native.grouped_gemm_tn_accum(dgu[:, I:], x, mg[E:], counts)
+    native.grouped_gemm_pair_wgrad(dgu, x, F_ops._main_grad(w_pair), counts)
     return native.grouped_gemm_pair_dgrad(dgu, w_pair, counts)
 
 

@@ -62,6 +62,7 @@ _SIGS = {
     "tlm_gemm_swiglu_bwd_grouped": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _LL, _LL, _I, _P]),
     "tlm_gemm_grouped_rows": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _LL, _LL, _LL, _LL, _I, _I, _I, _P]),
     "tlm_gemm_grouped_k": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _LL, _LL, _LL, _LL, _I, _P]),
+    "tlm_gemm_grouped_k_pair": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _LL, _LL, _P]),
     "tlm_embedding_fwd": (_I, [_P, _P, _P, _I, _I, _LL, _P]),
     "tlm_embedding_bwd": (_I, [_P, _P, _P, _I, _I, _LL, _P]),
     "tlm_add_rmsnorm_fwd": (_I, [_P, _P, _P, _P, _P, _P, _I, _I, _F, _P]),
@@ -549,6 +550,20 @@ def grouped_gemm_tn_accum(dy: torch.Tensor, x: torch.Tensor, acc: torch.Tensor, 
     rs, _ = _grouping(counts, dy.device)
     _check(lib().tlm_gemm_grouped_k(dy.data_ptr(), x.data_ptr(), acc.data_ptr(), rs.data_ptr(), E, R, N, K, lda, ldb,
                                     K, N * K, EPI_F32_ACC, _stream()), "grouped_gemm_tn_accum")
+
+
+def grouped_gemm_pair_wgrad(dgu: torch.Tensor, x: torch.Tensor, acc: torch.Tensor, counts) -> None:
+    """Weight gradients of both projections of `grouped_gemm_pair_fwd` in one launch: `acc [2E, I, D]` fp32,
+    `acc[e] += dgu[rows_e, :I]^T @ x[rows_e]`, `acc[E + e] += dgu[rows_e, I:]^T @ x[rows_e]`."""
+    R, I2, lda = _rows(dgu)
+    R2, D, ldb = _rows(x)
+    E2, I = acc.shape[0], acc.shape[1]
+    assert R == R2 and I2 == 2 * I and acc.shape == (E2, I, D) and acc.dtype == torch.float32 and acc.is_contiguous()
+    if R == 0:
+        return
+    rs, _ = _grouping(counts, dgu.device)
+    _check(lib().tlm_gemm_grouped_k_pair(dgu.data_ptr(), x.data_ptr(), acc.data_ptr(), rs.data_ptr(), E2 // 2, R, I, D, lda, ldb,
+                                         _stream()), "grouped_gemm_pair_wgrad")
 
 
 def grouped_gemm_nt_scatter(x: torch.Tensor, weight: torch.Tensor, counts, dest_rank: torch.Tensor,
