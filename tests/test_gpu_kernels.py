@@ -225,6 +225,32 @@ def test_gemm_swiglu_epilogues(nat, gemm_mode, M, I, K):
     assert _rel_err(dgu, ref) < 6e-3
 
 
+@pytest.mark.parametrize("rows,D", [(1, 1280), (37, 2304), (700, 3072), (5, 4096), (3, 4352)])
+def test_add_rmsnorm_of_wide_rows(nat, rows, D):
+    """Rows shared by several warps (1280 = 5 x 256, 2304 = 3 x 768, 3072 = 4 x 768, ...; 4352 = 17 x 256 is too many warps and
+    takes the shared-memory form), with and without an incoming residual gradient."""
+    g = torch.Generator(device="cuda").manual_seed(90)
+    x, gx = (torch.randn(rows, D, device="cuda", generator=g) for _ in range(2))
+    d, gh, w = _rand(rows, D, seed=91), _rand(rows, D, seed=92), _rand(D, seed=93)
+    x_new, h, rstd = nat.add_rmsnorm_fwd(x, d, w, 1e-6)
+    xd = x.double() + d.double()
+    r = (xd.pow(2).mean(-1, keepdim=True) + 1e-6).rsqrt()
+    assert ((x_new.double() - xd).norm() / xd.norm()).item() < 1e-7
+    assert ((rstd.double() - r[:, 0]).abs() / r[:, 0]).max().item() < 1e-6
+    ref_h = xd * r * w.double()
+    assert ((h.double() - ref_h).norm() / ref_h.norm()).item() < 2.5e-3
+    gw = gh.double() * w.double()
+    branch = r * (gw - xd * r * (gw * xd * r).mean(-1, keepdim=True))
+    for inc in (gx, None):
+        mg = torch.full((D,), 3.0, device="cuda")
+        got, got_d = nat.add_rmsnorm_bwd(inc, gh, x_new, rstd, w, mg, True)
+        ref = branch if inc is None else inc.double() + branch
+        assert ((got.double() - ref).norm() / ref.norm()).item() < 1e-6
+        assert ((got_d.double() - ref).norm() / ref.norm()).item() < 2.5e-3
+        dw = (gh.double() * xd * r).sum(0)
+        assert ((mg.double() - 3.0 - dw).norm() / dw.norm()).item() < 3e-6
+
+
 def test_swiglu(nat):
     gu = _rand(77, 2 * 384, seed=13)
     act = nat.swiglu_fwd(gu)

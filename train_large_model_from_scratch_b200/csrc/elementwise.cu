@@ -139,6 +139,70 @@ add_rmsnorm_fwd_reg_kernel(const float* __restrict__ x, const __nv_bfloat16* __r
   }
 }
 
+// Rows wider than a warp's registers: a block of W warps shares a row of D = W * NV * 256 columns, each lane owns NV groups of
+// 8 columns, and one block-wide sum per row joins the warps. Bound by HBM bandwidth; it replaces rows staged in shared memory
+// (one warp per row), where a warp's 3072-wide row kept too few loads in flight: in a training step 8192 x 3072 forward 67 ->
+// 48 us (6.3 TB/s), backward 199 -> 70 us (5.8 TB/s); 4096 x 4096 alone 64 -> 33 and 201 -> 47 us. See rms_split for W and NV.
+constexpr int RMS_WIDE_MAX_WARPS = 16;
+
+__device__ __forceinline__ float rms_block_sum(float v, float* red, int warps, int warp, int lane) {
+  v = warp_sum(v);
+  if (lane == 0) red[warp] = v;
+  __syncthreads();
+  float t = 0.f;
+  for (int i = 0; i < warps; ++i) t += red[i];
+  return t;
+}
+
+template <int NV>
+__global__ void __launch_bounds__(RMS_WIDE_MAX_WARPS * 32)
+add_rmsnorm_fwd_wide_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
+                            const __nv_bfloat16* __restrict__ w, float* __restrict__ x_new,
+                            __nv_bfloat16* __restrict__ h, float* __restrict__ rstd_out, int rows, int D, float eps) {
+  __shared__ float red[2][RMS_WIDE_MAX_WARPS];
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c0 = (warp * NV * 32 + lane) * 8;
+  int par = 0;
+  for (int r = blockIdx.x; r < rows; r += gridDim.x, par ^= 1) {
+    const long long base = (long long)r * D + c0;
+    float4 a[NV], b[NV];
+    uint4 d[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      a[k] = *reinterpret_cast<const float4*>(x + base + k * 256);
+      b[k] = *reinterpret_cast<const float4*>(x + base + k * 256 + 4);
+      if (delta != nullptr) d[k] = *reinterpret_cast<const uint4*>(delta + base + k * 256);
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      if (delta != nullptr) {
+        const float2 d0 = unpack_bf16(d[k].x), d1 = unpack_bf16(d[k].y), d2 = unpack_bf16(d[k].z), d3 = unpack_bf16(d[k].w);
+        a[k].x += d0.x; a[k].y += d0.y; a[k].z += d1.x; a[k].w += d1.y;
+        b[k].x += d2.x; b[k].y += d2.y; b[k].z += d3.x; b[k].w += d3.y;
+        float4* o = reinterpret_cast<float4*>(x_new + base + k * 256);
+        o[0] = a[k]; o[1] = b[k];
+      }
+      ss += a[k].x * a[k].x + a[k].y * a[k].y + a[k].z * a[k].z + a[k].w * a[k].w +
+            b[k].x * b[k].x + b[k].y * b[k].y + b[k].z * b[k].z + b[k].w * b[k].w;
+    }
+    ss = rms_block_sum(ss, red[par], warps, warp, lane);       // two buffers: the next row's sums cannot overtake this read
+    const float rstd = rsqrtf(ss / (float)D + eps);
+    if (threadIdx.x == 0) rstd_out[r] = rstd;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const uint4 wv = *reinterpret_cast<const uint4*>(w + c0 + k * 256);
+      const float2 w0 = unpack_bf16(wv.x), w1 = unpack_bf16(wv.y), w2 = unpack_bf16(wv.z), w3 = unpack_bf16(wv.w);
+      uint4 o;
+      o.x = pack_bf16(a[k].x * rstd * w0.x, a[k].y * rstd * w0.y);
+      o.y = pack_bf16(a[k].z * rstd * w1.x, a[k].w * rstd * w1.y);
+      o.z = pack_bf16(b[k].x * rstd * w2.x, b[k].y * rstd * w2.y);
+      o.w = pack_bf16(b[k].z * rstd * w3.x, b[k].w * rstd * w3.y);
+      *reinterpret_cast<uint4*>(h + base + k * 256) = o;
+    }
+  }
+}
+
 // g_x = g_xnew + rstd * (gh*w - xhat * mean(gh*w*xhat)); g_delta = bf16(g_x);
 // dw[c] += sum_rows gh*xhat. Each warp keeps a private dw row in shared memory;
 // the block folds them and issues one atomicAdd per column.
@@ -286,6 +350,85 @@ add_rmsnorm_bwd_reg_kernel(const float* __restrict__ g_xnew, const __nv_bfloat16
 #pragma unroll
       for (int j = 0; j < 8; ++j) atomicAdd(dw_out + (lane + 32 * k) * 8 + j, dw[k * 8 + j]);
   }
+}
+
+// Wide rows (see add_rmsnorm_fwd_wide_kernel). The row's x, g_h and incoming gradient are all requested before the first use;
+// the dweight partial sums stay in registers over all rows of the block and leave with one vector reduction per 4 columns.
+template <int NV>
+__global__ void __launch_bounds__(RMS_WIDE_MAX_WARPS * 32)
+add_rmsnorm_bwd_wide_kernel(const float* __restrict__ g_xnew, const __nv_bfloat16* __restrict__ g_h,
+                            const float* __restrict__ x_new, const float* __restrict__ rstd_in,
+                            const __nv_bfloat16* __restrict__ w, float* __restrict__ g_x,
+                            __nv_bfloat16* __restrict__ g_delta, float* __restrict__ dw_out, int rows, int D) {
+  __shared__ float red[2][RMS_WIDE_MAX_WARPS];
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c0 = (warp * NV * 32 + lane) * 8;
+  float dw[NV * 8];
+#pragma unroll
+  for (int i = 0; i < NV * 8; ++i) dw[i] = 0.f;
+  int par = 0;
+  for (int r = blockIdx.x; r < rows; r += gridDim.x, par ^= 1) {
+    const long long base = (long long)r * D + c0;
+    const float rstd = rstd_in[r];
+    float4 xa[NV], xb[NV], ga[NV], gb[NV];
+    uint4 gv[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      xa[k] = *reinterpret_cast<const float4*>(x_new + base + k * 256);
+      xb[k] = *reinterpret_cast<const float4*>(x_new + base + k * 256 + 4);
+      gv[k] = *reinterpret_cast<const uint4*>(g_h + base + k * 256);
+    }
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      if (g_xnew != nullptr) {
+        ga[k] = *reinterpret_cast<const float4*>(g_xnew + base + k * 256);
+        gb[k] = *reinterpret_cast<const float4*>(g_xnew + base + k * 256 + 4);
+      } else {
+        ga[k] = make_float4(0.f, 0.f, 0.f, 0.f); gb[k] = ga[k];
+      }
+    }
+    float dot = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const uint4 wv = *reinterpret_cast<const uint4*>(w + c0 + k * 256);
+      const float2 g0 = unpack_bf16(gv[k].x), g1 = unpack_bf16(gv[k].y), g2 = unpack_bf16(gv[k].z), g3 = unpack_bf16(gv[k].w);
+      const float2 w0 = unpack_bf16(wv.x), w1 = unpack_bf16(wv.y), w2 = unpack_bf16(wv.z), w3 = unpack_bf16(wv.w);
+      const float xs[8] = {xa[k].x, xa[k].y, xa[k].z, xa[k].w, xb[k].x, xb[k].y, xb[k].z, xb[k].w};
+      const float gs[8] = {g0.x, g0.y, g1.x, g1.y, g2.x, g2.y, g3.x, g3.y};
+      const float ws[8] = {w0.x, w0.y, w1.x, w1.y, w2.x, w2.y, w3.x, w3.y};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float xhat = xs[j] * rstd;
+        dw[k * 8 + j] = fmaf(gs[j], xhat, dw[k * 8 + j]);
+        dot = fmaf(gs[j] * ws[j], xhat, dot);
+      }
+    }
+    dot = rms_block_sum(dot, red[par], warps, warp, lane) / (float)D;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const uint4 wv = *reinterpret_cast<const uint4*>(w + c0 + k * 256);
+      const float2 g0 = unpack_bf16(gv[k].x), g1 = unpack_bf16(gv[k].y), g2 = unpack_bf16(gv[k].z), g3 = unpack_bf16(gv[k].w);
+      const float2 w0 = unpack_bf16(wv.x), w1 = unpack_bf16(wv.y), w2 = unpack_bf16(wv.z), w3 = unpack_bf16(wv.w);
+      const float xs[8] = {xa[k].x, xa[k].y, xa[k].z, xa[k].w, xb[k].x, xb[k].y, xb[k].z, xb[k].w};
+      const float gs[8] = {g0.x, g0.y, g1.x, g1.y, g2.x, g2.y, g3.x, g3.y};
+      const float ws[8] = {w0.x, w0.y, w1.x, w1.y, w2.x, w2.y, w3.x, w3.y};
+      const float gi[8] = {ga[k].x, ga[k].y, ga[k].z, ga[k].w, gb[k].x, gb[k].y, gb[k].z, gb[k].w};
+      float o[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = gi[j] + rstd * (gs[j] * ws[j] - xs[j] * rstd * dot);
+      float4* out = reinterpret_cast<float4*>(g_x + base + k * 256);
+      out[0] = make_float4(o[0], o[1], o[2], o[3]);
+      out[1] = make_float4(o[4], o[5], o[6], o[7]);
+      if (g_delta != nullptr)
+        *reinterpret_cast<uint4*>(g_delta + base + k * 256) =
+            make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7]));
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+#pragma unroll
+    for (int j = 0; j < 8; j += 4)
+      atomicAdd(reinterpret_cast<float4*>(dw_out + c0 + k * 256 + j), make_float4(dw[k * 8 + j], dw[k * 8 + j + 1], dw[k * 8 + j + 2], dw[k * 8 + j + 3]));
 }
 
 // ------------------------------------------------------------------ RoPE (in place)
@@ -629,6 +772,16 @@ TLM_API int tlm_embedding_bwd(const long long* idx, const float* dx, float* grad
   return launch_status();
 }
 
+// Wide rows: D = warps * nv * 256 with at most RMS_WIDE_MAX_WARPS warps per block; nv groups of 8 columns per lane, the
+// largest up to max_nv that divides. nv == 0: the width takes the kernels that stage rows in shared memory.
+struct RmsSplit { int nv, warps; };
+static RmsSplit rms_split(int D, int max_nv) {
+  if (D % 256 == 0)
+    for (int nv = max_nv; nv >= 1; --nv)
+      if (D / 256 % nv == 0 && D / 256 / nv <= RMS_WIDE_MAX_WARPS) return {nv, D / 256 / nv};
+  return {0, 0};
+}
+
 TLM_API int tlm_add_rmsnorm_fwd(const float* x, const void* delta, const void* w, float* x_new, void* h, float* rstd,
                                 int rows, int D, float eps, cudaStream_t st) {
   if (D % 256 == 0 && D / 256 <= 8 && D / 256 != 5 && D / 256 != 7) {
@@ -636,6 +789,16 @@ TLM_API int tlm_add_rmsnorm_fwd(const float* x, const void* delta, const void* w
 #define TLM_RMS_CASE(NV) case NV: add_rmsnorm_fwd_reg_kernel<NV><<<grid, 256, 0, st>>>(x, (const __nv_bfloat16*)delta, \
       (const __nv_bfloat16*)w, x_new, (__nv_bfloat16*)h, rstd, rows, eps); break;
     switch (D / 256) { TLM_RMS_CASE(1) TLM_RMS_CASE(2) TLM_RMS_CASE(3) TLM_RMS_CASE(4) TLM_RMS_CASE(6) TLM_RMS_CASE(8) }
+#undef TLM_RMS_CASE
+    count_launch();
+    return launch_status();
+  }
+  const RmsSplit sp = rms_split(D, 4);
+  if (sp.nv > 0) {
+    const int grid = grid_for(rows, 1, 64 / sp.warps);
+#define TLM_RMS_CASE(NV) case NV: add_rmsnorm_fwd_wide_kernel<NV><<<grid, sp.warps * 32, 0, st>>>(x, (const __nv_bfloat16*)delta, \
+      (const __nv_bfloat16*)w, x_new, (__nv_bfloat16*)h, rstd, rows, D, eps); break;
+    switch (sp.nv) { TLM_RMS_CASE(1) TLM_RMS_CASE(2) TLM_RMS_CASE(3) TLM_RMS_CASE(4) }
 #undef TLM_RMS_CASE
     count_launch();
     return launch_status();
@@ -664,6 +827,16 @@ TLM_API int tlm_add_rmsnorm_bwd(const float* g_xnew, const void* g_h, const floa
 #define TLM_RMS_CASE(NV) case NV: add_rmsnorm_bwd_reg_kernel<NV><<<grid, 256, 0, st>>>(g_xnew, (const __nv_bfloat16*)g_h, x_new, rstd, \
       (const __nv_bfloat16*)w, g_x, (__nv_bfloat16*)g_delta, dw, rows); break;
     switch (D / 256) { TLM_RMS_CASE(1) TLM_RMS_CASE(2) TLM_RMS_CASE(3) TLM_RMS_CASE(4) TLM_RMS_CASE(6) }
+#undef TLM_RMS_CASE
+    count_launch();
+    return launch_status();
+  }
+  const RmsSplit sp = rms_split(D, 3);          // 4 groups would not fit the registers
+  if (sp.nv > 0 && (reinterpret_cast<uintptr_t>(dw) & 15) == 0) {
+    const int grid = grid_for(rows, 1, sp.warps >= 16 ? 1 : 16 / sp.warps);
+#define TLM_RMS_CASE(NV) case NV: add_rmsnorm_bwd_wide_kernel<NV><<<grid, sp.warps * 32, 0, st>>>(g_xnew, (const __nv_bfloat16*)g_h, x_new, rstd, \
+      (const __nv_bfloat16*)w, g_x, (__nv_bfloat16*)g_delta, dw, rows, D); break;
+    switch (sp.nv) { TLM_RMS_CASE(1) TLM_RMS_CASE(2) TLM_RMS_CASE(3) }
 #undef TLM_RMS_CASE
     count_launch();
     return launch_status();
