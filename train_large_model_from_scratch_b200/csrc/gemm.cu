@@ -697,11 +697,9 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
               for (int i = 0; i < 32; i += 2) {
                 const uint32_t gw = pack_bf16(__uint_as_float(g[i]), __uint_as_float(g[i + 1]));
                 const uint32_t uw = pack_bf16(__uint_as_float(u[i]), __uint_as_float(u[i + 1]));
-                const float2 gf = unpack_bf16(gw), uf = unpack_bf16(uw);
                 pg[part * 16 + (i >> 1)] = gw;
                 pu[part * 16 + (i >> 1)] = uw;
-                pa[part * 16 + (i >> 1)] = pack_bf16(__fdividef(gf.x, 1.f + __expf(-gf.x)) * uf.x,
-                                                     __fdividef(gf.y, 1.f + __expf(-gf.y)) * uf.y);
+                pa[part * 16 + (i >> 1)] = swiglu2(gw, uw);
               }
             }
             const int col = t.n0 + h * 64;
@@ -742,38 +740,33 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             // all of this slab's gate / up loads are issued before the first store (the compiler must assume the
             // stores may alias them, so it would not hoist them itself); they overlap the staging above
             uint4 gv[8], uv[8];
+            const long long first = (long long)(row0 + sub_row) * 2 * p.N + col + chunk * 8;      // C and aux share the layout [M, 2 N]
+            const int rows_left = col + chunk * 8 < p.N ? t.m_end - (row0 + sub_row) : 0;
+            const __nv_bfloat16* gp = p.aux + first;
+            __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(p.C) + first;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              const int grow = row0 + i * 4 + sub_row;
               gv[i] = make_uint4(0, 0, 0, 0); uv[i] = gv[i];
-              if (grow < t.m_end && col + chunk * 8 < p.N) {
-                const __nv_bfloat16* gp = p.aux + (long long)grow * 2 * p.N + col + chunk * 8;
-                gv[i] = *reinterpret_cast<const uint4*>(gp);
-                uv[i] = *reinterpret_cast<const uint4*>(gp + p.N);
+              if (i * 4 < rows_left) {
+                gv[i] = *reinterpret_cast<const uint4*>(gp + (long long)i * 8 * p.N);
+                uv[i] = *reinterpret_cast<const uint4*>(gp + (long long)i * 8 * p.N + p.N);
               }
             }
             __syncwarp();
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int r = i * 4 + sub_row;                   // row within the warp's 32
-              const int grow = row0 + r;
               const uint32_t off = r * 128 + ((chunk ^ (r & 7)) << 4);
-              const bool live = grow < t.m_end && col + chunk * 8 < p.N;
               const uint4 dv = *reinterpret_cast<const uint4*>(buf + off);
               const uint32_t dw[4] = {dv.x, dv.y, dv.z, dv.w}, gw[4] = {gv[i].x, gv[i].y, gv[i].z, gv[i].w},
                              uw[4] = {uv[i].x, uv[i].y, uv[i].z, uv[i].w};
               uint32_t og[4], ou[4];
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const float2 dd = unpack_bf16(dw[k]), a = unpack_bf16(gw[k]), bb = unpack_bf16(uw[k]);
-                const float s0 = __fdividef(1.f, 1.f + __expf(-a.x)), s1 = __fdividef(1.f, 1.f + __expf(-a.y));
-                og[k] = pack_bf16(dd.x * bb.x * s0 * (1.f + a.x * (1.f - s0)), dd.y * bb.y * s1 * (1.f + a.y * (1.f - s1)));
-                ou[k] = pack_bf16(dd.x * a.x * s0, dd.y * a.y * s1);
-              }
-              if (live) {                                      // 8 lanes write one 128-byte row piece of d(gate) and of d(up)
-                __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(p.C) + (long long)grow * p.ldc + col + chunk * 8;
-                *reinterpret_cast<uint4*>(op) = make_uint4(og[0], og[1], og[2], og[3]);
-                *reinterpret_cast<uint4*>(op + p.N) = make_uint4(ou[0], ou[1], ou[2], ou[3]);
+              for (int k = 0; k < 4; ++k) swiglu_bwd2(dw[k], gw[k], uw[k], og[k], ou[k]);
+              if (i * 4 < rows_left) {                         // 8 lanes write one 128-byte row piece of d(gate) and of d(up)
+                __nv_bfloat16* o = op + (long long)i * 8 * p.N;
+                *reinterpret_cast<uint4*>(o) = make_uint4(og[0], og[1], og[2], og[3]);
+                *reinterpret_cast<uint4*>(o + p.N) = make_uint4(ou[0], ou[1], ou[2], ou[3]);
               }
             }
             __syncwarp();
