@@ -169,6 +169,46 @@ def test_gemm_heads_rope_epilogue(nat, gemm_mode, hd, Hq, Hkv, B, T, K):
     assert _rel_err(out[:, :, Hq + Hkv:], ref[:, :, Hq + Hkv:]) < 6e-3
 
 
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("hd,Hq,Hkv,B,T,K", [(64, 4, 2, 3, 33, 192), (64, 12, 4, 3, 1001, 768), (32, 8, 2, 2, 37, 192), (128, 2, 1, 5, 7, 256),
+                                              (64, 3, 1, 1, 1, 64), (128, 8, 4, 3, 335, 256), (32, 32, 4, 2, 777, 128)])
+def test_gemm_heads_any_number_of_rows(nat, mode, hd, Hq, Hkv, B, T, K):
+    """Batch entries whose row count is no multiple of 32 (a warp's rows cross entries)."""
+    import ctypes
+    from train_large_model_from_scratch_b200.ops import oracle
+    Ht = Hq + 2 * Hkv
+    x, w = _rand(B * T, K, seed=82), _rand(Ht * hd, K, scale=0.05, seed=83)
+    cos, sin = (t.contiguous() for t in oracle.rope_tables(torch.arange(7, 7 + T, device="cuda"), hd, 10000.0, "reference"))
+    out = torch.full((B * T * Ht * hd + 64,), 7.0, dtype=torch.bfloat16, device="cuda")
+    dst = (ctypes.c_void_p * 1)(out.data_ptr())
+    was = nat.set_gemm_pairs(mode)
+    nat.gemm_heads(x, w, False, dst, 1, B, T, T, Ht, 0, Hq, Hkv, Hq, Hkv, hd, Hq + Hkv, nat.rope_table_fp16(cos, sin), tables=(cos, sin))
+    nat.set_gemm_pairs(was)
+    nat.raise_on_device_status()
+    ref = (x.double() @ w.double().t()).view(B, T, Ht, hd)
+    ref[:, :, :Hq + Hkv] = oracle.rope(ref[:, :, :Hq + Hkv], cos.double(), sin.double())
+    got = out[:B * T * Ht * hd].view(B, T, Ht, hd).double()
+    assert ((got - ref).norm() / ref.norm()).item() < 2.5e-3 and bool((out[B * T * Ht * hd:] == 7.0).all())
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("M,I,K", [(1, 8, 64), (333, 200, 192), (130, 2056, 768), (3003, 2056, 256), (256, 136, 4096)])
+def test_swiglu_epilogues_of_any_width(nat, mode, M, I, K):
+    """An MLP width that is no multiple of 128: the last tile's gate columns must not reach the up half (nor the rows below)."""
+    x, w, wd, dy = _rand(M, K, seed=84), _rand(2 * I, K, scale=0.05, seed=85), _rand(K, I, scale=0.05, seed=86), _rand(M, K, seed=87)
+    was = nat.set_gemm_pairs(mode)
+    gu, act = nat.gemm_swiglu(x, w)
+    dgu = nat.gemm_swiglu_bwd(dy, wd, gu)
+    nat.set_gemm_pairs(was)
+    nat.raise_on_device_status()
+    assert _rel_err(gu, x.float() @ w.float().t()) < 6e-3
+    g, u = gu.float().chunk(2, dim=-1)
+    sig = torch.sigmoid(g)
+    assert _rel_err(act, g * sig * u) < 6e-3
+    d = (dy.float() @ wd.float()).bfloat16().float()
+    assert _rel_err(dgu, torch.cat([d * u * sig * (1 + g * (1 - sig)), d * g * sig], dim=-1)) < 6e-3
+
+
 def test_gemm_heads_scatter_plan(nat, gemm_mode):
     """Two destinations (both local buffers here) with the Ulysses head plan and a row offset; MN-major weight."""
     import ctypes

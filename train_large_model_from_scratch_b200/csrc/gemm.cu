@@ -46,7 +46,8 @@ constexpr int PAIR_STAGE_BYTES = A_BYTES + B_BYTES / 2;
 constexpr int GEMM_SMEM_PAIR = PAIR_STAGES * PAIR_STAGE_BYTES + EPI_BYTES + 1024 + TAIL_BYTES;
 
 enum Epilogue { EPI_BF16 = 0, EPI_F32_ACC = 1, EPI_F32 = 2, EPI_HEADS = 3, EPI_SWIGLU = 4, EPI_SWIGLU_BWD = 5, EPI_LSE = 6,
-                EPI_ROWS = 7 /* bf16 rows stored at looked-up (buffer, row): the expert-parallel combine */ };
+                EPI_ROWS = 7 /* bf16 rows stored at looked-up (buffer, row): the expert-parallel combine */,
+                EPI_HEADS_ANY = 8 /* EPI_HEADS to one destination for any rows_per_batch, fp32 rotation tables */ };
 
 // Destinations of the head-scatter epilogue: one 4-D map (hd, heads, T, B; box 64 x 1 x 32 x 1)
 // per rank of the sequence-parallel group; entry 0 alone when the output stays local.
@@ -81,6 +82,11 @@ struct GemmParams {
   int hd, rows_per_batch, row_off, Hq, Hkv, q_l, kv_l, n_rot, kv_rep;
   const __half2* cs;        // [rows_per_batch, hd] (cos, sin) pairs in fp16: |error| < 2^-11, below the bf16 rounding of
                             // the rotated outputs, and half the table bytes of two fp32 tables
+  // EPI_HEADS_ANY: a warp's 32 rows may belong to several batch entries. Such a warp stores its rows one by one instead of
+  // with TMA tile stores, at C = [batch, heads_rows, heads_pitch, hd]; cos / sin come from fp32 tables [rows_per_batch, hd].
+  const float* cosT;
+  const float* sinT;
+  int heads_rows, heads_pitch;
   // EPI_SWIGLU (MLP forward): B is the fused [2 I, K] weight (gate rows, then up rows), N = I. A tile holds the
   //   SAME 128 columns of gate and of up (two 128-row B boxes), and the epilogue writes three bf16 tiles:
   //   gate and up into C = gate_up [M, 2 I] (kept for backward) and silu(gate) * up into act [M, I].
@@ -478,6 +484,41 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     for (int tile = worker; tile < total_tiles && ok; tile += n_workers) {
       TileCoord t = get_tile(tile, grp);
       if (!t.valid) continue;
+      // EPI_HEADS_ANY: this lane's own batch entry and position, and its row of the fp32 tables: 32 (cos, sin) of the lower and
+      // of the upper half-head columns [c, c + n). Requested before the accumulator is waited for and kept for all heads of
+      // the tile: fetched per head, these row-per-lane loads made the epilogue three times as long as the main loop.
+      const int lane_row = t.m0 + q * 32 + lane, lane_b = EPI == EPI_HEADS_ANY ? lane_row / p.rows_per_batch : 0;
+      const int lane_t = EPI == EPI_HEADS_ANY ? lane_row - lane_b * p.rows_per_batch : 0;
+      float tab_cl[EPI == EPI_HEADS_ANY ? 32 : 1], tab_sl[EPI == EPI_HEADS_ANY ? 32 : 1], tab_ch[EPI == EPI_HEADS_ANY ? 32 : 1], tab_sh[EPI == EPI_HEADS_ANY ? 32 : 1];
+      auto load_tab = [&](int c, int n) {
+        if constexpr (EPI == EPI_HEADS_ANY) {
+          const float* cp = p.cosT + (long long)lane_t * p.hd + c;
+          const float* sp = p.sinT + (long long)lane_t * p.hd + c;
+          const int half = p.hd >> 1;
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            if (i < n) {
+              *reinterpret_cast<float4*>(tab_cl + i) = *reinterpret_cast<const float4*>(cp + i);
+              *reinterpret_cast<float4*>(tab_sl + i) = *reinterpret_cast<const float4*>(sp + i);
+              *reinterpret_cast<float4*>(tab_ch + i) = *reinterpret_cast<const float4*>(cp + half + i);
+              *reinterpret_cast<float4*>(tab_sh + i) = *reinterpret_cast<const float4*>(sp + half + i);
+            }
+          }
+        }
+      };
+      auto rotate_any = [&](uint32_t* lo, uint32_t* hi, int n) {
+        if constexpr (EPI == EPI_HEADS_ANY) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            if (i < n) {
+              const float a = __uint_as_float(lo[i]), b = __uint_as_float(hi[i]);
+              lo[i] = __float_as_uint(a * tab_cl[i] - b * tab_sl[i]);
+              hi[i] = __float_as_uint(b * tab_ch[i] + a * tab_sh[i]);
+            }
+          }
+        }
+      };
+      if (EPI == EPI_HEADS_ANY && t.n0 / p.hd < p.n_rot) load_tab(0, p.hd == 32 ? 16 : 32);
       if (EPI == EPI_SWIGLU_BWD) {
         // gate / up of the NEXT tile start moving into L2 now, a whole tile time before they are read
         auto prefetch_aux = [&](const TileCoord& tt) {
@@ -501,15 +542,27 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       const int row = t.m0 + q * 32 + lane;
       const bool row_ok = row < t.m_end;
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
-      if (EPI == EPI_HEADS) {
+      if (EPI == EPI_HEADS || EPI == EPI_HEADS_ANY) {
+        constexpr bool ANY = EPI == EPI_HEADS_ANY;
         // One head (hd columns) at a time: TMEM -> RoPE -> bf16 -> swizzled staging tile(s) -> TMA store into
-        // the head owner's packed tensor. The warp's 32 rows belong to one batch entry (rows_per_batch % 32 == 0).
+        // the head owner's packed tensor. The warp's 32 rows belong to one batch entry (EPI_HEADS: rows_per_batch % 32 == 0).
         uint8_t* ebuf = smem_al + STAGES * STAGE_BYTES + (warp - 2) * 2 * EPI_BUF_BYTES;
         const uint32_t ebuf_s = smem_base + STAGES * STAGE_BYTES + (warp - 2) * 2 * EPI_BUF_BYTES;
         const int grow = t.m0 + q * 32;
-        const bool rows_ok = grow < p.M;                       // warp-uniform (M % 32 == 0)
+        const bool rows_ok = grow < p.M;                       // warp-uniform (EPI_HEADS: M % 32 == 0)
         const int bi = grow / p.rows_per_batch, t0 = grow - bi * p.rows_per_batch;
-        const int hd = p.hd, half = hd >> 1;
+        const int hd = p.hd;
+        // EPI_HEADS_ANY: does the warp's tile store cover exactly its rows?
+        const bool tile_store = !ANY || (t0 + 32 <= p.rows_per_batch && grow + 32 <= p.M);
+        auto put_row = [&](const uint32_t* r, int slot, int c) {       // 32 columns of this lane's row
+          if (lane_row >= p.M) return;
+          uint4* out = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.C) +
+              (((long long)lane_b * p.heads_rows + p.row_off + lane_t) * p.heads_pitch + slot) * p.hd + c);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            out[i] = make_uint4(pack_bf16(__uint_as_float(r[8 * i]), __uint_as_float(r[8 * i + 1])), pack_bf16(__uint_as_float(r[8 * i + 2]), __uint_as_float(r[8 * i + 3])),
+                                pack_bf16(__uint_as_float(r[8 * i + 4]), __uint_as_float(r[8 * i + 5])), pack_bf16(__uint_as_float(r[8 * i + 6]), __uint_as_float(r[8 * i + 7])));
+        };
         const int n_heads = p.Hq + 2 * p.Hkv;
         const uint4* csrow = reinterpret_cast<const uint4*>(p.cs + (long long)(t0 + lane) * hd);   // 4 (cos, sin) pairs per 16 bytes
         // rotate 32 (lo, hi) column pairs with their (cos, sin) entries: lo = columns [c, c+32), hi = [c+half, c+half+32)
@@ -546,8 +599,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         };
         const int heads_per_tile = BN / hd;
         uint32_t cs_lo[32], cs_hi[32];                       // hd 64: the row's whole table, shared by the tile's heads
-        if (hd == 64 && rows_ok && t.n0 / hd < p.n_rot) { load_cs(cs_lo, 0); load_cs(cs_hi, 32); }
-        if (hd == 32 && rows_ok && t.n0 / hd < p.n_rot) load_cs(cs_lo, 0);
+        if (!ANY && hd == 64 && rows_ok && t.n0 / hd < p.n_rot) { load_cs(cs_lo, 0); load_cs(cs_hi, 32); }
+        if (!ANY && hd == 32 && rows_ok && t.n0 / hd < p.n_rot) load_cs(cs_lo, 0);
 #pragma unroll 1
         for (int hh = 0; hh < heads_per_tile; ++hh) {
           const int head = t.n0 / hd + hh;
@@ -572,7 +625,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             __syncwarp();
             tmem_ld_wait();
             if (live) {
-              if (rot) {
+              if (ANY && rot) rotate_any(r0, r0 + 16, 16);
+              if (!ANY && rot) {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {                    // pairs (i, i + 16) with their own table entries
                   const float2 l = __half22float2(*reinterpret_cast<const __half2*>(&cs_lo[i]));
@@ -582,12 +636,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
                   r0[i + 16] = __float_as_uint(b * h.x + a * h.y);
                 }
               }
-              stage32(r0, ebuf + bsel * EPI_BUF_BYTES, 0);
+              if (tile_store) stage32(r0, ebuf + bsel * EPI_BUF_BYTES, 0);
+              else put_row(r0, slot, 0);
             }
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              if (live)
+              if (live && tile_store)
                 for (int c = 0; c < copies; ++c)
                   asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
                                ::"l"((uint64_t)(dst_maps + dest + c)), "r"(ebuf_s + bsel * EPI_BUF_BYTES), "r"(0), "r"(slot),
@@ -603,14 +658,19 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             __syncwarp();
             tmem_ld_wait();
             if (live) {
-              if (rot) rotate(r0, r1, cs_lo, cs_hi);
-              stage32(r0, ebuf + bsel * EPI_BUF_BYTES, 0);
-              stage32(r1, ebuf + bsel * EPI_BUF_BYTES, 4);
+              if (rot) { if (ANY) rotate_any(r0, r1, 32); else rotate(r0, r1, cs_lo, cs_hi); }
+              if (tile_store) {
+                stage32(r0, ebuf + bsel * EPI_BUF_BYTES, 0);
+                stage32(r1, ebuf + bsel * EPI_BUF_BYTES, 4);
+              } else {
+                put_row(r0, slot, 0);
+                put_row(r1, slot, 32);
+              }
             }
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              if (live)
+              if (live && tile_store)
                 for (int c = 0; c < copies; ++c)
                   asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
                                ::"l"((uint64_t)(dst_maps + dest + c)), "r"(ebuf_s + bsel * EPI_BUF_BYTES), "r"(0), "r"(slot),
@@ -621,21 +681,30 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             __syncwarp();
 #pragma unroll 1
-            for (int part = 0; part < 2; ++part) {              // columns [32 part, +32) pair with [64 + 32 part, +32)
+            for (int pi = 0; pi < 2; ++pi) {                    // columns [32 part, +32) pair with [64 + 32 part, +32)
+              // EPI_HEADS_ANY: the second head starts with the part whose tables the first one ended with
+              const int part = ANY ? pi ^ (hh & 1) : pi;
+              if (ANY && pi == 1 && rot) load_tab(part * 32, 32);
               uint32_t r0[32], r1[32];
               tmem_ld32(taddr + hh * 128 + part * 32, r0);
               tmem_ld32(taddr + hh * 128 + 64 + part * 32, r1);
               tmem_ld_wait();
               if (live) {
-                if (rot) { load_cs(cs_lo, part * 32); load_cs(cs_hi, 64 + part * 32); rotate(r0, r1, cs_lo, cs_hi); }
-                stage32(r0, ebuf, part * 4);
-                stage32(r1, ebuf + EPI_BUF_BYTES, part * 4);
+                if (ANY) { if (rot) rotate_any(r0, r1, 32); }
+                else if (rot) { load_cs(cs_lo, part * 32); load_cs(cs_hi, 64 + part * 32); rotate(r0, r1, cs_lo, cs_hi); }
+                if (tile_store) {
+                  stage32(r0, ebuf, part * 4);
+                  stage32(r1, ebuf + EPI_BUF_BYTES, part * 4);
+                } else {
+                  put_row(r0, slot, part * 32);
+                  put_row(r1, slot, 64 + part * 32);
+                }
               }
             }
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              if (live) {
+              if (live && tile_store) {
                 for (int c = 0; c < copies; ++c)
 #pragma unroll
                   for (int s2 = 0; s2 < 2; ++s2)
@@ -658,12 +727,16 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         // warps whose 32 rows all belong to the tile's row range use TMA tile stores; a warp that straddles the end
         // of its group (grouped mode) stores its rows one by one: `base` / `ld` locate the same tensor for that
         const bool whole = row0 + 32 <= t.m_end;               // warp-uniform
-        auto put = [&](const uint32_t* w, const CUtensorMap* map, int col, __nv_bfloat16* base, long long ld) {
+        // `which`: middle coordinate of the map (gate | up are one [M, 2, I] tensor, so a slab past column I is clipped there
+        // and never reaches the other half); `base` already points at that half
+        auto put = [&](const uint32_t* w, const CUtensorMap* map, int col, int which, __nv_bfloat16* base, long long ld) {
+          if (col >= p.N) return;                              // warp-uniform
           if (!whole) {
             if (row0 + lane < t.m_end) {
               uint4* dst = reinterpret_cast<uint4*>(base + (long long)(row0 + lane) * ld + col);
 #pragma unroll
-              for (int ch = 0; ch < 8; ++ch) dst[ch] = make_uint4(w[4 * ch], w[4 * ch + 1], w[4 * ch + 2], w[4 * ch + 3]);
+              for (int ch = 0; ch < 8; ++ch)
+                if (col + ch * 8 < p.N) dst[ch] = make_uint4(w[4 * ch], w[4 * ch + 1], w[4 * ch + 2], w[4 * ch + 3]);
             }
             return;
           }
@@ -677,13 +750,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
           __syncwarp();
           if (lane == 0) {
             if (row0 < p.M)
-              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-                           ::"l"((uint64_t)map), "r"(ebuf_s + bsel * EPI_BUF_BYTES), "r"(col), "r"(row0) : "memory");
+              asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+                           ::"l"((uint64_t)map), "r"(ebuf_s + bsel * EPI_BUF_BYTES), "r"(col), "r"(which), "r"(row0) : "memory");
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
           bsel ^= 1;
         };
-        if (EPI == EPI_SWIGLU) {
+        if constexpr (EPI == EPI_SWIGLU) {
 #pragma unroll 1
           for (int h = 0; h < 2; ++h) {                      // two 64-column halves of the tile's 128 act columns
             uint32_t pg[32], pu[32], pa[32];
@@ -703,9 +776,9 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
               }
             }
             const int col = t.n0 + h * 64;
-            put(pg, &tmC, col, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc);
-            put(pu, &tmC, p.N + col, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc);
-            put(pa, dst_maps, col, p.act, p.ld_act);
+            put(pg, &tmC, col, 0, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc);
+            put(pu, &tmC, col, 1, reinterpret_cast<__nv_bfloat16*>(p.C) + p.N, p.ldc);
+            put(pa, dst_maps, col, 0, p.act, p.ld_act);
           }
         } else {
           // d(act) leaves tensor memory one row per lane, but the derivative is elementwise, so the warp stages
@@ -998,7 +1071,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       }
       if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
-    if ((((EPI == EPI_BF16 || EPI == EPI_F32_ACC) && p.tma_store) || EPI == EPI_HEADS || EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_BWD) && lane == 0)
+    if ((((EPI == EPI_BF16 || EPI == EPI_F32_ACC) && p.tma_store) || EPI == EPI_HEADS || EPI == EPI_HEADS_ANY || EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_BWD) && lane == 0)
       asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 
@@ -1020,11 +1093,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 }
 
 // Same main loop, head-scatter epilogue: the output maps (one per destination rank) replace the C map.
-template <bool B_MN, bool GATED = false>
+template <bool B_MN, bool GATED = false, int EPI = EPI_HEADS>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_heads_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const __grid_constant__ HeadDstMaps dst, const GemmParams p) {
-  gemm_body<false, B_MN, EPI_HEADS, GATED>(tmA, tmB, tmA, p, dst.m);
+  gemm_body<false, B_MN, EPI, GATED>(tmA, tmB, tmA, p, dst.m);
 }
 
 // MLP forward / backward with the SwiGLU math in the epilogue: `tmC` is the [M, 2 I] tensor the epilogue
@@ -1049,11 +1122,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmC, const GemmParams p) {
   gemm_body<A_MN, B_MN, EPI, false, true, GROUP>(tmA, tmB, tmC, p, nullptr);
 }
-template <bool B_MN>
+template <bool B_MN, int EPI = EPI_HEADS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_heads_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                        const __grid_constant__ HeadDstMaps dst, const GemmParams p) {
-  gemm_body<false, B_MN, EPI_HEADS, false, true>(tmA, tmB, tmA, p, dst.m);
+  gemm_body<false, B_MN, EPI, false, true>(tmA, tmB, tmA, p, dst.m);
 }
 template <int GROUP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
@@ -1204,11 +1277,11 @@ static int dispatch(bool a_mn, bool b_mn, int epi, const CUtensorMap& ma, const 
   return -2;
 }
 
-template <bool B_MN, bool GATED = false>
+template <bool B_MN, bool GATED = false, int EPI = EPI_HEADS>
 static int launch_heads(const CUtensorMap& ma, const CUtensorMap& mb, const HeadDstMaps& dst, const GemmParams& p,
                         int tiles, cudaStream_t st) {
   static bool configured = false;
-  auto kern = gemm_heads_kernel<B_MN, GATED>;
+  auto kern = gemm_heads_kernel<B_MN, GATED, EPI>;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
     if (e != cudaSuccess) return (int)e;
@@ -1221,11 +1294,11 @@ static int launch_heads(const CUtensorMap& ma, const CUtensorMap& mb, const Head
   return launch_status();
 }
 
-template <bool B_MN>
+template <bool B_MN, int EPI = EPI_HEADS>
 static int launch_heads_pair(const CUtensorMap& ma, const CUtensorMap& mb, const HeadDstMaps& dst, const GemmParams& p,
                              int tiles, cudaStream_t st) {
   static bool configured = false;
-  auto kern = gemm_heads_pair_kernel<B_MN>;
+  auto kern = gemm_heads_pair_kernel<B_MN, EPI>;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_PAIR);
     if (e != cudaSuccess) return (int)e;
@@ -1256,13 +1329,17 @@ TLM_API int tlm_gemm_set_pair(int mode) {
 //   N = (Hq + 2 Hkv) * hd;  dst_ptrs[r]: bf16 [batch, dst_rows, dst_heads, hd] on rank r (peer-mapped
 //   addresses are fine: the stores are TMA tile stores without multicast);  cs: fp16 (cos, sin) pairs
 //   [rows_per_batch, hd, 2] for the heads below n_rot.
-// Requirements: hd in {32, 64, 128}, rows_per_batch % 32 == 0, n_dst <= 8, Hq % q_l == 0, Hkv % kv_l == 0.
+// Requirements: hd in {32, 64, 128}, n_dst <= 8, Hq % q_l == 0, Hkv % kv_l == 0; rows_per_batch % 32 == 0 unless there is
+// one destination, x W^T and, for rotated heads, the fp32 tables cosT / sinT [rows_per_batch, hd] (used then instead of cs).
 TLM_API int tlm_gemm_heads(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, int b_mn,
                            void* const* dst_ptrs, int n_dst, int batch, int rows_per_batch, int dst_rows, int dst_heads,
                            int row_off, int Hq, int Hkv, int q_l, int kv_l, int hd, int n_rot, const void* cs,
-                           int kv_rep, cudaStream_t stream) {
+                           int kv_rep, const float* cosT, const float* sinT, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if ((hd != 32 && hd != 64 && hd != 128) || rows_per_batch % 32 != 0 || n_dst < 1 || n_dst > MAX_HEAD_DST) return -4;
+  if ((hd != 32 && hd != 64 && hd != 128) || n_dst < 1 || n_dst > MAX_HEAD_DST) return -4;
+  const bool f32_tables = n_rot == 0 || (cosT != nullptr && sinT != nullptr);
+  const bool any_rows = rows_per_batch % 32 != 0;
+  if (any_rows && (n_dst != 1 || b_mn || !f32_tables)) return -4;
   if (M != batch * rows_per_batch || N != (Hq + 2 * Hkv) * hd || q_l <= 0 || Hq % q_l != 0) return -5;
   if (kv_rep < 1) kv_rep = 1;
   if (kv_rep > 1) {                     // replicated KV heads: every destination holds exactly one k and one v head
@@ -1272,7 +1349,7 @@ TLM_API int tlm_gemm_heads(const void* A, const void* B, int M, int N, int K, lo
     if (Hkv > 0 && (kv_l <= 0 || Hkv % kv_l != 0)) return -5;
     if (Hq / q_l > n_dst || (Hkv > 0 && Hkv / kv_l > n_dst)) return -5;
   }
-  if (n_rot > 0 && cs == nullptr) return -5;
+  if (n_rot > 0 && cs == nullptr && !any_rows) return -5;
   GemmParams p{};
   if (!b_mn) take_pending_waits(p);               // x W^T: may be the first reader of its weights after an optimizer step
   const bool pair = use_pair(M) && p.wait_flags[0] == nullptr;
@@ -1292,48 +1369,56 @@ TLM_API int tlm_gemm_heads(const void* A, const void* B, int M, int N, int K, lo
   p.split_k = 1; p.k_chunk = K;
   p.hd = hd; p.rows_per_batch = rows_per_batch; p.row_off = row_off; p.Hq = Hq; p.Hkv = Hkv;
   p.q_l = q_l; p.kv_l = kv_l > 0 ? kv_l : 1; p.n_rot = n_rot; p.cs = (const __half2*)cs; p.kv_rep = kv_rep;
+  p.cosT = cosT; p.sinT = sinT; p.heads_rows = dst_rows; p.heads_pitch = dst_heads; p.C = dst_ptrs[0];
   if (pair) {
     const int ptiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
+    if (any_rows) return launch_heads_pair<false, EPI_HEADS_ANY>(ma, mb, dst, p, ptiles, stream);
     return b_mn ? launch_heads_pair<true>(ma, mb, dst, p, ptiles, stream) : launch_heads_pair<false>(ma, mb, dst, p, ptiles, stream);
   }
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+  if (any_rows)
+    return p.wait_flags[0] != nullptr ? launch_heads<false, true, EPI_HEADS_ANY>(ma, mb, dst, p, tiles, stream)
+                                      : launch_heads<false, false, EPI_HEADS_ANY>(ma, mb, dst, p, tiles, stream);
   if (!b_mn && p.wait_flags[0] != nullptr) return launch_heads<false, true>(ma, mb, dst, p, tiles, stream);
   return b_mn ? launch_heads<true>(ma, mb, dst, p, tiles, stream) : launch_heads<false>(ma, mb, dst, p, tiles, stream);
 }
 
-static int store_map_bf16(CUtensorMap* m, void* base, long long rows, long long cols, long long ld) {
-  uint64_t dims[2] = {(uint64_t)cols, (uint64_t)rows}, strides[1] = {(uint64_t)ld * 2};
-  uint32_t box[2] = {64, 32};
-  return make_tmap_bf16(m, base, 2, dims, strides, box);
+// [rows, parts, cols] bf16, contiguous: one 64 x 32 slab of one part per store
+static int store_map_bf16(CUtensorMap* m, void* base, long long rows, long long parts, long long cols) {
+  uint64_t dims[3] = {(uint64_t)cols, (uint64_t)parts, (uint64_t)rows}, strides[2] = {(uint64_t)cols * 2, (uint64_t)(parts * cols) * 2};
+  uint32_t box[3] = {64, 1, 32};
+  return make_tmap_bf16(m, base, 3, dims, strides, box);
 }
 
 // gate_up[M, 2 I] = x[M, K] * w_gu[2 I, K]^T  and  act[M, I] = silu(gate) * up, in one kernel.
-// Requirements: I % 128 == 0, contiguous outputs (row pitches 2 I and I).
+// Requirements: I % 8 == 0, contiguous outputs (row pitches 2 I and I). In the last tile of a width that is no multiple of
+// 128 the gate rows of B run on into the up rows; those columns are clipped by the stores.
 TLM_API int tlm_gemm_swiglu(const void* x, const void* w_gu, void* gate_up, void* act, int M, int I, int K,
                             long long lda, long long ldb, cudaStream_t stream) {
   if (M <= 0 || I <= 0 || K <= 0) return 0;
-  if (I % 128 != 0) return -4;
+  if (I % 8 != 0) return -4;
+  const bool pair = use_pair(M);
   Operand oa{x, M, K, lda, false, 0, 0}, ob{w_gu, 2LL * I, K, ldb, false, 1, 2LL * I * K};
   CUtensorMap ma, mb, mc, md;
   int e = build_map(&ma, oa, BM);
   if (e) return e;
   e = build_map(&mb, ob, 128);
   if (e) return e;
-  e = store_map_bf16(&mc, gate_up, M, 2LL * I, 2LL * I);
+  e = store_map_bf16(&mc, gate_up, M, 2, I);
   if (e) return e;
-  e = store_map_bf16(&md, act, M, I, I);
+  e = store_map_bf16(&md, act, M, 1, I);
   if (e) return e;
   GemmParams p{};
   p.M = M; p.N = I; p.K = K; p.C = gate_up; p.ldc = 2LL * I; p.status = status_word(); p.split_k = 1; p.k_chunk = K;
   p.act = (__nv_bfloat16*)act; p.ld_act = I;
-  if (use_pair(M)) {               // the B map's 128-row boxes serve both forms: rank 0 loads gate rows, rank 1 up rows
+  if (pair) {                      // the B map's 128-row boxes serve both forms: rank 0 loads gate rows, rank 1 up rows
     static bool pconfigured = false;
     if (!pconfigured) {
       cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_pair_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_PAIR);
       if (ce != cudaSuccess) return (int)ce;
       pconfigured = true;
     }
-    const int pgrid = pair_grid((long long)((M + 2 * BM - 1) / (2 * BM)) * (I / 128));
+    const int pgrid = pair_grid((long long)((M + 2 * BM - 1) / (2 * BM)) * ((I + 127) / 128));
     gemm_swiglu_pair_kernel<0><<<pgrid, GEMM_THREADS, GEMM_SMEM_PAIR, stream>>>(ma, mb, mc, md, p);
     count_launch();
     return launch_status();
@@ -1344,7 +1429,7 @@ TLM_API int tlm_gemm_swiglu(const void* x, const void* w_gu, void* gate_up, void
     if (ce != cudaSuccess) return (int)ce;
     configured = true;
   }
-  const int tiles = ((M + BM - 1) / BM) * (I / 128);
+  const int tiles = ((M + BM - 1) / BM) * ((I + 127) / 128);
   const int grid = tiles < num_sms() ? tiles : num_sms();
   gemm_swiglu_kernel<0><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ma, mb, mc, md, p);
   count_launch();
@@ -1357,18 +1442,19 @@ TLM_API int tlm_gemm_swiglu_bwd(const void* dy, const void* w_down, const void* 
                                 int D, long long lda, long long ldb, cudaStream_t stream) {
   if (M <= 0 || I <= 0 || D <= 0) return 0;
   if (I % 8 != 0) return -4;
+  const bool pair = use_pair(M);
   Operand oa{dy, M, D, lda, false, 0, 0}, ob{w_down, I, D, ldb, true, 1, (long long)I * D};
   CUtensorMap ma, mb, mc;
   int e = build_map(&ma, oa, BM);
   if (e) return e;
   e = build_map(&mb, ob, BN);
   if (e) return e;
-  e = store_map_bf16(&mc, d_gate_up, M, 2LL * I, 2LL * I);
+  e = store_map_bf16(&mc, d_gate_up, M, 2, I);
   if (e) return e;
   GemmParams p{};
   p.M = M; p.N = I; p.K = D; p.C = d_gate_up; p.ldc = 2LL * I; p.status = status_word(); p.split_k = 1; p.k_chunk = D;
   p.aux = (const __nv_bfloat16*)gate_up;
-  if (use_pair(M)) {               // MN-major B: 64-wide boxes in both forms
+  if (pair) {                      // MN-major B: 64-wide boxes in both forms
     static bool pconfigured = false;
     if (!pconfigured) {
       cudaError_t ce = cudaFuncSetAttribute(gemm_swiglu_bwd_pair_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_PAIR);
@@ -1433,9 +1519,9 @@ TLM_API int tlm_gemm_swiglu_grouped(const void* x, const void* w_pair, void* gat
   if (e) return e;
   e = build_map(&mb, ob, 128);
   if (e) return e;
-  e = store_map_bf16(&mc, gate_up, R, 2LL * I, 2LL * I);
+  e = store_map_bf16(&mc, gate_up, R, 2, I);
   if (e) return e;
-  e = store_map_bf16(&md, act, R, I, I);
+  e = store_map_bf16(&md, act, R, 1, I);
   if (e) return e;
   GemmParams p{};
   p.M = R; p.N = I; p.K = K; p.C = gate_up; p.ldc = 2LL * I; p.status = status_word(); p.split_k = 1; p.k_chunk = K;
@@ -1470,7 +1556,7 @@ TLM_API int tlm_gemm_swiglu_bwd_grouped(const void* dy, const void* w_down, cons
   if (e) return e;
   e = build_map(&mb, ob, BN);
   if (e) return e;
-  e = store_map_bf16(&mc, d_gate_up, R, 2LL * I, 2LL * I);
+  e = store_map_bf16(&mc, d_gate_up, R, 2, I);
   if (e) return e;
   GemmParams p{};
   p.M = R; p.N = I; p.K = D; p.C = d_gate_up; p.ldc = 2LL * I; p.status = status_word(); p.split_k = 1; p.k_chunk = D;

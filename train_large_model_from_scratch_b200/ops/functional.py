@@ -179,7 +179,7 @@ class _QKVProject(torch.autograd.Function):
         import ctypes
         dst = (ctypes.c_void_p * 1)(out.data_ptr())
         native.gemm_heads(h, weight, False, dst, 1, B, T, T, Ht, 0, n_q, n_kv, n_q, max(n_kv, 1), hd,
-                          n_q + n_kv, cs)
+                          n_q + n_kv, cs, tables=(cos, sin))
         return out
 
     @staticmethod
@@ -205,7 +205,8 @@ class _QKVAttention(torch.autograd.Function):
         qkv = torch.empty(B, T, Ht, hd, dtype=torch.bfloat16, device=h.device)
         import ctypes
         dst = (ctypes.c_void_p * 1)(qkv.data_ptr())
-        native.gemm_heads(h, weight, False, dst, 1, B, T, T, Ht, 0, n_q, n_kv, n_q, max(n_kv, 1), hd, n_q + n_kv, cs)
+        native.gemm_heads(h, weight, False, dst, 1, B, T, T, Ht, 0, n_q, n_kv, n_q, max(n_kv, 1), hd, n_q + n_kv, cs,
+                          tables=(cos, sin))
         o, lse = native.flash_attn_fwd(qkv, n_q, n_kv, True)
         ctx.save_for_backward(h, qkv, o, lse, cos, sin)
         ctx.weight, ctx.meta = weight, (n_q, n_kv)
@@ -234,7 +235,7 @@ def qkv_project_fused_ok(h: torch.Tensor, weight: torch.Tensor | None, hd: int, 
 
 def qkv_project(h, weight, cos, sin, cs, B: int, T: int, n_q: int, n_kv: int, hd: int) -> torch.Tensor:
     """CUDA only (check `qkv_project_fused_ok` first). `cs` = `native.rope_table_fp16(cos, sin)`."""
-    return _QKVProject.apply(h, weight, cos, sin, cs, B, T, n_q, n_kv, hd)
+    return _QKVProject.apply(h, weight, cos.contiguous(), sin.contiguous(), cs, B, T, n_q, n_kv, hd)
 
 
 # --------------------------------------------------------------------------- attention

@@ -55,7 +55,7 @@ _SIGS = {
     "tlm_get_deterministic": (_I, []),
     "tlm_gemm_set_pair": (_I, [_I]),
     "tlm_gemm": (_I, [_P, _P, _P, _I, _I, _I, _LL, _LL, _LL, _I, _I, _I, _P]),
-    "tlm_gemm_heads": (_I, [_P, _P, _I, _I, _I, _LL, _LL, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P]),
+    "tlm_gemm_heads": (_I, [_P, _P, _I, _I, _I, _LL, _LL, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P, _P, _P]),
     "tlm_gemm_swiglu": (_I, [_P, _P, _P, _P, _I, _I, _I, _LL, _LL, _P]),
     "tlm_gemm_swiglu_bwd": (_I, [_P, _P, _P, _P, _I, _I, _I, _LL, _LL, _P]),
     "tlm_gemm_swiglu_grouped": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _LL, _LL, _I, _P]),
@@ -263,8 +263,9 @@ def gemm_tn_accum(dy: torch.Tensor, x: torch.Tensor, acc: torch.Tensor) -> None:
 
 def heads_epilogue_ok(hd: int, rows_per_batch: int, n_dst: int = 1) -> bool:
     """Shapes the head-scatter GEMM epilogue supports."""
-    # head dim 32 only without an exchange (one destination): the attention kernels' scatter forms take 64 / 128
-    return (hd in (64, 128) or (hd == 32 and n_dst == 1)) and rows_per_batch % 32 == 0 and 1 <= n_dst <= 8
+    # head dim 32 only without an exchange (one destination): the attention kernels' scatter forms take 64 / 128. With one
+    # destination a batch entry may have any number of rows (the caller then passes the fp32 `tables` to `gemm_heads`)
+    return (hd in (64, 128) or (hd == 32 and n_dst == 1)) and (rows_per_batch % 32 == 0 or n_dst == 1) and 1 <= n_dst <= 8
 
 
 def rope_table_fp16(cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
@@ -275,15 +276,19 @@ def rope_table_fp16(cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
 
 def gemm_heads(x: torch.Tensor, w: torch.Tensor, b_mn: bool, dst_ptrs, n_dst: int, batch: int, rows_per_batch: int,
                dst_rows: int, dst_heads: int, row_off: int, n_q: int, n_kv: int, q_l: int, kv_l: int, hd: int,
-               n_rot: int, cs: torch.Tensor | None, kv_rep: int = 1) -> None:
+               n_rot: int, cs: torch.Tensor | None, kv_rep: int = 1, tables=None) -> None:
     """Projection GEMM with the head-scatter epilogue (`csrc/gemm.cu`, `tlm_gemm_heads`):
     `x [batch*rows_per_batch, K]` times `w` (`[N, K]`, or `[K, N]` when `b_mn`), N = (n_q + 2 n_kv) * hd;
     head h of row (b, t) -> RoPE (heads < n_rot, table `cs` from `rope_table_fp16`) ->
     `dst[owner(h)][b, row_off + t, slot(h), :]`.
     `dst_ptrs` is a ctypes array of `n_dst` device addresses (this rank's own tensor or peers' buffers).
     `kv_rep > 1` (fewer KV heads than destinations): k / v head j goes to the `kv_rep` destinations
-    `j * kv_rep .. j * kv_rep + kv_rep - 1`, slots `q_l` and `q_l + 1`."""
+    `j * kv_rep .. j * kv_rep + kv_rep - 1`, slots `q_l` and `q_l + 1`. `tables` (optional): the fp32 `(cos, sin)`
+    `[rows_per_batch, hd]` that `cs` was made from; batch entries whose row
+    count is no multiple of 32 rotate with them."""
     M, K, lda = _rows(x)
+    cos, sin = tables if tables is not None else (None, None)
+    assert tables is None or all(t.dtype == torch.float32 and t.shape == (rows_per_batch, hd) and t.is_contiguous() for t in tables)
     if b_mn:
         K2, N, ldb = _rows(w)
     else:
@@ -292,11 +297,11 @@ def gemm_heads(x: torch.Tensor, w: torch.Tensor, b_mn: bool, dst_ptrs, n_dst: in
     assert cs is None or (cs.dtype == torch.float16 and cs.shape == (rows_per_batch, hd, 2) and cs.is_contiguous())
     _check(lib().tlm_gemm_heads(x.data_ptr(), w.data_ptr(), M, N, K, lda, ldb, int(b_mn), dst_ptrs, n_dst, batch,
                                 rows_per_batch, dst_rows, dst_heads, row_off, n_q, n_kv, q_l, kv_l, hd, n_rot,
-                                _ptr(cs), int(kv_rep), _stream()), "gemm_heads")
+                                _ptr(cs), int(kv_rep), _ptr(cos), _ptr(sin), _stream()), "gemm_heads")
 
 
 def swiglu_epilogue_ok(I: int) -> bool:
-    return I % 128 == 0
+    return I % 8 == 0
 
 
 def gemm_swiglu(x: torch.Tensor, w_gu: torch.Tensor):
