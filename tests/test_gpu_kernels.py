@@ -169,11 +169,38 @@ def test_gemm_heads_rope_epilogue(nat, gemm_mode, hd, Hq, Hkv, B, T, K):
     assert _rel_err(out[:, :, Hq + Hkv:], ref[:, :, Hq + Hkv:]) < 6e-3
 
 
+@pytest.mark.parametrize("bn,split", [(64, 1), (64, 2), (64, 4), (64, 8), (128, 1), (128, 2), (128, 4), (128, 8)])
+@pytest.mark.parametrize("M,N,K", [(8, 8, 512), (128, 64, 576), (129, 136, 1000), (333, 264, 4104)])
+def test_small_tile_gemm(nat, bn, split, M, N, K):
+    """128 x 64 / 128 x 128 tiles with the reduction shared by a cluster: every layout, ragged rows, columns and k-blocks
+    that do not divide by the cluster. The fp32 sums of S parts have no larger error than one sum over K."""
+    def run(a, b, c, lda, ldb, a_mn, b_mn, epi):
+        nat._check(nat.lib().tlm_gemm_split(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, lda, ldb, c.stride(0), a_mn, b_mn,
+                                            epi, bn, split, nat._stream()), "gemm_split")
+    x, w = _rand(M, K, seed=80), _rand(N, K, seed=81)
+    ref = x.double() @ w.double().t()
+    out = torch.full((M + 3, N + 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    run(x, w, out, K, K, 0, 0, nat.EPI_BF16)
+    assert ((out[:M, :N].double() - ref).norm() / ref.norm()).item() < 2.5e-3          # bf16 rounding: 2^-9 / sqrt(3) = 1.1e-3 rms
+    assert bool((out[M:] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
+    wt = w.t().contiguous()
+    out.fill_(7.0)
+    run(x, wt, out, K, N, 0, 1, nat.EPI_BF16)
+    assert ((out[:M, :N].double() - ref).norm() / ref.norm()).item() < 2.5e-3
+    if M % 8 == 0:
+        xt = x.t().contiguous()
+        acc = torch.full((M + 3, N), 2.0, device="cuda")
+        run(xt, wt, acc, M, N, 1, 1, nat.EPI_F32_ACC)
+        assert ((acc[:M].double() - 2.0 - ref).norm() / ref.norm()).item() < 2e-6      # fp32 accumulation over K <= 4104
+        assert bool((acc[M:] == 2.0).all())
+
+
 @pytest.mark.parametrize("mode", [0, 1, 2])
 @pytest.mark.parametrize("hd,Hq,Hkv,B,T,K", [(64, 4, 2, 3, 33, 192), (64, 12, 4, 3, 1001, 768), (32, 8, 2, 2, 37, 192), (128, 2, 1, 5, 7, 256),
                                               (64, 3, 1, 1, 1, 64), (128, 8, 4, 3, 335, 256), (32, 32, 4, 2, 777, 128)])
 def test_gemm_heads_any_number_of_rows(nat, mode, hd, Hq, Hkv, B, T, K):
-    """Batch entries whose row count is no multiple of 32 (a warp's rows cross entries)."""
+    """Batch entries whose row count is no multiple of 32 (a warp's rows cross entries), on the small tiles (mode 1) and on
+    the wide ones."""
     import ctypes
     from train_large_model_from_scratch_b200.ops import oracle
     Ht = Hq + 2 * Hkv

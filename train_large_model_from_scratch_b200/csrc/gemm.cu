@@ -22,6 +22,7 @@
 // Every mbarrier wait is bounded; on a timeout the CTA records a status code,
 // every role leaves its loop, and the CTA still frees its tensor memory.
 #include "common.cuh"
+#include "gemm_split.h"
 #include <cuda_fp16.h>
 
 namespace tlm {
@@ -1153,6 +1154,8 @@ static bool pair_enabled() {
   }
   return g_pair_mode != 0;
 }
+// gemm_split.cu's small tiles are considered in the default mode only, so that modes 0 and 2 name one kernel form each
+static bool small_tiles() { return pair_enabled() && g_pair_mode == 1; }
 static bool use_pair(int M) { return pair_enabled() && M >= 2 * BM && num_sms() >= 2; }
 // row-grouped GEMMs: a pair tile's second half is wasted at the end of every group, so pairs need large groups
 // (mode 2, set by tests: pairs for every row-grouped launch, so that small ragged groups exercise that path)
@@ -1177,6 +1180,13 @@ static int for_group_chunks(GemmParams p, int groups, const int* row_start, int 
     if (e) return e;
   }
   return 0;
+}
+// Estimated time (us) of a product on this file's tiles of `tile_n` output columns, for the choice against gemm_split.cu:
+// 5.4 us around the main loops (fp32 accumulation 7.2), 0.28 us per k-block of a tile, one wave of tiles after another.
+static double wide_cost(int M, int N, int tile_n, int K, bool pair, int splits = 0) {
+  const int tile_m = pair ? 2 * BM : BM, walkers = pair ? num_sms() / 2 : num_sms();
+  const long long items = (long long)((M + tile_m - 1) / tile_m) * ((N + tile_n - 1) / tile_n) * (splits > 0 ? splits : 1);
+  return (splits > 0 ? 7.2 : 5.4) + (double)((items + walkers - 1) / walkers) * ((K + BK - 1) / BK) * 0.28;
 }
 // Operand description: `ptr` points at element (0,0); K-major operands are
 // [rows, K] with leading dimension `ld`; MN-major operands are [K, rows] with
@@ -1316,7 +1326,7 @@ static int launch_heads_pair(const CUtensorMap& ma, const CUtensorMap& mb, const
 using namespace tlm;
 
 // CTA-pair GEMMs at run time (tests and A/B measurements): 0 off, 1 on, 2 on and also for row-grouped GEMMs with
-// small groups. Returns the previous setting.
+// small groups; 0 and 2 keep small products on the wide tiles. Returns the previous setting.
 TLM_API int tlm_gemm_set_pair(int mode) {
   pair_enabled();
   const int was = g_pair_mode;
@@ -1353,6 +1363,14 @@ TLM_API int tlm_gemm_heads(const void* A, const void* B, int M, int N, int K, lo
   GemmParams p{};
   if (!b_mn) take_pending_waits(p);               // x W^T: may be the first reader of its weights after an optimizer step
   const bool pair = use_pair(M) && p.wait_flags[0] == nullptr;
+  if (small_tiles() && p.wait_flags[0] == nullptr && n_dst == 1 && kv_rep == 1 && !b_mn && f32_tables) {
+    SplitGemm g{};
+    g.A = A; g.B = B; g.M = M; g.N = N; g.K = K; g.lda = lda; g.ldb = ldb; g.epi = SPLIT_HEADS; g.C = dst_ptrs[0];
+    g.ldc = hd; g.hd = hd; g.rows_per_batch = rows_per_batch; g.dst_rows = dst_rows; g.dst_heads = dst_heads;
+    g.row_off = row_off; g.n_rot = n_rot; g.cosT = cosT; g.sinT = sinT;
+    const SplitPlan plan = split_plan(g, wide_cost(M, N, BN, K, pair));
+    if (plan.bn) return split_run(g, plan, stream);
+  }
   Operand oa{A, M, K, lda, false, 0, 0}, ob{B, N, K, ldb, b_mn != 0, 1, (long long)N * K};
   CUtensorMap ma, mb;
   int e = build_map(&ma, oa, BM);
@@ -1398,6 +1416,13 @@ TLM_API int tlm_gemm_swiglu(const void* x, const void* w_gu, void* gate_up, void
   if (M <= 0 || I <= 0 || K <= 0) return 0;
   if (I % 8 != 0) return -4;
   const bool pair = use_pair(M);
+  if (small_tiles()) {
+    SplitGemm g{};
+    g.A = x; g.B = w_gu; g.M = M; g.N = I; g.K = K; g.lda = lda; g.ldb = ldb; g.epi = SPLIT_SWIGLU; g.C = gate_up;
+    g.ldc = 2LL * I; g.act = act;
+    const SplitPlan plan = split_plan(g, wide_cost(M, I, 128, K, pair));
+    if (plan.bn) return split_run(g, plan, stream);
+  }
   Operand oa{x, M, K, lda, false, 0, 0}, ob{w_gu, 2LL * I, K, ldb, false, 1, 2LL * I * K};
   CUtensorMap ma, mb, mc, md;
   int e = build_map(&ma, oa, BM);
@@ -1443,6 +1468,13 @@ TLM_API int tlm_gemm_swiglu_bwd(const void* dy, const void* w_down, const void* 
   if (M <= 0 || I <= 0 || D <= 0) return 0;
   if (I % 8 != 0) return -4;
   const bool pair = use_pair(M);
+  if (small_tiles()) {
+    SplitGemm g{};
+    g.A = dy; g.B = w_down; g.M = M; g.N = I; g.K = D; g.lda = lda; g.ldb = ldb; g.b_mn = true; g.epi = SPLIT_SWIGLU_BWD;
+    g.C = d_gate_up; g.ldc = 2LL * I; g.aux = gate_up;
+    const SplitPlan plan = split_plan(g, wide_cost(M, I, BN, D, pair));
+    if (plan.bn) return split_run(g, plan, stream);
+  }
   Operand oa{dy, M, D, lda, false, 0, 0}, ob{w_down, I, D, ldb, true, 1, (long long)I * D};
   CUtensorMap ma, mb, mc;
   int e = build_map(&ma, oa, BM);
@@ -1633,6 +1665,14 @@ TLM_API int tlm_gemm(const void* A, const void* B, void* C, int M, int N, int K,
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.status = status_word(); p.groups = 0;
   if (!a_mn && !b_mn && epi == EPI_BF16) take_pending_waits(p);     // x W^T: may be the first reader of its weights
   const bool pair = use_pair(M) && p.wait_flags[0] == nullptr;
+  SplitGemm g{};
+  g.A = A; g.B = B; g.M = M; g.N = N; g.K = K; g.lda = lda; g.ldb = ldb; g.a_mn = a_mn != 0; g.b_mn = b_mn != 0;
+  g.epi = epi; g.C = C; g.ldc = ldc;
+  const bool small_tiles_ok = small_tiles() && p.wait_flags[0] == nullptr && ((epi == EPI_BF16 && !a_mn) || (epi == EPI_F32_ACC && a_mn && b_mn));
+  if (small_tiles_ok && epi == EPI_BF16) {
+    const SplitPlan plan = split_plan(g, wide_cost(M, N, BN, K, pair));
+    if (plan.bn) return split_run(g, plan, stream);
+  }
   Operand oa{A, M, K, lda, a_mn != 0, 0, 0}, ob{B, N, K, ldb, b_mn != 0, 1, (long long)N * K};
   CUtensorMap ma, mb;
   int e = build_map(&ma, oa, BM);
@@ -1671,6 +1711,10 @@ TLM_API int tlm_gemm(const void* A, const void* B, void* C, int M, int N, int K,
       p.k_chunk = per * BK;
       p.split_k = (kblocks + per - 1) / per;
     }
+  }
+  if (small_tiles_ok && epi == EPI_F32_ACC) {
+    const SplitPlan plan = split_plan(g, wide_cost(M, N, BN, p.k_chunk, pair, p.split_k));
+    if (plan.bn) return split_run(g, plan, stream);
   }
   return dispatch(a_mn != 0, b_mn != 0, epi, ma, mb, p, tiles * p.split_k, stream, pair);
 }

@@ -1,0 +1,374 @@
+// Small bf16 GEMMs: C[M,N] (=|+=) A[M,K] * B[N,K]^T with few output tiles.
+//
+// gemm.cu's 128 x 256 (pairs: 256 x 256) tiles leave most SMs without work when M and N are small, and whoever has a
+// tile walks the whole reduction alone: the data gradient of a 50304-wide LM head over 512 tokens of width 256 was two
+// tiles of 786 k-blocks. Here a tile is 128 x 64 or 128 x 128 and a cluster of S = 1, 2, 4 or 8 CTAs shares its
+// reduction, each CTA an equal share of the k-blocks. Every CTA leaves its fp32 partial tile in its own shared memory,
+// and after a cluster barrier CTA r adds up rows [128 r / S, 128 (r + 1) / S) of all S partials (distributed shared
+// memory, fixed order, so the result does not depend on timing) and applies the epilogue. No workspace, no second
+// launch, no atomics.
+//
+// Roles as in gemm.cu: warp 0 TMA producer, warp 1 MMA issuer and tensor-memory owner, warps 2-5 move the accumulator
+// to shared memory; then all six warps reduce and store. Two CTAs fit an SM, so one's prologue and epilogue run beside
+// the other's main loop. Waits are bounded.
+#include "common.cuh"
+#include "gemm_split.h"
+
+namespace tlm {
+
+constexpr int SP_BM = 128, SP_BK = 64, SP_THREADS = 192;
+constexpr int SP_A_BYTES = SP_BM * SP_BK * 2;
+constexpr int SP_BOX_MN = 64 * SP_BK * 2;                 // one 64(mn) x 64(k) MN-major box
+
+template <int BN>
+struct SplitCfg {
+  static constexpr int STAGES = BN == 64 ? 4 : 3;         // 96 KB ring either way: two CTAs per SM (192 KB measured the same)
+  static constexpr int STAGE_BYTES = SP_A_BYTES + BN * SP_BK * 2;
+  static constexpr int PITCH = BN + 4;                    // floats per row of the partial tile (reuses the ring)
+  static constexpr int RING = STAGES * STAGE_BYTES;
+  static constexpr int SMEM = RING + 1024 /*align slack*/ + 256 /*barriers*/;
+  static_assert(SP_BM * PITCH * 4 <= RING, "the partial tile reuses the operand ring");
+};
+
+struct SplitParams {
+  SplitGemm g;
+  int tiles_m, tiles_n;
+  unsigned int* status;
+};
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+template <bool A_MN, bool B_MN, int EPI, int BN, int S>
+__global__ void __launch_bounds__(SP_THREADS, 2)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const SplitParams p) {
+  using C = SplitCfg<BN>;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* sal = smem_raw + (sbase - smem_u32(smem_raw));
+  // barriers: full[0..STAGES), empty[STAGES..2 STAGES), accumulator full
+  const uint32_t bar0 = sbase + C::RING;
+  auto full_bar = [&](int s) { return bar0 + 8u * s; };
+  auto empty_bar = [&](int s) { return bar0 + 8u * (C::STAGES + s); };
+  const uint32_t acc_bar = bar0 + 8u * (2 * C::STAGES);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sal + C::RING + 8 * (2 * C::STAGES + 1));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const SplitGemm& g = p.g;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = S > 1 ? (int)cluster_ctarank() : 0;
+  const int tile = (int)blockIdx.x / S;
+  const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
+  constexpr int TILE_N = EPI == SPLIT_SWIGLU ? BN / 2 : BN;       // output columns (SwiGLU: as many of gate and of up)
+  const int m0 = tm * SP_BM, n0 = tn * TILE_N;
+  const int kblocks = (g.K + SP_BK - 1) / SP_BK;
+  const int kb_lo = (int)((long long)kblocks * rank / S), kb_hi = (int)((long long)kblocks * (rank + 1) / S);
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2 * C::STAGES + 1; ++i) mbar_init(bar0 + 8u * i, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+  }
+  if (warp == 1) { tmem_alloc(smem_u32(tmem_slot), BN); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0; uint32_t phase = 0;
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait(empty_bar(stage), phase ^ 1u, 81, abort_flag, p.status)) break;
+        const int k0 = kb * SP_BK;
+        const uint32_t sa = sbase + stage * C::STAGE_BYTES, sb = sa + SP_A_BYTES, fb = full_bar(stage);
+        mbar_expect_tx(fb, C::STAGE_BYTES);
+        if (A_MN) {
+#pragma unroll
+          for (int j = 0; j < SP_BM / 64; ++j) tma_load_2d(sa + j * SP_BOX_MN, &tmA, fb, m0 + 64 * j, k0);
+        } else {
+          tma_load_2d(sa, &tmA, fb, k0, m0);
+        }
+        if (B_MN) {
+#pragma unroll
+          for (int j = 0; j < BN / 64; ++j) tma_load_2d(sb + j * SP_BOX_MN, &tmB, fb, n0 + 64 * j, k0);
+        } else if (EPI == SPLIT_SWIGLU) {         // gate rows, then the matching up rows
+          tma_load_2d(sb, &tmB, fb, k0, n0);
+          tma_load_2d(sb + BN * SP_BK, &tmB, fb, k0, g.N + n0);
+        } else {
+          tma_load_2d(sb, &tmB, fb, k0, n0);
+        }
+        if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = umma_idesc_bf16(SP_BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      int stage = 0; uint32_t phase = 0;
+      bool ok = true;
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait(full_bar(stage), phase, 82, abort_flag, p.status)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t sa = sbase + stage * C::STAGE_BYTES, sb = sa + SP_A_BYTES;
+        const uint64_t ad = A_MN ? umma_smem_desc(sa, SP_BOX_MN, 1024) : umma_smem_desc(sa, 16, 1024);
+        const uint64_t bd = B_MN ? umma_smem_desc(sb, SP_BOX_MN, 1024) : umma_smem_desc(sb, 16, 1024);
+        umma_bf16(tmem, ad, bd, idesc, kb > kb_lo);
+#pragma unroll
+        for (int kk = 1; kk < SP_BK / 16; ++kk)
+          umma_bf16_acc(tmem, umma_desc_advance(ad, kk * (A_MN ? 2048 : 32)), umma_desc_advance(bd, kk * (B_MN ? 2048 : 32)), idesc);
+        umma_commit(empty_bar(stage));
+        if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
+      }
+      if (ok) umma_commit(acc_bar);
+    }
+  } else {
+    // accumulator -> this CTA's partial tile in shared memory (every operand read of the ring has retired by then)
+    const int row = (warp & 3) * 32 + lane;
+    if (mbar_wait(acc_bar, 0, 83, abort_flag, p.status)) {
+      tc_fence_after();
+      const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+      float* dst = reinterpret_cast<float*>(sal) + row * C::PITCH;
+#pragma unroll
+      for (int c = 0; c < BN; c += 32) {
+        uint32_t r[32];
+        tmem_ld32(taddr + c, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(dst + c + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+      }
+    }
+    tc_fence_before();
+  }
+  __syncwarp();
+  if (S > 1) cluster_sync_all(); else __syncthreads();
+
+  // ---- sum of the S partial tiles, in place: this CTA's rows of its own partial are read by nobody else. Neighbouring lanes
+  // read neighbouring 16-byte pieces, which is what the shared-memory network between SMs wants (S = 8, 32-byte pieces read
+  // by the epilogue itself: 3 us more).
+  constexpr int ROWS = SP_BM / S;
+  if constexpr (S > 1) {
+    constexpr int P4 = BN / 4;
+    for (int i = threadIdx.x; i < ROWS * P4; i += SP_THREADS) {
+      const int r = rank * ROWS + i / P4, c = (i % P4) * 4;
+      if (m0 + r >= g.M) break;                              // rows ascend with i
+      const uint32_t off = sbase + (uint32_t)(r * C::PITCH + c) * 4u;
+      float4 a[S];
+#pragma unroll
+      for (int s = 0; s < S; ++s) a[s] = ld_cluster_f4(mapa_shared(off, (uint32_t)s));
+#pragma unroll
+      for (int s = 1; s < S; ++s) { a[0].x += a[s].x; a[0].y += a[s].y; a[0].z += a[s].z; a[0].w += a[s].w; }
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(sal) + r * C::PITCH + c) = a[0];
+    }
+    __syncthreads();
+  }
+
+  // ---- epilogue, 8 columns per item
+  constexpr bool PAIRED = EPI == SPLIT_HEADS || EPI == SPLIT_SWIGLU;      // items own 8 columns and their 8 partner columns
+  constexpr int PER_ROW = PAIRED ? BN / 16 : BN / 8;
+  auto load8 = [&](int r, int c, float* v) {
+    const float* src = reinterpret_cast<const float*>(sal) + r * C::PITCH + c;
+    *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(src);
+    *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(src + 4);
+  };
+  auto pack8 = [](const float* v) {
+    return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+  };
+  const int half = EPI == SPLIT_HEADS ? g.hd >> 1 : 0;
+  for (int i = threadIdx.x; i < ROWS * PER_ROW; i += SP_THREADS) {
+    const int r = rank * ROWS + i / PER_ROW, ch = i % PER_ROW;
+    const long long row = m0 + r;
+    if (row >= g.M) break;                                   // rows ascend with i
+    float v[8];
+    if constexpr (EPI == SPLIT_BF16 || EPI == SPLIT_F32_ACC) {
+      const int col = n0 + ch * 8;
+      if (col >= g.N) continue;
+      if constexpr (EPI == SPLIT_BF16) {
+        load8(r, ch * 8, v);
+        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.C) + row * g.ldc + col) = pack8(v);
+      } else {
+        float4* out = reinterpret_cast<float4*>(reinterpret_cast<float*>(g.C) + row * g.ldc + col);
+        float4 o0 = out[0], o1 = out[1];
+        load8(r, ch * 8, v);
+        o0.x += v[0]; o0.y += v[1]; o0.z += v[2]; o0.w += v[3]; o1.x += v[4]; o1.y += v[5]; o1.z += v[6]; o1.w += v[7];
+        out[0] = o0; out[1] = o1;
+      }
+    } else if constexpr (EPI == SPLIT_HEADS) {
+      const int per_half = half >> 3;                        // 8-column pieces of half a head
+      const int hh = ch / per_half, j = (ch - hh * per_half) * 8, c = hh * g.hd + j;
+      if (n0 + c >= g.N) continue;                           // N is a multiple of hd
+      const int head = n0 / g.hd + hh;
+      const int bi = (int)(row / g.rows_per_batch), t = (int)(row - (long long)bi * g.rows_per_batch);
+      const bool rot = head < g.n_rot;
+      float cl[8], sl[8], chh[8], sh[8], u[8];
+      if (rot) {
+        const float* cp = g.cosT + (long long)t * g.hd + j;
+        const float* sp = g.sinT + (long long)t * g.hd + j;
+#pragma unroll
+        for (int k = 0; k < 8; k += 4) {
+          *reinterpret_cast<float4*>(cl + k) = *reinterpret_cast<const float4*>(cp + k);
+          *reinterpret_cast<float4*>(sl + k) = *reinterpret_cast<const float4*>(sp + k);
+          *reinterpret_cast<float4*>(chh + k) = *reinterpret_cast<const float4*>(cp + half + k);
+          *reinterpret_cast<float4*>(sh + k) = *reinterpret_cast<const float4*>(sp + half + k);
+        }
+      }
+      load8(r, c, v);
+      load8(r, c + half, u);
+      if (rot) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float a = v[k], b = u[k];
+          v[k] = a * cl[k] - b * sl[k];
+          u[k] = b * chh[k] + a * sh[k];
+        }
+      }
+      __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(g.C) + (((long long)bi * g.dst_rows + g.row_off + t) * g.dst_heads + head) * g.hd + j;
+      *reinterpret_cast<uint4*>(out) = pack8(v);
+      *reinterpret_cast<uint4*>(out + half) = pack8(u);
+    } else if constexpr (EPI == SPLIT_SWIGLU) {
+      const int col = n0 + ch * 8;
+      if (col >= g.N) continue;
+      float u[8];
+      load8(r, ch * 8, v);
+      load8(r, BN / 2 + ch * 8, u);
+      // as in gemm.cu: the products are rounded to bf16 first, so the numbers equal those of separate kernels
+      const uint4 gp = pack8(v), up = pack8(u);
+      const uint32_t gw[4] = {gp.x, gp.y, gp.z, gp.w}, uw[4] = {up.x, up.y, up.z, up.w};
+      uint32_t o[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) o[k] = swiglu2(gw[k], uw[k]);
+      __nv_bfloat16* gu = reinterpret_cast<__nv_bfloat16*>(g.C) + row * g.ldc + col;
+      *reinterpret_cast<uint4*>(gu) = gp;
+      *reinterpret_cast<uint4*>(gu + g.N) = up;
+      *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.act) + row * g.N + col) = make_uint4(o[0], o[1], o[2], o[3]);
+    } else {
+      const int col = n0 + ch * 8;
+      if (col >= g.N) continue;
+      const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(g.aux) + row * 2 * g.N + col;
+      const uint4 gv = *reinterpret_cast<const uint4*>(gp), uv = *reinterpret_cast<const uint4*>(gp + g.N);
+      load8(r, ch * 8, v);
+      const uint4 dv = pack8(v);
+      const uint32_t dw[4] = {dv.x, dv.y, dv.z, dv.w}, gw[4] = {gv.x, gv.y, gv.z, gv.w}, uw[4] = {uv.x, uv.y, uv.z, uv.w};
+      uint32_t og[4], ou[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) swiglu_bwd2(dw[k], gw[k], uw[k], og[k], ou[k]);
+      __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(g.C) + row * g.ldc + col;
+      *reinterpret_cast<uint4*>(out) = make_uint4(og[0], og[1], og[2], og[3]);
+      *reinterpret_cast<uint4*>(out + g.N) = make_uint4(ou[0], ou[1], ou[2], ou[3]);
+    }
+  }
+
+  // no CTA leaves while another may still read its partial tile
+  __syncwarp();
+  if (S > 1) cluster_sync_all(); else __syncthreads();
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, BN); }
+}
+
+// ---- host side ----------------------------------------------------------------------------------
+template <bool A_MN, bool B_MN, int EPI, int BN, int S>
+static int launch_split(const CUtensorMap& ma, const CUtensorMap& mb, const SplitParams& p, cudaStream_t st) {
+  auto kern = gemm_split_kernel<A_MN, B_MN, EPI, BN, S>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg<BN>::SMEM);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(p.tiles_m * p.tiles_n * S));
+  cfg.blockDim = dim3(SP_THREADS);
+  cfg.dynamicSmemBytes = SplitCfg<BN>::SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = S; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = S > 1 ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ma, mb, p);
+  count_launch();
+  return e != cudaSuccess ? (int)e : launch_status();
+}
+
+static int split_map(CUtensorMap* m, const void* ptr, long long rows, long long k, long long ld, bool mn, int box_rows) {
+  uint64_t dims[2] = {(uint64_t)(mn ? rows : k), (uint64_t)(mn ? k : rows)}, strides[1] = {(uint64_t)ld * 2};
+  uint32_t box[2] = {64, (uint32_t)(mn ? SP_BK : box_rows)};
+  return make_tmap_bf16(m, ptr, 2, dims, strides, box);
+}
+
+int split_run(const SplitGemm& g, const SplitPlan& plan, cudaStream_t st) {
+  const int bn = plan.bn, tile_n = g.epi == SPLIT_SWIGLU ? bn / 2 : bn;
+  const int kblocks = (g.K + SP_BK - 1) / SP_BK;
+  if ((bn != 64 && bn != 128) || plan.split < 1 || plan.split > kblocks) return -4;
+  if (g.N % 8 != 0 || g.ldc % 8 != 0 || (reinterpret_cast<uintptr_t>(g.C) & 15)) return -4;
+  if (g.epi == SPLIT_HEADS && (g.hd > bn || bn % g.hd != 0 || g.hd % 16 != 0)) return -4;
+  CUtensorMap ma, mb;
+  int e = split_map(&ma, g.A, g.M, g.K, g.lda, g.a_mn, SP_BM);
+  if (e) return e;
+  e = split_map(&mb, g.B, g.epi == SPLIT_SWIGLU ? 2LL * g.N : g.N, g.K, g.ldb, g.b_mn, tile_n);
+  if (e) return e;
+  SplitParams p{g, (g.M + SP_BM - 1) / SP_BM, (g.N + tile_n - 1) / tile_n, status_word()};
+#define TLM_SPLIT_S(A, B, E, BN)                                   \
+  switch (plan.split) {                                            \
+    case 1: return launch_split<A, B, E, BN, 1>(ma, mb, p, st);    \
+    case 2: return launch_split<A, B, E, BN, 2>(ma, mb, p, st);    \
+    case 4: return launch_split<A, B, E, BN, 4>(ma, mb, p, st);    \
+    case 8: return launch_split<A, B, E, BN, 8>(ma, mb, p, st);    \
+    default: return -4;                                            \
+  }
+#define TLM_SPLIT(A, B, E)                                                                             \
+  if (g.a_mn == A && g.b_mn == B && g.epi == E) {                                                      \
+    if (bn == 64) TLM_SPLIT_S(A, B, E, 64) else TLM_SPLIT_S(A, B, E, 128)                              \
+  }
+  TLM_SPLIT(false, false, SPLIT_BF16) TLM_SPLIT(false, true, SPLIT_BF16) TLM_SPLIT(true, true, SPLIT_F32_ACC)
+  TLM_SPLIT(false, false, SPLIT_HEADS) TLM_SPLIT(false, false, SPLIT_SWIGLU) TLM_SPLIT(false, true, SPLIT_SWIGLU_BWD)
+#undef TLM_SPLIT
+#undef TLM_SPLIT_S
+  return -2;
+}
+
+// Estimated time in us, fitted to 30 shapes (M 16 - 4096, N 256 - 3072, K 256 - 50304, operands in L2): a k-block takes
+// 0.24 us (64 columns) or 0.27 us (128 columns) of a CTA, what 24 / 32 KB take at the 64 B per clock that an SM gets out of
+// L2, and no less than all CTAs' blocks take at 14 TB/s out of the whole L2; plus what surrounds the main loop and the
+// exchange of the partial tiles. A weight gradient has to win clearly: its C is read by the SMs here, while the wide tiles
+// leave through TMA reduce-add, which matters once C comes from HBM.
+SplitPlan split_plan(const SplitGemm& g, double wide_us) {
+  SplitPlan best{0, 0};
+  if (g.N % 8 != 0 || g.ldc % 8 != 0 || (reinterpret_cast<uintptr_t>(g.C) & 15)) return best;
+  const long long kblocks = (g.K + SP_BK - 1) / SP_BK, slots = 2LL * num_sms();
+  static const double exchange[2][4] = {{0.0, 1.5, 1.3, 2.8}, {0.0, 2.2, 2.0, 2.3}};       // S = 1, 2, 4, 8
+  double best_us = g.epi == SPLIT_F32_ACC ? 0.85 * wide_us : wide_us;
+  for (int bn = 64; bn <= 128; bn *= 2) {
+    if (g.epi == SPLIT_HEADS && (g.hd > bn || bn % g.hd != 0)) continue;
+    const int tile_n = g.epi == SPLIT_SWIGLU ? bn / 2 : bn;
+    const long long tiles = (long long)((g.M + SP_BM - 1) / SP_BM) * ((g.N + tile_n - 1) / tile_n);
+    for (int i = 0, s = 1; s <= 8 && s <= kblocks; ++i, s *= 2) {
+      const long long ctas = tiles * s, resident = ctas < slots ? ctas : slots;
+      if (ctas > (s > 1 ? num_sms() : slots)) continue;          // a second wave of clusters costs more than it saves
+      const double alone = bn == 64 ? 0.24 : 0.27, shared = (double)resident * (bn == 64 ? 24576.0 : 32768.0) / 14e6;
+      const double us = (bn == 64 ? 3.4 : 3.8) + (g.a_mn ? 1.0 : 0.0) + exchange[bn / 128][i] +
+                        (double)((kblocks + s - 1) / s) * (alone > shared ? alone : shared);
+      if (us < best_us) { best_us = us; best = {bn, s}; }
+    }
+  }
+  return best;
+}
+
+}  // namespace tlm
+
+using namespace tlm;
+
+// tlm_gemm (same arguments) with the tile width and the split given: for tests and measurements.
+TLM_API int tlm_gemm_split(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                           long long ldc, int a_mn, int b_mn, int epi, int bn, int split, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (epi != SPLIT_BF16 && epi != SPLIT_F32_ACC) return -2;
+  SplitGemm g{};
+  g.A = A; g.B = B; g.M = M; g.N = N; g.K = K; g.lda = lda; g.ldb = ldb; g.a_mn = a_mn != 0; g.b_mn = b_mn != 0;
+  g.epi = epi; g.C = C; g.ldc = ldc;
+  return split_run(g, SplitPlan{bn, split}, stream);
+}

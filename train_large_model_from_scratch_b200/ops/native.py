@@ -55,6 +55,7 @@ _SIGS = {
     "tlm_get_deterministic": (_I, []),
     "tlm_gemm_set_pair": (_I, [_I]),
     "tlm_gemm": (_I, [_P, _P, _P, _I, _I, _I, _LL, _LL, _LL, _I, _I, _I, _P]),
+    "tlm_gemm_split": (_I, [_P, _P, _P, _I, _I, _I, _LL, _LL, _LL, _I, _I, _I, _I, _I, _P]),
     "tlm_gemm_heads": (_I, [_P, _P, _I, _I, _I, _LL, _LL, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P, _P, _P]),
     "tlm_gemm_swiglu": (_I, [_P, _P, _P, _P, _I, _I, _I, _LL, _LL, _P]),
     "tlm_gemm_swiglu_bwd": (_I, [_P, _P, _P, _P, _I, _I, _I, _LL, _LL, _P]),
@@ -155,7 +156,8 @@ def set_deterministic(on: bool) -> None:
 def set_gemm_pairs(mode) -> int:
     """Plain GEMMs of at least 256 rows, and row-grouped GEMMs with large groups, run as CTA pairs (`cta_group::2`, one
     256 x 256 tile per two SMs). `mode`: 0 / False off (also `TLM_GEMM_PAIR=0`), 1 / True on (the default), 2 on and
-    also for row-grouped GEMMs with small groups. Returns the previous mode. For tests and A/B measurements."""
+    also for row-grouped GEMMs with small groups. Modes 0 and 2 also keep products with few output tiles on the wide tiles
+    instead of `csrc/gemm_split.cu`. Returns the previous mode. For tests and A/B measurements."""
     return int(lib().tlm_gemm_set_pair(int(mode)))
 
 
@@ -284,7 +286,7 @@ def gemm_heads(x: torch.Tensor, w: torch.Tensor, b_mn: bool, dst_ptrs, n_dst: in
     `dst_ptrs` is a ctypes array of `n_dst` device addresses (this rank's own tensor or peers' buffers).
     `kv_rep > 1` (fewer KV heads than destinations): k / v head j goes to the `kv_rep` destinations
     `j * kv_rep .. j * kv_rep + kv_rep - 1`, slots `q_l` and `q_l + 1`. `tables` (optional): the fp32 `(cos, sin)`
-    `[rows_per_batch, hd]` that `cs` was made from; batch entries whose row
+    `[rows_per_batch, hd]` that `cs` was made from; products too small for the wide tiles and batch entries whose row
     count is no multiple of 32 rotate with them."""
     M, K, lda = _rows(x)
     cos, sin = tables if tables is not None else (None, None)
