@@ -120,3 +120,30 @@ def test_results_do_not_depend_on_the_block_order(group, monkeypatch):
     assert rel < 5e-3, rel                                                 # dQ: fp32 adds from several blocks, any order
     ref = _ref(qkv, Hq, Hkv)
     assert (o1.float() - ref).abs().max().item() < 2e-2
+
+
+@pytest.mark.parametrize("hd", [32, 128])
+@pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 1, 1, 1), (2, 127, 2, 1), (1, 129, 4, 4), (2, 513, 6, 2), (1, 1025, 8, 1)])
+def test_narrow_and_wide_heads_at_the_edges_of_tiles(hd, B, T, Hq, Hkv):
+    """Head dim 32 (its own 64-byte-swizzled tiles) and 128 (dQ takes turns with dP in tensor memory, two Q tiles and one dO
+    tile in shared memory): one step, first and last steps, several query heads per KV head. P and dS are rounded to bf16
+    (2^-9) before their products and the results once more, so 1e-2 bounds the relative error of every part."""
+    from train_large_model_from_scratch_b200.ops import native
+    g = torch.Generator(device="cuda").manual_seed(7)
+    qkv = torch.randn(B, T, Hq + 2 * Hkv, hd, device="cuda", generator=g).to(torch.bfloat16)
+    do = torch.randn(B, T, Hq, hd, device="cuda", generator=g).to(torch.bfloat16)
+    o, lse = native.flash_attn_fwd(qkv, Hq, Hkv, True)
+    dqkv = native.flash_attn_bwd(do, qkv, o, lse, Hq, Hkv, True)
+    native.raise_on_device_status()
+    x = qkv.double().requires_grad_()
+    q = x[:, :, :Hq].permute(0, 2, 1, 3)
+    k, v = (x[:, :, a:a + Hkv].permute(0, 2, 1, 3).repeat_interleave(Hq // Hkv, 1) for a in (Hq, Hq + Hkv))
+    s = (q @ k.transpose(-1, -2) / math.sqrt(hd)).masked_fill(torch.ones(T, T, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    ref = (torch.softmax(s, -1) @ v).permute(0, 2, 1, 3)
+    ref.backward(do.double())
+    assert ((o.double() - ref).norm() / ref.norm()).item() < 1e-2
+    for name, sl in (("dq", slice(0, Hq)), ("dk", slice(Hq, Hq + Hkv)), ("dv", slice(Hq + Hkv, None))):
+        a, b = dqkv[:, :, sl].double(), x.grad[:, :, sl]
+        # a single position attends to itself alone: dS is exactly zero up to rounding of dP - delta
+        bound = 1e-2 * b.norm().item() if T > 1 or name == "dv" else 1e-2 * do.double().norm().item()
+        assert (a - b).norm().item() < bound, (name, (a - b).norm().item(), b.norm().item())

@@ -39,16 +39,13 @@ struct AttnFwdParams {
   // peer-mapped addresses, plain 16-byte stores). n_dst == 0 disables it.
   __nv_bfloat16* o_dst[AT_MAX_DST];
   int n_dst, dst_rows, dst_heads, dst_head0;
-  // Head dim of the tensors in memory. It equals the kernel's HD except for hd = 32, which runs on the
-  // HD = 64 kernel: the TMA boxes stay 64 wide and the 32 columns past the end of a head are
-  // out-of-bounds zero fill, so Q K^T is unchanged and the upper half of O is never stored.
-  int hd;
+  int hd;                  // head dim of the tensors in memory (= the kernel's HD)
   int head_group;          // heads per group of the heavy-first block order (see heavy_first_decode)
 };
 
 template <int HD>
 struct AttnFwdSmem {
-  static constexpr int KB = HD / 64;                   // 64-wide blocks along hd
+  static constexpr int KB = HD == 128 ? 2 : 1;         // blocks along hd (64 wide; HD 32: one of 32)
   static constexpr int Q_BYTES = AT_BQ * HD * 2;
   static constexpr int KV_BYTES = AT_BKV * HD * 2;
   static constexpr int OFF_Q = 0;
@@ -66,7 +63,7 @@ struct AttnFwdSmem {
 constexpr float RESCALE_LOG2 = 8.0f;
 
 template <int HD>
-__global__ void __launch_bounds__(AT_THREADS, HD == 64 ? 2 : 1)
+__global__ void __launch_bounds__(AT_THREADS, HD <= 64 ? 2 : 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const AttnFwdParams p) {
   using L = AttnFwdSmem<HD>;
   constexpr int KB = L::KB;
@@ -142,12 +139,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const AttnFwdParams 
       constexpr uint32_t idesc_o = umma_idesc_bf16(AT_BQ, HD, 0, 1);
       // descriptors are built once per tile and advanced with one add per MMA: this thread's instruction
       // stream is what feeds the tensor pipe
-      const uint64_t dq = umma_smem_desc(sbase + L::OFF_Q, 16, 1024);
+      const uint64_t dq = attn_desc_k<HD>(sbase + L::OFF_Q);
       auto issue_s = [&](int j) -> bool {
         const int st = j & 1;
         if (!mbar_wait(bar(1 + st), (uint32_t)(j >> 1) & 1u, 13, abort_flag, p.status)) return false;
         tc_fence_after();
-        const uint64_t dk = umma_smem_desc(sbase + L::OFF_K + st * L::KV_BYTES, 16, 1024);
+        const uint64_t dk = attn_desc_k<HD>(sbase + L::OFF_K + st * L::KV_BYTES);
         umma_bf16(tmem + S_COL, dq, dk, idesc_s, 0);
 #pragma unroll
         for (int t = 1; t < HD / 16; ++t) {
@@ -170,10 +167,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const AttnFwdParams 
         if (!mbar_wait(bar(8), par, 14, abort_flag, p.status)) break;                        // P written
         if (!mbar_wait(bar(3 + st), (uint32_t)(j >> 1) & 1u, 15, abort_flag, p.status)) break;   // V landed
         tc_fence_after();
-        const uint64_t dv = umma_smem_desc(sbase + L::OFF_V + st * L::KV_BYTES, 16384, 1024);   // MN-major: 16 kv rows per step
+        const uint64_t dv = attn_desc_mn<HD>(sbase + L::OFF_V + st * L::KV_BYTES);   // MN-major: 16 kv rows per step
 #pragma unroll
         for (int t = 0; t < AT_BKV / 16; ++t)                   // 16 kv = 8 columns of packed pairs per step
-          umma_bf16_ts(tmem + O_COL, tmem + P_COL + t * 8, umma_desc_advance(dv, t * 2048), idesc_o, (j > 0) | (t > 0));
+          umma_bf16_ts(tmem + O_COL, tmem + P_COL + t * 8, umma_desc_advance(dv, t * attn_mn_step<HD>()), idesc_o, (j > 0) | (t > 0));
         umma_commit(bar(9));                                    // O updated, P free
         umma_commit(bar(5 + st));                               // V stage free
       }
@@ -294,12 +291,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const AttnFwdParams 
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, TMEM_COLS); }
 }
 
-// 4-D map over the packed tensor: dims (hd, heads, T, B); box (64, 1, rows, 1). For hd = 32 the box is wider
-// than the tensor's inner extent; the excess columns are zero fill.
-int make_qkv_map(CUtensorMap* map, const void* base, int B, int T, int heads, int hd, int box_rows) {
+// 4-D map over the packed tensor: dims (hd, heads, T, B); box (cols, 1, rows, 1). A box wider than hd = 32 is
+// filled with zeros (loads) or clipped (stores) there.
+int make_qkv_map(CUtensorMap* map, const void* base, int B, int T, int heads, int hd, int box_rows, int box_cols) {
   uint64_t dims[4] = {(uint64_t)hd, (uint64_t)heads, (uint64_t)T, (uint64_t)B};
   uint64_t strides[3] = {(uint64_t)hd * 2, (uint64_t)heads * hd * 2, (uint64_t)T * heads * hd * 2};
-  uint32_t box[4] = {64, 1, (uint32_t)box_rows, 1};
+  uint32_t box[4] = {(uint32_t)box_cols, 1, (uint32_t)box_rows, 1};
   return make_tmap_bf16(map, base, 4, dims, strides, box);
 }
 
@@ -328,7 +325,7 @@ static int attn_fwd_impl(const void* qkv, void* o, float* lse, int B, int T, int
   if (Hq % Hkv != 0) return -5;
   if (n_dst < 0 || n_dst > AT_MAX_DST || (n_dst > 0 && (dst_rows <= 0 || (long long)dst_rows * n_dst < T))) return -6;
   CUtensorMap map;
-  int e = make_qkv_map(&map, qkv, B, T, Hq + 2 * Hkv, hd, AT_BQ);
+  int e = make_qkv_map(&map, qkv, B, T, Hq + 2 * Hkv, hd, AT_BQ, hd == 32 ? 32 : 64);
   if (e) return e;
   AttnFwdParams p{};
   p.o = (__nv_bfloat16*)o; p.lse = lse; p.B = B; p.T = T; p.Hq = Hq; p.Hkv = Hkv;
@@ -338,7 +335,7 @@ static int attn_fwd_impl(const void* qkv, void* o, float* lse, int B, int T, int
   // a head's Q, K, V and O rows; in-step timing at B 8, T 4096, 16 heads of 64: groups of 16 - 32 heads are best
   // (0.45 ms against 0.49 ms with each head's tiles adjacent), all 128 heads at once lose that again to L2 misses
   p.head_group = attn_head_group("TLM_ATTN_FWD_GROUP", 8LL * T * hd, 48LL << 20, B * Hq);
-  return hd == 128 ? launch_fwd<128>(map, p, st) : launch_fwd<64>(map, p, st);
+  return hd == 128 ? launch_fwd<128>(map, p, st) : hd == 64 ? launch_fwd<64>(map, p, st) : launch_fwd<32>(map, p, st);
 }
 
 TLM_API int tlm_attn_fwd(const void* qkv, void* o, float* lse, int B, int T, int Hq, int Hkv, int hd, float scale,

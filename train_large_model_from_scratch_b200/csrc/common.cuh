@@ -323,6 +323,29 @@ __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t smem_addr, uint32_t 
   d |= (uint64_t)2 << 61;        // SWIZZLE_128B
   return d;
 }
+// Tiles of 32 bf16 columns, 64-byte swizzle: rows of 64 B, 8-row (K-major) or 8-k (MN-major) groups 512 B apart. One tile
+// is 32 wide in its contiguous direction, so there is no second stride.
+__device__ __forceinline__ uint64_t umma_smem_desc_sw64(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(512 >> 4) << 32;
+  d |= (uint64_t)1 << 46;        // descriptor version (Blackwell)
+  d |= (uint64_t)4 << 61;        // SWIZZLE_64B
+  return d;
+}
+// Operand tiles of the attention kernels: [128 rows][HD columns], HD 32 in one 64-byte-swizzled block, HD 64 / 128 in 64-wide
+// 128-byte-swizzled blocks 16 KB apart. K-major view (reduction over the columns) and MN-major view (reduction over the rows).
+template <int HD>
+__device__ __forceinline__ uint64_t attn_desc_k(uint32_t addr) {
+  return HD == 32 ? umma_smem_desc_sw64(addr) : umma_smem_desc(addr, 16, 1024);
+}
+template <int HD>
+__device__ __forceinline__ uint64_t attn_desc_mn(uint32_t addr) {
+  return HD == 32 ? umma_smem_desc_sw64(addr) : umma_smem_desc(addr, 16384, 1024);
+}
+template <int HD>
+constexpr uint32_t attn_mn_step() { return HD == 32 ? 1024 : 2048; }      // bytes of 16 rows of such a block
 // Descriptor of the same tile `byte_off` bytes further on. The start-address field holds (addr >> 4) in its
 // low 14 bits and shared-memory addresses stay below 2^18, so the field cannot carry into its neighbours and
 // the whole update is one add. The thread that issues the MMAs is a serial bottleneck (one instruction
@@ -433,8 +456,8 @@ int num_sms();
 // (read on every call: a handful of launches per step); clamped to [1, n_heads].
 int attn_head_group(const char* env, long long bytes_per_head, long long budget_bytes, int n_heads);
 
-// 4-D bf16 map over a packed [B, T, heads, hd] tensor: dims (hd, heads, T, B), box (64, 1, box_rows, 1).
-int make_qkv_map(CUtensorMap* map, const void* base, int B, int T, int heads, int hd, int box_rows);
+// 4-D bf16 map over a packed [B, T, heads, hd] tensor: dims (hd, heads, T, B), box (box_cols, 1, box_rows, 1).
+int make_qkv_map(CUtensorMap* map, const void* base, int B, int T, int heads, int hd, int box_rows, int box_cols = 64);
 
 // Packed fp32 pairs (sm_100: one issue slot for two lanes of fma / add / mul). The softmax warps of the attention
 // kernels are bound by instruction issue, so their scale-and-shift, row-sum and dS arithmetic runs on pairs.

@@ -98,8 +98,11 @@ static int make_tmap(CUtensorMap* map, CUtensorMapDataType dtype, const void* ba
     estr[i] = 1;
     if (i + 1 < rank) gstr[i] = strides_bytes[i];
   }
+  // boxes of 64-byte rows (32 bf16 columns) take the 64-byte swizzle, wider ones the 128-byte swizzle
+  const bool half_rows = dtype == CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 && box[0] == 32;
+  const CUtensorMapSwizzle swizzle = half_rows ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
   CUresult r = enc(map, dtype, (cuuint32_t)rank, const_cast<void*>(base), gdim, gstr, bdim,
-                   estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     fprintf(stderr, "tlm: cuTensorMapEncodeTiled failed (%d): rank %d base %p dims", (int)r, rank, base);

@@ -1,6 +1,5 @@
 """CUDA attention entry points used by `ops.native`: the tcgen05 flash-attention
-kernels for head dims 32, 64 and 128 (32 runs on the 64-wide kernel with
-zero-filled upper columns).
+kernels for head dims 32, 64 and 128.
 
 Other head dims (and non-causal calls) go to the library SDPA kernels through
 ATen (a library call, like a cuBLAS GEMM).
