@@ -41,6 +41,30 @@ def test_dense_model_matches_cpu_oracle(heads):
         assert c > 0.98, (name, c)
 
 
+@pytest.mark.parametrize("T,over", [(33, {}), (257, dict(num_attention_heads=8)), (1, {}), (160, dict(num_attention_heads=2, num_key_value_heads=1)),
+                                    (300, dict(intermediate_size=520, num_layer=3)), (512, dict(num_layer=1))])
+def test_blocks_issued_in_one_call_equal_the_per_op_path(T, over):
+    """Without gradients the blocks run as one native call with the same kernels: bit-identical logits and loss. A forward hook
+    on a sub-module (which the one call could not run) selects the per-op path and still fires."""
+    from train_large_model_from_scratch_b200.ops import native
+    model = _build("cuda", torch.bfloat16, **over).eval()
+    data = torch.randint(0, 4096, (3, T + 1), generator=torch.Generator().manual_seed(3)).cuda()
+    x, y = data[:, :-1].contiguous(), data[:, 1:].contiguous()
+    with torch.no_grad():
+        assert model._one_call_ok(model.wte(x), T)
+        logits, _, _ = model(x)
+        _, loss, _ = model(x, y)
+        seen = []
+        handle = model.blocks[0].mlp.register_forward_hook(lambda *a: seen.append(1))
+        logits_ref, _, _ = model(x)
+        _, loss_ref, _ = model(x, y)
+        handle.remove()
+    native.raise_on_device_status()
+    assert len(seen) == 2 and torch.equal(logits, logits_ref) and abs(loss.item() - loss_ref.item()) < 1e-5
+    logits_grad, _, _ = model(x)                                           # gradients on: per-op path, same values
+    assert logits_grad.requires_grad and torch.equal(logits, logits_grad.detach())
+
+
 def test_training_reduces_loss_on_fixed_batch():
     from train_large_model_from_scratch_b200.parallel.zero1.distributed_optimizer import FusedAdamW
     model = _build("cuda", torch.bfloat16)

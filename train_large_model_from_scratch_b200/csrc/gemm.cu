@@ -777,8 +777,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
               }
             }
             const int col = t.n0 + h * 64;
-            put(pg, &tmC, col, 0, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc);
-            put(pu, &tmC, col, 1, reinterpret_cast<__nv_bfloat16*>(p.C) + p.N, p.ldc);
+            if (p.C != nullptr) {                            // kept for the backward only
+              put(pg, &tmC, col, 0, reinterpret_cast<__nv_bfloat16*>(p.C), p.ldc);
+              put(pu, &tmC, col, 1, reinterpret_cast<__nv_bfloat16*>(p.C) + p.N, p.ldc);
+            }
             put(pa, dst_maps, col, 0, p.act, p.ld_act);
           }
         } else {
@@ -1409,7 +1411,8 @@ static int store_map_bf16(CUtensorMap* m, void* base, long long rows, long long 
 }
 
 // gate_up[M, 2 I] = x[M, K] * w_gu[2 I, K]^T  and  act[M, I] = silu(gate) * up, in one kernel.
-// Requirements: I % 8 == 0, contiguous outputs (row pitches 2 I and I). In the last tile of a width that is no multiple of
+// Requirements: I % 8 == 0, contiguous outputs (row pitches 2 I and I). gate_up may be null (forward without gradients:
+// evaluation at 32768 x 4096, K 1024 then stores a third as much). In the last tile of a width that is no multiple of
 // 128 the gate rows of B run on into the up rows; those columns are clipped by the stores.
 TLM_API int tlm_gemm_swiglu(const void* x, const void* w_gu, void* gate_up, void* act, int M, int I, int K,
                             long long lda, long long ldb, cudaStream_t stream) {
@@ -1429,9 +1432,10 @@ TLM_API int tlm_gemm_swiglu(const void* x, const void* w_gu, void* gate_up, void
   if (e) return e;
   e = build_map(&mb, ob, 128);
   if (e) return e;
-  e = store_map_bf16(&mc, gate_up, M, 2, I);
-  if (e) return e;
   e = store_map_bf16(&md, act, M, 1, I);
+  if (e) return e;
+  mc = md;                                        // unused without gate_up
+  if (gate_up != nullptr) e = store_map_bf16(&mc, gate_up, M, 2, I);
   if (e) return e;
   GemmParams p{};
   p.M = M; p.N = I; p.K = K; p.C = gate_up; p.ldc = 2LL * I; p.status = status_word(); p.split_k = 1; p.k_chunk = K;

@@ -242,9 +242,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       uint32_t o[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) o[k] = swiglu2(gw[k], uw[k]);
-      __nv_bfloat16* gu = reinterpret_cast<__nv_bfloat16*>(g.C) + row * g.ldc + col;
-      *reinterpret_cast<uint4*>(gu) = gp;
-      *reinterpret_cast<uint4*>(gu + g.N) = up;
+      if (g.C != nullptr) {
+        __nv_bfloat16* gu = reinterpret_cast<__nv_bfloat16*>(g.C) + row * g.ldc + col;
+        *reinterpret_cast<uint4*>(gu) = gp;
+        *reinterpret_cast<uint4*>(gu + g.N) = up;
+      }
       *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.act) + row * g.N + col) = make_uint4(o[0], o[1], o[2], o[3]);
     } else {
       const int col = n0 + ch * 8;

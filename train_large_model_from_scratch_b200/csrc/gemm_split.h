@@ -14,7 +14,7 @@ struct SplitGemm {
   long long lda, ldb;
   bool a_mn, b_mn;
   int epi;
-  void* C;                       // bf16 or fp32 result (pitch ldc); SwiGLU: gate|up / d(gate)|d(up), pitch ldc = 2 N
+  void* C;                       // bf16 or fp32 result (pitch ldc); SwiGLU: gate|up (or null) / d(gate)|d(up), pitch ldc = 2 N
   long long ldc;
   void* act;                     // SPLIT_SWIGLU: silu(gate) * up, [M, N]
   const void* aux;               // SPLIT_SWIGLU_BWD: gate|up, [M, 2 N]

@@ -164,7 +164,11 @@ class GPT(nn.Module):
         x = self.wte(idx)
         delta = None
         aux_total = None
-        for i, block in enumerate(self.blocks):
+        blocks = self.blocks
+        if not torch.is_grad_enabled() and self._one_call_ok(x, T):
+            x, delta = self._blocks_forward(x, B, T)
+            blocks = ()
+        for i, block in enumerate(blocks):
             g = self._group_of_block.get(i) if hooks is not None else None
             if g is not None:
                 hooks.before_group(g)                   # the group's first GEMM waits for the group's parameters
@@ -189,6 +193,39 @@ class GPT(nn.Module):
         if aux_total is not None:
             loss = loss + aux_total * (loss_scale / sp)
         return logits, loss, logging_loss
+
+    def _one_call_ok(self, x: torch.Tensor, T: int) -> bool:
+        """Whether the blocks' forward can be issued as one native call: no gradients, one GPU, dense bf16 blocks as this
+        class built them (fused weights, no replaced or hooked sub-module). Everything else takes the per-op path."""
+        from torch.nn.modules import module as nn_module
+        if (not x.is_cuda or x.dtype != torch.float32 or self.use_moe or self.comm_hooks is not None or len(self.blocks) == 0
+                or parallel_state.get_sep_world_size() > 1
+                or nn_module._global_forward_hooks or nn_module._global_forward_pre_hooks):
+            return False
+        first = self.blocks[0]
+        for block in self.blocks:
+            if type(block) is not Block or type(block.attn) is not Attention or type(block.mlp) is not MLP:
+                return False
+            attn, mlp = block.attn, block.mlp
+            if (attn.training and attn.dropout > 0.0) or not F_ops.swiglu_mlp_fused_ok(attn.q_proj.weight, mlp._gate_up_weight) \
+                    or not F_ops.qkv_project_fused_ok(attn.q_proj.weight, attn._qkv_weight, attn.head_dim, T):
+                return False
+            for m in (block, attn, mlp, block.ln_1, block.ln_2):
+                if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
+                    return False
+            for n in (block.ln_1, block.ln_2):
+                if type(n) is not LayerNorm or n.weight.dtype != torch.bfloat16 or n.variance_epsilon != first.ln_1.variance_epsilon:
+                    return False
+        return True
+
+    def _blocks_forward(self, x: torch.Tensor, B: int, T: int):
+        from ..ops import native
+        attn = self.blocks[0].attn
+        weights = [(b.ln_1.weight, b.attn._qkv_weight, b.attn.c_proj.weight, b.ln_2.weight, b.mlp._gate_up_weight, b.mlp.down_proj.weight)
+                   for b in self.blocks]
+        cos, sin = attn._rope(T, x.device)
+        return native.blocks_forward(x, weights, B, T, attn.num_attention_heads, attn.num_key_value_heads, attn.head_dim,
+                                     self.blocks[0].ln_1.variance_epsilon, attn._rope_fp16(T, x.device), cos, sin)
 
     # ------------------------------------------------------------------ bookkeeping
     def zero_grad_buffers(self) -> None:

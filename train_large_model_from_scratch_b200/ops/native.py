@@ -57,6 +57,7 @@ _SIGS = {
     "tlm_gemm": (_I, [_P, _P, _P, _I, _I, _I, _LL, _LL, _LL, _I, _I, _I, _P]),
     "tlm_gemm_split": (_I, [_P, _P, _P, _I, _I, _I, _LL, _LL, _LL, _I, _I, _I, _I, _I, _P]),
     "tlm_gemm_heads": (_I, [_P, _P, _I, _I, _I, _LL, _LL, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P, _P, _P]),
+    "tlm_blocks_forward": (_I, [_P, _I] + [_P] * 10 + [_I] * 7 + [_F, _F] + [_P] * 4),
     "tlm_gemm_swiglu": (_I, [_P, _P, _P, _P, _I, _I, _I, _LL, _LL, _P]),
     "tlm_gemm_swiglu_bwd": (_I, [_P, _P, _P, _P, _I, _I, _I, _LL, _LL, _P]),
     "tlm_gemm_swiglu_grouped": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _I, _LL, _LL, _I, _P]),
@@ -330,6 +331,32 @@ def gemm_swiglu_bwd(dy: torch.Tensor, w_down: torch.Tensor, gu: torch.Tensor) ->
     _check(lib().tlm_gemm_swiglu_bwd(dy.data_ptr(), w_down.data_ptr(), gu.data_ptr(), dgu.data_ptr(), M, I, D, lda, ldb,
                                      _stream()), "gemm_swiglu_bwd")
     return dgu
+
+
+def blocks_forward(x: torch.Tensor, weights, B: int, T: int, n_q: int, n_kv: int, hd: int, eps: float, cs: torch.Tensor,
+                   cos: torch.Tensor, sin: torch.Tensor):
+    """A run of dense blocks without gradients in one call (`csrc/forward.cu`). `weights`: per block first norm, q|k|v,
+    output projection, second norm, gate|up, down. Returns the residual stream `[B*T, D]` fp32 (`x` itself is kept) and
+    the last branch output, not added to it yet."""
+    M, D = x.shape
+    I = weights[0][5].shape[1]
+    assert x.is_contiguous() and x.dtype == torch.float32 and M == B * T and D == n_q * hd
+    for norm1, qkv, out, norm2, gate_up, down in weights:
+        for w, shape in ((norm1, (D,)), (qkv, ((n_q + 2 * n_kv) * hd, D)), (out, (D, D)), (norm2, (D,)), (gate_up, (2 * I, D)), (down, (D, I))):
+            assert w.shape == shape and w.dtype == torch.bfloat16 and w.is_contiguous()
+    assert cs.shape == (T, hd, 2) and cs.dtype == torch.float16 and cs.is_contiguous()
+    assert all(t.shape == (T, hd) and t.dtype == torch.float32 and t.is_contiguous() for t in (cos, sin))
+    bf = dict(dtype=torch.bfloat16, device=x.device)
+    xa, xb = torch.empty_like(x), torch.empty_like(x)
+    delta, h, o, act = (torch.empty(M, n, **bf) for n in (D, D, D, I))
+    qkv = torch.empty(M, (n_q + 2 * n_kv) * hd, **bf)
+    stats = torch.empty(M * (n_q + 1), dtype=torch.float32, device=x.device)           # log-sum-exp of every head's rows, 1 / rms
+    ptrs = (ctypes.c_void_p * (6 * len(weights)))(*[w.data_ptr() for block in weights for w in block])
+    _check(lib().tlm_blocks_forward(ctypes.cast(ptrs, ctypes.c_void_p), len(weights), x.data_ptr(), xa.data_ptr(), xb.data_ptr(),
+                                    delta.data_ptr(), h.data_ptr(), qkv.data_ptr(), o.data_ptr(), act.data_ptr(), stats.data_ptr(),
+                                    stats.data_ptr() + 4 * M * n_q, B, T, D, n_q, n_kv, hd, I, eps, hd ** -0.5, cs.data_ptr(),
+                                    cos.data_ptr(), sin.data_ptr(), _stream()), "blocks_forward")
+    return xa, delta
 
 
 def gemm_raw(a, b, c, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi) -> None:
