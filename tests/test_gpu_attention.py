@@ -122,11 +122,12 @@ def test_results_do_not_depend_on_the_block_order(group, monkeypatch):
     assert (o1.float() - ref).abs().max().item() < 2e-2
 
 
-@pytest.mark.parametrize("hd", [32, 128])
-@pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 1, 1, 1), (2, 127, 2, 1), (1, 129, 4, 4), (2, 513, 6, 2), (1, 1025, 8, 1)])
-def test_narrow_and_wide_heads_at_the_edges_of_tiles(hd, B, T, Hq, Hkv):
+@pytest.mark.parametrize("hd", [32, 64, 128])
+@pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 1, 1, 1), (2, 127, 2, 1), (1, 129, 4, 4), (2, 513, 6, 2), (1, 1025, 8, 1), (1, 1025, 1, 1), (3, 1001, 12, 4)])
+def test_backward_at_the_edges_of_tiles_and_splits(hd, B, T, Hq, Hkv):
     """Head dim 32 (its own 64-byte-swizzled tiles) and 128 (dQ takes turns with dP in tensor memory, two Q tiles and one dO
-    tile in shared memory): one step, first and last steps, several query heads per KV head. P and dS are rounded to bf16
+    tile in shared memory): one step, first and last steps, several query heads per KV head. Few KV tiles share their steps
+    between the CTAs of a cluster (2, 4 or 8 in the later cases; with one query head some CTAs get no step). P and dS are rounded to bf16
     (2^-9) before their products and the results once more, so 1e-2 bounds the relative error of every part."""
     from train_large_model_from_scratch_b200.ops import native
     g = torch.Generator(device="cuda").manual_seed(7)

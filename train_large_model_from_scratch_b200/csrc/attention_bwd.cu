@@ -19,8 +19,9 @@
 //      Two softmax warpgroups (one thread per query row, half of the KV columns
 //      each) turn S, dP into P, dS; dQ tiles are added to an fp32 buffer with
 //      TMA reduce-add tile stores because several KV tiles contribute to one query row.
-//      For hd = 64 the next step's S / dP MMAs are issued while the softmax
-//      warps still work on the current step.
+//      For hd 32 and 64 the next step's S / dP MMAs are issued while the softmax
+//      warps still work on the current step; hd 128 has its own order (see the HD 128 loops).
+//      With few KV tiles a cluster of CTAs shares a tile's steps (SPLIT, see split_for).
 //   3. dq (fp32, [B,Hq,T,hd]) -> bf16 into dqkv; with RoPE tables this pass also applies the transposed rotation to
 //      dQ (from the fp32 accumulator) and to the dK slots the main kernel wrote, so the packed gradient that leaves
 //      is the gradient of the UN-rotated q and k and no separate RoPE pass runs.
@@ -32,6 +33,7 @@
 // Every wait is bounded; on a timeout the CTA records a status code, leaves its
 // loops and still releases its tensor memory.
 #include "common.cuh"
+#include <cstdlib>
 
 namespace tlm {
 
@@ -62,6 +64,7 @@ struct AttnBwdParams {
   // 16-byte stores).
   __nv_bfloat16* dst[AB_MAX_DST];
   int n_dst, dst_rows, dst_heads, dst_q0, dst_k0, dst_v0;
+  int split;               // SPLIT instantiation: CTAs of the cluster that share one KV tile's steps
   int head_group;          // (batch, KV head) pairs per group of the heavy-first block order (see heavy_first_decode)
 };
 
@@ -84,7 +87,9 @@ struct AttnBwdCfg {
   // dQ staging: one [32 rows][32 fp32] swizzled box per softmax warp (HD 128: the warp's own parts of P and dS instead)
   static constexpr int OFF_DQS = OFF_DS + PD_BYTES;
   static constexpr int DQS_BYTES = HD <= 64 ? 8 * 4096 : 0;
+  static constexpr int PART_PITCH = 2 * HD + 4;          // SPLIT: floats per row of this CTA's dV | dK, from OFF_Q on
   static constexpr int OFF_BAR = OFF_DQS + DQS_BYTES;
+  static_assert(OFF_Q + AB_TILE * PART_PITCH * 4 <= OFF_BAR, "the partial dV | dK fits behind K and V");
   static constexpr int TOTAL = OFF_BAR + 256 + 1024;
   static constexpr uint32_t S_COL = 0, DP_COL = 128, DV_COL = 256, DK_COL = 256 + HD;
   // hd 64: dQ has two 64-column buffers (steps alternate), so dQ of step it can be issued while the softmax
@@ -210,7 +215,9 @@ __global__ void attn_dq_convert_kernel(const float* __restrict__ dq_acc, __nv_bf
   }
 }
 
-template <int HD, bool SCATTER>
+// SPLIT: a cluster of p.split CTAs works on one KV tile, each on its share of the (query head, query tile) steps; every CTA
+// leaves its fp32 dV | dK in its own shared memory and the cluster adds them up, in fixed order. See split_for.
+template <int HD, bool SCATTER, bool SPLIT>
 __global__ void __launch_bounds__(AB_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
                 const __grid_constant__ CUtensorMap tm_dq, const AttnBwdParams p) {
@@ -232,11 +239,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_tiles = (p.T + AB_TILE - 1) / AB_TILE;
   int j, bh;                                                  // KV tile (tile 0 has the most query tiles), (batch, KV head)
-  heavy_first_decode((int)blockIdx.x, n_tiles, p.B * p.Hkv, p.head_group, j, bh);
+  const int split = SPLIT ? p.split : 1, rank = SPLIT ? (int)cluster_ctarank() : 0;
+  heavy_first_decode((int)blockIdx.x / split, n_tiles, p.B * p.Hkv, p.head_group, j, bh);
   const int b = bh / p.Hkv, kvh = bh % p.Hkv;
   const int rep = p.Hq / p.Hkv;
   const int per_head = n_tiles - j;                           // query tiles j..n_tiles-1
-  const int n_it = rep * per_head;
+  const int it0 = SPLIT ? rep * per_head * rank / split : 0;                                       // this CTA's steps
+  const int n_it = SPLIT ? rep * per_head * (rank + 1) / split - it0 : rep * per_head;             // (SPLIT: may be none)
   const int heads_total = p.Hq + 2 * p.Hkv;
 
   if (threadIdx.x == 0) {
@@ -264,7 +273,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
       }
       if constexpr (!C::PIPELINED) {
         for (int it = 0; it < n_it; ++it) {
-          const int st = it & 1, hq = kvh * rep + it / per_head, qi = j + it % per_head;
+          const int st = it & 1, hq = kvh * rep + (it0 + it) / per_head, qi = j + (it0 + it) % per_head;
           if (!mbar_wait(bar(13 + st), ((uint32_t)(it >> 1) & 1u) ^ 1u, 21, abort_flag, p.status)) break;
           mbar_expect_tx(bar(10 + st), C::TILE_BYTES);
 #pragma unroll
@@ -281,7 +290,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
         const int st = it % C::STAGES;
         const uint32_t ph = (uint32_t)(it / C::STAGES) & 1u;
         if (!mbar_wait(bar(13 + st), ph ^ 1u, 21, abort_flag, p.status)) break;
-        const int hq = kvh * rep + it / per_head, qi = j + it % per_head;
+        const int hq = kvh * rep + (it0 + it) / per_head, qi = j + (it0 + it) % per_head;
         mbar_expect_tx(bar(10 + st), 2 * C::TILE_BYTES);
 #pragma unroll
         for (int kb = 0; kb < KB; ++kb) {
@@ -340,7 +349,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
         umma_commit(bar(5));
         return true;
       };
-      if (ok) ok = C::PIPELINED ? issue_s_dp(0) : issue_s(0);
+      if (ok && (!SPLIT || n_it > 0)) ok = C::PIPELINED ? issue_s_dp(0) : issue_s(0);
       for (int it = 0; it < n_it && ok; ++it) {
         const int st = it % C::STAGES;
         const uint32_t par = (uint32_t)it & 1u;
@@ -409,7 +418,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
     const int out0 = HD == 32 ? 0 : half * (HD / 2);         // first of this warp's OUT_COLS columns
     auto flush_dq = [&](int it) {
       if (HD != 32 || half == (it & 1)) {
-      const int hq = kvh * rep + it / per_head, qi = j + it % per_head;
+      const int hq = kvh * rep + (it0 + it) / per_head, qi = j + (it0 + it) % per_head;
       const int y0 = qi * AB_TILE + q4 * 32;                 // first of this warp's 32 query rows
 #pragma unroll
       for (int c = 0; c < C::OUT_COLS; c += 32) {
@@ -461,7 +470,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
     if constexpr (!C::PIPELINED) {
       for (int it = 0; it < n_it; ++it) {
         const uint32_t par = (uint32_t)it & 1u;
-        const int hq = kvh * rep + it / per_head, qi = j + it % per_head;
+        const int hq = kvh * rep + (it0 + it) / per_head, qi = j + (it0 + it) % per_head;
         const int t_row = qi * AB_TILE + row;
         const bool row_ok = t_row < p.T;
         const float lse2 = row_ok ? p.lse[((long long)b * p.Hq + hq) * p.T + t_row] * LOG2E : INFINITY;
@@ -516,7 +525,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
     } else
     for (int it = 0; it < n_it; ++it) {
       const uint32_t par = (uint32_t)it & 1u;
-      const int hq = kvh * rep + it / per_head, qi = j + it % per_head;
+      const int hq = kvh * rep + (it0 + it) / per_head, qi = j + (it0 + it) % per_head;
       const int t_row = qi * AB_TILE + row;
       const bool row_ok = t_row < p.T;
       const float lse2 = row_ok ? p.lse[((long long)b * p.Hq + hq) * p.T + t_row] * LOG2E : INFINITY;
@@ -561,7 +570,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
       {
         if (mbar_wait(bar(8), (uint32_t)(n_it - 1) & 1u, 31, abort_flag, p.status)) { tc_fence_after(); flush_dq(n_it - 1); } else ok = false;
       }
-      if (ok) {
+      if (ok && !SPLIT) {
         if constexpr (SCATTER) {
           // dV, dK accumulators -> bf16 rows of the packed gradient tensor
           tc_fence_after();
@@ -664,6 +673,59 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
       }
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");      // dQ reductions have left shared memory and landed
+    if constexpr (SPLIT) {
+      // this CTA's dV | dK, over the Q / dO ring (and for HD 128 the dQ boxes, so every warp's must have been read)
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      tc_fence_after();
+      float* part = reinterpret_cast<float*>(sal + C::OFF_Q) + row * C::PART_PITCH;
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        if (HD == 32 && which != half) continue;
+#pragma unroll
+        for (int c = 0; c < C::OUT_COLS; c += 32) {
+          uint32_t r[32];
+          tmem_ld32(t_lane + (which == 0 ? C::DV_COL : C::DK_COL) + out0 + c, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            *reinterpret_cast<uint4*>(part + which * HD + out0 + c + i) =
+                n_it > 0 ? make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]) : make_uint4(0, 0, 0, 0);      // no step: nothing was accumulated
+        }
+      }
+    }
+  }
+  if constexpr (SPLIT) {
+    __syncwarp();
+    tc_fence_before();
+    cluster_sync_all();
+    // rows [128 rank / split, 128 (rank + 1) / split) of the sum, in place (nobody else reads these rows of this CTA's part)
+    float* base = reinterpret_cast<float*>(sal + C::OFF_Q);
+    const int rows = AB_TILE / split, r0 = rank * rows;
+    for (int i = threadIdx.x; i < rows * (HD / 2); i += AB_THREADS) {
+      const int r = r0 + i / (HD / 2), c = (i % (HD / 2)) * 4;
+      const uint32_t off = sbase + C::OFF_Q + (uint32_t)(r * C::PART_PITCH + c) * 4u;
+      float4 a[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q < split) a[q] = ld_cluster_f4(mapa_shared(off, (uint32_t)q));
+#pragma unroll
+      for (int q = 1; q < 8; ++q)
+        if (q < split) { a[0].x += a[q].x; a[0].y += a[q].y; a[0].z += a[q].z; a[0].w += a[q].w; }
+      *reinterpret_cast<float4*>(base + r * C::PART_PITCH + c) = a[0];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < rows * (HD / 4); i += AB_THREADS) {
+      const int r = r0 + i / (HD / 4), c = (i % (HD / 4)) * 8, t_row = j * AB_TILE + r;
+      if (t_row >= p.T) continue;
+      const bool is_k = c >= HD;
+      const float osc = is_k ? p.scale : 1.f;
+      const float* v = base + r * C::PART_PITCH + c;
+      uint4 o;
+      o.x = pack_bf16(v[0] * osc, v[1] * osc); o.y = pack_bf16(v[2] * osc, v[3] * osc);
+      o.z = pack_bf16(v[4] * osc, v[5] * osc); o.w = pack_bf16(v[6] * osc, v[7] * osc);
+      *reinterpret_cast<uint4*>(p.dqkv + (((long long)b * p.T + t_row) * heads_total + (is_k ? p.Hq : p.Hq + p.Hkv) + kvh) * p.hd + (c - (is_k ? HD : 0))) = o;
+    }
+    cluster_sync_all();                // no CTA leaves while another may still read its part
   }
 
   tc_fence_before();
@@ -671,20 +733,56 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, TMEM_COLS); }
 }
 
-template <int HD, bool SCATTER>
+// CTAs per KV tile. One CTA per KV tile walks over all its query heads and tiles, so the tile with the most steps bounds the
+// launch from below however idle the chip is. A cluster divides that, but every CTA of a cluster costs about 5.4 steps (12 us:
+// start-up and the exchange of dV and dK while its SM has no other CTA). The estimate is the longer of a CTA's own time and the
+// work per SM; it picked the fastest of 1, 2, 4, 8 on eleven of twelve measured shapes. With delta and conversion passes, in us:
+// 1 x 8192, 8 / 1 heads of 64 961 -> 274; 4 x 777, 16 / 2 126 -> 60; 3 x 1001, 12 / 4 66 -> 49; 2 x 256, 8 / 2 of 32 26 -> 17.
+static int split_for(int n_tiles, int heads_kv, int rep) {
+  const char* v = getenv("TLM_ATTN_BWD_SPLIT");          // 1, 2, 4 or 8: for tests and measurements
+  const int forced = v != nullptr ? atoi(v) : 0;
+  if (forced == 1 || forced == 2 || forced == 4 || forced == 8) return forced;
+  const double heaviest = (double)rep * n_tiles, tiles = (double)n_tiles * heads_kv, total = heaviest * (n_tiles + 1) / 2 * heads_kv;
+  const double sms = num_sms();
+  int best = 1;
+  double best_cost = heaviest > total / sms ? heaviest : total / sms;
+  for (int s = 2; s <= 8; s *= 2) {
+    const double own = heaviest / s + 3.0, shared = (total + 5.4 * tiles * s) / sms, cost = own > shared ? own : shared;
+    if (cost < best_cost) { best_cost = cost; best = s; }
+  }
+  return best;
+}
+
+template <int HD, bool SCATTER, bool SPLIT = false>
 static int launch_bwd(const CUtensorMap& mq, const CUtensorMap& mdo, const CUtensorMap& mdq, const AttnBwdParams& p,
                       cudaStream_t st) {
   using C = AttnBwdCfg<HD>;
+  auto kern = attn_bwd_kernel<HD, SCATTER, SPLIT>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<HD, SCATTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::TOTAL);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
   const int grid = ((p.T + AB_TILE - 1) / AB_TILE) * p.B * p.Hkv;
-  attn_bwd_kernel<HD, SCATTER><<<grid, AB_THREADS, C::TOTAL, st>>>(mq, mdo, mdq, p);
+  if (!SPLIT) {
+    kern<<<grid, AB_THREADS, C::TOTAL, st>>>(mq, mdo, mdq, p);
+    count_launch();
+    return launch_status();
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(grid * p.split));
+  cfg.blockDim = dim3(AB_THREADS);
+  cfg.dynamicSmemBytes = C::TOTAL;
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = p.split; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, mq, mdo, mdq, p);
   count_launch();
-  return launch_status();
+  return e != cudaSuccess ? (int)e : launch_status();
 }
 
 }  // namespace tlm
@@ -736,8 +834,13 @@ static int attn_bwd_impl(const void* qkv, const void* o, const void* dout, const
     if (e) return e;
   }
   if (n_dst > 0) e = hd == 128 ? launch_bwd<128, true>(mq, mdo, mdq, p, st) : launch_bwd<64, true>(mq, mdo, mdq, p, st);
-  else e = hd == 128 ? launch_bwd<128, false>(mq, mdo, mdq, p, st) : hd == 64 ? launch_bwd<64, false>(mq, mdo, mdq, p, st)
-                                                                              : launch_bwd<32, false>(mq, mdo, mdq, p, st);
+  else {
+    p.split = split_for((T + AB_TILE - 1) / AB_TILE, B * Hkv, Hq / Hkv);
+    if (p.split > 1) e = hd == 128 ? launch_bwd<128, false, true>(mq, mdo, mdq, p, st) : hd == 64 ? launch_bwd<64, false, true>(mq, mdo, mdq, p, st)
+                                                                                                   : launch_bwd<32, false, true>(mq, mdo, mdq, p, st);
+    else e = hd == 128 ? launch_bwd<128, false>(mq, mdo, mdq, p, st) : hd == 64 ? launch_bwd<64, false>(mq, mdo, mdq, p, st)
+                                                                                : launch_bwd<32, false>(mq, mdo, mdq, p, st);
+  }
   if (e) return e;
   // without a return scatter the main kernel has written un-rotated dK into dqkv: this pass rotates it in place
   const int rot_k = (n_dst == 0 && cosT != nullptr) ? Hkv : 0;

@@ -36,13 +36,6 @@ struct SplitParams {
   unsigned int* status;
 };
 
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-  return v;
-}
-
 template <bool A_MN, bool B_MN, int EPI, int BN, int S>
 __global__ void __launch_bounds__(SP_THREADS, 2)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const SplitParams p) {
