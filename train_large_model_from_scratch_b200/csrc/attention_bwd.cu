@@ -5,7 +5,7 @@
 // so the QKV projection's dgrad/wgrad GEMMs consume one tensor.
 //
 // Three launches:
-//   1. delta[b,h,t] = sum_d do*o
+//   1. delta[b,h,t] = sum_d do*o; the dQ accumulator is zeroed on the way
 //   2. main kernel: one CTA per (128-row KV tile, batch, KV head). K and V stay in
 //      shared memory; the CTA walks over every query head of the group and every
 //      query tile at or below the diagonal. Per step five MMAs run on the
@@ -46,7 +46,7 @@ struct AttnBwdDst {
 
 struct AttnBwdParams {
   __nv_bfloat16* dqkv;
-  float* dq_acc;            // [B,Hq,T,hd] fp32, zeroed by the launcher
+  float* dq_acc;            // [B,Hq,T,hd] fp32, zeroed by the delta kernel
   const float* lse;
   const float* delta;
   int B, T, Hq, Hkv;
@@ -108,7 +108,7 @@ constexpr int DELTA_T = 32, DELTA_THREADS = 256;
 
 __global__ void __launch_bounds__(DELTA_THREADS)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
-                  float* __restrict__ delta, int B, int T, int Hq, int hd) {
+                  float* __restrict__ delta, float* __restrict__ dq_acc, int B, int T, int Hq, int hd) {
   extern __shared__ float delta_s[];                       // [Hq][DELTA_T + 1]
   const int tiles_t = (T + DELTA_T - 1) / DELTA_T;
   const int b = blockIdx.x / tiles_t, t0 = (blockIdx.x % tiles_t) * DELTA_T;
@@ -117,6 +117,12 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
   const int sub = threadIdx.x % lpr, slot = threadIdx.x / lpr, slots = DELTA_THREADS / lpr;
   const int rows = nt * Hq;                                // row rr = tl * Hq + h
   const long long base = ((long long)b * T + t0) * Hq * hd;
+  // this slab of the dQ accumulator starts at zero: stores that nothing waits for, beside the loads of the row sums
+  const int vec_h = nt * hd / 4;                           // float4 of one head: its nt rows are contiguous
+  for (int h = 0; h < Hq; ++h) {
+    float4* z = reinterpret_cast<float4*>(dq_acc + (((long long)b * Hq + h) * T + t0) * hd);
+    for (int i = threadIdx.x; i < vec_h; i += DELTA_THREADS) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
   const uint4* op = reinterpret_cast<const uint4*>(o + base) + sub;
   const uint4* dp = reinterpret_cast<const uint4*>(dout + base) + sub;
   for (int rb = 0; rb < rows; rb += 4 * slots) {          // trip count is uniform: the shuffles below need whole warps
@@ -153,17 +159,21 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
 // (j + hd / 2) per thread so that the transposed rotation (see AttnBwdParams) can be applied on the way.
 // `rot_k` (only without a head -> sequence return): the Hkv k-head slots of dqkv, written as bf16 by the main kernel, are
 // rotated in place by further work items (heads Hq .. Hq + Hkv - 1).
+// Index: 32 bits while the items fit (three 64-bit divisions per item took longer than the item's 64 bytes).
+template <typename Index>
 __global__ void attn_dq_convert_kernel(const float* __restrict__ dq_acc, __nv_bfloat16* __restrict__ dqkv, int B, int T,
                                        int Hq, int heads_total, int hd, float scale, const float* __restrict__ cosT,
                                        const float* __restrict__ sinT, const AttnBwdDst d, int dst_q0, int rot_k) {
-  const int half = hd / 2, vec = half / 8;
+  const int half = hd / 2, vec_log = hd == 32 ? 1 : hd == 64 ? 2 : 3;          // hd / 16 items per row
   const int heads = Hq + rot_k;
-  const long long total = (long long)B * heads * T * vec;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int j = (int)(i % vec) * 8;
-    long long r = i / vec;
-    const int t = (int)(r % T); r /= T;
-    const int h = (int)(r % heads); const long long b = r / heads;
+  const Index total = ((Index)B * heads * T) << vec_log, step = (Index)gridDim.x * blockDim.x;
+  for (Index i = blockIdx.x * (Index)blockDim.x + threadIdx.x; i < total; i += step) {
+    const int j = (int)(i & ((1 << vec_log) - 1)) * 8;
+    Index r = i >> vec_log;
+    const Index bh = r / (Index)T;
+    const int t = (int)(r - bh * (Index)T);
+    const long long b = (long long)(bh / (Index)heads);
+    const int h = (int)(bh - (Index)b * heads);
     float lo[8], hi[8];
     if (h < Hq) {
       const float* src = dq_acc + (((long long)b * Hq + h) * T + t) * hd + j;
@@ -798,13 +808,10 @@ static int attn_bwd_impl(const void* qkv, const void* o, const void* dout, const
                          int dst_heads, int dst_q0, int dst_k0, int dst_v0, cudaStream_t st) {
   if (hd != 32 && hd != 64 && hd != 128) return -4;
   if (Hq % Hkv != 0) return -5;
-  const long long rows = (long long)B * T * Hq;
   if ((size_t)Hq * (DELTA_T + 1) * 4 > 48 * 1024) return -6;
   attn_delta_kernel<<<B * ((T + DELTA_T - 1) / DELTA_T), DELTA_THREADS, (size_t)Hq * (DELTA_T + 1) * 4, st>>>(
-      (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, B, T, Hq, hd);
+      (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, dq_acc, B, T, Hq, hd);
   count_launch();
-  cudaError_t ce = cudaMemsetAsync(dq_acc, 0, (size_t)rows * hd * 4, st);
-  if (ce != cudaSuccess) return (int)ce;
   CUtensorMap mq, mdo;
   const int box_cols = hd == 32 && n_dst == 0 ? 32 : 64;
   int e = make_qkv_map(&mq, qkv, B, T, Hq + 2 * Hkv, hd, AB_TILE, box_cols);
@@ -844,11 +851,14 @@ static int attn_bwd_impl(const void* qkv, const void* o, const void* dout, const
   if (e) return e;
   // without a return scatter the main kernel has written un-rotated dK into dqkv: this pass rotates it in place
   const int rot_k = (n_dst == 0 && cosT != nullptr) ? Hkv : 0;
-  long long items = (long long)B * T * (Hq + rot_k) * (hd / 16);
-  int cb = (int)((items + 255) / 256);
-  if (cb > num_sms() * 16) cb = num_sms() * 16;
-  attn_dq_convert_kernel<<<cb, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dqkv, B, T, Hq, Hq + 2 * Hkv, hd, scale, cosT, sinT, dd, dst_q0,
-                                             rot_k);
+  const long long items = (long long)B * T * (Hq + rot_k) * (hd / 16);
+  int cb = (int)((items + 255) / 256 < num_sms() * 16 ? (items + 255) / 256 : num_sms() * 16);
+  if (items + 256LL * cb < (1LL << 32))
+    attn_dq_convert_kernel<unsigned><<<cb, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dqkv, B, T, Hq, Hq + 2 * Hkv, hd, scale, cosT, sinT, dd,
+                                                         dst_q0, rot_k);
+  else
+    attn_dq_convert_kernel<long long><<<cb, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dqkv, B, T, Hq, Hq + 2 * Hkv, hd, scale, cosT, sinT, dd,
+                                                          dst_q0, rot_k);
   count_launch();
   return launch_status();
 }
