@@ -6,7 +6,7 @@
 // reduction, each CTA an equal share of the k-blocks. Every CTA leaves its fp32 partial tile in its own shared memory,
 // and after a cluster barrier CTA r adds up rows [128 r / S, 128 (r + 1) / S) of all S partials (distributed shared
 // memory, fixed order, so the result does not depend on timing) and applies the epilogue. No workspace, no second
-// launch, no atomics.
+// launch, no atomics between the parts.
 //
 // Roles as in gemm.cu: warp 0 TMA producer, warp 1 MMA issuer and tensor-memory owner, warps 2-5 move the accumulator
 // to shared memory; then all six warps reduce and store. Two CTAs fit an SM, so one's prologue and epilogue run beside
@@ -173,10 +173,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
   };
   const int half = EPI == SPLIT_HEADS ? g.hd >> 1 : 0;
+  // read-only loads (rotation tables, gate / up) of four items in flight: one after the other, their latency was most of
+  // the epilogue
+#pragma unroll 4
   for (int i = threadIdx.x; i < ROWS * PER_ROW; i += SP_THREADS) {
     const int r = rank * ROWS + i / PER_ROW, ch = i % PER_ROW;
     const long long row = m0 + r;
-    if (row >= g.M) break;                                   // rows ascend with i
+    if (row >= g.M) continue;
     float v[8];
     if constexpr (EPI == SPLIT_BF16 || EPI == SPLIT_F32_ACC) {
       const int col = n0 + ch * 8;
@@ -185,11 +188,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         load8(r, ch * 8, v);
         *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.C) + row * g.ldc + col) = pack8(v);
       } else {
-        float4* out = reinterpret_cast<float4*>(reinterpret_cast<float*>(g.C) + row * g.ldc + col);
-        float4 o0 = out[0], o1 = out[1];
+        // one reduction per element: nothing waits for C, and the result does not depend on timing
+        float* out = reinterpret_cast<float*>(g.C) + row * g.ldc + col;
         load8(r, ch * 8, v);
-        o0.x += v[0]; o0.y += v[1]; o0.z += v[2]; o0.w += v[3]; o1.x += v[4]; o1.y += v[5]; o1.z += v[6]; o1.w += v[7];
-        out[0] = o0; out[1] = o1;
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(out), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(out + 4), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
       }
     } else if constexpr (EPI == SPLIT_HEADS) {
       const int per_half = half >> 3;                        // 8-column pieces of half a head
@@ -204,10 +207,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         const float* sp = g.sinT + (long long)t * g.hd + j;
 #pragma unroll
         for (int k = 0; k < 8; k += 4) {
-          *reinterpret_cast<float4*>(cl + k) = *reinterpret_cast<const float4*>(cp + k);
-          *reinterpret_cast<float4*>(sl + k) = *reinterpret_cast<const float4*>(sp + k);
-          *reinterpret_cast<float4*>(chh + k) = *reinterpret_cast<const float4*>(cp + half + k);
-          *reinterpret_cast<float4*>(sh + k) = *reinterpret_cast<const float4*>(sp + half + k);
+          *reinterpret_cast<float4*>(cl + k) = __ldg(reinterpret_cast<const float4*>(cp + k));
+          *reinterpret_cast<float4*>(sl + k) = __ldg(reinterpret_cast<const float4*>(sp + k));
+          *reinterpret_cast<float4*>(chh + k) = __ldg(reinterpret_cast<const float4*>(cp + half + k));
+          *reinterpret_cast<float4*>(sh + k) = __ldg(reinterpret_cast<const float4*>(sp + half + k));
         }
       }
       load8(r, c, v);
@@ -245,7 +248,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       const int col = n0 + ch * 8;
       if (col >= g.N) continue;
       const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(g.aux) + row * 2 * g.N + col;
-      const uint4 gv = *reinterpret_cast<const uint4*>(gp), uv = *reinterpret_cast<const uint4*>(gp + g.N);
+      const uint4 gv = __ldg(reinterpret_cast<const uint4*>(gp)), uv = __ldg(reinterpret_cast<const uint4*>(gp + g.N));
       load8(r, ch * 8, v);
       const uint4 dv = pack8(v);
       const uint32_t dw[4] = {dv.x, dv.y, dv.z, dv.w}, gw[4] = {gv.x, gv.y, gv.z, gv.w}, uw[4] = {uv.x, uv.y, uv.z, uv.w};
@@ -329,8 +332,7 @@ int split_run(const SplitGemm& g, const SplitPlan& plan, cudaStream_t st) {
 // Estimated time in us, fitted to 30 shapes (M 16 - 4096, N 256 - 3072, K 256 - 50304, operands in L2): a k-block takes
 // 0.24 us (64 columns) or 0.27 us (128 columns) of a CTA, what 24 / 32 KB take at the 64 B per clock that an SM gets out of
 // L2, and no less than all CTAs' blocks take at 14 TB/s out of the whole L2; plus what surrounds the main loop and the
-// exchange of the partial tiles. A weight gradient has to win clearly: its C is read by the SMs here, while the wide tiles
-// leave through TMA reduce-add, which matters once C comes from HBM.
+// exchange of the partial tiles. A weight gradient has to win clearly: the wide tiles add to C with whole TMA boxes.
 SplitPlan split_plan(const SplitGemm& g, double wide_us) {
   SplitPlan best{0, 0};
   if (g.N % 8 != 0 || g.ldc % 8 != 0 || (reinterpret_cast<uintptr_t>(g.C) & 15)) return best;
