@@ -438,6 +438,22 @@ def test_grouped_pair_weight_gradients(nat, gemm_mode, counts, I, D):
         r += c
 
 
+@pytest.mark.parametrize("M,E,k", [(1, 1, 1), (127, 33, 8), (129, 128, 8), (300, 256, 2), (64, 8, 8)])
+def test_moe_route_ties_zeros_and_infinities(nat, M, E, k):
+    """Few distinct logits, both zeros and -inf among them: the k largest, lower expert id first among equals, as a stable sort."""
+    g = torch.Generator(device="cuda").manual_seed(95)
+    values = torch.tensor([-float("inf"), -2.0, -0.0, 0.0, 0.5, 3.0], device="cuda").bfloat16()
+    logits = values[torch.randint(0, 6, (M, E), device="cuda", generator=g)]
+    logits[:, 0] = 0.25                                   # never only -inf
+    w, ex, counts, base, pos, order = nat.moe_route(logits, k)
+    nat.raise_on_device_status()
+    val, idx = torch.sort(logits.float() + 0.0, dim=-1, descending=True, stable=True)
+    assert torch.equal(ex.long(), idx[:, :k])
+    torch.testing.assert_close(w, torch.softmax(val[:, :k], -1), rtol=1e-5, atol=1e-7)
+    assert torch.equal(counts.long(), torch.bincount(idx[:, :k].reshape(-1), minlength=E))
+    assert torch.equal(order.long(), torch.argsort(idx[:, :k].reshape(-1), stable=True))
+
+
 @pytest.mark.parametrize("M,E,k", [(300, 8, 2), (129, 128, 8), (64, 4, 1), (1000, 40, 3)])
 def test_moe_route_and_row_movement(nat, M, E, k):
     """Device routing (top-k, softmax of the winners, stable expert-major order) and the gather / combine /
