@@ -109,6 +109,7 @@ constexpr int DELTA_T = 32, DELTA_THREADS = 256;
 __global__ void __launch_bounds__(DELTA_THREADS)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
                   float* __restrict__ delta, float* __restrict__ dq_acc, int B, int T, int Hq, int hd) {
+  griddep_wait();
   extern __shared__ float delta_s[];                       // [Hq][DELTA_T + 1]
   const int tiles_t = (T + DELTA_T - 1) / DELTA_T;
   const int b = blockIdx.x / tiles_t, t0 = (blockIdx.x % tiles_t) * DELTA_T;
@@ -164,6 +165,7 @@ template <typename Index>
 __global__ void attn_dq_convert_kernel(const float* __restrict__ dq_acc, __nv_bfloat16* __restrict__ dqkv, int B, int T,
                                        int Hq, int heads_total, int hd, float scale, const float* __restrict__ cosT,
                                        const float* __restrict__ sinT, const AttnBwdDst d, int dst_q0, int rot_k) {
+  griddep_wait();
   const int half = hd / 2, vec_log = hd == 32 ? 1 : hd == 64 ? 2 : 3;          // hd / 16 items per row
   const int heads = Hq + rot_k;
   const Index total = ((Index)B * heads * T) << vec_log, step = (Index)gridDim.x * blockDim.x;
@@ -271,6 +273,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  griddep_wait();
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
@@ -775,24 +778,7 @@ static int launch_bwd(const CUtensorMap& mq, const CUtensorMap& mdo, const CUten
     configured = true;
   }
   const int grid = ((p.T + AB_TILE - 1) / AB_TILE) * p.B * p.Hkv;
-  if (!SPLIT) {
-    kern<<<grid, AB_THREADS, C::TOTAL, st>>>(mq, mdo, mdq, p);
-    count_launch();
-    return launch_status();
-  }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(grid * p.split));
-  cfg.blockDim = dim3(AB_THREADS);
-  cfg.dynamicSmemBytes = C::TOTAL;
-  cfg.stream = st;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = p.split; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, mq, mdo, mdq, p);
-  count_launch();
-  return e != cudaSuccess ? (int)e : launch_status();
+  return launch_overlapped(kern, dim3((unsigned)(grid * (SPLIT ? p.split : 1))), dim3(AB_THREADS), C::TOTAL, st, SPLIT ? p.split : 1, mq, mdo, mdq, p);
 }
 
 }  // namespace tlm
@@ -809,9 +795,9 @@ static int attn_bwd_impl(const void* qkv, const void* o, const void* dout, const
   if (hd != 32 && hd != 64 && hd != 128) return -4;
   if (Hq % Hkv != 0) return -5;
   if ((size_t)Hq * (DELTA_T + 1) * 4 > 48 * 1024) return -6;
-  attn_delta_kernel<<<B * ((T + DELTA_T - 1) / DELTA_T), DELTA_THREADS, (size_t)Hq * (DELTA_T + 1) * 4, st>>>(
+  int le = launch_overlapped(attn_delta_kernel, dim3(B * ((T + DELTA_T - 1) / DELTA_T)), dim3(DELTA_THREADS), (size_t)Hq * (DELTA_T + 1) * 4, st, 1,
       (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, dq_acc, B, T, Hq, hd);
-  count_launch();
+  if (le) return le;
   CUtensorMap mq, mdo;
   const int box_cols = hd == 32 && n_dst == 0 ? 32 : 64;
   int e = make_qkv_map(&mq, qkv, B, T, Hq + 2 * Hkv, hd, AB_TILE, box_cols);
@@ -853,14 +839,9 @@ static int attn_bwd_impl(const void* qkv, const void* o, const void* dout, const
   const int rot_k = (n_dst == 0 && cosT != nullptr) ? Hkv : 0;
   const long long items = (long long)B * T * (Hq + rot_k) * (hd / 16);
   int cb = (int)((items + 255) / 256 < num_sms() * 16 ? (items + 255) / 256 : num_sms() * 16);
-  if (items + 256LL * cb < (1LL << 32))
-    attn_dq_convert_kernel<unsigned><<<cb, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dqkv, B, T, Hq, Hq + 2 * Hkv, hd, scale, cosT, sinT, dd,
-                                                         dst_q0, rot_k);
-  else
-    attn_dq_convert_kernel<long long><<<cb, 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dqkv, B, T, Hq, Hq + 2 * Hkv, hd, scale, cosT, sinT, dd,
-                                                          dst_q0, rot_k);
-  count_launch();
-  return launch_status();
+  auto conv = items + 256LL * cb < (1LL << 32) ? attn_dq_convert_kernel<unsigned> : attn_dq_convert_kernel<long long>;
+  return launch_overlapped(conv, dim3(cb), dim3(256), 0, st, 1, (const float*)dq_acc, (__nv_bfloat16*)dqkv, B, T, Hq, Hq + 2 * Hkv, hd, scale, cosT, sinT,
+                           dd, dst_q0, rot_k);
 }
 
 TLM_API int tlm_attn_bwd(const void* qkv, const void* o, const void* dout, const float* lse, void* dqkv,

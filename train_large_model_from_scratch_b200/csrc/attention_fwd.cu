@@ -107,6 +107,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const AttnFwdParams 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  griddep_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -310,9 +311,7 @@ static int launch_fwd(const CUtensorMap& map, const AttnFwdParams& p, cudaStream
     configured = true;
   }
   const int grid = ((p.T + AT_BQ - 1) / AT_BQ) * p.B * p.Hq;
-  attn_fwd_kernel<HD><<<grid, AT_THREADS, L::TOTAL, st>>>(map, p);
-  count_launch();
-  return launch_status();
+  return launch_overlapped(attn_fwd_kernel<HD>, dim3(grid), dim3(AT_THREADS), L::TOTAL, st, 1, map, p);
 }
 
 }  // namespace tlm

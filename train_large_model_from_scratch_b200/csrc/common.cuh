@@ -28,6 +28,30 @@ inline void count_launch(int n = 1) { g_launches += (unsigned long long)n; }
 // code = (site << 8) | detail. `status_word()` returns the device-visible pointer.
 unsigned int* status_word();
 
+// Kernels launched through launch_overlapped may start while the kernel before them in the stream drains: their launch and
+// set-up (barriers, tensor memory, descriptor fetch) then run beside its tail. They call griddep_wait() before they touch
+// memory that another kernel reads or writes. No kernel signals its dependents early: a dependent starts only when every
+// block of the kernel before it has left, so the two never compete for tensor memory. A 333-token prompt through 12 layers
+// (87 launches) 1010 -> 793 us, an expert layer 859 -> 847 us; steps replayed as a graph did not change.
+#ifdef __CUDACC__
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+inline int launch_overlapped(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, P(args)...);
+  count_launch();
+  return (int)(e != cudaSuccess ? e : cudaPeekAtLastError());
+}
+#endif
+
 inline int launch_status() {
   cudaError_t e = cudaPeekAtLastError();
   return (int)e;

@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(256)
 add_rmsnorm_fwd_reg_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
                            const __nv_bfloat16* __restrict__ w, float* __restrict__ x_new,
                            __nv_bfloat16* __restrict__ h, float* __restrict__ rstd_out, int rows, float eps) {
+  griddep_wait();
   constexpr int D = NV * 256;
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int r = blockIdx.x * warps + warp; r < rows; r += gridDim.x * warps) {
@@ -159,6 +160,7 @@ __global__ void __launch_bounds__(RMS_WIDE_MAX_WARPS * 32)
 add_rmsnorm_fwd_wide_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
                             const __nv_bfloat16* __restrict__ w, float* __restrict__ x_new,
                             __nv_bfloat16* __restrict__ h, float* __restrict__ rstd_out, int rows, int D, float eps) {
+  griddep_wait();
   __shared__ float red[2][RMS_WIDE_MAX_WARPS];
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c0 = (warp * NV * 32 + lane) * 8;
@@ -281,6 +283,7 @@ add_rmsnorm_bwd_reg_kernel(const float* __restrict__ g_xnew, const __nv_bfloat16
                            const float* __restrict__ x_new, const float* __restrict__ rstd_in,
                            const __nv_bfloat16* __restrict__ w, float* __restrict__ g_x,
                            __nv_bfloat16* __restrict__ g_delta, float* __restrict__ dw_out, int rows) {
+  griddep_wait();
   constexpr int D = NV * 256;
   __shared__ float dw_s[8][D > 1024 ? 1 : D];       // block fold (only used when it fits; else atomics per warp)
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -360,6 +363,7 @@ add_rmsnorm_bwd_wide_kernel(const float* __restrict__ g_xnew, const __nv_bfloat1
                             const float* __restrict__ x_new, const float* __restrict__ rstd_in,
                             const __nv_bfloat16* __restrict__ w, float* __restrict__ g_x,
                             __nv_bfloat16* __restrict__ g_delta, float* __restrict__ dw_out, int rows, int D) {
+  griddep_wait();
   __shared__ float red[2][RMS_WIDE_MAX_WARPS];
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c0 = (warp * NV * 32 + lane) * 8;
@@ -786,8 +790,8 @@ TLM_API int tlm_add_rmsnorm_fwd(const float* x, const void* delta, const void* w
                                 int rows, int D, float eps, cudaStream_t st) {
   if (D % 256 == 0 && D / 256 <= 8 && D / 256 != 5 && D / 256 != 7) {
     const int grid = grid_for((rows + 7) / 8, 1, 8);
-#define TLM_RMS_CASE(NV) case NV: add_rmsnorm_fwd_reg_kernel<NV><<<grid, 256, 0, st>>>(x, (const __nv_bfloat16*)delta, \
-      (const __nv_bfloat16*)w, x_new, (__nv_bfloat16*)h, rstd, rows, eps); break;
+#define TLM_RMS_CASE(NV) case NV: return launch_overlapped(add_rmsnorm_fwd_reg_kernel<NV>, dim3(grid), dim3(256), 0, st, 1, x, (const __nv_bfloat16*)delta, \
+      (const __nv_bfloat16*)w, x_new, (__nv_bfloat16*)h, rstd, rows, eps);
     switch (D / 256) { TLM_RMS_CASE(1) TLM_RMS_CASE(2) TLM_RMS_CASE(3) TLM_RMS_CASE(4) TLM_RMS_CASE(6) TLM_RMS_CASE(8) }
 #undef TLM_RMS_CASE
     count_launch();
@@ -796,8 +800,8 @@ TLM_API int tlm_add_rmsnorm_fwd(const float* x, const void* delta, const void* w
   const RmsSplit sp = rms_split(D, 4);
   if (sp.nv > 0) {
     const int grid = grid_for(rows, 1, 64 / sp.warps);
-#define TLM_RMS_CASE(NV) case NV: add_rmsnorm_fwd_wide_kernel<NV><<<grid, sp.warps * 32, 0, st>>>(x, (const __nv_bfloat16*)delta, \
-      (const __nv_bfloat16*)w, x_new, (__nv_bfloat16*)h, rstd, rows, D, eps); break;
+#define TLM_RMS_CASE(NV) case NV: return launch_overlapped(add_rmsnorm_fwd_wide_kernel<NV>, dim3(grid), dim3(sp.warps * 32), 0, st, 1, x, (const __nv_bfloat16*)delta, \
+      (const __nv_bfloat16*)w, x_new, (__nv_bfloat16*)h, rstd, rows, D, eps);
     switch (sp.nv) { TLM_RMS_CASE(1) TLM_RMS_CASE(2) TLM_RMS_CASE(3) TLM_RMS_CASE(4) }
 #undef TLM_RMS_CASE
     count_launch();
@@ -824,8 +828,8 @@ TLM_API int tlm_add_rmsnorm_bwd(const float* g_xnew, const void* g_h, const floa
                                 cudaStream_t st) {
   if (D % 256 == 0 && D / 256 <= 6 && D / 256 != 5) {
     const int grid = grid_for((rows + 7) / 8, 1, 4);
-#define TLM_RMS_CASE(NV) case NV: add_rmsnorm_bwd_reg_kernel<NV><<<grid, 256, 0, st>>>(g_xnew, (const __nv_bfloat16*)g_h, x_new, rstd, \
-      (const __nv_bfloat16*)w, g_x, (__nv_bfloat16*)g_delta, dw, rows); break;
+#define TLM_RMS_CASE(NV) case NV: return launch_overlapped(add_rmsnorm_bwd_reg_kernel<NV>, dim3(grid), dim3(256), 0, st, 1, g_xnew, (const __nv_bfloat16*)g_h, x_new, rstd, \
+      (const __nv_bfloat16*)w, g_x, (__nv_bfloat16*)g_delta, dw, rows);
     switch (D / 256) { TLM_RMS_CASE(1) TLM_RMS_CASE(2) TLM_RMS_CASE(3) TLM_RMS_CASE(4) TLM_RMS_CASE(6) }
 #undef TLM_RMS_CASE
     count_launch();
@@ -834,8 +838,8 @@ TLM_API int tlm_add_rmsnorm_bwd(const float* g_xnew, const void* g_h, const floa
   const RmsSplit sp = rms_split(D, 3);          // 4 groups would not fit the registers
   if (sp.nv > 0 && (reinterpret_cast<uintptr_t>(dw) & 15) == 0) {
     const int grid = grid_for(rows, 1, sp.warps >= 16 ? 1 : 16 / sp.warps);
-#define TLM_RMS_CASE(NV) case NV: add_rmsnorm_bwd_wide_kernel<NV><<<grid, sp.warps * 32, 0, st>>>(g_xnew, (const __nv_bfloat16*)g_h, x_new, rstd, \
-      (const __nv_bfloat16*)w, g_x, (__nv_bfloat16*)g_delta, dw, rows, D); break;
+#define TLM_RMS_CASE(NV) case NV: return launch_overlapped(add_rmsnorm_bwd_wide_kernel<NV>, dim3(grid), dim3(sp.warps * 32), 0, st, 1, g_xnew, (const __nv_bfloat16*)g_h, x_new, rstd, \
+      (const __nv_bfloat16*)w, g_x, (__nv_bfloat16*)g_delta, dw, rows, D);
     switch (sp.nv) { TLM_RMS_CASE(1) TLM_RMS_CASE(2) TLM_RMS_CASE(3) }
 #undef TLM_RMS_CASE
     count_launch();

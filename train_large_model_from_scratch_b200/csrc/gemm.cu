@@ -253,6 +253,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     if (PAIR) { tmem_alloc_pair(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish_pair(); }
     else { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
   }
+  griddep_wait();
   if (GROUP == 1 && warp == 2) {
     // exclusive prefix sum of the groups' row-tile counts: lane l owns groups [8 l, 8 l + 8)
     constexpr int PER = MAX_GROUPS / 32;
@@ -1230,9 +1231,7 @@ static int launch_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensor
   }
   int grid = tiles < num_sms() ? tiles : num_sms();
   if (grid <= 0) return 0;
-  kern<<<grid, GEMM_THREADS, GEMM_SMEM, st>>>(ma, mb, mc, p);
-  count_launch();
-  return launch_status();
+  return launch_overlapped(kern, dim3(grid), dim3(GEMM_THREADS), GEMM_SMEM, st, 1, ma, mb, mc, p);
 }
 
 template <bool A_MN, bool B_MN, int EPI, int GROUP = 0>
@@ -1247,9 +1246,7 @@ static int launch_pair_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUt
   }
   const int grid = pair_grid(tiles);
   if (grid <= 0) return 0;
-  kern<<<grid, GEMM_THREADS, GEMM_SMEM_PAIR, st>>>(ma, mb, mc, p);
-  count_launch();
-  return launch_status();
+  return launch_overlapped(kern, dim3(grid), dim3(GEMM_THREADS), GEMM_SMEM_PAIR, st, 1, ma, mb, mc, p);
 }
 
 // `pair`: `tiles` counts 256-row tiles and the B map was built with 128-row boxes (see pair_maps)
@@ -1301,9 +1298,7 @@ static int launch_heads(const CUtensorMap& ma, const CUtensorMap& mb, const Head
   }
   int grid = tiles < num_sms() ? tiles : num_sms();
   if (grid <= 0) return 0;
-  kern<<<grid, GEMM_THREADS, GEMM_SMEM, st>>>(ma, mb, dst, p);
-  count_launch();
-  return launch_status();
+  return launch_overlapped(kern, dim3(grid), dim3(GEMM_THREADS), GEMM_SMEM, st, 1, ma, mb, dst, p);
 }
 
 template <bool B_MN, int EPI = EPI_HEADS>
@@ -1318,9 +1313,7 @@ static int launch_heads_pair(const CUtensorMap& ma, const CUtensorMap& mb, const
   }
   const int grid = pair_grid(tiles);
   if (grid <= 0) return 0;
-  kern<<<grid, GEMM_THREADS, GEMM_SMEM_PAIR, st>>>(ma, mb, dst, p);
-  count_launch();
-  return launch_status();
+  return launch_overlapped(kern, dim3(grid), dim3(GEMM_THREADS), GEMM_SMEM_PAIR, st, 1, ma, mb, dst, p);
 }
 
 }  // namespace tlm
@@ -1448,9 +1441,7 @@ TLM_API int tlm_gemm_swiglu(const void* x, const void* w_gu, void* gate_up, void
       pconfigured = true;
     }
     const int pgrid = pair_grid((long long)((M + 2 * BM - 1) / (2 * BM)) * ((I + 127) / 128));
-    gemm_swiglu_pair_kernel<0><<<pgrid, GEMM_THREADS, GEMM_SMEM_PAIR, stream>>>(ma, mb, mc, md, p);
-    count_launch();
-    return launch_status();
+    return launch_overlapped(gemm_swiglu_pair_kernel<0>, dim3(pgrid), dim3(GEMM_THREADS), GEMM_SMEM_PAIR, stream, 1, ma, mb, mc, md, p);
   }
   static bool configured = false;
   if (!configured) {
@@ -1460,9 +1451,7 @@ TLM_API int tlm_gemm_swiglu(const void* x, const void* w_gu, void* gate_up, void
   }
   const int tiles = ((M + BM - 1) / BM) * ((I + 127) / 128);
   const int grid = tiles < num_sms() ? tiles : num_sms();
-  gemm_swiglu_kernel<0><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ma, mb, mc, md, p);
-  count_launch();
-  return launch_status();
+  return launch_overlapped(gemm_swiglu_kernel<0>, dim3(grid), dim3(GEMM_THREADS), GEMM_SMEM, stream, 1, ma, mb, mc, md, p);
 }
 
 // d(gate_up)[M, 2 I] from dy[M, D], w_down[D, I] (row pitch ldb) and the saved gate_up[M, 2 I]:
@@ -1498,9 +1487,7 @@ TLM_API int tlm_gemm_swiglu_bwd(const void* dy, const void* w_down, const void* 
       pconfigured = true;
     }
     const int pgrid = pair_grid((long long)((M + 2 * BM - 1) / (2 * BM)) * ((I + BN - 1) / BN));
-    gemm_swiglu_bwd_pair_kernel<0><<<pgrid, GEMM_THREADS_WIDE, GEMM_SMEM_PAIR, stream>>>(ma, mb, mc, p);
-    count_launch();
-    return launch_status();
+    return launch_overlapped(gemm_swiglu_bwd_pair_kernel<0>, dim3(pgrid), dim3(GEMM_THREADS_WIDE), GEMM_SMEM_PAIR, stream, 1, ma, mb, mc, p);
   }
   static bool configured = false;
   if (!configured) {
@@ -1510,9 +1497,7 @@ TLM_API int tlm_gemm_swiglu_bwd(const void* dy, const void* w_down, const void* 
   }
   const int tiles = ((M + BM - 1) / BM) * ((I + BN - 1) / BN);
   const int grid = tiles < num_sms() ? tiles : num_sms();
-  gemm_swiglu_bwd_kernel<0><<<grid, GEMM_THREADS_WIDE, GEMM_SMEM, stream>>>(ma, mb, mc, p);
-  count_launch();
-  return launch_status();
+  return launch_overlapped(gemm_swiglu_bwd_kernel<0>, dim3(grid), dim3(GEMM_THREADS_WIDE), GEMM_SMEM, stream, 1, ma, mb, mc, p);
 }
 
 // Arms a "parameters ready" gate for the next forward-projection GEMM launched through this library (tlm_gemm with
@@ -1571,10 +1556,8 @@ TLM_API int tlm_gemm_swiglu_grouped(const void* x, const void* w_pair, void* gat
     configured = true;
   }
   return for_group_chunks(p, groups, row_start, R, max_rows_per_group, I / 128, pair, [&](const GemmParams& q, int tiles) {
-    if (pair) gemm_swiglu_pair_kernel<1><<<pair_grid(tiles), GEMM_THREADS, GEMM_SMEM_PAIR, stream>>>(ma, mb, mc, md, q);
-    else gemm_swiglu_kernel<1><<<tiles < num_sms() ? tiles : num_sms(), GEMM_THREADS, GEMM_SMEM, stream>>>(ma, mb, mc, md, q);
-    count_launch();
-    return launch_status();
+    if (pair) return launch_overlapped(gemm_swiglu_pair_kernel<1>, dim3(pair_grid(tiles)), dim3(GEMM_THREADS), GEMM_SMEM_PAIR, stream, 1, ma, mb, mc, md, q);
+    return launch_overlapped(gemm_swiglu_kernel<1>, dim3(tiles < num_sms() ? tiles : num_sms()), dim3(GEMM_THREADS), GEMM_SMEM, stream, 1, ma, mb, mc, md, q);
   });
 }
 
@@ -1606,10 +1589,8 @@ TLM_API int tlm_gemm_swiglu_bwd_grouped(const void* dy, const void* w_down, cons
     configured = true;
   }
   return for_group_chunks(p, groups, row_start, R, max_rows_per_group, (I + BN - 1) / BN, pair, [&](const GemmParams& q, int tiles) {
-    if (pair) gemm_swiglu_bwd_pair_kernel<1><<<pair_grid(tiles), GEMM_THREADS_WIDE, GEMM_SMEM_PAIR, stream>>>(ma, mb, mc, q);
-    else gemm_swiglu_bwd_kernel<1><<<tiles < num_sms() ? tiles : num_sms(), GEMM_THREADS_WIDE, GEMM_SMEM, stream>>>(ma, mb, mc, q);
-    count_launch();
-    return launch_status();
+    if (pair) return launch_overlapped(gemm_swiglu_bwd_pair_kernel<1>, dim3(pair_grid(tiles)), dim3(GEMM_THREADS_WIDE), GEMM_SMEM_PAIR, stream, 1, ma, mb, mc, q);
+    return launch_overlapped(gemm_swiglu_bwd_kernel<1>, dim3(tiles < num_sms() ? tiles : num_sms()), dim3(GEMM_THREADS_WIDE), GEMM_SMEM, stream, 1, ma, mb, mc, q);
   });
 }
 

@@ -73,6 +73,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  griddep_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -277,19 +278,7 @@ static int launch_split(const CUtensorMap& ma, const CUtensorMap& mb, const Spli
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(p.tiles_m * p.tiles_n * S));
-  cfg.blockDim = dim3(SP_THREADS);
-  cfg.dynamicSmemBytes = SplitCfg<BN>::SMEM;
-  cfg.stream = st;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = S; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = S > 1 ? 1 : 0;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ma, mb, p);
-  count_launch();
-  return e != cudaSuccess ? (int)e : launch_status();
+  return launch_overlapped(kern, dim3((unsigned)(p.tiles_m * p.tiles_n * S)), dim3(SP_THREADS), SplitCfg<BN>::SMEM, st, S, ma, mb, p);
 }
 
 static int split_map(CUtensorMap* m, const void* ptr, long long rows, long long k, long long ld, bool mn, int box_rows) {
