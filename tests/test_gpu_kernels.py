@@ -292,7 +292,7 @@ def test_gemm_swiglu_epilogues(nat, gemm_mode, M, I, K):
     assert _rel_err(dgu, ref) < 6e-3
 
 
-@pytest.mark.parametrize("rows,D", [(1, 1280), (37, 2304), (700, 3072), (5, 4096), (3, 4352)])
+@pytest.mark.parametrize("rows,D", [(1, 1280), (9, 1536), (37, 2304), (700, 3072), (5, 4096), (3, 4352)])
 def test_add_rmsnorm_of_wide_rows(nat, rows, D):
     """Rows shared by several warps (1280 = 5 x 256, 2304 = 3 x 768, 3072 = 4 x 768, ...; 4352 = 17 x 256 is too many warps and
     takes the shared-memory form), with and without an incoming residual gradient."""
