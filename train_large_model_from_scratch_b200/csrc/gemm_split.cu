@@ -320,14 +320,19 @@ int split_run(const SplitGemm& g, const SplitPlan& plan, cudaStream_t st) {
 
 // Estimated time in us, fitted to 30 shapes (M 16 - 4096, N 256 - 3072, K 256 - 50304, operands in L2): a k-block takes
 // 0.24 us (64 columns) or 0.27 us (128 columns) of a CTA, what 24 / 32 KB take at the 64 B per clock that an SM gets out of
-// L2, and no less than all CTAs' blocks take at 14 TB/s out of the whole L2; plus what surrounds the main loop and the
+// L2, and no less than all CTAs' blocks take at 14 TB/s out of the whole L2 (7.5 TB/s when the operands do not stay in it:
+// 2560 x 512, K 50304 on 80 CTAs took 273 us against 224 us on wide tiles), 1.3 times as long when the rows of a K-major
+// operand do not start on 128-byte lines (2436 x 512, K 1384: 16.4 us, wide tiles 14.5); plus what surrounds the main loop and the
 // exchange of the partial tiles. A weight gradient has to win clearly: the wide tiles add to C with whole TMA boxes.
 SplitPlan split_plan(const SplitGemm& g, double wide_us) {
   SplitPlan best{0, 0};
   if (g.N % 8 != 0 || g.ldc % 8 != 0 || (reinterpret_cast<uintptr_t>(g.C) & 15)) return best;
   const long long kblocks = (g.K + SP_BK - 1) / SP_BK, slots = 2LL * num_sms();
+  const double operand_bytes = 2.0 * g.K * ((double)g.M + (g.epi == SPLIT_SWIGLU ? 2.0 : 1.0) * g.N);
+  const double lines = (!g.a_mn && g.lda % 64 != 0) || (!g.b_mn && g.ldb % 64 != 0) ? 1.3 : 1.0;
+  const double l2_rate = operand_bytes > 64e6 ? 7.5e6 : 14e6;          // bytes per us
   static const double exchange[2][4] = {{0.0, 1.5, 1.3, 2.8}, {0.0, 2.2, 2.0, 2.3}};       // S = 1, 2, 4, 8
-  double best_us = g.epi == SPLIT_F32_ACC ? 0.85 * wide_us : wide_us;
+  double best_us = (g.epi == SPLIT_F32_ACC ? 0.85 : 0.95) * wide_us;
   for (int bn = 64; bn <= 128; bn *= 2) {
     if (g.epi == SPLIT_HEADS && (g.hd > bn || bn % g.hd != 0)) continue;
     const int tile_n = g.epi == SPLIT_SWIGLU ? bn / 2 : bn;
@@ -335,9 +340,9 @@ SplitPlan split_plan(const SplitGemm& g, double wide_us) {
     for (int i = 0, s = 1; s <= 8 && s <= kblocks; ++i, s *= 2) {
       const long long ctas = tiles * s, resident = ctas < slots ? ctas : slots;
       if (ctas > (s > 1 ? num_sms() : slots)) continue;          // a second wave of clusters costs more than it saves
-      const double alone = bn == 64 ? 0.24 : 0.27, shared = (double)resident * (bn == 64 ? 24576.0 : 32768.0) / 14e6;
+      const double alone = bn == 64 ? 0.24 : 0.27, shared = (double)resident * (bn == 64 ? 24576.0 : 32768.0) / l2_rate;
       const double us = (bn == 64 ? 3.4 : 3.8) + (g.a_mn ? 1.0 : 0.0) + exchange[bn / 128][i] +
-                        (double)((kblocks + s - 1) / s) * (alone > shared ? alone : shared);
+                        (double)((kblocks + s - 1) / s) * lines * (alone > shared ? alone : shared);
       if (us < best_us) { best_us = us; best = {bn, s}; }
     }
   }
