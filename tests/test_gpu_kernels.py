@@ -215,7 +215,8 @@ def test_gemm_heads_any_number_of_rows(nat, mode, hd, Hq, Hkv, B, T, K):
     ref = (x.double() @ w.double().t()).view(B, T, Ht, hd)
     ref[:, :, :Hq + Hkv] = oracle.rope(ref[:, :, :Hq + Hkv], cos.double(), sin.double())
     got = out[:B * T * Ht * hd].view(B, T, Ht, hd).double()
-    assert ((got - ref).norm() / ref.norm()).item() < 2.5e-3 and bool((out[B * T * Ht * hd:] == 7.0).all())
+    # one bf16 rounding is 1.7e-3 rms; head dim 128 rounds before and after the rotation: sqrt(2) * 1.7e-3 = 2.4e-3
+    assert ((got - ref).norm() / ref.norm()).item() < (3e-3 if hd == 128 else 2.5e-3) and bool((out[B * T * Ht * hd:] == 7.0).all())
 
 
 @pytest.mark.parametrize("mode", [0, 1, 2])

@@ -5,7 +5,7 @@
 // so the QKV projection's dgrad/wgrad GEMMs consume one tensor.
 //
 // Three launches:
-//   1. delta[b,h,t] = sum_d do*o; the dQ accumulator is zeroed on the way
+//   1. delta[b,h,t] = sum_d do*o; the dQ accumulator is zeroed on the way (few rows: by a memset)
 //   2. main kernel: one CTA per (128-row KV tile, batch, KV head). K and V stay in
 //      shared memory; the CTA walks over every query head of the group and every
 //      query tile at or below the diagonal. Per step five MMAs run on the
@@ -46,7 +46,7 @@ struct AttnBwdDst {
 
 struct AttnBwdParams {
   __nv_bfloat16* dqkv;
-  float* dq_acc;            // [B,Hq,T,hd] fp32, zeroed by the delta kernel
+  float* dq_acc;            // [B,Hq,T,hd] fp32, zeroed before the main kernel
   const float* lse;
   const float* delta;
   int B, T, Hq, Hkv;
@@ -120,7 +120,7 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
   const long long base = ((long long)b * T + t0) * Hq * hd;
   // this slab of the dQ accumulator starts at zero: stores that nothing waits for, beside the loads of the row sums
   const int vec_h = nt * hd / 4;                           // float4 of one head: its nt rows are contiguous
-  for (int h = 0; h < Hq; ++h) {
+  for (int h = 0; dq_acc != nullptr && h < Hq; ++h) {
     float4* z = reinterpret_cast<float4*>(dq_acc + (((long long)b * Hq + h) * T + t0) * hd);
     for (int i = threadIdx.x; i < vec_h; i += DELTA_THREADS) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
@@ -795,8 +795,15 @@ static int attn_bwd_impl(const void* qkv, const void* o, const void* dout, const
   if (hd != 32 && hd != 64 && hd != 128) return -4;
   if (Hq % Hkv != 0) return -5;
   if ((size_t)Hq * (DELTA_T + 1) * 4 > 48 * 1024) return -6;
-  int le = launch_overlapped(attn_delta_kernel, dim3(B * ((T + DELTA_T - 1) / DELTA_T)), dim3(DELTA_THREADS), (size_t)Hq * (DELTA_T + 1) * 4, st, 1,
-      (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, dq_acc, B, T, Hq, hd);
+  // Few blocks would take longer over the zeroes than a memset (48 heads of 64, 16 rows: one block, 3 us more)
+  const int delta_blocks = B * ((T + DELTA_T - 1) / DELTA_T);
+  const bool fused_zero = delta_blocks >= num_sms();
+  if (!fused_zero) {
+    const cudaError_t ce = cudaMemsetAsync(dq_acc, 0, (size_t)B * T * Hq * hd * 4, st);
+    if (ce != cudaSuccess) return (int)ce;
+  }
+  int le = launch_overlapped(attn_delta_kernel, dim3(delta_blocks), dim3(DELTA_THREADS), (size_t)Hq * (DELTA_T + 1) * 4, st, 1,
+      (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, fused_zero ? dq_acc : nullptr, B, T, Hq, hd);
   if (le) return le;
   CUtensorMap mq, mdo;
   const int box_cols = hd == 32 && n_dst == 0 ? 32 : 64;
