@@ -245,3 +245,22 @@ def test_attention_dropout_trains_and_is_off_in_eval():
             plain.eval()
             _, loss_pe, _ = plain(idx, tgt)
         assert abs(float(loss_e) - float(loss_pe)) < 1e-6
+
+
+def test_shapes_of_the_fused_paths():
+    """Which calls take the fused projection and SwiGLU kernels, and that a model on the CPU never takes the one-call forward."""
+    from train_large_model_from_scratch_b200.models import GPT
+    from train_large_model_from_scratch_b200.ops import native
+    from train_large_model_from_scratch_b200.training.config import ModelConfig
+    for hd in (32, 64, 128):
+        assert all(native.heads_epilogue_ok(hd, rows) for rows in (1, 31, 32, 1001, 4096))      # one destination: any rows
+    assert native.heads_epilogue_ok(64, 64, 2) and not native.heads_epilogue_ok(64, 33, 2) and not native.heads_epilogue_ok(32, 64, 2)
+    assert not native.heads_epilogue_ok(48, 64) and not native.heads_epilogue_ok(64, 64, 9)
+    assert native.swiglu_epilogue_ok(2056) and native.swiglu_epilogue_ok(8) and not native.swiglu_epilogue_ok(2052)
+    assert not native.grouped_swiglu_ok(2056)                                                   # experts keep whole 128-column tiles
+    model = GPT(ModelConfig(num_layer=1, hidden_size=64, num_attention_heads=1, num_key_value_heads=1, intermediate_size=64,
+                            vocab_size=64, block_size=32), device="cpu").eval()
+    ids = torch.arange(8)[None]
+    with torch.no_grad():
+        assert not model._one_call_ok(model.wte(ids), 8)
+        assert model(ids)[0].shape == (1, 8, 64)
