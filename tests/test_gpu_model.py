@@ -65,6 +65,23 @@ def test_blocks_issued_in_one_call_equal_the_per_op_path(T, over):
     assert logits_grad.requires_grad and torch.equal(logits, logits_grad.detach())
 
 
+def test_strided_weights_stay_on_the_per_op_path():
+    """A projection whose weight is a slice of a wider tensor: the per-op kernels take its row pitch, the one call does not."""
+    from train_large_model_from_scratch_b200.ops import native
+    model = _build("cuda", torch.bfloat16).eval()
+    x = torch.randint(0, 4096, (2, 64), generator=torch.Generator().manual_seed(4)).cuda()
+    with torch.no_grad():
+        ref, _, _ = model(x)
+        w = model.blocks[1].attn.c_proj.weight
+        wide = torch.zeros(w.shape[0], w.shape[1] + 64, dtype=w.dtype, device="cuda")
+        wide[:, :w.shape[1]] = w
+        model.blocks[1].attn.c_proj.weight = torch.nn.Parameter(wide[:, :w.shape[1]])
+        assert not model._one_call_ok(model.wte(x), 64)
+        got, _, _ = model(x)
+    native.raise_on_device_status()
+    assert torch.equal(got, ref)
+
+
 def test_training_reduces_loss_on_fixed_batch():
     from train_large_model_from_scratch_b200.parallel.zero1.distributed_optimizer import FusedAdamW
     model = _build("cuda", torch.bfloat16)

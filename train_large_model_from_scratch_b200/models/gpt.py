@@ -202,7 +202,12 @@ class GPT(nn.Module):
                 or parallel_state.get_sep_world_size() > 1
                 or nn_module._global_forward_hooks or nn_module._global_forward_pre_hooks):
             return False
-        first = self.blocks[0]
+        def form(block):                       # what the one call takes from the first block
+            attn = block.attn
+            return (attn.num_attention_heads, attn.num_key_value_heads, attn.head_dim, block.mlp._gate_up_weight.shape,
+                    attn.config.rope_theta, attn.config.rope_variant, block.ln_1.variance_epsilon)
+
+        first = None
         for block in self.blocks:
             if type(block) is not Block or type(block.attn) is not Attention or type(block.mlp) is not MLP:
                 return False
@@ -213,9 +218,14 @@ class GPT(nn.Module):
             for m in (block, attn, mlp, block.ln_1, block.ln_2):
                 if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
                     return False
-            for n in (block.ln_1, block.ln_2):
-                if type(n) is not LayerNorm or n.weight.dtype != torch.bfloat16 or n.variance_epsilon != first.ln_1.variance_epsilon:
+            if type(block.ln_1) is not LayerNorm or type(block.ln_2) is not LayerNorm or block.ln_1.variance_epsilon != block.ln_2.variance_epsilon:
+                return False
+            for w in (block.ln_1.weight, attn._qkv_weight, attn.c_proj.weight, block.ln_2.weight, mlp._gate_up_weight, mlp.down_proj.weight):
+                if w.dtype != torch.bfloat16 or not w.is_contiguous():
                     return False
+            first = first if first is not None else form(block)
+            if form(block) != first:
+                return False
         return True
 
     def _blocks_forward(self, x: torch.Tensor, B: int, T: int):
