@@ -148,3 +148,27 @@ def test_backward_at_the_edges_of_tiles_and_splits(hd, B, T, Hq, Hkv):
         # a single position attends to itself alone: dS is exactly zero up to rounding of dP - delta
         bound = 1e-2 * b.norm().item() if T > 1 or name == "dv" else 1e-2 * do.double().norm().item()
         assert (a - b).norm().item() < bound, (name, (a - b).norm().item(), b.norm().item())
+
+
+@pytest.mark.parametrize("hd", [32, 64, 128])
+@pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 130, 2, 1), (2, 257, 3, 3), (1, 1001, 6, 2)])
+def test_backward_with_any_split_of_a_tile(hd, B, T, Hq, Hkv, monkeypatch):
+    """1, 2, 4 and 8 CTAs per KV tile, set by hand instead of by the rule (which looks at the chip's SM count): the last tile's
+    rows end inside a CTA's share and inside a warp, with 8 CTAs some have no step. Bounds as in the test above."""
+    from train_large_model_from_scratch_b200.ops import native
+    g = torch.Generator(device="cuda").manual_seed(11)
+    qkv = torch.randn(B, T, Hq + 2 * Hkv, hd, device="cuda", generator=g).to(torch.bfloat16)
+    do = torch.randn(B, T, Hq, hd, device="cuda", generator=g).to(torch.bfloat16)
+    o, lse = native.flash_attn_fwd(qkv, Hq, Hkv, True)
+    x = qkv.double().requires_grad_()
+    q = x[:, :, :Hq].permute(0, 2, 1, 3)
+    k, v = (x[:, :, a:a + Hkv].permute(0, 2, 1, 3).repeat_interleave(Hq // Hkv, 1) for a in (Hq, Hq + Hkv))
+    s = (q @ k.transpose(-1, -2) / math.sqrt(hd)).masked_fill(torch.ones(T, T, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    (torch.softmax(s, -1) @ v).permute(0, 2, 1, 3).backward(do.double())
+    for split in (1, 2, 4, 8):
+        monkeypatch.setenv("TLM_ATTN_BWD_SPLIT", str(split))
+        dqkv = native.flash_attn_bwd(do, qkv, o, lse, Hq, Hkv, True)
+        native.raise_on_device_status()
+        for name, sl in (("dq", slice(0, Hq)), ("dk", slice(Hq, Hq + Hkv)), ("dv", slice(Hq + Hkv, None))):
+            a, b = dqkv[:, :, sl].double(), x.grad[:, :, sl]
+            assert ((a - b).norm() / b.norm()).item() < 1e-2, (split, name)

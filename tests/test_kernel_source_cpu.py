@@ -1,0 +1,36 @@
+"""Rules of the CUDA sources that no test on a GPU can show to be broken: what a compiler happens to do right today."""
+import glob
+import os
+import re
+
+import train_large_model_from_scratch_b200 as pkg
+
+SRC = os.path.join(os.path.dirname(pkg.__file__), "csrc")
+
+
+def _source(name):
+    with open(os.path.join(SRC, name)) as f:
+        return f.read()
+
+
+def _body(text, start):
+    """The braced block that opens at or after `start`."""
+    i = text.index("{", start)
+    depth, j = 0, i
+    while True:
+        depth += {"{": 1, "}": -1}.get(text[j], 0)
+        j += 1
+        if depth == 0:
+            return text[i:j]
+
+
+def test_cluster_barriers_join_their_warp_first():
+    """`barrier.cluster.*.aligned` needs all lanes of a warp at the instruction; callers leave loops lane by lane (the rows of
+    a sequence's last tile), so the one helper that issues it joins the warp itself, and nobody issues it elsewhere."""
+    common = _source("common.cuh")
+    body = _body(common, common.index("void cluster_sync_all()"))
+    assert body.index("__syncwarp();") < body.index("barrier.cluster.arrive")
+    for path in glob.glob(os.path.join(SRC, "*.cu*")):
+        text = _source(os.path.basename(path))
+        n = len(re.findall(r"barrier\.cluster\.arrive", text))
+        assert n == (1 if path.endswith("common.cuh") else 0), path

@@ -395,7 +395,10 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+// Every thread of the cluster. The `.aligned` form needs a whole warp at the instruction together, and callers come out of
+// loops whose lanes leave at different turns, so the warp is joined here.
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // shared::cluster address of the same shared-memory offset in CTA `rank` of this cluster
