@@ -34,3 +34,22 @@ def test_cluster_barriers_join_their_warp_first():
         text = _source(os.path.basename(path))
         n = len(re.findall(r"barrier\.cluster\.arrive", text))
         assert n == (1 if path.endswith("common.cuh") else 0), path
+
+
+def test_kernels_that_start_early_read_through_plain_loads():
+    """A kernel that calls `griddep_wait` lives from before the kernel in front of it has finished writing. The read-only load
+    path (`__ldg`, or what the compiler may make of a `const ... __restrict__` argument) is for memory that nothing writes in a
+    kernel's whole life, and a compiler need not keep such loads behind the wait."""
+    waiting = 0
+    for path in glob.glob(os.path.join(SRC, "*.cu")):
+        text = _source(os.path.basename(path))
+        for m in re.finditer(r"__global__", text):
+            signature, body = text[m.start():text.index("{", m.start())], _body(text, m.start())
+            if "griddep_wait();" in body:
+                waiting += 1
+                assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", signature), signature
+                assert "__ldg" not in body and "ld.global.nc" not in body, signature
+    assert waiting >= 8
+    gemm = _source("gemm.cu")                              # its kernels share one body
+    body = _body(gemm, gemm.index("void gemm_body("))
+    assert "griddep_wait();" in body and "__ldg" not in body and "ld.global.nc" not in body

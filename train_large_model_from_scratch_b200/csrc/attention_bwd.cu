@@ -107,7 +107,7 @@ struct AttnBwdCfg {
 constexpr int DELTA_T = 32, DELTA_THREADS = 256;
 
 __global__ void __launch_bounds__(DELTA_THREADS)
-attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
+attn_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* dout,
                   float* __restrict__ delta, float* __restrict__ dq_acc, int B, int T, int Hq, int hd) {
   griddep_wait();
   extern __shared__ float delta_s[];                       // [Hq][DELTA_T + 1]
@@ -162,9 +162,9 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
 // rotated in place by further work items (heads Hq .. Hq + Hkv - 1).
 // Index: 32 bits while the items fit (three 64-bit divisions per item took longer than the item's 64 bytes).
 template <typename Index>
-__global__ void attn_dq_convert_kernel(const float* __restrict__ dq_acc, __nv_bfloat16* __restrict__ dqkv, int B, int T,
-                                       int Hq, int heads_total, int hd, float scale, const float* __restrict__ cosT,
-                                       const float* __restrict__ sinT, const AttnBwdDst d, int dst_q0, int rot_k) {
+__global__ void attn_dq_convert_kernel(const float* dq_acc, __nv_bfloat16* __restrict__ dqkv, int B, int T,
+                                       int Hq, int heads_total, int hd, float scale, const float* cosT,
+                                       const float* sinT, const AttnBwdDst d, int dst_q0, int rot_k) {
   griddep_wait();
   const int half = hd / 2, vec_log = hd == 32 ? 1 : hd == 64 ? 2 : 3;          // hd / 16 items per row
   const int heads = Hq + rot_k;

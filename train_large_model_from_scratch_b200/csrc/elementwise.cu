@@ -91,8 +91,8 @@ __global__ void add_rmsnorm_fwd_kernel(const float* __restrict__ x, const __nv_b
 // row before the first use, so one warp keeps NV * 3 sixteen-byte loads in flight; no shared memory.
 template <int NV>
 __global__ void __launch_bounds__(256)
-add_rmsnorm_fwd_reg_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
-                           const __nv_bfloat16* __restrict__ w, float* __restrict__ x_new,
+add_rmsnorm_fwd_reg_kernel(const float* x, const __nv_bfloat16* delta,
+                           const __nv_bfloat16* w, float* __restrict__ x_new,
                            __nv_bfloat16* __restrict__ h, float* __restrict__ rstd_out, int rows, float eps) {
   griddep_wait();
   constexpr int D = NV * 256;
@@ -157,8 +157,8 @@ __device__ __forceinline__ float rms_block_sum(float v, float* red, int warps, i
 
 template <int NV>
 __global__ void __launch_bounds__(RMS_WIDE_MAX_WARPS * 32)
-add_rmsnorm_fwd_wide_kernel(const float* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
-                            const __nv_bfloat16* __restrict__ w, float* __restrict__ x_new,
+add_rmsnorm_fwd_wide_kernel(const float* x, const __nv_bfloat16* delta,
+                            const __nv_bfloat16* w, float* __restrict__ x_new,
                             __nv_bfloat16* __restrict__ h, float* __restrict__ rstd_out, int rows, int D, float eps) {
   griddep_wait();
   __shared__ float red[2][RMS_WIDE_MAX_WARPS];
@@ -279,9 +279,9 @@ __global__ void add_rmsnorm_bwd_kernel(const float* __restrict__ g_xnew, const _
 // global memory, no shared-memory traffic in the row loop.
 template <int NV>
 __global__ void __launch_bounds__(256, 2)
-add_rmsnorm_bwd_reg_kernel(const float* __restrict__ g_xnew, const __nv_bfloat16* __restrict__ g_h,
-                           const float* __restrict__ x_new, const float* __restrict__ rstd_in,
-                           const __nv_bfloat16* __restrict__ w, float* __restrict__ g_x,
+add_rmsnorm_bwd_reg_kernel(const float* g_xnew, const __nv_bfloat16* g_h,
+                           const float* x_new, const float* rstd_in,
+                           const __nv_bfloat16* w, float* __restrict__ g_x,
                            __nv_bfloat16* __restrict__ g_delta, float* __restrict__ dw_out, int rows) {
   griddep_wait();
   constexpr int D = NV * 256;
@@ -352,9 +352,9 @@ add_rmsnorm_bwd_reg_kernel(const float* __restrict__ g_xnew, const __nv_bfloat16
 // the dweight partial sums stay in registers over all rows of the block and leave with one vector reduction per 4 columns.
 template <int NV>
 __global__ void __launch_bounds__(RMS_WIDE_MAX_WARPS * 32)
-add_rmsnorm_bwd_wide_kernel(const float* __restrict__ g_xnew, const __nv_bfloat16* __restrict__ g_h,
-                            const float* __restrict__ x_new, const float* __restrict__ rstd_in,
-                            const __nv_bfloat16* __restrict__ w, float* __restrict__ g_x,
+add_rmsnorm_bwd_wide_kernel(const float* g_xnew, const __nv_bfloat16* g_h,
+                            const float* x_new, const float* rstd_in,
+                            const __nv_bfloat16* w, float* __restrict__ g_x,
                             __nv_bfloat16* __restrict__ g_delta, float* __restrict__ dw_out, int rows, int D) {
   griddep_wait();
   __shared__ float red[2][RMS_WIDE_MAX_WARPS];

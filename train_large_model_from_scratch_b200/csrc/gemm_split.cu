@@ -174,91 +174,113 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
   };
   const int half = EPI == SPLIT_HEADS ? g.hd >> 1 : 0;
-  // read-only loads (rotation tables, gate / up) of four items in flight: one after the other, their latency was most of
-  // the epilogue
-#pragma unroll 4
-  for (int i = threadIdx.x; i < ROWS * PER_ROW; i += SP_THREADS) {
-    const int r = rank * ROWS + i / PER_ROW, ch = i % PER_ROW;
-    const long long row = m0 + r;
-    if (row >= g.M) continue;
-    float v[8];
-    if constexpr (EPI == SPLIT_BF16 || EPI == SPLIT_F32_ACC) {
-      const int col = n0 + ch * 8;
-      if (col >= g.N) continue;
-      if constexpr (EPI == SPLIT_BF16) {
+  // What other kernels wrote (rotation tables, gate / up) comes through plain loads: the read-only path may only be used for
+  // memory that nothing writes while this kernel lives, and it lives from before griddep_wait. A plain load does not pass a
+  // store, so the loads of BATCH items are issued before the first of their stores; one after the other, their latency was
+  // most of the epilogue.
+  constexpr int BATCH = EPI == SPLIT_HEADS ? 2 : EPI == SPLIT_SWIGLU_BWD ? 4 : 1;
+  constexpr int ITEMS = ROWS * PER_ROW;
+  float4 pre[EPI == SPLIT_HEADS ? BATCH * 8 : 1];            // per item: cos, sin of the lower, cos, sin of the upper columns
+  uint4 pre_gu[EPI == SPLIT_SWIGLU_BWD ? BATCH * 2 : 1];     // per item: gate, up
+  for (int i0 = threadIdx.x; i0 < ITEMS; i0 += BATCH * SP_THREADS) {
+    if constexpr (BATCH > 1) {
+#pragma unroll
+      for (int u = 0; u < BATCH; ++u) {
+        const int i = i0 + u * SP_THREADS, r = rank * ROWS + i / PER_ROW, ch = i % PER_ROW;
+        const long long row = m0 + r;
+        if (i >= ITEMS || row >= g.M) continue;
+        if constexpr (EPI == SPLIT_HEADS) {
+          const int per_half = half >> 3, hh = ch / per_half, j = (ch - hh * per_half) * 8;
+          if (n0 + hh * g.hd >= g.N || n0 / g.hd + hh >= g.n_rot) continue;
+          const long long at = (long long)(row % g.rows_per_batch) * g.hd + j;
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            pre[u * 8 + k] = *reinterpret_cast<const float4*>(g.cosT + at + 4 * k);
+            pre[u * 8 + 2 + k] = *reinterpret_cast<const float4*>(g.sinT + at + 4 * k);
+            pre[u * 8 + 4 + k] = *reinterpret_cast<const float4*>(g.cosT + at + half + 4 * k);
+            pre[u * 8 + 6 + k] = *reinterpret_cast<const float4*>(g.sinT + at + half + 4 * k);
+          }
+        } else {
+          if (n0 + ch * 8 >= g.N) continue;
+          const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(g.aux) + row * 2 * g.N + n0 + ch * 8;
+          pre_gu[u * 2] = *reinterpret_cast<const uint4*>(gp);
+          pre_gu[u * 2 + 1] = *reinterpret_cast<const uint4*>(gp + g.N);
+        }
+      }
+    }
+#pragma unroll
+    for (int ub = 0; ub < BATCH; ++ub) {
+      const int i = i0 + ub * SP_THREADS, r = rank * ROWS + i / PER_ROW, ch = i % PER_ROW;
+      const long long row = m0 + r;
+      if (i >= ITEMS || row >= g.M) continue;
+      float v[8];
+      if constexpr (EPI == SPLIT_BF16 || EPI == SPLIT_F32_ACC) {
+        const int col = n0 + ch * 8;
+        if (col >= g.N) continue;
+        if constexpr (EPI == SPLIT_BF16) {
+          load8(r, ch * 8, v);
+          *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.C) + row * g.ldc + col) = pack8(v);
+        } else {
+          // one reduction per element: nothing waits for C, and the result does not depend on timing
+          float* out = reinterpret_cast<float*>(g.C) + row * g.ldc + col;
+          load8(r, ch * 8, v);
+          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(out), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(out + 4), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+        }
+      } else if constexpr (EPI == SPLIT_HEADS) {
+        const int per_half = half >> 3;                        // 8-column pieces of half a head
+        const int hh = ch / per_half, j = (ch - hh * per_half) * 8, c = hh * g.hd + j;
+        if (n0 + c >= g.N) continue;                           // N is a multiple of hd
+        const int head = n0 / g.hd + hh;
+        const int bi = (int)(row / g.rows_per_batch), t = (int)(row - (long long)bi * g.rows_per_batch);
+        const bool rot = head < g.n_rot;
+        float u[8];
+        load8(r, c, v);
+        load8(r, c + half, u);
+        if (rot) {
+          const float *cl = reinterpret_cast<const float*>(pre + ub * 8), *sl = cl + 8, *chh = cl + 16, *sh = cl + 24;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const float a = v[k], b = u[k];
+            v[k] = a * cl[k] - b * sl[k];
+            u[k] = b * chh[k] + a * sh[k];
+          }
+        }
+        __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(g.C) + (((long long)bi * g.dst_rows + g.row_off + t) * g.dst_heads + head) * g.hd + j;
+        *reinterpret_cast<uint4*>(out) = pack8(v);
+        *reinterpret_cast<uint4*>(out + half) = pack8(u);
+      } else if constexpr (EPI == SPLIT_SWIGLU) {
+        const int col = n0 + ch * 8;
+        if (col >= g.N) continue;
+        float u[8];
         load8(r, ch * 8, v);
-        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.C) + row * g.ldc + col) = pack8(v);
+        load8(r, BN / 2 + ch * 8, u);
+        // as in gemm.cu: the products are rounded to bf16 first, so the numbers equal those of separate kernels
+        const uint4 gp = pack8(v), up = pack8(u);
+        const uint32_t gw[4] = {gp.x, gp.y, gp.z, gp.w}, uw[4] = {up.x, up.y, up.z, up.w};
+        uint32_t o[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) o[k] = swiglu2(gw[k], uw[k]);
+        if (g.C != nullptr) {
+          __nv_bfloat16* gu = reinterpret_cast<__nv_bfloat16*>(g.C) + row * g.ldc + col;
+          *reinterpret_cast<uint4*>(gu) = gp;
+          *reinterpret_cast<uint4*>(gu + g.N) = up;
+        }
+        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.act) + row * g.N + col) = make_uint4(o[0], o[1], o[2], o[3]);
       } else {
-        // one reduction per element: nothing waits for C, and the result does not depend on timing
-        float* out = reinterpret_cast<float*>(g.C) + row * g.ldc + col;
+        const int col = n0 + ch * 8;
+        if (col >= g.N) continue;
+        const uint4 gv = pre_gu[ub * 2], uv = pre_gu[ub * 2 + 1];
         load8(r, ch * 8, v);
-        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(out), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
-        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(out + 4), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
-      }
-    } else if constexpr (EPI == SPLIT_HEADS) {
-      const int per_half = half >> 3;                        // 8-column pieces of half a head
-      const int hh = ch / per_half, j = (ch - hh * per_half) * 8, c = hh * g.hd + j;
-      if (n0 + c >= g.N) continue;                           // N is a multiple of hd
-      const int head = n0 / g.hd + hh;
-      const int bi = (int)(row / g.rows_per_batch), t = (int)(row - (long long)bi * g.rows_per_batch);
-      const bool rot = head < g.n_rot;
-      float cl[8], sl[8], chh[8], sh[8], u[8];
-      if (rot) {
-        const float* cp = g.cosT + (long long)t * g.hd + j;
-        const float* sp = g.sinT + (long long)t * g.hd + j;
+        const uint4 dv = pack8(v);
+        const uint32_t dw[4] = {dv.x, dv.y, dv.z, dv.w}, gw[4] = {gv.x, gv.y, gv.z, gv.w}, uw[4] = {uv.x, uv.y, uv.z, uv.w};
+        uint32_t og[4], ou[4];
 #pragma unroll
-        for (int k = 0; k < 8; k += 4) {
-          *reinterpret_cast<float4*>(cl + k) = __ldg(reinterpret_cast<const float4*>(cp + k));
-          *reinterpret_cast<float4*>(sl + k) = __ldg(reinterpret_cast<const float4*>(sp + k));
-          *reinterpret_cast<float4*>(chh + k) = __ldg(reinterpret_cast<const float4*>(cp + half + k));
-          *reinterpret_cast<float4*>(sh + k) = __ldg(reinterpret_cast<const float4*>(sp + half + k));
-        }
+        for (int k = 0; k < 4; ++k) swiglu_bwd2(dw[k], gw[k], uw[k], og[k], ou[k]);
+        __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(g.C) + row * g.ldc + col;
+        *reinterpret_cast<uint4*>(out) = make_uint4(og[0], og[1], og[2], og[3]);
+        *reinterpret_cast<uint4*>(out + g.N) = make_uint4(ou[0], ou[1], ou[2], ou[3]);
       }
-      load8(r, c, v);
-      load8(r, c + half, u);
-      if (rot) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float a = v[k], b = u[k];
-          v[k] = a * cl[k] - b * sl[k];
-          u[k] = b * chh[k] + a * sh[k];
-        }
-      }
-      __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(g.C) + (((long long)bi * g.dst_rows + g.row_off + t) * g.dst_heads + head) * g.hd + j;
-      *reinterpret_cast<uint4*>(out) = pack8(v);
-      *reinterpret_cast<uint4*>(out + half) = pack8(u);
-    } else if constexpr (EPI == SPLIT_SWIGLU) {
-      const int col = n0 + ch * 8;
-      if (col >= g.N) continue;
-      float u[8];
-      load8(r, ch * 8, v);
-      load8(r, BN / 2 + ch * 8, u);
-      // as in gemm.cu: the products are rounded to bf16 first, so the numbers equal those of separate kernels
-      const uint4 gp = pack8(v), up = pack8(u);
-      const uint32_t gw[4] = {gp.x, gp.y, gp.z, gp.w}, uw[4] = {up.x, up.y, up.z, up.w};
-      uint32_t o[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) o[k] = swiglu2(gw[k], uw[k]);
-      if (g.C != nullptr) {
-        __nv_bfloat16* gu = reinterpret_cast<__nv_bfloat16*>(g.C) + row * g.ldc + col;
-        *reinterpret_cast<uint4*>(gu) = gp;
-        *reinterpret_cast<uint4*>(gu + g.N) = up;
-      }
-      *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.act) + row * g.N + col) = make_uint4(o[0], o[1], o[2], o[3]);
-    } else {
-      const int col = n0 + ch * 8;
-      if (col >= g.N) continue;
-      const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(g.aux) + row * 2 * g.N + col;
-      const uint4 gv = __ldg(reinterpret_cast<const uint4*>(gp)), uv = __ldg(reinterpret_cast<const uint4*>(gp + g.N));
-      load8(r, ch * 8, v);
-      const uint4 dv = pack8(v);
-      const uint32_t dw[4] = {dv.x, dv.y, dv.z, dv.w}, gw[4] = {gv.x, gv.y, gv.z, gv.w}, uw[4] = {uv.x, uv.y, uv.z, uv.w};
-      uint32_t og[4], ou[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) swiglu_bwd2(dw[k], gw[k], uw[k], og[k], ou[k]);
-      __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(g.C) + row * g.ldc + col;
-      *reinterpret_cast<uint4*>(out) = make_uint4(og[0], og[1], og[2], og[3]);
-      *reinterpret_cast<uint4*>(out + g.N) = make_uint4(ou[0], ou[1], ou[2], ou[3]);
     }
   }
 
