@@ -219,6 +219,42 @@ def test_gemm_heads_any_number_of_rows(nat, mode, hd, Hq, Hkv, B, T, K):
     assert ((got - ref).norm() / ref.norm()).item() < (3e-3 if hd == 128 else 2.5e-3) and bool((out[B * T * Ht * hd:] == 7.0).all())
 
 
+@pytest.mark.parametrize("hd,T", [(64, 64), (64, 33), (128, 96), (128, 33), (32, 50)])
+def test_rotation_tables_that_start_anywhere(nat, hd, T):
+    """The fused projection reads the fp32 tables in 16-byte pieces. Tables that are views into a longer buffer at an odd
+    offset give the same results, forward and backward; the kernel's own entry point falls back to the fp16 table where
+    that can do, and refuses otherwise."""
+    import ctypes
+    from train_large_model_from_scratch_b200.ops import functional as F_ops, oracle
+    B, Hq, Hkv, K = 2, 4, 2, 128
+    Ht = Hq + 2 * Hkv
+    x, w = _rand(B * T, K, seed=90), _rand(Ht * hd, K, scale=0.05, seed=91)
+    cos, sin = (t.contiguous() for t in oracle.rope_tables(torch.arange(T, device="cuda"), hd, 10000.0, "reference"))
+    cs = nat.rope_table_fp16(cos, sin)
+    odd = [torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view(T, hd) for t in (cos, sin)]
+    assert all(t.is_contiguous() and t.data_ptr() % 16 == 4 for t in odd)
+    outs = []
+    for c, s in ((cos, sin), odd):
+        h = x.clone().requires_grad_()
+        w.main_grad = torch.zeros(w.shape, device="cuda")
+        o = F_ops.qkv_attention(h, w, c, s, cs, B, T, Hq, Hkv, hd)
+        o.backward(torch.ones_like(o))
+        outs.append((o.detach(), h.grad, w.main_grad))
+    nat.raise_on_device_status()
+    assert torch.equal(outs[0][0], outs[1][0])
+    assert _rel_err(outs[1][1], outs[0][1]) < 5e-3 and _rel_err(outs[1][2], outs[0][2]) < 5e-3      # dQ: fp32 adds in any order
+    out = torch.empty(B, T, Ht, hd, dtype=torch.bfloat16, device="cuda")
+    args = (x, w, False, (ctypes.c_void_p * 1)(out.data_ptr()), 1, B, T, T, Ht, 0, Hq, Hkv, Hq, Hkv, hd, Hq + Hkv, cs)
+    if T % 32:
+        with pytest.raises(nat.NativeError):
+            nat.gemm_heads(*args, tables=tuple(odd))
+    else:
+        nat.gemm_heads(*args, tables=tuple(odd))
+        ref = (x.float() @ w.float().t()).view(B, T, Ht, hd)
+        ref[:, :, :Hq + Hkv] = oracle.rope(ref[:, :, :Hq + Hkv], cos, sin)
+        assert _rel_err(out, ref) < 6e-3
+
+
 @pytest.mark.parametrize("mode", [0, 1, 2])
 @pytest.mark.parametrize("M,I,K", [(1, 8, 64), (333, 200, 192), (130, 2056, 768), (3003, 2056, 256), (256, 136, 4096)])
 def test_swiglu_epilogues_of_any_width(nat, mode, M, I, K):

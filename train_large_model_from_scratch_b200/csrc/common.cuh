@@ -55,6 +55,8 @@ inline int launch_overlapped(void (*kern)(P...), dim3 grid, dim3 block, size_t s
 }
 #endif
 
+inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 inline int launch_status() {
   cudaError_t e = cudaPeekAtLastError();
   return (int)e;

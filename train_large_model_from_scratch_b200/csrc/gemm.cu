@@ -1340,14 +1340,16 @@ TLM_API int tlm_rope(void* qkv, const float* cosT, const float* sinT, long long 
 //   addresses are fine: the stores are TMA tile stores without multicast);  cs: fp16 (cos, sin) pairs
 //   [rows_per_batch, hd, 2] for the heads below n_rot.
 // Requirements: hd in {32, 64, 128}, n_dst <= 8, Hq % q_l == 0, Hkv % kv_l == 0; rows_per_batch % 32 == 0 unless there is
-// one destination, x W^T and, for rotated heads, the fp32 tables cosT / sinT [rows_per_batch, hd] (used then instead of cs).
+// one destination, x W^T and, for rotated heads, the fp32 tables cosT / sinT [rows_per_batch, hd], 16-byte aligned (used then
+// instead of cs).
 TLM_API int tlm_gemm_heads(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, int b_mn,
                            void* const* dst_ptrs, int n_dst, int batch, int rows_per_batch, int dst_rows, int dst_heads,
                            int row_off, int Hq, int Hkv, int q_l, int kv_l, int hd, int n_rot, const void* cs,
                            int kv_rep, const float* cosT, const float* sinT, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((hd != 32 && hd != 64 && hd != 128) || n_dst < 1 || n_dst > MAX_HEAD_DST) return -4;
-  const bool f32_tables = n_rot == 0 || (cosT != nullptr && sinT != nullptr);
+  // read in 16-byte pieces: tables that do not start on one count as absent (cs is enough where rows_per_batch % 32 == 0)
+  const bool f32_tables = n_rot == 0 || (cosT != nullptr && sinT != nullptr && aligned16(cosT) && aligned16(sinT));
   const bool any_rows = rows_per_batch % 32 != 0;
   if (any_rows && (n_dst != 1 || b_mn || !f32_tables)) return -4;
   if (M != batch * rows_per_batch || N != (Hq + 2 * Hkv) * hd || q_l <= 0 || Hq % q_l != 0) return -5;

@@ -224,9 +224,16 @@ class _QKVAttention(torch.autograd.Function):
         return dh, None, None, None, None, None, None, None, None, None
 
 
+def _table(t: torch.Tensor) -> torch.Tensor:
+    """A rotation table as the kernels read it, in 16-byte pieces: contiguous and 16-byte aligned (a view of one long
+    position table may be neither)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def qkv_attention(h, weight, cos, sin, cs, B: int, T: int, n_q: int, n_kv: int, hd: int) -> torch.Tensor:
     """CUDA only (same conditions as `qkv_project`): projection + RoPE + causal attention -> `[B, T, n_q, hd]`."""
-    return _QKVAttention.apply(h, weight, cos.contiguous(), sin.contiguous(), cs, B, T, n_q, n_kv, hd)
+    return _QKVAttention.apply(h, weight, _table(cos), _table(sin), cs, B, T, n_q, n_kv, hd)
 
 
 def qkv_project_fused_ok(h: torch.Tensor, weight: torch.Tensor | None, hd: int, T: int) -> bool:
@@ -235,7 +242,7 @@ def qkv_project_fused_ok(h: torch.Tensor, weight: torch.Tensor | None, hd: int, 
 
 def qkv_project(h, weight, cos, sin, cs, B: int, T: int, n_q: int, n_kv: int, hd: int) -> torch.Tensor:
     """CUDA only (check `qkv_project_fused_ok` first). `cs` = `native.rope_table_fp16(cos, sin)`."""
-    return _QKVProject.apply(h, weight, cos.contiguous(), sin.contiguous(), cs, B, T, n_q, n_kv, hd)
+    return _QKVProject.apply(h, weight, _table(cos), _table(sin), cs, B, T, n_q, n_kv, hd)
 
 
 # --------------------------------------------------------------------------- attention
