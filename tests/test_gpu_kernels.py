@@ -255,6 +255,38 @@ def test_rotation_tables_that_start_anywhere(nat, hd, T):
         assert _rel_err(out, ref) < 6e-3
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+def test_gemm_heads_clips_rows_and_heads_past_the_destination(nat, mode):
+    """A destination with fewer rows per entry, or fewer heads, than the product has: what does not fit is dropped (the TMA
+    stores clip it), also where the product is small enough for the small tiles, whose own stores would not. Where rows
+    are stored one by one (entries that are no multiple of 32 rows) such a call is refused."""
+    import ctypes
+    from train_large_model_from_scratch_b200.ops import oracle
+    B, T, Hq, Hkv, hd, K = 2, 64, 4, 2, 64, 128
+    Ht = Hq + 2 * Hkv
+    x, w = _rand(B * T, K, seed=92), _rand(Ht * hd, K, scale=0.05, seed=93)
+    cos, sin = (t.contiguous() for t in oracle.rope_tables(torch.arange(T, device="cuda"), hd, 10000.0, "reference"))
+    ref = (x.float() @ w.float().t()).view(B, T, Ht, hd)
+    ref[:, :, :Hq + Hkv] = oracle.rope(ref[:, :, :Hq + Hkv], cos, sin)
+    was = nat.set_gemm_pairs(mode)
+    try:
+        for rows, heads, off in ((40, Ht, 0), (T, Ht - 2, 0), (80, Ht, 32)):
+            buf = torch.full((B * rows * heads + 4096, hd), 7.0, dtype=torch.bfloat16, device="cuda")
+            dst = (ctypes.c_void_p * 1)(buf.data_ptr())
+            nat.gemm_heads(x, w, False, dst, 1, B, T, rows, heads, off, Hq, Hkv, Hq, Hkv, hd, Hq + Hkv,
+                           nat.rope_table_fp16(cos, sin), tables=(cos, sin))
+            nat.raise_on_device_status()
+            got, n = buf[:B * rows * heads].view(B, rows, heads, hd), min(T, rows - off)
+            assert _rel_err(got[:, off:off + n], ref[:, :n, :heads]) < 6e-3
+            assert bool((got[:, :off] == 7.0).all()) and bool((buf[B * rows * heads:] == 7.0).all())
+        out = torch.empty(B, T, Ht, hd, dtype=torch.bfloat16, device="cuda")
+        with pytest.raises(nat.NativeError):
+            nat.gemm_heads(x[:66], w, False, (ctypes.c_void_p * 1)(out.data_ptr()), 1, 2, 33, 32, Ht, 0, Hq, Hkv, Hq, Hkv, hd, Hq + Hkv,
+                           None, tables=(cos[:33], sin[:33]))
+    finally:
+        nat.set_gemm_pairs(was)
+
+
 @pytest.mark.parametrize("mode", [0, 1, 2])
 @pytest.mark.parametrize("M,I,K", [(1, 8, 64), (333, 200, 192), (130, 2056, 768), (3003, 2056, 256), (256, 136, 4096)])
 def test_swiglu_epilogues_of_any_width(nat, mode, M, I, K):

@@ -1351,7 +1351,9 @@ TLM_API int tlm_gemm_heads(const void* A, const void* B, int M, int N, int K, lo
   // read in 16-byte pieces: tables that do not start on one count as absent (cs is enough where rows_per_batch % 32 == 0)
   const bool f32_tables = n_rot == 0 || (cosT != nullptr && sinT != nullptr && aligned16(cosT) && aligned16(sinT));
   const bool any_rows = rows_per_batch % 32 != 0;
-  if (any_rows && (n_dst != 1 || b_mn || !f32_tables)) return -4;
+  // rows and heads past the destination's are clipped by the TMA tile stores; the forms that store row by row must have none
+  const bool inside = row_off >= 0 && row_off + rows_per_batch <= dst_rows && Hq + 2 * Hkv <= dst_heads;
+  if (any_rows && (n_dst != 1 || b_mn || !f32_tables || !inside)) return -4;
   if (M != batch * rows_per_batch || N != (Hq + 2 * Hkv) * hd || q_l <= 0 || Hq % q_l != 0) return -5;
   if (kv_rep < 1) kv_rep = 1;
   if (kv_rep > 1) {                     // replicated KV heads: every destination holds exactly one k and one v head
@@ -1366,7 +1368,7 @@ TLM_API int tlm_gemm_heads(const void* A, const void* B, int M, int N, int K, lo
   GemmParams p{};
   if (!b_mn) take_pending_waits(p);               // x W^T: may be the first reader of its weights after an optimizer step
   const bool pair = use_pair(M) && p.wait_flags[0] == nullptr;
-  if (small_tiles() && p.wait_flags[0] == nullptr && n_dst == 1 && kv_rep == 1 && !b_mn && f32_tables) {
+  if (small_tiles() && p.wait_flags[0] == nullptr && n_dst == 1 && kv_rep == 1 && !b_mn && f32_tables && inside) {
     SplitGemm g{};
     g.A = A; g.B = B; g.M = M; g.N = N; g.K = K; g.lda = lda; g.ldb = ldb; g.epi = SPLIT_HEADS; g.C = dst_ptrs[0];
     g.ldc = hd; g.hd = hd; g.rows_per_batch = rows_per_batch; g.dst_rows = dst_rows; g.dst_heads = dst_heads;
