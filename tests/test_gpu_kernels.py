@@ -305,6 +305,27 @@ def test_swiglu_epilogues_of_any_width(nat, mode, M, I, K):
     assert _rel_err(dgu, torch.cat([d * u * sig * (1 + g * (1 - sig)), d * g * sig], dim=-1)) < 6e-3
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+def test_swiglu_epilogues_refuse_misaligned_tensors(nat, mode):
+    """Their 16-byte accesses need aligned tensors: an `act`, `gate_up` or saved `gate_up` that is not is an error, on the
+    wide tiles (whose tensor maps cannot be made) as on the small ones."""
+    M, I, K = 64, 64, 64
+    x, w, wd = _rand(M, K, seed=94), _rand(2 * I, K, seed=95), _rand(K, I, seed=96)
+    flat = torch.zeros(M * 2 * I + 8, dtype=torch.bfloat16, device="cuda")
+    odd, good = flat.data_ptr() + 2, torch.zeros(M * 2 * I, dtype=torch.bfloat16, device="cuda")
+    was = nat.set_gemm_pairs(mode)
+    try:
+        fwd = lambda gu, act: nat.lib().tlm_gemm_swiglu(x.data_ptr(), w.data_ptr(), gu, act, M, I, K, K, K, nat._stream())
+        bwd = lambda gu, out: nat.lib().tlm_gemm_swiglu_bwd(x.data_ptr(), wd.data_ptr(), gu, out, M, I, K, K, I, nat._stream())
+        assert fwd(odd, good.data_ptr()) != 0 and fwd(good.data_ptr(), odd) != 0
+        assert bwd(odd, good.data_ptr()) != 0 and bwd(good.data_ptr(), odd) != 0
+        assert fwd(good.data_ptr(), flat.data_ptr()) == 0
+    finally:
+        nat.set_gemm_pairs(was)
+    nat.raise_on_device_status()
+    assert bool((flat[M * I:] == 0).all())
+
+
 def test_gemm_heads_scatter_plan(nat, gemm_mode):
     """Two destinations (both local buffers here) with the Ulysses head plan and a row offset; MN-major weight."""
     import ctypes

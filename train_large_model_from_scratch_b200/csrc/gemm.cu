@@ -1475,7 +1475,7 @@ TLM_API int tlm_gemm_swiglu(const void* x, const void* w_gu, void* gate_up, void
 TLM_API int tlm_gemm_swiglu_bwd(const void* dy, const void* w_down, const void* gate_up, void* d_gate_up, int M, int I,
                                 int D, long long lda, long long ldb, cudaStream_t stream) {
   if (M <= 0 || I <= 0 || D <= 0) return 0;
-  if (I % 8 != 0) return -4;
+  if (I % 8 != 0 || !aligned16(gate_up)) return -4;          // gate | up is read in 16-byte pieces
   const bool pair = use_pair(M);
   if (small_tiles()) {
     SplitGemm g{};

@@ -309,11 +309,16 @@ static int split_map(CUtensorMap* m, const void* ptr, long long rows, long long 
   return make_tmap_bf16(m, ptr, 2, dims, strides, box);
 }
 
+// everything the epilogues load and store in 16-byte pieces (absent tensors are null)
+static bool aligned_ok(const SplitGemm& g) {
+  return g.N % 8 == 0 && g.ldc % 8 == 0 && aligned16(g.C) && aligned16(g.act) && aligned16(g.aux) && aligned16(g.cosT) && aligned16(g.sinT);
+}
+
 int split_run(const SplitGemm& g, const SplitPlan& plan, cudaStream_t st) {
   const int bn = plan.bn, tile_n = g.epi == SPLIT_SWIGLU ? bn / 2 : bn;
   const int kblocks = (g.K + SP_BK - 1) / SP_BK;
   if ((bn != 64 && bn != 128) || plan.split < 1 || plan.split > kblocks) return -4;
-  if (g.N % 8 != 0 || g.ldc % 8 != 0 || (reinterpret_cast<uintptr_t>(g.C) & 15)) return -4;
+  if (!aligned_ok(g)) return -4;
   if (g.epi == SPLIT_HEADS && (g.hd > bn || bn % g.hd != 0 || g.hd % 16 != 0)) return -4;
   CUtensorMap ma, mb;
   int e = split_map(&ma, g.A, g.M, g.K, g.lda, g.a_mn, SP_BM);
@@ -348,7 +353,7 @@ int split_run(const SplitGemm& g, const SplitPlan& plan, cudaStream_t st) {
 // exchange of the partial tiles. A weight gradient has to win clearly: the wide tiles add to C with whole TMA boxes.
 SplitPlan split_plan(const SplitGemm& g, double wide_us) {
   SplitPlan best{0, 0};
-  if (g.N % 8 != 0 || g.ldc % 8 != 0 || (reinterpret_cast<uintptr_t>(g.C) & 15)) return best;
+  if (!aligned_ok(g)) return best;
   const long long kblocks = (g.K + SP_BK - 1) / SP_BK, slots = 2LL * num_sms();
   const double operand_bytes = 2.0 * g.K * ((double)g.M + (g.epi == SPLIT_SWIGLU ? 2.0 : 1.0) * g.N);
   const double lines = (!g.a_mn && g.lda % 64 != 0) || (!g.b_mn && g.ldb % 64 != 0) ? 1.3 : 1.0;
