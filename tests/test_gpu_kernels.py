@@ -486,6 +486,36 @@ def test_grouped_gemms(nat, gemm_mode, counts, N, K):
         r += c
 
 
+@pytest.mark.parametrize("counts,N,K", [([130, 0, 64, 257], 512, 256), ([5, 300, 1, 90], 264, 72), ([700, 0, 1300, 257], 512, 256)])
+def test_grouped_gemms_with_every_store(nat, gemm_mode, counts, N, K):
+    """The grouped entry points take the kind of store as an argument: bf16, fp32, and fp32 added to what is there."""
+    R, E = sum(counts), len(counts)
+    x, w, dy = _rand(R, K, seed=100), _rand(E, N, K, seed=101), _rand(R, N, seed=102)
+    rs = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32, device="cuda")
+    grp = torch.repeat_interleave(torch.arange(E, device="cuda"), torch.tensor(counts, device="cuda"))
+    def rows(a, out, n, k, b_mn, epi):
+        nat._check(nat.lib().tlm_gemm_grouped_rows(a.data_ptr(), w.data_ptr(), out.data_ptr(), rs.data_ptr(), E, R, n, k, k, K,
+                                                   N * K, n, b_mn, epi, R, nat._stream()), "grouped_rows")
+    nt = torch.cat([x[grp == e].float() @ w[e].float().t() for e in range(E)])
+    nn = torch.cat([dy[grp == e].float() @ w[e].float() for e in range(E)])
+    out = torch.full((R, N), 3.0, device="cuda")
+    rows(x, out, N, K, 0, nat.EPI_F32)
+    assert _rel_err(out, nt) < 1e-4
+    rows(x, out, N, K, 0, nat.EPI_F32_ACC)
+    assert _rel_err(out, 2 * nt) < 1e-4
+    out = torch.full((R, K), 3.0, device="cuda")
+    rows(dy, out, K, N, 1, nat.EPI_F32)
+    assert _rel_err(out, nn) < 1e-4
+    for epi, dtype, tol in ((nat.EPI_F32, torch.float32, 1e-4), (nat.EPI_BF16, torch.bfloat16, 6e-3)):
+        got = torch.full((E, N, K), 3.0, dtype=dtype, device="cuda")
+        nat._check(nat.lib().tlm_gemm_grouped_k(dy.data_ptr(), x.data_ptr(), got.data_ptr(), rs.data_ptr(), E, R, N, K, N, K, K, N * K,
+                                                epi, nat._stream()), "grouped_k")
+        for e, c in enumerate(counts):
+            ref = dy[grp == e].float().t() @ x[grp == e].float()
+            assert _rel_err(got[e], ref) < tol if c else bool((got[e] == 3.0).all()), (epi, e)
+    nat.raise_on_device_status()
+
+
 @pytest.mark.parametrize("E", [255, 256, 257, 300])
 def test_row_grouped_gemms_around_the_group_limit_of_a_launch(nat, gemm_mode, E):
     """256 groups fit one launch's tile list, more run as several launches: ragged groups (empty ones, one of more than

@@ -1281,7 +1281,8 @@ static int dispatch(bool a_mn, bool b_mn, int epi, const CUtensorMap& ma, const 
   TLM_CASE(true, true, EPI_BF16, 0) TLM_CASE(false, true, EPI_F32, 0) TLM_CASE(false, false, EPI_LSE, 0)
   TLM_CASE(false, false, EPI_BF16, 1) TLM_CASE(false, true, EPI_BF16, 1)
   TLM_CASE(false, false, EPI_ROWS, 1) TLM_CASE(false, true, EPI_ROWS, 1)
-  TLM_CASE(true, true, EPI_F32_ACC, 2)
+  TLM_CASE(false, false, EPI_F32, 1) TLM_CASE(false, true, EPI_F32, 1) TLM_CASE(false, false, EPI_F32_ACC, 1)
+  TLM_CASE(true, true, EPI_F32_ACC, 2) TLM_CASE(true, true, EPI_F32, 2) TLM_CASE(true, true, EPI_BF16, 2)
 #undef TLM_CASE
   return -2;
 }
@@ -1724,7 +1725,8 @@ TLM_API int tlm_gemm(const void* A, const void* B, void* C, int M, int N, int K,
 // groups+1 ints, ascending, row_start[groups] == M); group g multiplies by
 // B[g] ([N,K] K-major or [K,N] MN-major, `b_group_stride` elements apart).
 // `max_rows_per_group` bounds the per-group tile count (a host-known bound,
-// e.g. M); tiles beyond a group's real row count exit immediately.
+// e.g. M); it only sizes the grid, the kernel walks the tiles that exist.
+// epi: EPI_BF16, EPI_F32 (plain stores) or, with K-major B, EPI_F32_ACC.
 TLM_API int tlm_gemm_grouped_rows(const void* A, const void* B, void* C, const int* row_start, int groups, int M,
                                   int N, int K, long long lda, long long ldb, long long b_group_stride,
                                   long long ldc, int b_mn, int epi, int max_rows_per_group, cudaStream_t stream) {
@@ -1821,6 +1823,7 @@ static int grouped_k(const void* A, const void* B, void* C, const int* row_start
 // Grouped wgrad: C[g] ([M,N] fp32, `c_group_stride` apart) += A[rows_g, M]^T * B[rows_g, N]
 // where rows_g = [row_start[g], row_start[g+1]) is the reduction range.
 // A is stored [R, M] and B [R, N] (both MN-major with respect to the product).
+// epi: EPI_F32_ACC, or EPI_F32 / EPI_BF16, which store the products (an empty group's matrix is left alone).
 TLM_API int tlm_gemm_grouped_k(const void* A, const void* B, void* C, const int* row_start, int groups, int R,
                                int M, int N, long long lda, long long ldb, long long ldc, long long c_group_stride,
                                int epi, cudaStream_t stream) {
