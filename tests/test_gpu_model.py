@@ -65,6 +65,55 @@ def test_blocks_issued_in_one_call_equal_the_per_op_path(T, over):
     assert logits_grad.requires_grad and torch.equal(logits, logits_grad.detach())
 
 
+def _replace(model, where, seen, monkeypatch):
+    """Put a wrapper that counts its calls in one of the places the per-op path goes through."""
+    from train_large_model_from_scratch_b200.models.modules.attn import Attention
+    from train_large_model_from_scratch_b200.models.modules.norm import LayerNorm
+    from train_large_model_from_scratch_b200.ops import attention_cuda, functional as F_ops, native
+    owner, name = {"instance add_norm": (model.blocks[1].ln_2, "add_norm"), "instance forward": (model.blocks[1].mlp, "forward"),
+                   "class add_norm": (LayerNorm, "add_norm"), "class forward": (Attention, "forward"), "op": (F_ops, "linear"),
+                   "kernel": (native, "flash_attn_fwd"), "attention": (attention_cuda, "fwd")}[where]
+    stock = getattr(owner, name)
+
+    def wrapper(*args, **kwargs):
+        seen.append(where)
+        return stock(*args, **kwargs)
+    monkeypatch.setattr(owner, name, wrapper)
+
+
+@pytest.mark.parametrize("where", ["instance add_norm", "instance forward", "class add_norm", "class forward", "op", "kernel", "attention"])
+def test_what_a_program_replaced_is_called_without_gradients_too(where, monkeypatch):
+    """The one native call knows nothing of a method or an op that the program replaced, on one module, on a class or in the
+    op modules: such a program gets the per-op path, which calls the replacement, and the one call again afterwards."""
+    from train_large_model_from_scratch_b200.ops import native
+    model = _build("cuda", torch.bfloat16).eval()
+    x = torch.randint(0, 4096, (2, 64), generator=torch.Generator().manual_seed(5)).cuda()
+    seen = []
+    with torch.no_grad():
+        ref, _, _ = model(x)
+        with monkeypatch.context() as m:
+            _replace(model, where, seen, m)
+            assert not model._one_call_ok(model.wte(x), 64)
+            got, _, _ = model(x)
+        if not where.startswith("instance"):
+            assert model._one_call_ok(model.wte(x), 64)
+    native.raise_on_device_status()
+    assert seen and torch.equal(got, ref)
+
+
+def test_forward_mode_tangents_are_not_dropped():
+    """The ops have no forward-mode rule and say so; a weight with a tangent must not go into the one call, which would
+    return logits without one."""
+    import torch.autograd.forward_ad as fwad
+    model = _build("cuda", torch.bfloat16).eval()
+    x = torch.randint(0, 4096, (2, 64), generator=torch.Generator().manual_seed(6)).cuda()
+    with torch.no_grad(), fwad.dual_level():
+        w = model.blocks[0].ln_2.weight
+        dual = fwad.make_dual(w.detach(), torch.ones_like(w))
+        with pytest.raises((NotImplementedError, RuntimeError)):
+            torch.func.functional_call(model, {"blocks.0.ln_2.weight": dual}, (x,))
+
+
 def test_strided_weights_stay_on_the_per_op_path():
     """A projection whose weight is a slice of a wider tensor: the per-op kernels take its row pitch, the one call does not."""
     from train_large_model_from_scratch_b200.ops import native

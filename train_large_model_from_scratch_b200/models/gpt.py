@@ -15,7 +15,9 @@ from __future__ import annotations
 
 import torch
 import torch.nn as nn
+from torch.autograd import forward_ad
 
+from ..ops import attention_cuda, native
 from ..ops import functional as F_ops
 from ..parallel import parallel_state
 from ..parallel.flat import EXPERT_LOCAL_PARAM_SUFFIXES, flatten_model
@@ -53,6 +55,25 @@ class Block(nn.Module):
         if self.use_moe:
             m = m[0]
         return x, m
+
+
+def _per_op_parts():
+    """What a dense block's forward calls on the per-op path, as `(owner, name)`."""
+    yield from ((Block, "forward"), (Attention, "forward"), (Attention, "_rope"), (Attention, "_rope_fp16"), (MLP, "forward"),
+                (LayerNorm, "add_norm"), (Block, "__call__"), (Attention, "__call__"), (MLP, "__call__"))
+    for name in ("add_rmsnorm", "qkv_attention", "linear", "swiglu_mlp"):
+        yield F_ops, name
+    for fn in ("_AddRMSNorm", "_QKVAttention", "_Linear", "_SwiGLUMLP"):
+        yield F_ops, fn
+        yield getattr(F_ops, fn), "forward"
+    for name in ("add_rmsnorm_fwd", "gemm_heads", "flash_attn_fwd", "gemm_nt", "gemm_swiglu"):
+        yield native, name
+    yield attention_cuda, "fwd"
+
+
+# as this package defines them: a program that has put something else in one of these places gets the per-op path
+_STOCK_PARTS = tuple((owner, name, getattr(owner, name)) for owner, name in _per_op_parts())
+_REPLACEABLE = {"forward", "add_norm", "_rope", "_rope_fp16", "_compiled_call_impl"}      # attributes set on one module
 
 
 class _GroupBoundary(torch.autograd.Function):
@@ -195,12 +216,15 @@ class GPT(nn.Module):
         return logits, loss, logging_loss
 
     def _one_call_ok(self, x: torch.Tensor, T: int) -> bool:
-        """Whether the blocks' forward can be issued as one native call: no gradients, one GPU, dense bf16 blocks as this
-        class built them (fused weights, no replaced or hooked sub-module). Everything else takes the per-op path."""
+        """Whether the blocks' forward can be issued as one native call: no gradients of either mode, no tracing, one GPU,
+        dense bf16 blocks as this class built them (fused weights, no hooked sub-module, nothing replaced of what the
+        per-op path calls: see `_per_op_parts`). Everything else takes the per-op path."""
         from torch.nn.modules import module as nn_module
         if (not x.is_cuda or x.dtype != torch.float32 or self.use_moe or self.comm_hooks is not None or len(self.blocks) == 0
                 or parallel_state.get_sep_world_size() > 1
-                or nn_module._global_forward_hooks or nn_module._global_forward_pre_hooks):
+                or nn_module._global_forward_hooks or nn_module._global_forward_pre_hooks
+                or forward_ad._current_level >= 0 or torch.jit.is_tracing()
+                or any(getattr(owner, name) is not part for owner, name, part in _STOCK_PARTS)):
             return False
         def form(block):                       # what the one call takes from the first block
             attn = block.attn
@@ -216,7 +240,7 @@ class GPT(nn.Module):
                     or not F_ops.qkv_project_fused_ok(attn.q_proj.weight, attn._qkv_weight, attn.head_dim, T):
                 return False
             for m in (block, attn, mlp, block.ln_1, block.ln_2):
-                if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
+                if m._forward_hooks or m._forward_pre_hooks or not _REPLACEABLE.isdisjoint(m.__dict__):
                     return False
             if type(block.ln_1) is not LayerNorm or type(block.ln_2) is not LayerNorm or block.ln_1.variance_epsilon != block.ln_2.variance_epsilon:
                 return False
@@ -229,7 +253,6 @@ class GPT(nn.Module):
         return True
 
     def _blocks_forward(self, x: torch.Tensor, B: int, T: int):
-        from ..ops import native
         attn = self.blocks[0].attn
         weights = [(b.ln_1.weight, b.attn._qkv_weight, b.attn.c_proj.weight, b.ln_2.weight, b.mlp._gate_up_weight, b.mlp.down_proj.weight)
                    for b in self.blocks]
