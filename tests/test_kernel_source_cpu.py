@@ -53,3 +53,12 @@ def test_kernels_that_start_early_read_through_plain_loads():
     gemm = _source("gemm.cu")                              # its kernels share one body
     body = _body(gemm, gemm.index("void gemm_body("))
     assert "griddep_wait();" in body and "__ldg" not in body and "ld.global.nc" not in body
+
+
+def test_a_width_without_a_kernel_is_an_error():
+    """The norms pick their kernel with a `switch` whose every case launches and returns; should a width ever get there
+    without a case, the call has to fail instead of reporting a launch that did not happen."""
+    text = _source("elementwise.cu")
+    switches = [m.end() for m in re.finditer(r"switch \((?:D / 256|sp\.nv)\) \{[^\n]*\}\n#undef TLM_RMS_CASE\n", text)]
+    assert len(switches) == 4
+    assert all(text[at:].lstrip().startswith("return -4;") for at in switches)

@@ -787,8 +787,7 @@ TLM_API int tlm_add_rmsnorm_fwd(const float* x, const void* delta, const void* w
       (const __nv_bfloat16*)w, x_new, (__nv_bfloat16*)h, rstd, rows, eps);
     switch (D / 256) { TLM_RMS_CASE(1) TLM_RMS_CASE(2) TLM_RMS_CASE(3) TLM_RMS_CASE(4) TLM_RMS_CASE(6) TLM_RMS_CASE(8) }
 #undef TLM_RMS_CASE
-    count_launch();
-    return launch_status();
+    return -4;
   }
   const RmsSplit sp = rms_split(D, 4);
   if (sp.nv > 0) {
@@ -797,8 +796,7 @@ TLM_API int tlm_add_rmsnorm_fwd(const float* x, const void* delta, const void* w
       (const __nv_bfloat16*)w, x_new, (__nv_bfloat16*)h, rstd, rows, D, eps);
     switch (sp.nv) { TLM_RMS_CASE(1) TLM_RMS_CASE(2) TLM_RMS_CASE(3) TLM_RMS_CASE(4) }
 #undef TLM_RMS_CASE
-    count_launch();
-    return launch_status();
+    return -4;
   }
   int warps = 8;
   while (warps > 1 && (size_t)warps * D * 4 > 200 * 1024) warps >>= 1;
@@ -825,8 +823,7 @@ TLM_API int tlm_add_rmsnorm_bwd(const float* g_xnew, const void* g_h, const floa
       (const __nv_bfloat16*)w, g_x, (__nv_bfloat16*)g_delta, dw, rows);
     switch (D / 256) { TLM_RMS_CASE(1) TLM_RMS_CASE(2) TLM_RMS_CASE(3) TLM_RMS_CASE(4) }
 #undef TLM_RMS_CASE
-    count_launch();
-    return launch_status();
+    return -4;
   }
   const RmsSplit sp = rms_split(D, 3);          // 4 groups would not fit the registers
   if (sp.nv > 0 && (reinterpret_cast<uintptr_t>(dw) & 15) == 0) {
@@ -838,8 +835,7 @@ TLM_API int tlm_add_rmsnorm_bwd(const float* g_xnew, const void* g_h, const floa
       (const __nv_bfloat16*)w, g_x, (__nv_bfloat16*)g_delta, dw, rows, D);
     switch (sp.nv) { TLM_RMS_CASE(1) TLM_RMS_CASE(2) TLM_RMS_CASE(3) }
 #undef TLM_RMS_CASE
-    count_launch();
-    return launch_status();
+    return -4;
   }
   int warps = 8;
   while (warps > 1 && (size_t)warps * 2 * D * 4 > 200 * 1024) warps >>= 1;
