@@ -195,6 +195,65 @@ def test_small_tile_gemm(nat, bn, split, M, N, K):
         assert bool((acc[M:] == 2.0).all())
 
 
+SPLIT_PLANS = [(64, 1), (64, 2), (64, 4), (64, 8), (128, 1), (128, 2), (128, 4), (128, 8)]
+
+
+@pytest.mark.parametrize("bn,split", SPLIT_PLANS)
+@pytest.mark.parametrize("hd,Hq,Hkv,B,T,K", [(32, 5, 1, 3, 50, 520), (64, 3, 1, 2, 129, 1000), (64, 1, 1, 1, 7, 512), (128, 2, 1, 5, 33, 576)])
+def test_small_tile_heads(nat, bn, split, hd, Hq, Hkv, B, T, K):
+    """The head / rotation epilogue on every tile width and split, not only where the cost rule picks one: heads that do not
+    fill the last tile, rows that end inside a CTA's share, entries of any length. One bf16 rounding: 1.7e-3 rms."""
+    from train_large_model_from_scratch_b200.ops import oracle
+    Ht, M = Hq + 2 * Hkv, B * T
+    x, w = _rand(M, K, seed=110), _rand(Ht * hd, K, scale=0.05, seed=111)
+    cos, sin = (t.contiguous() for t in oracle.rope_tables(torch.arange(3, 3 + T, device="cuda"), hd, 10000.0, "reference"))
+    out = torch.full((M * Ht * hd + 4096,), 7.0, dtype=torch.bfloat16, device="cuda")
+    code = nat.lib().tlm_gemm_split_heads(x.data_ptr(), w.data_ptr(), out[2048:].data_ptr(), M, Ht * hd, K, hd, T, Hq + Hkv,
+                                          cos.data_ptr(), sin.data_ptr(), bn, split, nat._stream())
+    if hd > bn:                                           # a head has to fit a tile
+        assert code != 0
+        return
+    assert code == 0
+    nat.raise_on_device_status()
+    ref = (x.double() @ w.double().t()).view(B, T, Ht, hd)
+    ref[:, :, :Hq + Hkv] = oracle.rope(ref[:, :, :Hq + Hkv], cos.double(), sin.double())
+    got = out[2048:2048 + M * Ht * hd].view(B, T, Ht, hd).double()
+    assert ((got - ref).norm() / ref.norm()).item() < 2.5e-3
+    assert (got - ref).abs().max().item() <= 2.0 ** -8 * ref.abs().max().item()             # no row or head in the wrong place
+    assert bool((out[:2048] == 7.0).all()) and bool((out[2048 + M * Ht * hd:] == 7.0).all())
+
+
+@pytest.mark.parametrize("bn,split", SPLIT_PLANS)
+@pytest.mark.parametrize("M,I,K", [(1, 8, 512), (129, 72, 1000), (200, 264, 576), (333, 136, 4104)])
+def test_small_tile_swiglu(nat, bn, split, M, I, K):
+    """SwiGLU forward (with and without gate | up kept) and backward on every tile width and split: widths that end inside a
+    tile, ragged rows and k-blocks. gate, up and d(act) are rounded to bf16 first (1.7e-3 rms), the results once more."""
+    x, w, wd, dy = _rand(M, K, seed=112), _rand(2 * I, K, scale=0.05, seed=113), _rand(K, I, scale=0.05, seed=114), _rand(M, K, seed=115)
+    def guarded(n):
+        t = torch.full((n + 2048,), 7.0, dtype=torch.bfloat16, device="cuda")
+        return t, t[1024:1024 + n], lambda: bool((t[:1024] == 7.0).all()) and bool((t[1024 + n:] == 7.0).all())
+    gu_buf, gu, gu_ok = guarded(M * 2 * I)
+    act_buf, act, act_ok = guarded(M * I)
+    act2_buf, act2, act2_ok = guarded(M * I)
+    d_buf, d, d_ok = guarded(M * 2 * I)
+    run = lambda *a: nat._check(nat.lib().tlm_gemm_split_swiglu(*a, bn, split, nat._stream()), "gemm_split_swiglu")
+    run(x.data_ptr(), w.data_ptr(), gu.data_ptr(), act.data_ptr(), None, M, I, K, 0)
+    run(x.data_ptr(), w.data_ptr(), None, act2.data_ptr(), None, M, I, K, 0)
+    run(dy.data_ptr(), wd.data_ptr(), d.data_ptr(), None, gu.data_ptr(), M, I, K, 1)
+    nat.raise_on_device_status()
+    assert gu_ok() and act_ok() and act2_ok() and d_ok() and torch.equal(act, act2)
+    gu = gu.view(M, 2 * I).double()
+    ref = x.double() @ w.double().t()
+    assert ((gu - ref).norm() / ref.norm()).item() < 2.5e-3
+    g, u = gu.chunk(2, dim=-1)
+    sig = torch.sigmoid(g)
+    ref = g * sig * u
+    assert ((act.view(M, I).double() - ref).norm() / ref.norm()).item() < 2.5e-3
+    da = (dy.double() @ wd.double())
+    ref = torch.cat([da * u * sig * (1 + g * (1 - sig)), da * g * sig], dim=-1)
+    assert ((d.view(M, 2 * I).double() - ref).norm() / ref.norm()).item() < 4e-3            # two roundings: sqrt(2) * 1.7e-3
+
+
 @pytest.mark.parametrize("mode", [0, 1, 2])
 @pytest.mark.parametrize("hd,Hq,Hkv,B,T,K", [(64, 4, 2, 3, 33, 192), (64, 12, 4, 3, 1001, 768), (32, 8, 2, 2, 37, 192), (128, 2, 1, 5, 7, 256),
                                               (64, 3, 1, 1, 1, 64), (128, 8, 4, 3, 335, 256), (32, 32, 4, 2, 777, 128)])

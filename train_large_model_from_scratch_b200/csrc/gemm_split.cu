@@ -390,3 +390,24 @@ TLM_API int tlm_gemm_split(const void* A, const void* B, void* C, int M, int N, 
   g.epi = epi; g.C = C; g.ldc = ldc;
   return split_run(g, SplitPlan{bn, split}, stream);
 }
+// The fused epilogues with the plan given, for the same purpose. heads: C = [M / rows, rows, N / hd, hd], the first n_rot heads
+// rotated; forward SwiGLU: C = gate|up [M, 2 N] (or null), act [M, N]; backward: A = dy, B = w_down [K, N], aux = gate|up,
+// C = d(gate)|d(up).
+TLM_API int tlm_gemm_split_heads(const void* A, const void* B, void* C, int M, int N, int K, int hd, int rows, int n_rot,
+                                 const float* cosT, const float* sinT, int bn, int split, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (hd <= 0 || N % hd != 0 || rows <= 0 || M % rows != 0 || (n_rot > 0 && (cosT == nullptr || sinT == nullptr))) return -5;
+  SplitGemm g{};
+  g.A = A; g.B = B; g.M = M; g.N = N; g.K = K; g.lda = K; g.ldb = K; g.epi = SPLIT_HEADS; g.C = C; g.ldc = hd;
+  g.hd = hd; g.rows_per_batch = rows; g.dst_rows = rows; g.dst_heads = N / hd; g.n_rot = n_rot; g.cosT = cosT; g.sinT = sinT;
+  return split_run(g, SplitPlan{bn, split}, stream);
+}
+TLM_API int tlm_gemm_split_swiglu(const void* A, const void* B, void* C, void* act, const void* aux, int M, int N, int K,
+                                  int backward, int bn, int split, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (backward ? (C == nullptr || aux == nullptr) : act == nullptr) return -5;
+  SplitGemm g{};
+  g.A = A; g.B = B; g.M = M; g.N = N; g.K = K; g.lda = K; g.ldb = backward ? N : K; g.b_mn = backward != 0;
+  g.epi = backward ? SPLIT_SWIGLU_BWD : SPLIT_SWIGLU; g.C = C; g.ldc = 2LL * N; g.act = act; g.aux = aux;
+  return split_run(g, SplitPlan{bn, split}, stream);
+}
