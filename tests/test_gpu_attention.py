@@ -172,3 +172,41 @@ def test_backward_with_any_split_of_a_tile(hd, B, T, Hq, Hkv, monkeypatch):
         for name, sl in (("dq", slice(0, Hq)), ("dk", slice(Hq, Hq + Hkv)), ("dv", slice(Hq + Hkv, None))):
             a, b = dqkv[:, :, sl].double(), x.grad[:, :, sl]
             assert ((a - b).norm() / b.norm()).item() < 1e-2, (split, name)
+
+
+@pytest.mark.parametrize("hd", [32, 64, 128])
+@pytest.mark.parametrize("T,n_dst,rows", [(256, 2, 128), (200, 3, 72)])
+def test_scatter_forms_into_local_buffers(hd, T, n_dst, rows):
+    """The forms that store O, and in the backward dQ / dK / dV, into the sequence owners' tensors, with all owners' tensors on
+    this GPU: the same numbers as the packed forms, at the right rows and heads and nowhere else."""
+    import ctypes
+    from train_large_model_from_scratch_b200.ops import attention_cuda, native, oracle
+    B, Hq, Hkv = 2, 4, 2
+    g = torch.Generator(device="cuda").manual_seed(13)
+    qkv = torch.randn(B, T, Hq + 2 * Hkv, hd, device="cuda", generator=g).to(torch.bfloat16)
+    do = torch.randn(B, T, Hq, hd, device="cuda", generator=g).to(torch.bfloat16)
+    cos, sin = (t.contiguous() for t in oracle.rope_tables(torch.arange(T, device="cuda"), hd, 10000.0, "reference"))
+    o, lse = native.flash_attn_fwd(qkv, Hq, Hkv, True)
+    dqkv = native.flash_attn_bwd(do, qkv, o, lse, Hq, Hkv, True, rope=(cos, sin))
+
+    def owners(heads):
+        bufs = [torch.full((B, rows, heads, hd), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(n_dst)]
+        return bufs, (ctypes.c_void_p * n_dst)(*[b.data_ptr() for b in bufs])
+    bufs, ptrs = owners(Hq + 3)
+    o2, lse2 = attention_cuda.fwd_scatter(qkv, Hq, Hkv, ptrs, n_dst, rows, Hq + 3, 2)
+    assert torch.equal(o, o2) and torch.equal(lse, lse2)
+    got = torch.cat(bufs, dim=1)
+    assert torch.equal(got[:, :T, 2:2 + Hq], o) and bool((got[:, T:] == 7.0).all())
+    assert bool((got[:, :, :2] == 7.0).all()) and bool((got[:, :, 2 + Hq:] == 7.0).all())
+    Ht = 2 * (Hq + 2 * Hkv)                                        # this group's heads among those of two groups
+    bufs, ptrs = owners(Ht)
+    attention_cuda.bwd_scatter(do, qkv, o, lse, Hq, Hkv, (cos, sin), ptrs, n_dst, rows, Ht, Hq, 2 * Hq + Hkv, 2 * Hq + 3 * Hkv)
+    native.raise_on_device_status()
+    got = torch.cat(bufs, dim=1)
+    assert bool((got[:, T:] == 7.0).all())
+    for at, sl in ((Hq, slice(0, Hq)), (2 * Hq + Hkv, slice(Hq, Hq + Hkv)), (2 * Hq + 3 * Hkv, slice(Hq + Hkv, None))):
+        a, b = got[:, :T, at:at + (sl.stop or Hq + 2 * Hkv) - sl.start].float(), dqkv[:, :, sl].float()
+        # dQ: fp32 adds in any order; dK: rotated before instead of after its rounding to bf16
+        assert ((a - b).norm() / b.norm()).item() < 5e-3, at
+    others = [h for h in range(Ht) if h not in (*range(Hq, 2 * Hq), *range(2 * Hq + Hkv, 2 * Hq + 2 * Hkv), *range(2 * Hq + 3 * Hkv, Ht))]
+    assert bool((got[:, :, others] == 7.0).all())
