@@ -346,8 +346,8 @@ int split_run(const SplitGemm& g, const SplitPlan& plan, cudaStream_t st) {
 }
 
 // Estimated time in us, fitted to 30 shapes (M 16 - 4096, N 256 - 3072, K 256 - 50304, operands in L2): a k-block takes
-// 0.24 us (64 columns) or 0.27 us (128 columns) of a CTA, what 24 / 32 KB take at the 64 B per clock that an SM gets out of
-// L2, and no less than all CTAs' blocks take at 14 TB/s out of the whole L2 (7.5 TB/s when the operands do not stay in it:
+// 0.24 us (64 columns) or 0.27 us (128 columns) of a CTA, fitted: 24 and 32 KB at 52 and 62 B per clock and SM out of L2 (at
+// 1.965 GHz; an SM gets no more than 64), and no less than all CTAs' blocks take at 14 TB/s out of the whole L2 (7.5 TB/s when the operands do not stay in it:
 // 2560 x 512, K 50304 on 80 CTAs took 273 us against 224 us on wide tiles), 1.3 times as long when the rows of a K-major
 // operand do not start on 128-byte lines (2436 x 512, K 1384: 16.4 us, wide tiles 14.5); plus what surrounds the main loop and the
 // exchange of the partial tiles. A weight gradient has to win clearly: the wide tiles add to C with whole TMA boxes.

@@ -49,7 +49,7 @@ def fwd(qkv: torch.Tensor, n_q: int, n_kv: int, causal: bool):
 
 def fwd_scatter(qkv: torch.Tensor, n_q: int, n_kv: int, dst_ptrs, n_dst: int, dst_rows: int, dst_heads: int,
                 dst_head0: int):
-    """Causal attention (head dims 64 / 128) whose epilogue also stores each output row into
+    """Causal attention (head dims 32 / 64 / 128) whose epilogue also stores each output row into
     `dst[t // dst_rows][b, t % dst_rows, dst_head0 + h, :]` (`dst_ptrs`: ctypes array of device addresses of
     bf16 `[B, dst_rows, dst_heads, hd]` tensors, typically peers' symmetric buffers)."""
     B, T, _, hd = qkv.shape

@@ -73,7 +73,7 @@ class _GroupedGateUp(torch.autograd.Function):
     """Gate and up projections of all local experts as ONE grouped GEMM writing `gate | up` side by side
     (`w_pair [2E, I, D]`: the gate matrices, then the up matrices; they are adjacent in the flat expert buffer).
     Backward: one grouped GEMM with the reduction running over both halves gives `dx` (no separate sum),
-    two grouped wgrad GEMMs accumulate into the two halves of the gradient buffer."""
+    the weight gradients accumulate into the two halves of the gradient buffer (one launch where I % 256 == 0, else two)."""
 
     @staticmethod
     def forward(ctx, x, w_pair, counts):
