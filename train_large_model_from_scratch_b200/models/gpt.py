@@ -73,7 +73,6 @@ def _per_op_parts():
 
 # as this package defines them: a program that has put something else in one of these places gets the per-op path
 _STOCK_PARTS = tuple((owner, name, getattr(owner, name)) for owner, name in _per_op_parts())
-_REPLACEABLE = {"forward", "add_norm", "_rope", "_rope_fp16", "_compiled_call_impl"}      # attributes set on one module
 
 
 class _GroupBoundary(torch.autograd.Function):
@@ -240,7 +239,9 @@ class GPT(nn.Module):
                     or not F_ops.qkv_project_fused_ok(attn.q_proj.weight, attn._qkv_weight, attn.head_dim, T):
                 return False
             for m in (block, attn, mlp, block.ln_1, block.ln_2):
-                if m._forward_hooks or m._forward_pre_hooks or not _REPLACEABLE.isdisjoint(m.__dict__):
+                own = m.__dict__               # attributes set on this one module
+                if (m._forward_hooks or m._forward_pre_hooks or "forward" in own or "add_norm" in own or "_rope" in own
+                        or "_rope_fp16" in own or "_compiled_call_impl" in own):
                     return False
             if type(block.ln_1) is not LayerNorm or type(block.ln_2) is not LayerNorm or block.ln_1.variance_epsilon != block.ln_2.variance_epsilon:
                 return False
