@@ -68,3 +68,38 @@ def test_save_resume_loss_parity_with_recorded_step(world):
     assert len(later) >= 3
     _close(whole["losses"], second["losses"], 3e-3, later)
     _close(whole["norms"], second["norms"], 3e-2, later)
+
+
+def _small_trainer():
+    from train_large_model_from_scratch_b200.training import Trainer
+    from train_large_model_from_scratch_b200.training.config import (CheckpointConfig, Config, DataConfig, LoggingConfig, ModelConfig,
+                                                                     OptimConfig, ParallelConfig, SeedConfig, TrainingConfig)
+    return Trainer(Config(
+        logging=LoggingConfig(exp_name="t", log_dir=tempfile.mkdtemp(prefix="tlm_gpu_")), seed=SeedConfig(),
+        data=DataConfig(use_mock_data=True, mock_data_num_samples=2),
+        train=TrainingConfig(total_batch_size=512, batch_size=2, seq_len=256, max_steps=100, max_epochs=None, debug=True).with_derived(),
+        optim=OptimConfig(max_lr=6e-4, min_lr=6e-5, warmup_steps=10), ckpt=CheckpointConfig(), parallel=ParallelConfig(),
+        model=ModelConfig(num_layer=2, hidden_size=256, num_attention_heads=4, num_key_value_heads=2, intermediate_size=512,
+                          vocab_size=2048, block_size=512)))
+
+
+def test_forward_at_another_length_between_recorded_steps():
+    """Scoring a prompt of another length between two steps replaces the rotation tables that the model caches; the recorded
+    step goes on reading the ones it was recorded with."""
+    data = torch.randint(0, 2048, (2, 257), generator=torch.Generator().manual_seed(8)).cuda()
+    batch = [{"input_ids": data[:, :-1].contiguous(), "labels": data[:, 1:].contiguous()}]
+    losses = []
+    for other_lengths in (False, True):
+        tr, run = _small_trainer(), []
+        for step in range(7):
+            run.append(float(tr.train_step(step, batches=batch)["loss"]))
+            if other_lengths and step >= 3:
+                logits, _, _ = tr.raw_model(data[:, :100])                 # with gradients on: every block's tables
+                del logits
+                junk = [torch.full((256, 64), 1e3, device="cuda") for _ in range(64)] + \
+                       [torch.full((256, 64, 2), 1e3, device="cuda", dtype=torch.float16) for _ in range(64)]
+                del junk
+        assert tr._graph is not None
+        losses.append(run)
+    for a, b in zip(*losses):
+        assert abs(a - b) < 5e-3 * a, losses

@@ -89,6 +89,7 @@ class Trainer:
         self._graph_in = None
         self._graph_out = None
         self._graph_launches = 0
+        self._graph_tables = None
         self._graph_eager_steps = 0
         self._graph_disabled = False
         self._prefetched = None            # next step's batches, already on their way to the device
@@ -464,6 +465,10 @@ class Trainer:
                     return True
                 self._graph_launches = native.launch_count() - before
                 self._graph = graph
+                # the recording reads the rotation tables at their addresses: a forward at another length replaces the
+                # modules' cached tables, which must not free these
+                self._graph_tables = [(b.attn._rope_cache, b.attn._rope_cache_fp16, b.attn._rope_cache_full)
+                                      for b in self.raw_model.blocks]
             self._graph.replay()
             native.add_launch_count(self._graph_launches)
             # the recording writes its results into the same two tensors every time: hand out copies
