@@ -88,7 +88,8 @@ __global__ void add_rmsnorm_fwd_kernel(const float* __restrict__ x, const __nv_b
 }
 
 // Register-resident variant for D = NV * 256: each lane owns NV groups of 8 columns and issues all loads of its
-// row before the first use, so one warp keeps NV * 3 sixteen-byte loads in flight; no shared memory.
+// row before the first use, so one warp keeps NV * 3 sixteen-byte loads in flight; no shared memory. The weights are requested
+// before the first store of h, for the same reason as in the backward (between the stores: 32768 x 1024 68 us, now 63).
 template <int NV>
 __global__ void __launch_bounds__(256)
 add_rmsnorm_fwd_reg_kernel(const float* x, const __nv_bfloat16* delta,
@@ -122,14 +123,19 @@ add_rmsnorm_fwd_reg_kernel(const float* x, const __nv_bfloat16* delta,
       ss += a[k].x * a[k].x + a[k].y * a[k].y + a[k].z * a[k].z + a[k].w * a[k].w +
             b[k].x * b[k].x + b[k].y * b[k].y + b[k].z * b[k].z + b[k].w * b[k].w;
     }
+    // w (D * 2 bytes, stays in L1) for all of the row's h, requested when delta's registers are free and not before: held over
+    // the sum they would cost a resident block
+    asm volatile("" ::: "memory");
+    uint4 wv[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) wv[k] = *reinterpret_cast<const uint4*>(w + (lane + 32 * k) * 8);
     ss = warp_sum(ss);
     const float rstd = rsqrtf(ss * (1.f / (float)D) + eps);
     if (lane == 0) rstd_out[r] = rstd;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
       const int c = (lane + 32 * k) * 8;
-      const uint4 wv = *reinterpret_cast<const uint4*>(w + c);            // D * 2 bytes, stays in L1
-      const float2 w0 = unpack_bf16(wv.x), w1 = unpack_bf16(wv.y), w2 = unpack_bf16(wv.z), w3 = unpack_bf16(wv.w);
+      const float2 w0 = unpack_bf16(wv[k].x), w1 = unpack_bf16(wv[k].y), w2 = unpack_bf16(wv[k].z), w3 = unpack_bf16(wv[k].w);
       uint4 o;
       o.x = pack_bf16(a[k].x * rstd * w0.x, a[k].y * rstd * w0.y);
       o.y = pack_bf16(a[k].z * rstd * w1.x, a[k].w * rstd * w1.y);
@@ -188,13 +194,15 @@ add_rmsnorm_fwd_wide_kernel(const float* x, const __nv_bfloat16* delta,
       ss += a[k].x * a[k].x + a[k].y * a[k].y + a[k].z * a[k].z + a[k].w * a[k].w +
             b[k].x * b[k].x + b[k].y * b[k].y + b[k].z * b[k].z + b[k].w * b[k].w;
     }
+    uint4 wv[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) wv[k] = *reinterpret_cast<const uint4*>(w + c0 + k * 256);
     ss = rms_block_sum(ss, red[par], warps, warp, lane);       // two buffers: the next row's sums cannot overtake this read
     const float rstd = rsqrtf(ss / (float)D + eps);
     if (threadIdx.x == 0) rstd_out[r] = rstd;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-      const uint4 wv = *reinterpret_cast<const uint4*>(w + c0 + k * 256);
-      const float2 w0 = unpack_bf16(wv.x), w1 = unpack_bf16(wv.y), w2 = unpack_bf16(wv.z), w3 = unpack_bf16(wv.w);
+      const float2 w0 = unpack_bf16(wv[k].x), w1 = unpack_bf16(wv[k].y), w2 = unpack_bf16(wv[k].z), w3 = unpack_bf16(wv[k].w);
       uint4 o;
       o.x = pack_bf16(a[k].x * rstd * w0.x, a[k].y * rstd * w0.y);
       o.y = pack_bf16(a[k].z * rstd * w1.x, a[k].w * rstd * w1.y);
@@ -274,65 +282,82 @@ __global__ void add_rmsnorm_bwd_kernel(const float* __restrict__ g_xnew, const _
   }
 }
 
-// Register-resident variant for D = NV * 256 (NV <= 4): each lane owns NV groups of 8
-// columns, keeps x_hat, g*w and its dweight partial sums in registers; one pass over
-// global memory, no shared-memory traffic in the row loop.
+// Register-resident variant for D = NV * 256 (NV <= 4): each lane owns NV groups of 8 columns and keeps them, the weights and
+// its dweight partial sums in registers; one pass over global memory, no shared-memory traffic in the row loop. Bound by HBM
+// bandwidth from a few thousand rows on, so every load of a row is requested before its first store: a plain load does not pass
+// a store, and read-only ones may not be used (see launch_overlapped). Requested one group after the other between the stores,
+// 32768 x 1024 took 96 us and 6224 x 1024 22.5 us.
+// Threads per block: up to 512 columns a warp's row, weights and sums leave room for two blocks of eight warps; at 768 and 1024
+// columns they take 144 to 168 registers per lane, three blocks of four warps.
+template <int NV> constexpr int rms_bwd_threads() { return NV <= 2 ? 256 : 128; }
+
 template <int NV>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(rms_bwd_threads<NV>(), NV <= 2 ? 2 : 3)
 add_rmsnorm_bwd_reg_kernel(const float* g_xnew, const __nv_bfloat16* g_h,
                            const float* x_new, const float* rstd_in,
                            const __nv_bfloat16* w, float* __restrict__ g_x,
                            __nv_bfloat16* __restrict__ g_delta, float* __restrict__ dw_out, int rows) {
   griddep_wait();
   constexpr int D = NV * 256;
-  __shared__ float dw_s[8][D];                      // block fold
+  __shared__ float dw_s[rms_bwd_threads<NV>() / 32][D];                      // block fold
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float dw[NV * 8];
 #pragma unroll
   for (int i = 0; i < NV * 8; ++i) dw[i] = 0.f;
+  uint4 wv[NV];                                     // the same columns of w for every row
+#pragma unroll
+  for (int k = 0; k < NV; ++k) wv[k] = *reinterpret_cast<const uint4*>(w + (lane + 32 * k) * 8);
   for (int r = blockIdx.x * warps + warp; r < rows; r += gridDim.x * warps) {
+    // all of the row's loads before its first store (a plain load does not pass one)
     const float rstd = rstd_in[r];
-    float xh[NV * 8], gw[NV * 8];
+    float4 xa[NV], xb[NV], ga[NV], gb[NV];
+    uint4 gv[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const long long at = (long long)r * D + (lane + 32 * k) * 8;
+      xa[k] = *reinterpret_cast<const float4*>(x_new + at);
+      xb[k] = *reinterpret_cast<const float4*>(x_new + at + 4);
+      gv[k] = *reinterpret_cast<const uint4*>(g_h + at);
+      ga[k] = make_float4(0.f, 0.f, 0.f, 0.f); gb[k] = ga[k];
+      if (g_xnew != nullptr) {
+        ga[k] = *reinterpret_cast<const float4*>(g_xnew + at);
+        gb[k] = *reinterpret_cast<const float4*>(g_xnew + at + 4);
+      }
+    }
     float dot = 0.f;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-      const int c = (lane + 32 * k) * 8;
-      const float4 a = *reinterpret_cast<const float4*>(x_new + (long long)r * D + c);
-      const float4 b = *reinterpret_cast<const float4*>(x_new + (long long)r * D + c + 4);
-      const uint4 gv = *reinterpret_cast<const uint4*>(g_h + (long long)r * D + c);
-      const float2 g0 = unpack_bf16(gv.x), g1 = unpack_bf16(gv.y), g2 = unpack_bf16(gv.z), g3 = unpack_bf16(gv.w);
-      const uint4 wv = *reinterpret_cast<const uint4*>(w + c);          // 2 KB table, stays in L1
-      const float2 w0 = unpack_bf16(wv.x), w1 = unpack_bf16(wv.y), w2 = unpack_bf16(wv.z), w3 = unpack_bf16(wv.w);
-      const float xs[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      const float2 g0 = unpack_bf16(gv[k].x), g1 = unpack_bf16(gv[k].y), g2 = unpack_bf16(gv[k].z), g3 = unpack_bf16(gv[k].w);
+      const float2 w0 = unpack_bf16(wv[k].x), w1 = unpack_bf16(wv[k].y), w2 = unpack_bf16(wv[k].z), w3 = unpack_bf16(wv[k].w);
+      float* xs[8] = {&xa[k].x, &xa[k].y, &xa[k].z, &xa[k].w, &xb[k].x, &xb[k].y, &xb[k].z, &xb[k].w};
       const float gs[8] = {g0.x, g0.y, g1.x, g1.y, g2.x, g2.y, g3.x, g3.y};
       const float ws[8] = {w0.x, w0.y, w1.x, w1.y, w2.x, w2.y, w3.x, w3.y};
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float xhat = xs[j] * rstd;
-        xh[k * 8 + j] = xhat;
+        const float xhat = *xs[j] * rstd;
+        *xs[j] = xhat;
         dw[k * 8 + j] = fmaf(gs[j], xhat, dw[k * 8 + j]);
-        const float t = gs[j] * ws[j];
-        gw[k * 8 + j] = t;
-        dot = fmaf(t, xhat, dot);
+        dot = fmaf(gs[j] * ws[j], xhat, dot);
       }
     }
     dot = warp_sum(dot) * (1.f / (float)D);
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-      const int c = (lane + 32 * k) * 8;
+      const long long at = (long long)r * D + (lane + 32 * k) * 8;
+      const float2 g0 = unpack_bf16(gv[k].x), g1 = unpack_bf16(gv[k].y), g2 = unpack_bf16(gv[k].z), g3 = unpack_bf16(gv[k].w);
+      const float2 w0 = unpack_bf16(wv[k].x), w1 = unpack_bf16(wv[k].y), w2 = unpack_bf16(wv[k].z), w3 = unpack_bf16(wv[k].w);
+      const float gs[8] = {g0.x, g0.y, g1.x, g1.y, g2.x, g2.y, g3.x, g3.y};
+      const float ws[8] = {w0.x, w0.y, w1.x, w1.y, w2.x, w2.y, w3.x, w3.y};
+      const float xh[8] = {xa[k].x, xa[k].y, xa[k].z, xa[k].w, xb[k].x, xb[k].y, xb[k].z, xb[k].w};
+      const float gi[8] = {ga[k].x, ga[k].y, ga[k].z, ga[k].w, gb[k].x, gb[k].y, gb[k].z, gb[k].w};
       float o[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = rstd * (gw[k * 8 + j] - xh[k * 8 + j] * dot);
-      if (g_xnew != nullptr) {
-        const float4 ga = *reinterpret_cast<const float4*>(g_xnew + (long long)r * D + c);
-        const float4 gb = *reinterpret_cast<const float4*>(g_xnew + (long long)r * D + c + 4);
-        o[0] += ga.x; o[1] += ga.y; o[2] += ga.z; o[3] += ga.w; o[4] += gb.x; o[5] += gb.y; o[6] += gb.z; o[7] += gb.w;
-      }
-      float4* out = reinterpret_cast<float4*>(g_x + (long long)r * D + c);
+      for (int j = 0; j < 8; ++j) o[j] = rstd * (gs[j] * ws[j] - xh[j] * dot) + gi[j];
+      float4* out = reinterpret_cast<float4*>(g_x + at);
       out[0] = make_float4(o[0], o[1], o[2], o[3]);
       out[1] = make_float4(o[4], o[5], o[6], o[7]);
       if (g_delta != nullptr)
-        *reinterpret_cast<uint4*>(g_delta + (long long)r * D + c) =
+        *reinterpret_cast<uint4*>(g_delta + at) =
             make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7]));
     }
   }
@@ -363,6 +388,9 @@ add_rmsnorm_bwd_wide_kernel(const float* g_xnew, const __nv_bfloat16* g_h,
   float dw[NV * 8];
 #pragma unroll
   for (int i = 0; i < NV * 8; ++i) dw[i] = 0.f;
+  uint4 wr[NV];                                            // the same columns of w for every row
+#pragma unroll
+  for (int k = 0; k < NV; ++k) wr[k] = *reinterpret_cast<const uint4*>(w + c0 + k * 256);
   int par = 0;
   for (int r = blockIdx.x; r < rows; r += gridDim.x, par ^= 1) {
     const long long base = (long long)r * D + c0;
@@ -387,7 +415,7 @@ add_rmsnorm_bwd_wide_kernel(const float* g_xnew, const __nv_bfloat16* g_h,
     float dot = 0.f;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-      const uint4 wv = *reinterpret_cast<const uint4*>(w + c0 + k * 256);
+      const uint4 wv = wr[k];
       const float2 g0 = unpack_bf16(gv[k].x), g1 = unpack_bf16(gv[k].y), g2 = unpack_bf16(gv[k].z), g3 = unpack_bf16(gv[k].w);
       const float2 w0 = unpack_bf16(wv.x), w1 = unpack_bf16(wv.y), w2 = unpack_bf16(wv.z), w3 = unpack_bf16(wv.w);
       const float xs[8] = {xa[k].x, xa[k].y, xa[k].z, xa[k].w, xb[k].x, xb[k].y, xb[k].z, xb[k].w};
@@ -403,7 +431,7 @@ add_rmsnorm_bwd_wide_kernel(const float* g_xnew, const __nv_bfloat16* g_h,
     dot = rms_block_sum(dot, red[par], warps, warp, lane) / (float)D;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-      const uint4 wv = *reinterpret_cast<const uint4*>(w + c0 + k * 256);
+      const uint4 wv = wr[k];
       const float2 g0 = unpack_bf16(gv[k].x), g1 = unpack_bf16(gv[k].y), g2 = unpack_bf16(gv[k].z), g3 = unpack_bf16(gv[k].w);
       const float2 w0 = unpack_bf16(wv.x), w1 = unpack_bf16(wv.y), w2 = unpack_bf16(wv.z), w3 = unpack_bf16(wv.w);
       const float xs[8] = {xa[k].x, xa[k].y, xa[k].z, xa[k].w, xb[k].x, xb[k].y, xb[k].z, xb[k].w};
@@ -818,9 +846,18 @@ TLM_API int tlm_add_rmsnorm_bwd(const float* g_xnew, const void* g_h, const floa
                                 const void* w, float* g_x, void* g_delta, float* dw, int rows, int D,
                                 cudaStream_t st) {
   if (D % 256 == 0 && D / 256 <= 4) {
-    const int grid = grid_for((rows + 7) / 8, 1, 4);
-#define TLM_RMS_CASE(NV) case NV: return launch_overlapped(add_rmsnorm_bwd_reg_kernel<NV>, dim3(grid), dim3(256), 0, st, 1, g_xnew, (const __nv_bfloat16*)g_h, x_new, rstd, \
-      (const __nv_bfloat16*)w, g_x, (__nv_bfloat16*)g_delta, dw, rows);
+    // Blocks of eight rows, one resident set of them (two for many rows, whose last blocks would else be a partial set); of four
+    // rows while that leaves SMs without one: every block adds all D columns into dw (1500 x 768 in blocks of four 5.9 us, of
+    // eight 4.9)
+    auto blocks = [&](int T, int per_sm) {
+      const int full = grid_for((rows + 7) / 8, 1, per_sm), some = (rows + 3) / 4;
+      return T == 256 || full >= num_sms() ? full : (some < num_sms() ? some : num_sms());
+    };
+#define TLM_RMS_CASE(NV) case NV: { \
+      constexpr int T = rms_bwd_threads<NV>(); \
+      const int grid = blocks(T, T == 256 ? 4 : rows < 16384 ? 3 : 6); \
+      return launch_overlapped(add_rmsnorm_bwd_reg_kernel<NV>, dim3(grid), dim3(T), 0, st, 1, g_xnew, (const __nv_bfloat16*)g_h, x_new, rstd, \
+                               (const __nv_bfloat16*)w, g_x, (__nv_bfloat16*)g_delta, dw, rows); }
     switch (D / 256) { TLM_RMS_CASE(1) TLM_RMS_CASE(2) TLM_RMS_CASE(3) TLM_RMS_CASE(4) }
 #undef TLM_RMS_CASE
     return -4;
