@@ -198,6 +198,21 @@ def test_small_tile_gemm(nat, bn, split, M, N, K):
 SPLIT_PLANS = [(64, 1), (64, 2), (64, 4), (64, 8), (128, 1), (128, 2), (128, 4), (128, 8)]
 
 
+@pytest.mark.parametrize("epi,M,N,K,small", [
+    (4, 16, 6000, 2048, False), (4, 24, 5632, 1536, False), (4, 64, 5632, 1536, True), (0, 8, 32000, 256, False),   # few rows
+    (1, 1024, 3872, 80, False), (1, 2688, 1024, 288, False), (1, 1024, 1024, 1512, True),                           # weight gradients
+    (0, 966, 1536, 6784, True), (0, 333, 1024, 4096, True), (0, 8192, 4096, 1024, False)])
+def test_small_tiles_where_they_measured_faster(nat, epi, M, N, K, small):
+    """The cost rule at shapes of both kinds (148 SMs): few rows of a narrow operand and many CTAs, weight gradients over few
+    tokens. The 128-wide tiles lose to the 64-wide ones in long reductions that come out of memory."""
+    if nat.lib().tlm_num_sms() != 148:
+        pytest.skip("the times behind the rule are those of 148 SMs")
+    plan = nat.lib().tlm_gemm_split_plan(M, N, K, epi)
+    assert (plan != 0) == small, divmod(plan, 16)
+    if (M, N, K) == (966, 1536, 6784):
+        assert divmod(plan, 16) == (64, 1)
+
+
 @pytest.mark.parametrize("bn,split", SPLIT_PLANS)
 @pytest.mark.parametrize("hd,Hq,Hkv,B,T,K", [(32, 5, 1, 3, 50, 520), (64, 3, 1, 2, 129, 1000), (64, 1, 1, 1, 7, 512), (128, 2, 1, 5, 33, 576)])
 def test_small_tile_heads(nat, bn, split, hd, Hq, Hkv, B, T, K):

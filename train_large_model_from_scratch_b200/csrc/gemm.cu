@@ -1721,6 +1721,17 @@ TLM_API int tlm_gemm(const void* A, const void* B, void* C, int M, int N, int K,
   return dispatch(a_mn != 0, b_mn != 0, epi, ma, mb, p, tiles * p.split_k, stream, pair);
 }
 
+// What the rule makes of a product of that size with contiguous operands (for tests): 16 * tile width + CTAs per tile of the
+// small-tile GEMM, 0 for the wide tiles. epi: a SplitEpilogue; weight gradients (SPLIT_F32_ACC) without split reduction.
+TLM_API int tlm_gemm_split_plan(int M, int N, int K, int epi) {
+  SplitGemm g{};
+  g.M = M; g.N = N; g.K = K; g.epi = epi; g.hd = 64;
+  g.a_mn = epi == SPLIT_F32_ACC; g.b_mn = epi == SPLIT_F32_ACC || epi == SPLIT_SWIGLU_BWD;
+  g.lda = g.a_mn ? M : K; g.ldb = g.b_mn ? N : K; g.ldc = N;
+  const SplitPlan plan = split_plan(g, wide_cost(M, N, epi == SPLIT_SWIGLU ? 128 : BN, K, use_pair(M), epi == SPLIT_F32_ACC ? 1 : 0));
+  return plan.bn ? 16 * plan.bn + plan.split : 0;
+}
+
 // Grouped forward / dgrad: rows of A and C are grouped (`row_start`, device,
 // groups+1 ints, ascending, row_start[groups] == M); group g multiplies by
 // B[g] ([N,K] K-major or [K,N] MN-major, `b_group_stride` elements apart).

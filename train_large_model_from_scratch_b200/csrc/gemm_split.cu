@@ -345,19 +345,26 @@ int split_run(const SplitGemm& g, const SplitPlan& plan, cudaStream_t st) {
   return -2;
 }
 
-// Estimated time in us, fitted to 30 shapes (M 16 - 4096, N 256 - 3072, K 256 - 50304, operands in L2): a k-block takes
-// 0.24 us (64 columns) or 0.27 us (128 columns) of a CTA, fitted: 24 and 32 KB at 52 and 62 B per clock and SM out of L2 (at
-// 1.965 GHz; an SM gets no more than 64), and no less than all CTAs' blocks take at 14 TB/s out of the whole L2 (7.5 TB/s when the operands do not stay in it:
-// 2560 x 512, K 50304 on 80 CTAs took 273 us against 224 us on wide tiles), 1.3 times as long when the rows of a K-major
-// operand do not start on 128-byte lines (2436 x 512, K 1384: 16.4 us, wide tiles 14.5); plus what surrounds the main loop and the
-// exchange of the partial tiles. A weight gradient has to win clearly: the wide tiles add to C with whole TMA boxes.
+// Estimated time in us, fitted to 380 products (M 1 - 8192, N 256 - 50304, K 8 - 8000; every plan and the wide tiles timed with
+// operands in L2 and with weights and gradients out of memory). A k-block takes 0.24 us (64 columns, four stages) or 0.33 us
+// (128 columns: 0.27 out of L2, 0.36 where three stages are not enough for the latency of memory: 966 x 1536, K 6784 took 41.5 us
+// on 128 columns, 33.7 on 64, 35.9 on wide tiles) of a CTA, and no less than all CTAs' blocks take at 17.6 TB/s out of the whole
+// L2 (7.5 TB/s when the operands do not stay in it: 2560 x 512, K 50304 on 80 CTAs took 273 us against 224 us on wide tiles),
+// 1.3 times as long when the rows of a K-major operand do not start on 128-byte lines (2436 x 512, K 1384: 16.4 us, wide tiles
+// 14.5); plus what surrounds the main loop and the exchange of the partial tiles. Few rows: when all of A is less than 128 KB, its
+// lines come from too few places in L2, and the CTAs wait for each other there, 3.5 ns each per k-block (6000 gate | up columns,
+// K 2048, on 188 CTAs: 28 us at 24 rows, 12.3 us at 32; wide tiles 14.8). A weight gradient's C is read and written by the
+// reductions, 4 bytes at 6.5 TB/s (1024 x 3872, K 80: 9.1 us, wide tiles 7.7), and has to win clearly: the wide tiles add
+// whole TMA boxes. Of the 380 products none is more than 4 % slower than on wide tiles (28 were without the last three terms).
 SplitPlan split_plan(const SplitGemm& g, double wide_us) {
   SplitPlan best{0, 0};
   if (!aligned_ok(g)) return best;
   const long long kblocks = (g.K + SP_BK - 1) / SP_BK, slots = 2LL * num_sms();
   const double operand_bytes = 2.0 * g.K * ((double)g.M + (g.epi == SPLIT_SWIGLU ? 2.0 : 1.0) * g.N);
   const double lines = (!g.a_mn && g.lda % 64 != 0) || (!g.b_mn && g.ldb % 64 != 0) ? 1.3 : 1.0;
-  const double l2_rate = operand_bytes > 64e6 ? 7.5e6 : 14e6;          // bytes per us
+  const double l2_rate = operand_bytes > 64e6 ? 7.5e6 : 17.6e6;        // bytes per us
+  const double per_cta = !g.a_mn && 2.0 * g.M * g.K < 131072.0 ? 0.0035 : 0.0;
+  const double c_us = g.epi == SPLIT_F32_ACC ? 4.0 * g.M * g.N / 6.5e6 : 0.0;
   static const double exchange[2][4] = {{0.0, 1.5, 1.3, 2.8}, {0.0, 2.2, 2.0, 2.3}};       // S = 1, 2, 4, 8
   double best_us = (g.epi == SPLIT_F32_ACC ? 0.85 : 0.95) * wide_us;
   for (int bn = 64; bn <= 128; bn *= 2) {
@@ -367,9 +374,12 @@ SplitPlan split_plan(const SplitGemm& g, double wide_us) {
     for (int i = 0, s = 1; s <= 8 && s <= kblocks; ++i, s *= 2) {
       const long long ctas = tiles * s, resident = ctas < slots ? ctas : slots;
       if (ctas > (s > 1 ? num_sms() : slots)) continue;          // a second wave of clusters costs more than it saves
-      const double alone = bn == 64 ? 0.24 : 0.27, shared = (double)resident * (bn == 64 ? 24576.0 : 32768.0) / l2_rate;
-      const double us = (bn == 64 ? 3.4 : 3.8) + (g.a_mn ? 1.0 : 0.0) + exchange[bn / 128][i] +
-                        (double)((kblocks + s - 1) / s) * lines * (alone > shared ? alone : shared);
+      double block = bn == 64 ? 0.24 : 0.33;
+      const double shared = (double)resident * (bn == 64 ? 24576.0 : 32768.0) / l2_rate, queue = (double)resident * per_cta;
+      if (shared > block) block = shared;
+      if (queue > block) block = queue;
+      const double us = (bn == 64 ? 3.4 : 3.8) + (g.a_mn ? 1.0 : 0.0) + exchange[bn / 128][i] + c_us +
+                        (double)((kblocks + s - 1) / s) * lines * block;
       if (us < best_us) { best_us = us; best = {bn, s}; }
     }
   }

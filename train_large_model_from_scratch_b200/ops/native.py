@@ -57,6 +57,7 @@ _SIGS = {
     "tlm_gemm": (_I, [_P, _P, _P, _I, _I, _I, _LL, _LL, _LL, _I, _I, _I, _P]),
     "tlm_gemm_split": (_I, [_P, _P, _P, _I, _I, _I, _LL, _LL, _LL, _I, _I, _I, _I, _I, _P]),
     "tlm_gemm_split_heads": (_I, [_P, _P, _P] + [_I] * 6 + [_P, _P, _I, _I, _P]),
+    "tlm_gemm_split_plan": (_I, [_I] * 4),
     "tlm_gemm_split_swiglu": (_I, [_P] * 5 + [_I] * 6 + [_P]),
     "tlm_gemm_heads": (_I, [_P, _P, _I, _I, _I, _LL, _LL, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P, _P, _P]),
     "tlm_blocks_forward": (_I, [_P, _I] + [_P] * 10 + [_I] * 7 + [_F, _F] + [_P] * 4),
