@@ -689,6 +689,29 @@ def test_moe_route_and_row_movement(nat, M, E, k):
     assert _rel_err(dl, lf.grad) < 1e-2
 
 
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("D", [8, 256, 264, 512, 768, 1032, 1280])
+def test_moe_combine_and_pair_dot_batches(nat, k, D):
+    """The batches of rows (combine) and of 512-byte pieces (pair-dot) in flight follow k and D: full, partly empty and several
+    batches, pairs that were dropped (place -1). Sums in fp32: one bf16 rounding of the combined row, 2^-9 / sqrt(3)."""
+    M = 37
+    g = torch.Generator(device="cuda").manual_seed(120)
+    pos = torch.randperm(M * k, device="cuda", generator=g).int()
+    dropped = torch.rand(M * k, device="cuda", generator=g) < 0.2
+    pos[dropped] = -1
+    y, d_out = _rand(M * k, D, seed=121), _rand(M, D, seed=122)
+    w = torch.rand(M, k, device="cuda", generator=g)
+    rows = y.double()[pos.long().clamp(min=0)].view(M, k, D) * (~dropped).view(M, k, 1)
+    for weights in (w, None):
+        out = nat.moe_combine(y, pos, weights, M, k).double()
+        ref = (rows * (1.0 if weights is None else w.double()[:, :, None])).sum(1)
+        assert ((out - ref).norm() / ref.norm()).item() < 2.5e-3
+    dw = nat.moe_pair_dot(d_out, y, pos, k)
+    ref = (d_out.double()[:, None, :] * rows).sum(-1).reshape(-1)
+    torch.testing.assert_close(dw.double(), ref, rtol=1e-4, atol=1e-3)
+    assert bool((dw[dropped] == 0).all())
+
+
 def test_grouped_gemm_row_scatter_epilogue(nat, gemm_mode):
     """Grouped GEMM whose epilogue stores each output row at a looked-up (buffer, row): two local buffers
     stand in for two ranks; rows flagged -1 are dropped."""
