@@ -227,7 +227,8 @@ __global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ x, const int
 // together (U = 4; fewer for k below 4, whose batches would be partly empty: 32768 tokens, k 2, 1024 columns took 40.7 us with
 // U = 4, 36.5 with 2; 16384, k 1, 1024 columns 13.0 and 9.1 with 1; 8192, k 8 27.5, one row after the other 30.3).
 template <int U>
-__global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ pos,
+__global__ void __launch_bounds__(256, U == 2 ? 6 : U == 1 ? 8 : 4)      // U 2: 38 registers and six blocks per SM (47 and five: 6000 x 1024 9.8 us, now 7.7)
+moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ pos,
                                    const float* __restrict__ w, __nv_bfloat16* __restrict__ out, int M, int D, int k) {
   const int lane = threadIdx.x & 31;
   const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
