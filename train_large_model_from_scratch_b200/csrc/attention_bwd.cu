@@ -6,30 +6,23 @@
 //
 // Three launches:
 //   1. delta[b,h,t] = sum_d do*o; the dQ accumulator is zeroed on the way (few rows: by a memset)
-//   2. main kernel: one CTA per (128-row KV tile, batch, KV head). K and V stay in
-//      shared memory; the CTA walks over every query head of the group and every
-//      query tile at or below the diagonal. Per step five MMAs run on the
-//      tensor cores:   S = Q K^T,  dP = dO V^T            (TMEM, fp32)
-//                      dV += P^T dO,  dK += dS^T Q         (TMEM accumulators)
-//                      dQ  = dS K                          (TMEM, flushed per step)
-//      P and dS are written once to shared memory as [q][kv] bf16 tiles in the
-//      swizzled operand layout; read as K-major they feed dQ, read as MN-major
-//      they are P^T / dS^T, and Q / dO / K / V tiles are used as loaded (MN-major
-//      where the product needs their transpose), so nothing is transposed.
-//      Two softmax warpgroups (one thread per query row, half of the KV columns
-//      each) turn S, dP into P, dS; dQ tiles are added to an fp32 buffer with
-//      TMA reduce-add tile stores because several KV tiles contribute to one query row.
-//      For hd 32 and 64 the next step's S / dP MMAs are issued while the softmax
-//      warps still work on the current step; hd 128 has its own order (see the HD 128 loops).
+//   2. main kernel: one CTA per (128-row KV tile, batch, KV head). The CTA walks over every query head of the group and
+//      every query tile at or below the diagonal. Per step five products run on the tensor cores, scores transposed:
+//                      S^T = K Q^T,  dP^T = V dO^T       (TMEM, fp32; rows = keys, columns = queries)
+//                      dV += P^T dO,  dK += dS^T Q       (TMEM accumulators; P^T / dS^T are TMEM operands)
+//                      dQ  = dS K                        (TMEM, flushed per step)
+//      so P never leaves tensor memory and only dS goes through shared memory, as the [kv][q] bf16 tile that dQ reads
+//      MN-major. Q / dO / K / V tiles are used as loaded.
+//      Warps: 0 loads (Q, dO by TMA; -lse log2 e and -delta of the step's rows by the warp), 1 issues the products,
+//      2 - 17 softmax (32 keys x 32 queries each: P, dS), 18 - 21 take dQ out: tiles are added to an fp32 buffer with TMA
+//      reduce-add tile stores because several KV tiles contribute to one query row.
 //      With few KV tiles a cluster of CTAs shares a tile's steps (SPLIT, see split_for).
 //   3. dq (fp32, [B,Hq,T,hd]) -> bf16 into dqkv; with RoPE tables this pass also applies the transposed rotation to
 //      dQ (from the fp32 accumulator) and to the dK slots the main kernel wrote, so the packed gradient that leaves
 //      is the gradient of the UN-rotated q and k and no separate RoPE pass runs.
 // A second instantiation of the main kernel (SCATTER) serves Ulysses sequence parallelism: its dK / dV epilogue
 // rotates dK itself and stores the rows straight into the sequence owners' packed gradient buffers, and the
-// conversion pass does the same for dQ. The plain instantiation carries none of that code: this kernel's main loop
-// is sensitive to anything that changes its register allocation, and in-step timing (not the isolated kernel
-// benchmark) decides what stays in it.
+// conversion pass does the same for dQ.
 // Every wait is bounded; on a timeout the CTA records a status code, leaves its
 // loops and still releases its tensor memory.
 #include "common.cuh"
@@ -37,7 +30,7 @@
 
 namespace tlm {
 
-constexpr int AB_TILE = 128, AB_THREADS = 320, AB_MAX_DST = 8;
+constexpr int AB_TILE = 128, AB_THREADS = 704, AB_MAX_DST = 8;
 
 struct AttnBwdDst {
   __nv_bfloat16* p[AB_MAX_DST];
@@ -47,6 +40,7 @@ struct AttnBwdDst {
 struct AttnBwdParams {
   __nv_bfloat16* dqkv;
   float* dq_acc;            // [B,Hq,T,hd] fp32, zeroed before the main kernel
+  const __nv_bfloat16* qkv;
   const float* lse;
   const float* delta;
   int B, T, Hq, Hkv;
@@ -66,39 +60,6 @@ struct AttnBwdParams {
   int n_dst, dst_rows, dst_heads, dst_q0, dst_k0, dst_v0;
   int split;               // SPLIT instantiation: CTAs of the cluster that share one KV tile's steps
   int head_group;          // (batch, KV head) pairs per group of the heavy-first block order (see heavy_first_decode)
-};
-
-template <int HD>
-struct AttnBwdCfg {
-  // Q / dO ring. Three stages for hd 64: the MMA warp issues S / dP of step it+1 before dV / dK / dQ of step
-  // it, so the load of step it+1 must have been started a whole step earlier (when step it-2 retired) for its
-  // latency to stay off the tensor pipe's critical path.
-  static constexpr int STAGES = HD <= 64 ? 3 : 2;        // of Q; HD 128 has room for one dO tile (see the HD 128 loops)
-  static constexpr int DO_STAGES = HD <= 64 ? 3 : 1;
-  static constexpr bool PIPELINED = HD <= 64;            // dQ has its own TMEM columns
-  static constexpr int TILE_BYTES = AB_TILE * HD * 2;
-  static constexpr int PD_BYTES = AB_TILE * AB_TILE * 2;
-  static constexpr int OFF_K = 0;
-  static constexpr int OFF_V = OFF_K + TILE_BYTES;
-  static constexpr int OFF_Q = OFF_V + TILE_BYTES;
-  static constexpr int OFF_DO = OFF_Q + STAGES * TILE_BYTES;
-  static constexpr int OFF_P = OFF_DO + DO_STAGES * TILE_BYTES;
-  static constexpr int OFF_DS = OFF_P + PD_BYTES;
-  // dQ staging: one [32 rows][32 fp32] swizzled box per softmax warp (HD 128: the warp's own parts of P and dS instead)
-  static constexpr int OFF_DQS = OFF_DS + PD_BYTES;
-  static constexpr int DQS_BYTES = HD <= 64 ? 8 * 4096 : 0;
-  static constexpr int PART_PITCH = 2 * HD + 4;          // SPLIT: floats per row of this CTA's dV | dK, from OFF_Q on
-  static constexpr int OFF_BAR = OFF_DQS + DQS_BYTES;
-  static_assert(OFF_Q + AB_TILE * PART_PITCH * 4 <= OFF_BAR, "the partial dV | dK fits behind K and V");
-  static constexpr int TOTAL = OFF_BAR + 256 + 1024;
-  static constexpr uint32_t S_COL = 0, DP_COL = 128, DV_COL = 256, DK_COL = 256 + HD;
-  // hd 64: dQ has two 64-column buffers (steps alternate), so dQ of step it can be issued while the softmax
-  // warps still drain dQ of step it-1. hd 128: dQ reuses the dP columns (no spare tensor memory).
-  static constexpr uint32_t DQ_COL = HD <= 64 ? 384 : 128;
-  static constexpr uint32_t DQ_BUF_COLS = HD <= 64 ? 64 : 0;
-  // columns of dQ, dK, dV one softmax warp carries out: half of the head, or with HD 32 all of it, in turns (a flush box
-  // is 32 columns wide)
-  static constexpr int OUT_COLS = HD == 32 ? 32 : HD / 2;
 };
 
 // delta[b, h, t] = sum_c o[b, t, h, c] * dout[b, t, h, c]. One block per (b, 32 consecutive t): that slab of o
@@ -227,6 +188,81 @@ __global__ void attn_dq_convert_kernel(const float* dq_acc, __nv_bfloat16* __res
   }
 }
 
+// What a step consists of, and what bounds it. Every step is taken in two halves of 64 query columns, each with its own eight
+// softmax warps and barriers: while one half's exponentials run, the other half's products do. For head dims 32 and 64 there
+// are three score tiles for the two halves, so a half's scores of its next step are there before its warps ask for them
+// (two tiles: 1048 us against 974 at the first shape below); dP^T of the next step is issued as soon as a half has published
+// P^T and dS^T, and its warps come to it only after their exponentials. Head dim 128 (WIDE) has 256 tensor-memory columns
+// beside dV and dK: scores of both halves, and dP^T in turns with dQ; a step's chain is dQ -> its way out, beside dV, dK and
+// the next scores -> dP^T -> dS, and the exponentials of the next step run beside the last link.
+// Cycles per 128 x 128 step, head dim 64 / 32: products 1664 / 832, exponentials 1024 (16 a cycle), shared memory 300 KB /
+// 184 KB at 128 B a cycle; measured 2640 / 2460, head dim 128 about 4700. Long runs are under the power cap at 1.5 - 1.7 GHz,
+// so what counts is energy: without the dQ reductions to L2 head dim 64 would take 8 % less, without any other part 2 - 4 %.
+// In us with the delta and conversion passes, in sequence, against the form before (scores [q][kv], P and dS through shared
+// memory, eight softmax warps that also flushed dQ, products issued by one lane's own code):
+//   B 8, T 4096, 16 / 8 heads of 64: 1115 -> 974     B 1, T 32768, the same: 7440 -> 6270
+//   B 8, T 4096, 32 / 4 heads of 32: 2083 -> 1520    B 2, T 4096, 24 / 8 heads of 128: 941 -> 774
+// The one lane was the largest part: every MMA operand then goes from an ordinary to a uniform register on its own, and a
+// step's products took 76 cycles each to issue, whatever their size (see umma_bf16_w).
+template <int HD>
+struct AttnBwdCfg {
+  static constexpr bool WIDE = HD == 128;
+  static constexpr int KB = WIDE ? 2 : 1;                     // 64-wide blocks of a tile (HD 32: one of 32)
+  static constexpr int STAGES = WIDE ? 2 : 3;                 // Q / lse / delta ring
+  static constexpr int DO_STAGES = WIDE ? 1 : 3;
+  static constexpr int DS_BUFS = WIDE ? 1 : 2;
+  static constexpr int NS = WIDE ? 2 : 3;                     // score tiles (half steps)
+  static constexpr bool KV_TMEM = HD == 32;                   // K and V as operands in tensor memory
+  static constexpr int TILE_BYTES = AB_TILE * HD * 2;
+  static constexpr int OFF_K = 0;
+  static constexpr int OFF_V = OFF_K + TILE_BYTES;
+  static constexpr int OFF_Q = OFF_V + (KV_TMEM ? 0 : TILE_BYTES);
+  static constexpr int OFF_DO = OFF_Q + STAGES * TILE_BYTES;
+  static constexpr int OFF_DS = OFF_DO + DO_STAGES * TILE_BYTES;   // buffers of [2 query halves][128 kv][64 q] bf16
+  static constexpr int DS_BYTES = AB_TILE * AB_TILE * 2;
+  static constexpr int OFF_DQS = OFF_DS + DS_BUFS * DS_BYTES;  // dQ staging: [32 rows][32 fp32] boxes of the four flush warps
+  static constexpr int BOXES = WIDE ? 2 : 1;
+  static constexpr int OFF_ROW = OFF_DQS + 4 * BOXES * 4096;
+  static constexpr int OFF_BAR = OFF_ROW + STAGES * 2 * AB_TILE * 4;
+  static constexpr int TOTAL = OFF_BAR + 256;
+  static_assert(TOTAL <= 232448, "shared memory of one block");
+  static constexpr int PART_PITCH = 2 * HD + 4;                // SPLIT: floats per row of this CTA's dV | dK, from OFF_Q on
+  static_assert(AB_TILE * PART_PITCH * 4 <= (WIDE ? OFF_ROW : OFF_DS) - OFF_Q, "the partial dV | dK fits behind K and V");
+  // tensor memory: NS tiles of S^T (a half step's P^T and dS^T replace them as bf16), two of dP^T, dV, dK, dQ, K and V.
+  // WIDE: dQ takes turns with dP^T.
+  static constexpr uint32_t S_COL = 0, DP_COL = NS * 64, DV_COL = DP_COL + 128, DK_COL = DV_COL + HD, DQ_COL = WIDE ? DP_COL : DK_COL + HD;
+  static constexpr uint32_t K_COL = DQ_COL + HD, V_COL = K_COL + HD / 2;
+  static_assert((WIDE ? DK_COL + HD : KV_TMEM ? V_COL + HD / 2 : DQ_COL + HD) <= 512, "tensor memory");
+  static constexpr int OUT_COLS = HD / 4;                      // columns of dV and of dK one softmax warp carries out
+};
+
+// P of 32 query columns of one KV row: scores from tensor memory, -lse of the columns from shared memory; columns below
+// `masked` come before the row (DIAG).
+template <bool DIAG>
+__device__ __forceinline__ void attn_bwd_p(uint32_t t_s, const float* nlse, float2 sc2, int masked, float2* pr) {
+#pragma unroll
+  for (int c = 0; c < 32; c += 16) {
+    uint32_t sv[16];
+    tmem_ld16(t_s + c, sv);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 16; i += 4) {
+      const float4 nl = *reinterpret_cast<const float4*>(nlse + c + i);
+      const float2 x = ffma2(make_float2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sc2, make_float2(nl.x, nl.y));
+      const float2 y = ffma2(make_float2(__uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3])), sc2, make_float2(nl.z, nl.w));
+      float2* o = pr + ((c + i) >> 1);
+      o[0] = make_float2(ex2_approx(x.x), ex2_approx(x.y));
+      o[1] = make_float2(ex2_approx(y.x), ex2_approx(y.y));
+      if (DIAG) {
+        if (c + i < masked) o[0].x = 0.f;
+        if (c + i + 1 < masked) o[0].y = 0.f;
+        if (c + i + 2 < masked) o[1].x = 0.f;
+        if (c + i + 3 < masked) o[1].y = 0.f;
+      }
+    }
+  }
+}
+
 // SPLIT: a cluster of p.split CTAs works on one KV tile, each on its share of the (query head, query tile) steps; every CTA
 // leaves its fp32 dV | dK in its own shared memory and the cluster adds them up, in fixed order. See split_for.
 template <int HD, bool SCATTER, bool SPLIT>
@@ -234,21 +270,23 @@ __global__ void __launch_bounds__(AB_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
                 const __grid_constant__ CUtensorMap tm_dq, const AttnBwdParams p) {
   using C = AttnBwdCfg<HD>;
-  constexpr int KB = HD == 128 ? 2 : 1;
   constexpr uint32_t TMEM_COLS = 512;
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* sal = smem_raw + (sbase - smem_u32(smem_raw));
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t sbase = smem_u32(smem_raw);
+  uint8_t* sal = smem_raw;
+  if (sbase & 1023u) {                                // swizzled tiles need a 1024-byte aligned base
+    if (threadIdx.x == 0) report_status(p.status, (20u << 8) | 2u);
+    return;
+  }
   const uint32_t bar0 = sbase + C::OFF_BAR;
-  // barriers: 0,1 dq_consumed[buffer]  4 kv_full  5 sdp_full  6 sdp_consumed  7 pds_full  8 dq_full
-  //           10.. qdo_full[stage]  13.. qdo_empty[stage]
-  // HD 128:   1 dq_consumed  4 kv_full  5 s_full  6 s_consumed  7 pds_full  8 dq_full  9 dp_full  10,11 q_full[stage]
-  //           12 do_full  13,14 q_empty[stage]  15 do_empty
+  // barriers; [n] of a half, buffer, stage or score tile
+  enum { KV_FULL = 0, KV_TMEM = 1, DP_FULL = 2 /* [2] */, PDS = 4 /* [2]: P^T, dS^T published */, DQ_FULL = 6 /* [2] */, DQ_FREE = 8,
+         RING_FULL = 9 /* [3] */, RING_EMPTY = 12 /* [3] */, S_FULL = 15 /* [3] */, DO_FULL = 18, DO_EMPTY = 19, ALL_DONE = 20, N_BARS = 21 };
   auto bar = [&](int i) { return bar0 + 8u * i; };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sal + C::OFF_BAR + 128);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sal + C::OFF_BAR + 192);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int n_tiles = (p.T + AB_TILE - 1) / AB_TILE;
   int j, bh;                                                  // KV tile (tile 0 has the most query tiles), (batch, KV head)
   const int split = SPLIT ? p.split : 1, rank = SPLIT ? (int)cluster_ctarank() : 0;
@@ -261,7 +299,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
   const int heads_total = p.Hq + 2 * p.Hkv;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 16; ++i) mbar_init(bar(i), (i == 0 || i == 1 || i == 6 || i == 7) ? 8 : 1);
+    for (int i = 0; i < N_BARS; ++i)
+      mbar_init(bar(i), i == KV_TMEM ? 16 : (i == PDS || i == PDS + 1) ? 8 : i == DQ_FREE ? 4 : (i >= RING_FULL && i < RING_EMPTY) ? 2 : 1);
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tm_qkv);
@@ -272,439 +311,387 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   griddep_wait();
 
   if (warp == 0) {
-    // ---------------------------------------------------------------- TMA producer
+    // ---------------------------------------------------------------- producer: Q, dO by TMA; -lse, -delta by the warp
     if (lane == 0) {
-      mbar_expect_tx(bar(4), 2 * C::TILE_BYTES);
+      mbar_expect_tx(bar(KV_FULL), (C::KV_TMEM ? 1 : 2) * C::TILE_BYTES);
 #pragma unroll
-      for (int kb = 0; kb < KB; ++kb) {
-        tma_load_4d(sbase + C::OFF_K + kb * 16384, &tm_qkv, bar(4), kb * 64, p.Hq + kvh, j * AB_TILE, b);
-        tma_load_4d(sbase + C::OFF_V + kb * 16384, &tm_qkv, bar(4), kb * 64, p.Hq + p.Hkv + kvh, j * AB_TILE, b);
+      for (int kb = 0; kb < C::KB; ++kb) {
+        tma_load_4d(sbase + C::OFF_K + kb * 16384, &tm_qkv, bar(KV_FULL), kb * 64, p.Hq + kvh, j * AB_TILE, b);
+        if (!C::KV_TMEM) tma_load_4d(sbase + C::OFF_V + kb * 16384, &tm_qkv, bar(KV_FULL), kb * 64, p.Hq + p.Hkv + kvh, j * AB_TILE, b);
       }
-      if constexpr (!C::PIPELINED) {
-        for (int it = 0; it < n_it; ++it) {
-          const int st = it & 1, hq = kvh * rep + (it0 + it) / per_head, qi = j + (it0 + it) % per_head;
-          if (!mbar_wait(bar(13 + st), ((uint32_t)(it >> 1) & 1u) ^ 1u, 21, abort_flag, p.status)) break;
-          mbar_expect_tx(bar(10 + st), C::TILE_BYTES);
+    }
+    for (int it = 0; it < n_it; ++it) {
+      const int st = it % C::STAGES;
+      const int hq = kvh * rep + (it0 + it) / per_head, qi = j + (it0 + it) % per_head;
+      if (!mbar_wait_warp(bar(RING_EMPTY + st), ((uint32_t)(it / C::STAGES) & 1u) ^ 1u, 21, abort_flag, p.status)) break;
+      if (lane == 0) {
+        mbar_expect_tx(bar(RING_FULL + st), (C::WIDE ? 1 : 2) * C::TILE_BYTES);
 #pragma unroll
-          for (int kb = 0; kb < KB; ++kb)
-            tma_load_4d(sbase + C::OFF_Q + st * C::TILE_BYTES + kb * 16384, &tm_qkv, bar(10 + st), kb * 64, hq, qi * AB_TILE, b);
-          if (!mbar_wait(bar(15), ((uint32_t)it & 1u) ^ 1u, 32, abort_flag, p.status)) break;
-          mbar_expect_tx(bar(12), C::TILE_BYTES);
+        for (int kb = 0; kb < C::KB; ++kb)
+          tma_load_4d(sbase + C::OFF_Q + st * C::TILE_BYTES + kb * 16384, &tm_qkv, bar(RING_FULL + st), kb * 64, hq, qi * AB_TILE, b);
+        if (!C::WIDE) tma_load_4d(sbase + C::OFF_DO + st * C::TILE_BYTES, &tm_do, bar(RING_FULL + st), 0, hq, qi * AB_TILE, b);
+      }
+      constexpr float LOG2E = 1.4426950408889634f;
+      const long long r0 = ((long long)b * p.Hq + hq) * p.T;
+      float* rows = reinterpret_cast<float*>(sal + C::OFF_ROW) + st * 2 * AB_TILE;
+      float l[4], d[4];
 #pragma unroll
-          for (int kb = 0; kb < KB; ++kb)
-            tma_load_4d(sbase + C::OFF_DO + kb * 16384, &tm_do, bar(12), kb * 64, hq, qi * AB_TILE, b);
-        }
-      } else
-      for (int it = 0; it < n_it; ++it) {
-        const int st = it % C::STAGES;
-        const uint32_t ph = (uint32_t)(it / C::STAGES) & 1u;
-        if (!mbar_wait(bar(13 + st), ph ^ 1u, 21, abort_flag, p.status)) break;
-        const int hq = kvh * rep + (it0 + it) / per_head, qi = j + (it0 + it) % per_head;
-        mbar_expect_tx(bar(10 + st), 2 * C::TILE_BYTES);
+      for (int k = 0; k < 4; ++k) {
+        const int t = qi * AB_TILE + 32 * k + lane;
+        l[k] = t < p.T ? p.lse[r0 + t] * -LOG2E : -INFINITY;               // rows past the end: P = 0
+        d[k] = t < p.T ? -p.delta[r0 + t] : 0.f;
+      }
 #pragma unroll
-        for (int kb = 0; kb < KB; ++kb) {
-          tma_load_4d(sbase + C::OFF_Q + st * C::TILE_BYTES + kb * 16384, &tm_qkv, bar(10 + st), kb * 64, hq, qi * AB_TILE, b);
-          tma_load_4d(sbase + C::OFF_DO + st * C::TILE_BYTES + kb * 16384, &tm_do, bar(10 + st), kb * 64, hq, qi * AB_TILE, b);
+      for (int k = 0; k < 4; ++k) { rows[32 * k + lane] = l[k]; rows[AB_TILE + 32 * k + lane] = d[k]; }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(RING_FULL + st));
+      if constexpr (C::WIDE) {
+        if (!mbar_wait_warp(bar(DO_EMPTY), ((uint32_t)it & 1u) ^ 1u, 35, abort_flag, p.status)) break;
+        if (lane == 0) {
+          mbar_expect_tx(bar(DO_FULL), C::TILE_BYTES);
+#pragma unroll
+          for (int kb = 0; kb < C::KB; ++kb)
+            tma_load_4d(sbase + C::OFF_DO + kb * 16384, &tm_do, bar(DO_FULL), kb * 64, hq, qi * AB_TILE, b);
         }
       }
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = umma_idesc_bf16(AB_TILE, AB_TILE, 0, 0);     // S, dP : A, B K-major
-      constexpr uint32_t idesc_t = umma_idesc_bf16(AB_TILE, HD, 1, 1);          // dV, dK: A, B MN-major
-      constexpr uint32_t idesc_q = umma_idesc_bf16(AB_TILE, HD, 0, 1);          // dQ    : A K-major, B MN-major
-      const uint32_t sk = sbase + C::OFF_K, sv = sbase + C::OFF_V, sp = sbase + C::OFF_P, sds = sbase + C::OFF_DS;
-      // descriptors of the resident K / V tiles and of the P / dS tiles, built once
-      const uint64_t dk_k = attn_desc_k<HD>(sk), dv_k = attn_desc_k<HD>(sv);                       // K-major views
-      const uint64_t dk_mn = attn_desc_mn<HD>(sk);                                                 // K as MN-major B (dQ)
-      const uint64_t dp_mn = umma_smem_desc(sp, 16384, 1024), dds_mn = umma_smem_desc(sds, 16384, 1024);
-      const uint64_t dds_k = umma_smem_desc(sds, 16, 1024);
-      auto issue_s_dp = [&](int it) -> bool {
-        const int st = it % C::STAGES;
-        if (!mbar_wait(bar(10 + st), (uint32_t)(it / C::STAGES) & 1u, 22, abort_flag, p.status)) return false;
+    const uint32_t el = elect_one();
+    constexpr uint32_t idesc_s = umma_idesc_bf16(AB_TILE, 64, 0, 0);          // S^T, dP^T of one half: B K-major
+    constexpr uint32_t idesc_t = umma_idesc_bf16(AB_TILE, HD, 0, 1);          // dV, dK: A from tensor memory, B MN-major
+    constexpr uint32_t idesc_q = umma_idesc_bf16(AB_TILE, HD, 1, 1);          // dQ    : A, B MN-major
+    const uint64_t dk_mn = attn_desc_mn<HD>(sbase + C::OFF_K);
+    // Half step h = 2 it + s: query columns 64 s .. 64 s + 63 of step it, scores in tile h % NS. Which tile and which ring stage
+    // is carried along instead of computed from h, and s is a constant of the unrolled body: both keep the operands uniform.
+    const uint64_t dk_k = attn_desc_k<HD>(sbase + C::OFF_K), dv_k = attn_desc_k<HD>(sbase + C::OFF_V);
+    const uint64_t q_k = attn_desc_k<HD>(sbase + C::OFF_Q), do_k = attn_desc_k<HD>(sbase + C::OFF_DO);
+    const uint64_t q_mn = attn_desc_mn<HD>(sbase + C::OFF_Q), do_mn = attn_desc_mn<HD>(sbase + C::OFF_DO);
+    auto issue_sp = [&](uint32_t d, uint32_t a_tmem, uint64_t a_smem, uint64_t db) {
+#pragma unroll
+      for (int t = 0; t < HD / 16; ++t) {
+        if constexpr (C::KV_TMEM) umma_bf16_ts_w(el, d, a_tmem + t * 8, umma_desc_advance(db, t * 32), idesc_s, t > 0);
+        else umma_bf16_w(el, d, umma_desc_advance(a_smem, t * 32), umma_desc_advance(db, t * 32), idesc_s, t > 0);
+      }
+    };
+    auto ring = [&](int it, int st) -> bool {
+      const bool r = mbar_wait_warp(bar(RING_FULL + st), (uint32_t)(it / C::STAGES) & 1u, 22, abort_flag, p.status);
+      tc_fence_after();
+      return r;
+    };
+    auto issue_s = [&](int sb, int st, int s) {
+      issue_sp(tmem + C::S_COL + sb * 64, tmem + C::K_COL, dk_k, umma_desc_advance(q_k, st * C::TILE_BYTES + s * (C::TILE_BYTES / 2)));
+      umma_commit_w(el, bar(S_FULL + sb));
+    };
+    auto issue_dp = [&](int st, int s) {
+      issue_sp(tmem + C::DP_COL + s * 64, tmem + C::V_COL, dv_k, umma_desc_advance(do_k, st * C::TILE_BYTES + s * (C::TILE_BYTES / 2)));
+      umma_commit_w(el, bar(DP_FULL + s));
+    };
+    bool ok = mbar_wait_warp(bar(KV_FULL), 0, 23, abort_flag, p.status);
+    if (ok && C::KV_TMEM) ok = mbar_wait_warp(bar(KV_TMEM), 0, 34, abort_flag, p.status);
+    tc_fence_after();
+    if constexpr (C::WIDE) {
+      // One order of five products a step; S^T and dP^T of both halves in one piece (half the reads of K and V).
+      constexpr uint32_t idesc_w = umma_idesc_bf16(AB_TILE, AB_TILE, 0, 0);
+      auto issue_kk = [&](uint32_t d, uint64_t a, uint64_t bm) {
+#pragma unroll
+        for (int t = 0; t < HD / 16; ++t) {
+          const uint32_t off = (t >> 2) * 16384 + (t & 3) * 32;
+          umma_bf16_w(el, d, umma_desc_advance(a, off), umma_desc_advance(bm, off), idesc_w, t > 0);
+        }
+      };
+      auto issue_dp_w = [&](int it) -> bool {
+        if (!mbar_wait_warp(bar(DO_FULL), (uint32_t)it & 1u, 36, abort_flag, p.status)) return false;
         tc_fence_after();
-        const uint64_t dq_k = attn_desc_k<HD>(sbase + C::OFF_Q + st * C::TILE_BYTES);
-        const uint64_t ddo_k = attn_desc_k<HD>(sbase + C::OFF_DO + st * C::TILE_BYTES);
-#pragma unroll
-        for (int t = 0; t < HD / 16; ++t) {
-          const uint32_t off = (t >> 2) * 16384 + (t & 3) * 32;
-          if (t == 0) umma_bf16(tmem + C::S_COL, dq_k, dk_k, idesc_s, 0);
-          else umma_bf16_acc(tmem + C::S_COL, umma_desc_advance(dq_k, off), umma_desc_advance(dk_k, off), idesc_s);
-        }
-#pragma unroll
-        for (int t = 0; t < HD / 16; ++t) {
-          const uint32_t off = (t >> 2) * 16384 + (t & 3) * 32;
-          if (t == 0) umma_bf16(tmem + C::DP_COL, ddo_k, dv_k, idesc_s, 0);
-          else umma_bf16_acc(tmem + C::DP_COL, umma_desc_advance(ddo_k, off), umma_desc_advance(dv_k, off), idesc_s);
-        }
-        umma_commit(bar(5));
+        issue_kk(tmem + C::DP_COL, dv_k, do_k);
+        umma_commit_w(el, bar(DP_FULL));
         return true;
       };
-      bool ok = mbar_wait(bar(4), 0, 23, abort_flag, p.status);
-      // HD 128: D[128 x 128] = A B^T over 128 columns, both K-major
-      auto issue_kk = [&](uint32_t d_col, uint64_t a, uint64_t bm) {
-#pragma unroll
-        for (int t = 0; t < HD / 16; ++t) {
-          const uint32_t off = (t >> 2) * 16384 + (t & 3) * 32;
-          if (t == 0) umma_bf16(tmem + d_col, a, bm, idesc_s, 0);
-          else umma_bf16_acc(tmem + d_col, umma_desc_advance(a, off), umma_desc_advance(bm, off), idesc_s);
-        }
-      };
-      auto issue_s = [&](int it) -> bool {
-        if (!mbar_wait(bar(10 + (it & 1)), (uint32_t)(it >> 1) & 1u, 22, abort_flag, p.status)) return false;
-        tc_fence_after();
-        issue_kk(C::S_COL, attn_desc_k<HD>(sbase + C::OFF_Q + (it & 1) * C::TILE_BYTES), dk_k);
-        umma_commit(bar(5));
-        return true;
-      };
-      if (ok && (!SPLIT || n_it > 0)) ok = C::PIPELINED ? issue_s_dp(0) : issue_s(0);
+      const uint64_t dds_mn = umma_smem_desc(sbase + C::OFF_DS, 16384, 1024);
+      if (ok && n_it > 0 && (ok = ring(0, 0))) {
+        issue_kk(tmem + C::S_COL, dk_k, q_k);
+        umma_commit_w(el, bar(S_FULL));
+        ok = issue_dp_w(0);
+      }
       for (int it = 0; it < n_it && ok; ++it) {
-        const int st = it % C::STAGES;
-        const uint32_t par = (uint32_t)it & 1u;
-        if constexpr (C::PIPELINED) {
-          if (it + 1 < n_it) {
-            if (!mbar_wait(bar(6), par, 24, abort_flag, p.status)) break;          // S, dP of `it` are in registers
-            if (!issue_s_dp(it + 1)) break;
-          }
-        } else {
-          if (it + 1 < n_it) {
-            if (!mbar_wait(bar(6), par, 24, abort_flag, p.status)) break;          // S of `it` is in registers
-            if (!issue_s(it + 1)) break;
-          }
-          if (!mbar_wait(bar(12), par, 33, abort_flag, p.status)) break;           // dO landed
-          if (it > 0 && !mbar_wait(bar(1), par ^ 1u, 25, abort_flag, p.status)) break;   // dQ(it-1) read out of the dP columns
+        const int st = it & 1;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          if (!(ok = mbar_wait_warp(bar(PDS + s), (uint32_t)it & 1u, 26, abort_flag, p.status))) break;
           tc_fence_after();
-          issue_kk(C::DP_COL, attn_desc_k<HD>(sbase + C::OFF_DO), dv_k);
-          umma_commit(bar(9));
+          if (s == 1) {                                 // first, so that its way out runs beside the products after it
+#pragma unroll
+            for (int t = 0; t < AB_TILE / 16; ++t)
+              umma_bf16_w(el, tmem + C::DQ_COL, umma_desc_advance(dds_mn, t * 2048), umma_desc_advance(dk_mn, t * 2048), idesc_q, t > 0);
+            umma_commit_w(el, bar(DQ_FULL));
+          }
+          const uint64_t dq = umma_desc_advance(q_mn, st * C::TILE_BYTES + s * 8192), ddo = umma_desc_advance(do_mn, s * 8192);
+          const uint32_t t_s = tmem + C::S_COL + s * 64;
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+            umma_bf16_ts_w(el, tmem + C::DV_COL, t_s + (t >> 1) * 32 + (t & 1) * 8, umma_desc_advance(ddo, t * 2048), idesc_t, (it > 0) | (s > 0) | (t > 0));
+          if (s == 1) umma_commit_w(el, bar(DO_EMPTY));
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+            umma_bf16_ts_w(el, tmem + C::DK_COL, t_s + 16 + (t >> 1) * 32 + (t & 1) * 8, umma_desc_advance(dq, t * 2048), idesc_t, (it > 0) | (s > 0) | (t > 0));
         }
-        if (!mbar_wait(bar(7), par, 26, abort_flag, p.status)) break;              // P, dS published
-        // this step's dQ buffer was last used by step it-2: its flush is phase (it>>1)-1 of that buffer's barrier
-        if (C::PIPELINED && it > 1 && !mbar_wait(bar(it & 1), ((uint32_t)(it >> 1) & 1u) ^ 1u, 27, abort_flag, p.status)) break;
+        if (!ok) break;
+        umma_commit_w(el, bar(RING_EMPTY + st));
+        if (it + 1 < n_it) {
+          if (!(ok = ring(it + 1, st ^ 1))) break;
+          issue_kk(tmem + C::S_COL, dk_k, umma_desc_advance(q_k, (st ^ 1) * C::TILE_BYTES));
+          umma_commit_w(el, bar(S_FULL));
+          if (!(ok = mbar_wait_warp(bar(DQ_FREE), (uint32_t)it & 1u, 27, abort_flag, p.status))) break;     // dQ(it) is out of the dP columns
+          if (!(ok = issue_dp_w(it + 1))) break;
+        }
+      }
+    } else {
+      if (ok && n_it > 0 && (ok = ring(0, 0))) {
+        issue_s(0, 0, 0);
+        issue_dp(0, 0);
+        issue_s(1, 0, 1);
+        issue_dp(0, 1);
+        if (n_it > 1 && (ok = ring(1, 1))) issue_s(2, 1, 0);
+      }
+      int st = 0, sb = 0;
+      for (int it = 0; it < n_it && ok; ++it) {
+        const int st1 = st == C::STAGES - 1 ? 0 : st + 1, st2 = st1 == C::STAGES - 1 ? 0 : st1 + 1;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          if (!(ok = mbar_wait_warp(bar(PDS + s), (uint32_t)it & 1u, 26, abort_flag, p.status))) break;
+          tc_fence_after();
+          if (it + 1 < n_it) issue_dp(st1, s);           // needed first; its columns were read before P^T and dS^T were published
+          const uint64_t dq = umma_desc_advance(q_mn, st * C::TILE_BYTES + s * (C::TILE_BYTES / 2));
+          const uint64_t ddo = umma_desc_advance(do_mn, st * C::TILE_BYTES + s * (C::TILE_BYTES / 2));
+          const uint32_t t_s = tmem + C::S_COL + sb * 64;
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+            umma_bf16_ts_w(el, tmem + C::DV_COL, t_s + (t >> 1) * 32 + (t & 1) * 8, umma_desc_advance(ddo, t * attn_mn_step<HD>()), idesc_t, (it > 0) | (s > 0) | (t > 0));
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+            umma_bf16_ts_w(el, tmem + C::DK_COL, t_s + 16 + (t >> 1) * 32 + (t & 1) * 8, umma_desc_advance(dq, t * attn_mn_step<HD>()), idesc_t, (it > 0) | (s > 0) | (t > 0));
+          // the tensor pipe works in order: these scores replace the P^T / dS^T that were just read
+          if (s == 0) {
+            if (it + 1 < n_it) issue_s(sb, st1, 1);
+          } else if (it + 2 < n_it) {
+            if (!(ok = ring(it + 2, st2))) break;
+            issue_s(sb, st2, 0);
+          }
+          sb = sb == C::NS - 1 ? 0 : sb + 1;
+        }
+        if (!ok) break;
+        if (it > 0 && !(ok = mbar_wait_warp(bar(DQ_FREE), ((uint32_t)it & 1u) ^ 1u, 27, abort_flag, p.status))) break;     // dQ(it-1) is in registers
         tc_fence_after();
-        const uint64_t dq_mn = attn_desc_mn<HD>(sbase + C::OFF_Q + st * C::TILE_BYTES);
-        const uint64_t ddo_mn = attn_desc_mn<HD>(sbase + C::OFF_DO + (C::DO_STAGES > 1 ? st : 0) * C::TILE_BYTES);
-        // dV += P^T dO, dK += dS^T Q : reduction over 16 query rows per step
-        if (it == 0) {
-          umma_bf16(tmem + C::DV_COL, dp_mn, ddo_mn, idesc_t, 0);
-          umma_bf16(tmem + C::DK_COL, dds_mn, dq_mn, idesc_t, 0);
-        } else {
-          umma_bf16_acc(tmem + C::DV_COL, dp_mn, ddo_mn, idesc_t);
-          umma_bf16_acc(tmem + C::DK_COL, dds_mn, dq_mn, idesc_t);
-        }
+        const uint64_t dds_mn = umma_smem_desc(sbase + C::OFF_DS + (it & 1) * C::DS_BYTES, 16384, 1024);
 #pragma unroll
-        for (int t = 1; t < AB_TILE / 16; ++t) {
-          umma_bf16_acc(tmem + C::DV_COL, umma_desc_advance(dp_mn, t * 2048), umma_desc_advance(ddo_mn, t * attn_mn_step<HD>()), idesc_t);
-          umma_bf16_acc(tmem + C::DK_COL, umma_desc_advance(dds_mn, t * 2048), umma_desc_advance(dq_mn, t * attn_mn_step<HD>()), idesc_t);
-        }
-        // dQ = dS K : reduction over 16 kv rows per step
-        const uint32_t t_dq = tmem + C::DQ_COL + (uint32_t)(it & 1) * C::DQ_BUF_COLS;
-        umma_bf16(t_dq, dds_k, dk_mn, idesc_q, 0);
+        for (int t = 0; t < AB_TILE / 16; ++t)
+          umma_bf16_w(el, tmem + C::DQ_COL, umma_desc_advance(dds_mn, t * 2048), umma_desc_advance(dk_mn, t * attn_mn_step<HD>()), idesc_q, t > 0);
+        umma_commit_w(el, bar(DQ_FULL + (it & 1)));       // dQ ready, this dS buffer free
+        umma_commit_w(el, bar(RING_EMPTY + st));
+        st = st1;
+      }
+    }
+    if (ok && n_it > 0) umma_commit_w(el, bar(ALL_DONE));
+  } else if (warp < 18) {
+    // ---------------------------------------------------------------- softmax warps: 32 query columns of 32 KV rows each
+    const int q4 = warp & 3, g = (warp - 2) >> 2, s = g >> 1;
+    const int row = q4 * 32 + lane;                           // row of the KV tile
+    const int t_row = j * AB_TILE + row;
+    const uint32_t t_lane = tmem + ((uint32_t)(q4 * 32) << 16);
+    bool ok = true;
+    if constexpr (C::KV_TMEM) {   // K (warps of half 0) and V (half 1) rows become tensor-memory operands, half a row per warp
+      const int c0 = (g & 1) * (HD / 2);
+      const __nv_bfloat16* src = p.qkv + (((long long)b * p.T + t_row) * heads_total + p.Hq + s * p.Hkv + kvh) * p.hd + c0;
+      uint32_t w[HD / 4];
 #pragma unroll
-        for (int t = 1; t < AB_TILE / 16; ++t)
-          umma_bf16_acc(t_dq, umma_desc_advance(dds_k, (t >> 2) * 16384 + (t & 3) * 32),
-                        umma_desc_advance(dk_mn, t * attn_mn_step<HD>()), idesc_q);
-        umma_commit(bar(8));                        // dQ ready; P / dS and this Q / dO stage are free
-        umma_commit(bar(13 + st));
-        if (!C::PIPELINED) umma_commit(bar(15));
+      for (int c = 0; c < HD / 16; ++c) {
+        const uint4 v = t_row < p.T && c0 + c * 8 < p.hd ? reinterpret_cast<const uint4*>(src)[c] : make_uint4(0, 0, 0, 0);
+        w[4 * c] = v.x; w[4 * c + 1] = v.y; w[4 * c + 2] = v.z; w[4 * c + 3] = v.w;
+      }
+      const uint32_t col = (s == 0 ? C::K_COL : C::V_COL) + c0 / 2;
+      if constexpr (HD == 32) tmem_st8(t_lane + col, w);
+      else tmem_st16(t_lane + col, w);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(KV_TMEM));
+    }
+    const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
+    const int col0 = (g & 1) * 32;                             // of the half's 64 query columns
+    for (int it = 0; it < n_it; ++it) {
+      const int st = it % C::STAGES, qi = j + (it0 + it) % per_head;
+      const float* rows = reinterpret_cast<const float*>(sal + C::OFF_ROW) + st * 2 * AB_TILE + s * 64 + col0;
+      uint8_t* drow = sal + C::OFF_DS + (C::WIDE ? 0 : it & 1) * C::DS_BYTES + s * 16384 + row * 128;
+      if (!mbar_wait(bar(RING_FULL + st), (uint32_t)(it / C::STAGES) & 1u, 28, abort_flag, p.status)) { ok = false; break; }
+      const int h = 2 * it + s, sb = C::WIDE ? 0 : h % C::NS;
+      const uint32_t t_s = t_lane + C::S_COL + (C::WIDE ? s : sb) * 64 + col0, t_dp = t_lane + C::DP_COL + s * 64 + col0;
+      if (!mbar_wait(bar(S_FULL + sb), (uint32_t)(C::WIDE ? it : h / C::NS) & 1u, 29, abort_flag, p.status)) { ok = false; break; }
+      tc_fence_after();
+      float2 pr[16];
+      // two copies: the compare and select of the diagonal tiles doubled the instructions of a pair in all the others
+      if (qi == j) attn_bwd_p<true>(t_s, rows, sc2, row - s * 64 - col0, pr);
+      else attn_bwd_p<false>(t_s, rows, sc2, 0, pr);
+      {
+        uint32_t pp[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) pp[i] = pack_bf16(pr[i].x, pr[i].y);
+        tmem_st16(t_s, pp);
+      }
+      if (!mbar_wait(bar(DP_FULL + (C::WIDE ? 0 : s)), (uint32_t)it & 1u, 33, abort_flag, p.status)) { ok = false; break; }
+      tc_fence_after();
+      uint32_t dd[16];
+#pragma unroll
+      for (int c = 0; c < 32; c += 16) {
+        uint32_t dp[16];
+        tmem_ld16(t_dp + c, dp);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) {
+          const float4 nd = *reinterpret_cast<const float4*>(rows + AB_TILE + c + i);
+          // dS = P (dP - delta); the softmax scale is applied once, when dQ and dK leave their accumulators
+          const float2 d0 = fmul2(pr[(c + i) >> 1], fadd2(make_float2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1])), make_float2(nd.x, nd.y)));
+          const float2 d1 = fmul2(pr[((c + i) >> 1) + 1], fadd2(make_float2(__uint_as_float(dp[i + 2]), __uint_as_float(dp[i + 3])), make_float2(nd.z, nd.w)));
+          dd[(c + i) >> 1] = pack_bf16(d0.x, d0.y);
+          dd[((c + i) >> 1) + 1] = pack_bf16(d1.x, d1.y);
+        }
+      }
+      tmem_st16(t_s + 16, dd);
+      if (!C::WIDE && it > 1 && !mbar_wait(bar(DQ_FULL + (it & 1)), ((uint32_t)(it >> 1) & 1u) ^ 1u, 30, abort_flag, p.status)) { ok = false; break; }
+#pragma unroll
+      for (int ch = 0; ch < 4; ++ch)
+        *reinterpret_cast<uint4*>(drow + ((((col0 >> 3) + ch) ^ (row & 7)) << 4)) = make_uint4(dd[4 * ch], dd[4 * ch + 1], dd[4 * ch + 2], dd[4 * ch + 3]);
+      fence_proxy_async_smem();
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(PDS + s));
+    }
+    if (ok && n_it > 0) ok = mbar_wait(bar(ALL_DONE), 0, 31, abort_flag, p.status);
+    tc_fence_after();
+    constexpr int W = C::OUT_COLS;
+    const int out0 = g * W;                                    // first of this warp's columns of dV and dK
+    auto load_out = [&](uint32_t col, uint32_t* r) {
+      if constexpr (W == 8) tmem_ld8(t_lane + col, r);
+      else if constexpr (W == 16) tmem_ld16(t_lane + col, r);
+      else tmem_ld32(t_lane + col, r);
+      tmem_ld_wait();
+    };
+    if (ok && !SPLIT) {
+      // dV, dK accumulators -> bf16 rows of the packed gradient tensor
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        const float osc = which == 0 ? 1.f : p.scale;
+        __nv_bfloat16* dst = p.dqkv + (((long long)b * p.T + t_row) * heads_total + (which == 0 ? p.Hq + p.Hkv : p.Hq) + kvh) * p.hd + out0;
+        bool dst_ok = t_row < p.T && out0 < p.hd;
+        if (SCATTER && p.n_dst > 0) {
+          const int owner = t_row / p.dst_rows, tl = t_row - owner * p.dst_rows;
+          dst_ok = dst_ok && owner < p.n_dst;
+          if (dst_ok)
+            dst = p.dst[owner] + (((long long)b * p.dst_rows + tl) * p.dst_heads + (which == 0 ? p.dst_v0 : p.dst_k0) + kvh) * p.hd + out0;
+        }
+        uint32_t r[W];
+        load_out((which == 0 ? C::DV_COL : C::DK_COL) + out0, r);
+        if (SCATTER && which == 1 && p.cosT != nullptr && out0 < p.hd) {
+          // transposed RoPE on dK (fp32): column j pairs with j +- hd / 2 (the condition is the warp's, as the load needs)
+          const bool low = out0 < p.hd / 2;
+          const int pc = low ? out0 + p.hd / 2 : out0 - p.hd / 2;      // partner's first column
+          uint32_t q2[W];
+          load_out(C::DK_COL + pc, q2);
+          if (t_row < p.T) {
+            const float* cr = p.cosT + (long long)t_row * p.hd;
+            const float* sr = p.sinT + (long long)t_row * p.hd;
+#pragma unroll
+            for (int i = 0; i < W; ++i) {
+              const float a = __uint_as_float(r[i]), bb = __uint_as_float(q2[i]);
+              r[i] = __float_as_uint(low ? a * cr[out0 + i] + bb * sr[pc + i] : a * cr[out0 + i] - bb * sr[pc + i]);
+            }
+          }
+        }
+        if (dst_ok) {
+#pragma unroll
+          for (int i = 0; i < W; i += 8) {
+            uint4 v;
+            v.x = pack_bf16(__uint_as_float(r[i]) * osc, __uint_as_float(r[i + 1]) * osc);
+            v.y = pack_bf16(__uint_as_float(r[i + 2]) * osc, __uint_as_float(r[i + 3]) * osc);
+            v.z = pack_bf16(__uint_as_float(r[i + 4]) * osc, __uint_as_float(r[i + 5]) * osc);
+            v.w = pack_bf16(__uint_as_float(r[i + 6]) * osc, __uint_as_float(r[i + 7]) * osc);
+            *reinterpret_cast<uint4*>(dst + i) = v;
+          }
+        }
+      }
+    }
+    if constexpr (SPLIT) {
+      // this CTA's dV | dK, over the Q / dO ring: every MMA and every row of the ring has been read (WIDE: over the dQ boxes too)
+      if (C::WIDE) {
+        __syncwarp();
+        asm volatile("bar.sync 1, 640;" ::: "memory");
+      }
+      float* part = reinterpret_cast<float*>(sal + C::OFF_Q) + row * C::PART_PITCH + out0;
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        uint32_t r[W];
+        load_out((which == 0 ? C::DV_COL : C::DK_COL) + out0, r);
+#pragma unroll
+        for (int i = 0; i < W; i += 4)
+          *reinterpret_cast<uint4*>(part + which * HD + i) =
+              n_it > 0 ? make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]) : make_uint4(0, 0, 0, 0);      // no step: nothing was accumulated
       }
     }
   } else {
-    // ---------------------------------------------------------------- softmax warpgroups (warps 2..9)
-    const int q4 = warp & 3, half = (warp - 2) >> 2;
-    const int row = q4 * 32 + lane;
+    // ---------------------------------------------------------------- dQ of every step -> fp32 accumulator in global memory
+    const int q4 = warp & 3;
     const uint32_t t_lane = tmem + ((uint32_t)(q4 * 32) << 16);
-    constexpr float LOG2E = 1.4426950408889634f;
-    bool ok = true;
-
-    // dQ tile of step `it` -> fp32 accumulator in global memory. Each warp turns its [32 rows][HD/2 columns]
-    // part into swizzled [32][32 fp32] boxes in shared memory and one lane hands them to the TMA unit as
-    // reduce-add tile stores (several KV tiles add into the same query rows), so the SM issues one bulk
-    // operation per 4 KB instead of 256 vector atomics.
-    // HD 128 has no room for staging boxes: when dQ of a step is complete, so are all reads of its P and dS, and the two
-    // 4 KB pieces of P and dS that this warp writes serve as its boxes for the two 32-column pieces of dQ.
-    const int box0 = C::PIPELINED ? C::OFF_DQS + (warp - 2) * 4096 : C::OFF_P + (half * 4 + q4) * 4096;
-    const int out0 = HD == 32 ? 0 : half * (HD / 2);         // first of this warp's OUT_COLS columns
-    auto flush_dq = [&](int it) {
-      if (HD != 32 || half == (it & 1)) {
-      const int hq = kvh * rep + (it0 + it) / per_head, qi = j + (it0 + it) % per_head;
-      const int y0 = qi * AB_TILE + q4 * 32;                 // first of this warp's 32 query rows
-#pragma unroll
-      for (int c = 0; c < C::OUT_COLS; c += 32) {
-        uint32_t r[32];
-        tmem_ld32(t_lane + C::DQ_COL + (uint32_t)(it & 1) * C::DQ_BUF_COLS + out0 + c, r);
-        if (C::PIPELINED) {
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // staging box free again
-          __syncwarp();
-        }
-        tmem_ld_wait();
-        const int box = box0 + (C::PIPELINED ? 0 : (c >> 5) * (C::OFF_DS - C::OFF_P));
-        uint8_t* rowp = sal + box + lane * 128;
-#pragma unroll
-        for (int ch = 0; ch < 8; ++ch)
-          *reinterpret_cast<uint4*>(rowp + ((ch ^ (lane & 7)) << 4)) = make_uint4(r[4 * ch], r[4 * ch + 1], r[4 * ch + 2], r[4 * ch + 3]);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          if (y0 < p.T && out0 + c < p.hd)
-            asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
-                         ::"l"((uint64_t)&tm_dq), "r"(sbase + box), "r"(out0 + c), "r"(y0), "r"(b * p.Hq + hq) : "memory");
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        }
-      }
-      tc_fence_before();
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(C::PIPELINED ? bar(it & 1) : bar(1));
-    };
-
-    // HD 128. Tensor memory holds S, dP, dV and dK and nothing else, shared memory two Q tiles and one dO tile, so dQ takes
-    // turns with dP. A step's chain: flush dQ of the step before -> dP -> dS -> dV, dK, dQ; the next step's S and its
-    // exponentials run beside the last link. One step after the other (S, dP, softmax, dV, dK, dQ, flush, next load),
-    // 24 query / 8 KV heads and 2 x 4096 tokens took 1.11 ms, in this order 0.95 ms.
-    // P / dS stores of a step: 64 columns of this warp's rows
-    auto store_pds = [&](const uint32_t* pp, const uint32_t* dd) {
-      uint8_t* prow = sal + C::OFF_P + half * 16384 + row * 128;
-      uint8_t* drow = sal + C::OFF_DS + half * 16384 + row * 128;
-#pragma unroll
-      for (int ch = 0; ch < 8; ++ch) {
-        const int sw = (ch ^ (row & 7)) << 4;
-        *reinterpret_cast<uint4*>(prow + sw) = make_uint4(pp[4 * ch], pp[4 * ch + 1], pp[4 * ch + 2], pp[4 * ch + 3]);
-        *reinterpret_cast<uint4*>(drow + sw) = make_uint4(dd[4 * ch], dd[4 * ch + 1], dd[4 * ch + 2], dd[4 * ch + 3]);
-      }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(7));
-    };
-    if constexpr (!C::PIPELINED) {
-      for (int it = 0; it < n_it; ++it) {
-        const uint32_t par = (uint32_t)it & 1u;
-        const int hq = kvh * rep + (it0 + it) / per_head, qi = j + (it0 + it) % per_head;
-        const int t_row = qi * AB_TILE + row;
-        const bool row_ok = t_row < p.T;
-        const float lse2 = row_ok ? p.lse[((long long)b * p.Hq + hq) * p.T + t_row] * LOG2E : INFINITY;
-        const float dlt = row_ok ? p.delta[((long long)b * p.Hq + hq) * p.T + t_row] : 0.f;
-        const bool diag = (qi == j);
-        if (!mbar_wait(bar(5), par, 28, abort_flag, p.status)) { ok = false; break; }
-        tc_fence_after();
-        uint32_t pr[64];                              // fp32 scores, then probabilities
-        tmem_ld32(t_lane + C::S_COL + half * 64, pr);
-        tmem_ld32(t_lane + C::S_COL + half * 64 + 32, pr + 32);
-        tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(6));           // S may be overwritten
-        const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), nl2 = make_float2(-lse2, -lse2), nd2 = make_float2(-dlt, -dlt);
-#pragma unroll
-        for (int i = 0; i < 64; i += 2) {
-          const float2 x = ffma2(make_float2(__uint_as_float(pr[i]), __uint_as_float(pr[i + 1])), sc2, nl2);
-          float2 e = make_float2(ex2_approx(x.x), ex2_approx(x.y));
-          if (diag) {
-            if (half * 64 + i > row) e.x = 0.f;
-            if (half * 64 + i + 1 > row) e.y = 0.f;
-          }
-          pr[i] = __float_as_uint(e.x); pr[i + 1] = __float_as_uint(e.y);
-        }
-        if (it > 0) {
-          if (!mbar_wait(bar(8), par ^ 1u, 29, abort_flag, p.status)) { ok = false; break; }
-          tc_fence_after();
-          flush_dq(it - 1);
-        }
-        if (!mbar_wait(bar(9), par, 30, abort_flag, p.status)) { ok = false; break; }
-        tc_fence_after();
-        uint32_t pp[32], dd[32];
-#pragma unroll
-        for (int c = 0; c < 64; c += 32) {
-          uint32_t dp[32];
-          tmem_ld32(t_lane + C::DP_COL + half * 64 + c, dp);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const float2 e = make_float2(__uint_as_float(pr[c + i]), __uint_as_float(pr[c + i + 1]));
-            const float2 ds = fmul2(e, fadd2(make_float2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1])), nd2));
-            pp[(c + i) >> 1] = pack_bf16(e.x, e.y);
-            dd[(c + i) >> 1] = pack_bf16(ds.x, ds.y);
-          }
-        }
-        tc_fence_before();
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the boxes have been read
-        __syncwarp();
-        store_pds(pp, dd);
-      }
-    } else
+    const int box0 = C::OFF_DQS + q4 * C::BOXES * 4096;
     for (int it = 0; it < n_it; ++it) {
-      const uint32_t par = (uint32_t)it & 1u;
       const int hq = kvh * rep + (it0 + it) / per_head, qi = j + (it0 + it) % per_head;
-      const int t_row = qi * AB_TILE + row;
-      const bool row_ok = t_row < p.T;
-      const float lse2 = row_ok ? p.lse[((long long)b * p.Hq + hq) * p.T + t_row] * LOG2E : INFINITY;
-      const float dlt = row_ok ? p.delta[((long long)b * p.Hq + hq) * p.T + t_row] : 0.f;
-      const bool diag = (qi == j);
-      if (!mbar_wait(bar(5), par, 28, abort_flag, p.status)) { ok = false; break; }
+      const int y0 = qi * AB_TILE + q4 * 32;                  // first of this warp's 32 query rows
+      if (!mbar_wait(bar(DQ_FULL + (C::WIDE ? 0 : it & 1)), (uint32_t)(C::WIDE ? it : it >> 1) & 1u, 32, abort_flag, p.status)) break;
       tc_fence_after();
-      uint32_t pp[32], dd[32];                      // 64 columns of P and dS, packed bf16 pairs
+      constexpr int COLS = HD < 64 ? HD : 64;                 // in registers at a time
 #pragma unroll
-      for (int c = 0; c < 64; c += 32) {
-        uint32_t s[32], dp[32];
-        tmem_ld32(t_lane + C::S_COL + half * 64 + c, s);
-        tmem_ld32(t_lane + C::DP_COL + half * 64 + c, dp);
+      for (int c0 = 0; c0 < HD; c0 += COLS) {
+        uint32_t r[COLS];
+#pragma unroll
+        for (int c = 0; c < COLS; c += 32) tmem_ld32(t_lane + C::DQ_COL + c0 + c, r + c);
         tmem_ld_wait();
-        const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), nl2 = make_float2(-lse2, -lse2), nd2 = make_float2(-dlt, -dlt);
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float2 x = ffma2(make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), sc2, nl2);
-          float2 pr = make_float2(ex2_approx(x.x), ex2_approx(x.y));
-          if (diag) {
-            const int col = half * 64 + c + i;
-            if (col > row) pr.x = 0.f;
-            if (col + 1 > row) pr.y = 0.f;
-          }
-          // dS = P (dP - delta); the softmax scale is applied once, when dQ and dK leave their accumulators
-          const float2 ds = fmul2(pr, fadd2(make_float2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1])), nd2));
-          pp[(c + i) >> 1] = pack_bf16(pr.x, pr.y);
-          dd[(c + i) >> 1] = pack_bf16(ds.x, ds.y);
+        if (c0 + COLS == HD) {                                // all of it has been read: the columns are free
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(DQ_FREE));
         }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(6));           // S / dP columns may be overwritten
-      if (it > 0) {                                 // MMAs of step it-1 done: P / dS free, dQ(it-1) ready
-        if (!mbar_wait(bar(8), par ^ 1u, 29, abort_flag, p.status)) { ok = false; break; }
-        tc_fence_after();
-      }
-      store_pds(pp, dd);
-      if (it > 0) flush_dq(it - 1);
-    }
-    if (ok && n_it > 0) {
-      {
-        if (mbar_wait(bar(8), (uint32_t)(n_it - 1) & 1u, 31, abort_flag, p.status)) { tc_fence_after(); flush_dq(n_it - 1); } else ok = false;
-      }
-      if (ok && !SPLIT) {
-        if constexpr (SCATTER) {
-          // dV, dK accumulators -> bf16 rows of the packed gradient tensor
-          tc_fence_after();
-          const int t_row = j * AB_TILE + row;
-  #pragma unroll
-          for (int which = 0; which < 2; ++which) {
-            const int head = which == 0 ? p.Hq + p.Hkv + kvh : p.Hq + kvh;
-            const float osc = which == 0 ? 1.f : p.scale;
-            const uint32_t col0 = (which == 0 ? C::DV_COL : C::DK_COL) + half * (HD / 2);
-            __nv_bfloat16* dst = p.dqkv + (((long long)b * p.T + t_row) * heads_total + head) * p.hd + half * (HD / 2);
-            bool dst_ok = true;
-            if (p.n_dst > 0) {
-              const int owner = t_row / p.dst_rows, tl = t_row - owner * p.dst_rows;
-              dst_ok = owner < p.n_dst;
-              if (dst_ok)
-                dst = p.dst[owner] + (((long long)b * p.dst_rows + tl) * p.dst_heads + (which == 0 ? p.dst_v0 : p.dst_k0) + kvh) * p.hd
-                      + half * (HD / 2);
-            }
-  #pragma unroll
-            for (int c = 0; c < HD / 2; c += 32) {
-              uint32_t r[32];
-              tmem_ld32(t_lane + col0 + c, r);
-              tmem_ld_wait();
-              // transposed RoPE on dK (fp32): column j pairs with j +- hd / 2. `rot` is warp-uniform (the
-              // tensor-memory load of the partner columns must be executed by the whole warp).
-              const int colg = half * (HD / 2) + c;                      // first of this thread's 32 columns
-              const bool rot = which == 1 && p.cosT != nullptr && colg < p.hd;
-              uint32_t q2[32];
-              if (rot && p.hd == HD) {                                   // partner columns sit in the other half-row
-                tmem_ld32(t_lane + C::DK_COL + (1 - half) * (HD / 2) + c, q2);
-                tmem_ld_wait();
-              }
-              if (rot && t_row < p.T) {
-                const float* cr = p.cosT + (long long)t_row * p.hd;
-                const float* sr = p.sinT + (long long)t_row * p.hd;
-                if (p.hd == HD) {
-                  const int pc = (1 - half) * (HD / 2) + c;             // partner's first column
-  #pragma unroll
-                  for (int i = 0; i < 32; ++i) {
-                    const float a = __uint_as_float(r[i]), bb = __uint_as_float(q2[i]);
-                    r[i] = __float_as_uint(half == 0 ? a * cr[colg + i] + bb * sr[pc + i] : a * cr[colg + i] - bb * sr[pc + i]);
-                  }
-                } else {                                                // hd 32 on the 64-wide kernel: both halves are in r
-                  float o[32];
-  #pragma unroll
-                  for (int i = 0; i < 16; ++i) {
-                    const float a = __uint_as_float(r[i]), bb = __uint_as_float(r[i + 16]);
-                    o[i] = a * cr[i] + bb * sr[i + 16];
-                    o[i + 16] = bb * cr[i + 16] - a * sr[i];
-                  }
-  #pragma unroll
-                  for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(o[i]);
-                }
-              }
-              if (t_row < p.T && dst_ok && half * (HD / 2) + c < p.hd) {
-  #pragma unroll
-                for (int i = 0; i < 32; i += 8) {
-                  uint4 v;
-                  v.x = pack_bf16(__uint_as_float(r[i]) * osc, __uint_as_float(r[i + 1]) * osc);
-                  v.y = pack_bf16(__uint_as_float(r[i + 2]) * osc, __uint_as_float(r[i + 3]) * osc);
-                  v.z = pack_bf16(__uint_as_float(r[i + 4]) * osc, __uint_as_float(r[i + 5]) * osc);
-                  v.w = pack_bf16(__uint_as_float(r[i + 6]) * osc, __uint_as_float(r[i + 7]) * osc);
-                  *reinterpret_cast<uint4*>(dst + c + i) = v;
-                }
-              }
-            }
+#pragma unroll
+        for (int c = 0; c < COLS; c += 32 * C::BOXES) {
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // staging boxes free again
+          __syncwarp();
+#pragma unroll
+          for (int x = 0; x < C::BOXES; ++x) {
+            uint8_t* rowp = sal + box0 + x * 4096 + lane * 128;
+            const uint32_t* v = r + c + 32 * x;
+#pragma unroll
+            for (int ch = 0; ch < 8; ++ch)
+              *reinterpret_cast<uint4*>(rowp + ((ch ^ (lane & 7)) << 4)) = make_uint4(v[4 * ch], v[4 * ch + 1], v[4 * ch + 2], v[4 * ch + 3]);
           }
-
-        } else {
-          // dV, dK accumulators -> bf16 rows of the packed gradient tensor
-          tc_fence_after();
-          const int t_row = j * AB_TILE + row;
-  #pragma unroll
-          for (int which = 0; which < 2; ++which) {
-            if (HD == 32 && which != half) continue;                      // HD 32: half 0 carries dV, half 1 dK
-            const int head = which == 0 ? p.Hq + p.Hkv + kvh : p.Hq + kvh;
-            const float osc = which == 0 ? 1.f : p.scale;
-            const uint32_t col0 = (which == 0 ? C::DV_COL : C::DK_COL) + out0;
-            __nv_bfloat16* dst = p.dqkv + (((long long)b * p.T + t_row) * heads_total + head) * p.hd + out0;
-  #pragma unroll
-            for (int c = 0; c < C::OUT_COLS; c += 32) {
-              uint32_t r[32];
-              tmem_ld32(t_lane + col0 + c, r);
-              tmem_ld_wait();
-              if (t_row < p.T) {
-  #pragma unroll
-                for (int i = 0; i < 32; i += 8) {
-                  uint4 v;
-                  v.x = pack_bf16(__uint_as_float(r[i]) * osc, __uint_as_float(r[i + 1]) * osc);
-                  v.y = pack_bf16(__uint_as_float(r[i + 2]) * osc, __uint_as_float(r[i + 3]) * osc);
-                  v.z = pack_bf16(__uint_as_float(r[i + 4]) * osc, __uint_as_float(r[i + 5]) * osc);
-                  v.w = pack_bf16(__uint_as_float(r[i + 6]) * osc, __uint_as_float(r[i + 7]) * osc);
-                  *reinterpret_cast<uint4*>(dst + c + i) = v;
-                }
-              }
-            }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+#pragma unroll
+            for (int x = 0; x < C::BOXES; ++x)
+              if (y0 < p.T && c0 + c + 32 * x < p.hd)
+                asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+                             ::"l"((uint64_t)&tm_dq), "r"(sbase + box0 + x * 4096), "r"(c0 + c + 32 * x), "r"(y0), "r"(b * p.Hq + hq) : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
-
         }
       }
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");      // dQ reductions have left shared memory and landed
-    if constexpr (SPLIT) {
-      // this CTA's dV | dK, over the Q / dO ring (and for HD 128 the dQ boxes, so every warp's must have been read)
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      tc_fence_after();
-      float* part = reinterpret_cast<float*>(sal + C::OFF_Q) + row * C::PART_PITCH;
-#pragma unroll
-      for (int which = 0; which < 2; ++which) {
-        if (HD == 32 && which != half) continue;
-#pragma unroll
-        for (int c = 0; c < C::OUT_COLS; c += 32) {
-          uint32_t r[32];
-          tmem_ld32(t_lane + (which == 0 ? C::DV_COL : C::DK_COL) + out0 + c, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; i += 4)
-            *reinterpret_cast<uint4*>(part + which * HD + out0 + c + i) =
-                n_it > 0 ? make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]) : make_uint4(0, 0, 0, 0);      // no step: nothing was accumulated
-        }
-      }
+    if (SPLIT && C::WIDE) {
+      __syncwarp();
+      asm volatile("bar.sync 1, 640;" ::: "memory");
     }
   }
   if constexpr (SPLIT) {
@@ -769,16 +756,16 @@ static int split_for(int n_tiles, int heads_kv, int rep) {
 template <int HD, bool SCATTER, bool SPLIT = false>
 static int launch_bwd(const CUtensorMap& mq, const CUtensorMap& mdo, const CUtensorMap& mdq, const AttnBwdParams& p,
                       cudaStream_t st) {
-  using C = AttnBwdCfg<HD>;
+  constexpr int smem = AttnBwdCfg<HD>::TOTAL;
   auto kern = attn_bwd_kernel<HD, SCATTER, SPLIT>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
   const int grid = ((p.T + AB_TILE - 1) / AB_TILE) * p.B * p.Hkv;
-  return launch_overlapped(kern, dim3((unsigned)(grid * (SPLIT ? p.split : 1))), dim3(AB_THREADS), C::TOTAL, st, SPLIT ? p.split : 1, mq, mdo, mdq, p);
+  return launch_overlapped(kern, dim3((unsigned)(grid * (SPLIT ? p.split : 1))), dim3(AB_THREADS), smem, st, SPLIT ? p.split : 1, mq, mdo, mdq, p);
 }
 
 }  // namespace tlm
@@ -816,7 +803,7 @@ static int attn_bwd_impl(const void* qkv, const void* o, const void* dout, const
     return -6;
   if (n_dst == 0 && dqkv == nullptr) return -6;
   AttnBwdParams p{};
-  p.dqkv = (__nv_bfloat16*)dqkv; p.dq_acc = dq_acc; p.lse = lse; p.delta = delta; p.B = B; p.T = T; p.Hq = Hq; p.Hkv = Hkv;
+  p.qkv = (const __nv_bfloat16*)qkv; p.dqkv = (__nv_bfloat16*)dqkv; p.dq_acc = dq_acc; p.lse = lse; p.delta = delta; p.B = B; p.T = T; p.Hq = Hq; p.Hkv = Hkv;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status_word(); p.hd = hd; p.cosT = cosT; p.sinT = sinT;
   p.n_dst = n_dst; p.dst_rows = dst_rows; p.dst_heads = dst_heads; p.dst_q0 = dst_q0; p.dst_k0 = dst_k0; p.dst_v0 = dst_v0;
   // per (batch, KV head): Q, dO, dQ (fp32 accumulator + bf16 result) of its query heads, K, V, dK, dV; measured at
