@@ -806,8 +806,10 @@ static int attn_bwd_impl(const void* qkv, const void* o, const void* dout, const
   p.qkv = (const __nv_bfloat16*)qkv; p.dqkv = (__nv_bfloat16*)dqkv; p.dq_acc = dq_acc; p.lse = lse; p.delta = delta; p.B = B; p.T = T; p.Hq = Hq; p.Hkv = Hkv;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status_word(); p.hd = hd; p.cosT = cosT; p.sinT = sinT;
   p.n_dst = n_dst; p.dst_rows = dst_rows; p.dst_heads = dst_heads; p.dst_q0 = dst_q0; p.dst_k0 = dst_k0; p.dst_v0 = dst_v0;
-  // per (batch, KV head): Q, dO, dQ (fp32 accumulator + bf16 result) of its query heads, K, V, dK, dV; measured at
-  // B 8, T 4096, 16 / 8 heads of 64: 1.054 ms with groups of 8 - 16, 1.105 with each head's tiles adjacent, 1.12 with all 64
+  // per (batch, KV head): Q, dO, dQ (fp32 accumulator + bf16 result) of its query heads, K, V, dK, dV. In us with the delta and
+  // conversion passes: B 8, T 4096, 16 / 8 heads of 64: 930 with groups of 8 - 16, 957 with 32, 1040 with all 64.
+  // Groups of one size (even_group): 24 / 8 heads of 128, B 2, T 4096, in 4 x 4 instead of 5 + 5 + 5 + 1: 740 -> 652;
+  // 32 / 4 heads of 32, B 8, in 4 x 8 instead of 10 + 10 + 10 + 2: 1494 -> 1287
   p.head_group = attn_head_group("TLM_ATTN_BWD_GROUP", (long long)T * hd * (10LL * (Hq / Hkv) + 8), 112LL << 20, B * Hkv);
   AttnBwdDst dd{};
   dd.n = n_dst; dd.rows = dst_rows; dd.heads = dst_heads;

@@ -133,9 +133,11 @@ int num_sms() {
 int attn_head_group(const char* env, long long bytes_per_head, long long budget_bytes, int n_heads) {
   long long g = bytes_per_head > 0 ? budget_bytes / bytes_per_head : 1;
   const char* v = getenv(env);
-  if (v != nullptr && atoi(v) > 0) g = atoi(v);
+  const bool forced = v != nullptr && atoi(v) > 0;
+  if (forced) g = atoi(v);
   if (g > n_heads) g = n_heads;
-  return g < 1 ? 1 : (int)g;
+  if (g < 1) g = 1;
+  return (int)(forced ? g : even_group(n_heads, (int)g));
 }
 
 }  // namespace tlm
