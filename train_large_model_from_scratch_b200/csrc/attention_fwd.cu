@@ -8,7 +8,7 @@
 // One CTA owns 128 query rows of one (batch, head) and walks over 128-row KV
 // tiles up to the diagonal:
 //   warp 0     TMA: Q once, then K / V tiles into a 2-deep ring (128B swizzle)
-//   warp 1     one lane issues  S = Q K^T  (M128 N128) into TMEM, and after the
+//   warp 1     issues  S = Q K^T  (M128 N128) into TMEM, and after the
 //              softmax warps have published P:  O_j = P V  (M128 N=hd; V is
 //              consumed as an MN-major operand straight from its row-major tile)
 //   warps 2-5  one thread per query row: tcgen05.ld S, running max / sum with
@@ -86,7 +86,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const AttnFwdParams 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sal + L::OFF_BAR + 128);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int n_q_tiles = (p.T + AT_BQ - 1) / AT_BQ;
   int tile_rank, bh;
   heavy_first_decode((int)blockIdx.x, n_q_tiles, p.B * p.Hq, p.head_group, tile_rank, bh);
@@ -106,7 +106,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const AttnFwdParams 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   griddep_wait();
 
   if (warp == 0) {
@@ -135,46 +135,46 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const AttnFwdParams 
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = umma_idesc_bf16(AT_BQ, AT_BKV, 0, 0);
-      constexpr uint32_t idesc_o = umma_idesc_bf16(AT_BQ, HD, 0, 1);
-      // descriptors are built once per tile and advanced with one add per MMA: this thread's instruction
-      // stream is what feeds the tensor pipe
-      const uint64_t dq = attn_desc_k<HD>(sbase + L::OFF_Q);
-      auto issue_s = [&](int j) -> bool {
-        const int st = j & 1;
-        if (!mbar_wait(bar(1 + st), (uint32_t)(j >> 1) & 1u, 13, abort_flag, p.status)) return false;
-        tc_fence_after();
-        const uint64_t dk = attn_desc_k<HD>(sbase + L::OFF_K + st * L::KV_BYTES);
-        umma_bf16(tmem + S_COL, dq, dk, idesc_s, 0);
+    // The warp stays together and one lane issues, so that the operands are computed in uniform registers (see umma_bf16_w): as
+    // one lane's own code a tile's 12 MMAs took 76 cycles each, longer than they run. Long runs, in us: B 8, T 4096, 16 heads of
+    // 64 467 -> 432, 32 heads of 32 833 -> 765; B 2, 24 heads of 128 275 -> 264.
+    // Descriptors are built once per tile and advanced with one add per MMA.
+    const uint32_t el = elect_one();
+    constexpr uint32_t idesc_s = umma_idesc_bf16(AT_BQ, AT_BKV, 0, 0);
+    constexpr uint32_t idesc_o = umma_idesc_bf16(AT_BQ, HD, 0, 1);
+    const uint64_t dq = attn_desc_k<HD>(sbase + L::OFF_Q);
+    auto issue_s = [&](int j) -> bool {
+      const int st = j & 1;
+      if (!mbar_wait_warp(bar(1 + st), (uint32_t)(j >> 1) & 1u, 13, abort_flag, p.status)) return false;
+      tc_fence_after();
+      const uint64_t dk = attn_desc_k<HD>(sbase + L::OFF_K + st * L::KV_BYTES);
 #pragma unroll
-        for (int t = 1; t < HD / 16; ++t) {
-          const uint32_t off = (t >> 2) * 16384 + (t & 3) * 32;
-          umma_bf16_acc(tmem + S_COL, umma_desc_advance(dq, off), umma_desc_advance(dk, off), idesc_s);
-        }
-        umma_commit(bar(7));
-        umma_commit(bar(11 + st));                              // K stage free
-        return true;
-      };
-      bool ok = mbar_wait(bar(0), 0, 12, abort_flag, p.status);
-      if (ok) ok = issue_s(0);
-      for (int j = 0; j < n_kv && ok; ++j) {
-        const int st = j & 1;
-        const uint32_t par = (uint32_t)j & 1u;
-        if (j + 1 < n_kv) {                                     // S of the next tile overlaps this tile's softmax
-          if (!mbar_wait(bar(10), par, 18, abort_flag, p.status)) break;
-          if (!issue_s(j + 1)) break;
-        }
-        if (!mbar_wait(bar(8), par, 14, abort_flag, p.status)) break;                        // P written
-        if (!mbar_wait(bar(3 + st), (uint32_t)(j >> 1) & 1u, 15, abort_flag, p.status)) break;   // V landed
-        tc_fence_after();
-        const uint64_t dv = attn_desc_mn<HD>(sbase + L::OFF_V + st * L::KV_BYTES);   // MN-major: 16 kv rows per step
-#pragma unroll
-        for (int t = 0; t < AT_BKV / 16; ++t)                   // 16 kv = 8 columns of packed pairs per step
-          umma_bf16_ts(tmem + O_COL, tmem + P_COL + t * 8, umma_desc_advance(dv, t * attn_mn_step<HD>()), idesc_o, (j > 0) | (t > 0));
-        umma_commit(bar(9));                                    // O updated, P free
-        umma_commit(bar(5 + st));                               // V stage free
+      for (int t = 0; t < HD / 16; ++t) {
+        const uint32_t off = (t >> 2) * 16384 + (t & 3) * 32;
+        umma_bf16_w(el, tmem + S_COL, umma_desc_advance(dq, off), umma_desc_advance(dk, off), idesc_s, t > 0);
       }
+      umma_commit_w(el, bar(7));
+      umma_commit_w(el, bar(11 + st));                              // K stage free
+      return true;
+    };
+    bool ok = mbar_wait_warp(bar(0), 0, 12, abort_flag, p.status);
+    if (ok) ok = issue_s(0);
+    for (int j = 0; j < n_kv && ok; ++j) {
+      const int st = j & 1;
+      const uint32_t par = (uint32_t)j & 1u;
+      if (j + 1 < n_kv) {                                     // S of the next tile overlaps this tile's softmax
+        if (!mbar_wait_warp(bar(10), par, 18, abort_flag, p.status)) break;
+        if (!issue_s(j + 1)) break;
+      }
+      if (!mbar_wait_warp(bar(8), par, 14, abort_flag, p.status)) break;                        // P written
+      if (!mbar_wait_warp(bar(3 + st), (uint32_t)(j >> 1) & 1u, 15, abort_flag, p.status)) break;   // V landed
+      tc_fence_after();
+      const uint64_t dv = attn_desc_mn<HD>(sbase + L::OFF_V + st * L::KV_BYTES);   // MN-major: 16 kv rows per step
+#pragma unroll
+      for (int t = 0; t < AT_BKV / 16; ++t)                   // 16 kv = 8 columns of packed pairs per step
+        umma_bf16_ts_w(el, tmem + O_COL, tmem + P_COL + t * 8, umma_desc_advance(dv, t * attn_mn_step<HD>()), idesc_o, (j > 0) | (t > 0));
+      umma_commit_w(el, bar(9));                                    // O updated, P free
+      umma_commit_w(el, bar(5 + st));                               // V stage free
     }
   } else {
     const int q = warp & 3;
