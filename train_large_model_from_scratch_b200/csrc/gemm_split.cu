@@ -52,7 +52,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const SplitGemm& g = p.g;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int rank = S > 1 ? (int)cluster_ctarank() : 0;
   const int tile = (int)blockIdx.x / S;
   const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
@@ -72,7 +72,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   griddep_wait();
 
   if (warp == 0) {
@@ -102,25 +102,25 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16(SP_BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
-      int stage = 0; uint32_t phase = 0;
-      bool ok = true;
-      for (int kb = kb_lo; kb < kb_hi; ++kb) {
-        if (!mbar_wait(full_bar(stage), phase, 82, abort_flag, p.status)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t sa = sbase + stage * C::STAGE_BYTES, sb = sa + SP_A_BYTES;
-        const uint64_t ad = A_MN ? umma_smem_desc(sa, SP_BOX_MN, 1024) : umma_smem_desc(sa, 16, 1024);
-        const uint64_t bd = B_MN ? umma_smem_desc(sb, SP_BOX_MN, 1024) : umma_smem_desc(sb, 16, 1024);
-        umma_bf16(tmem, ad, bd, idesc, kb > kb_lo);
+    // by the whole warp (see umma_bf16_w): four MMAs of 48 (BN 64) or 64 cycles took 76 each to issue from one lane's own code.
+    // In us, weights out of memory: 333 x 1024 x 4096 11.6 -> 11.1, 333 x 1024 x 1024 7.2 -> 6.7, 512 x 256 x 256 3.7 -> 3.4
+    const uint32_t el = elect_one();
+    constexpr uint32_t idesc = umma_idesc_bf16(SP_BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+    int stage = 0; uint32_t phase = 0;
+    bool ok = true;
+    for (int kb = kb_lo; kb < kb_hi; ++kb) {
+      if (!mbar_wait_warp(full_bar(stage), phase, 82, abort_flag, p.status)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t sa = sbase + stage * C::STAGE_BYTES, sb = sa + SP_A_BYTES;
+      const uint64_t ad = A_MN ? umma_smem_desc(sa, SP_BOX_MN, 1024) : umma_smem_desc(sa, 16, 1024);
+      const uint64_t bd = B_MN ? umma_smem_desc(sb, SP_BOX_MN, 1024) : umma_smem_desc(sb, 16, 1024);
 #pragma unroll
-        for (int kk = 1; kk < SP_BK / 16; ++kk)
-          umma_bf16_acc(tmem, umma_desc_advance(ad, kk * (A_MN ? 2048 : 32)), umma_desc_advance(bd, kk * (B_MN ? 2048 : 32)), idesc);
-        umma_commit(empty_bar(stage));
-        if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
-      }
-      if (ok) umma_commit(acc_bar);
+      for (int kk = 0; kk < SP_BK / 16; ++kk)
+        umma_bf16_w(el, tmem, umma_desc_advance(ad, kk * (A_MN ? 2048 : 32)), umma_desc_advance(bd, kk * (B_MN ? 2048 : 32)), idesc, (kb > kb_lo) | (kk > 0));
+      umma_commit_w(el, empty_bar(stage));
+      if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
     }
+    if (ok) umma_commit_w(el, acc_bar);
   } else {
     // accumulator -> this CTA's partial tile in shared memory (every operand read of the ring has retired by then)
     const int row = (warp & 3) * 32 + lane;
