@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(DELTA_THREADS)
 attn_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* dout,
                   float* __restrict__ delta, float* __restrict__ dq_acc, int B, int T, int Hq, int hd) {
   griddep_wait();
+  griddep_launch();
   extern __shared__ float delta_s[];                       // [Hq][DELTA_T + 1]
   const int tiles_t = (T + DELTA_T - 1) / DELTA_T;
   const int b = blockIdx.x / tiles_t, t0 = (blockIdx.x % tiles_t) * DELTA_T;
@@ -127,6 +128,7 @@ __global__ void attn_dq_convert_kernel(const float* dq_acc, __nv_bfloat16* __res
                                        int Hq, int heads_total, int hd, float scale, const float* cosT,
                                        const float* sinT, const AttnBwdDst d, int dst_q0, int rot_k) {
   griddep_wait();
+  griddep_launch();
   const int half = hd / 2, vec_log = hd == 32 ? 1 : hd == 64 ? 2 : 3;          // hd / 16 items per row
   const int heads = Hq + rot_k;
   const Index total = ((Index)B * heads * T) << vec_log, step = (Index)gridDim.x * blockDim.x;
@@ -496,6 +498,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
       }
     }
     if (ok && n_it > 0) umma_commit_w(el, bar(ALL_DONE));
+    griddep_launch();
   } else if (warp < 18) {
     // ---------------------------------------------------------------- softmax warps: 32 query columns of 32 KV rows each
     const int q4 = warp & 3, g = (warp - 2) >> 2, s = g >> 1;

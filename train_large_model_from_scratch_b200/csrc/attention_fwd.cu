@@ -176,6 +176,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const AttnFwdParams 
       umma_commit_w(el, bar(9));                                    // O updated, P free
       umma_commit_w(el, bar(5 + st));                               // V stage free
     }
+    griddep_launch();
   } else {
     const int q = warp & 3;
     const int row = q * 32 + lane;                              // row inside the tile == TMEM lane

@@ -28,16 +28,25 @@ inline void count_launch(int n = 1) { g_launches += (unsigned long long)n; }
 // code = (site << 8) | detail. `status_word()` returns the device-visible pointer.
 unsigned int* status_word();
 
-// Kernels launched through launch_overlapped start when every block of the kernel before them in the stream has left, without
-// waiting for its writes to be flushed: no kernel signals its dependents earlier, so the two never compete for tensor memory.
-// What overlaps is the launch itself, and the set-up (barriers, tensor memory, descriptor fetch) with that flush. They call
-// griddep_wait() before they touch memory that another kernel reads or writes. A 333-token prompt through 12 layers
-// (87 launches) 1010 -> 793 us, an expert layer 859 -> 847 us; steps replayed as a graph did not change.
+// Kernels launched through launch_overlapped may start before the kernel in front of them in the stream is done, and call
+// griddep_wait() before they touch memory that another kernel reads or writes: it returns when that kernel has ended and its
+// writes can be seen (and, as that kernel waited in the same way, those before it). griddep_launch() lets the next kernel
+// start; it takes effect when every block of the grid has called it or ended, so no block of a grid is ever kept out by its
+// successor. A kernel that uses tensor memory calls it after its own allocation, in the warp that allocates: a block of the
+// next kernel that takes the rest of an SM's columns, or waits for them, then holds up nobody it waits for itself. The GEMM
+// and attention kernels call it when their last MMA has been issued, so that launch, barriers, tensor memory and descriptor
+// fetch of the next kernel run beside the epilogue; norms at their start. Called at the start by all of them (the next kernel's
+// blocks then sit on the few SMs that are free, two on one SM) a 333-token prompt took 703 us, not called 686, so 668.
+// A grid of more than one block per SM is launched without all this (and costs what it did): its early blocks pile up on the
+// SMs that happen to be free, eight norm blocks or two of the heaviest attention tiles on each; 3003-row norms 5.0 -> 6.3 us.
+// Steps of 512 tokens (tiny model) 1163 -> 1064 us, of 6006 tokens (8 layers of 768) 6930 -> 6580 us.
 // The kernel lives from before that wait, so what other kernels write is not read-only for its whole life: such kernels take
 // their inputs as plain pointers (no const __restrict__, from which the compiler may make read-only loads that need not stay
 // behind the wait; no __ldg).
+int num_sms();
 #ifdef __CUDACC__
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... P, typename... A>
 inline int launch_overlapped(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, A&&... args) {
   cudaLaunchConfig_t cfg{};
@@ -48,7 +57,7 @@ inline int launch_overlapped(void (*kern)(P...), dim3 grid, dim3 block, size_t s
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  cfg.numAttrs = cluster > 1 ? 2 : (int)grid.x > num_sms() ? 0 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, P(args)...);
   count_launch();
   return (int)(e != cudaSuccess ? e : cudaPeekAtLastError());
@@ -240,6 +249,13 @@ __device__ __forceinline__ void tma_load_4d(uint32_t smem_dst, const CUtensorMap
       "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
       ::"r"(smem_dst), "l"((uint64_t)map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
+}
+// The box of tma_load_2d into L2 only
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int c0, int c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"((uint64_t)map), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
@@ -524,8 +540,6 @@ int make_tmap_bf16(CUtensorMap* map, const void* base, int rank, const uint64_t*
 // same for fp32 elements (inner box extent <= 32 elements with the 128-byte swizzle)
 int make_tmap_f32(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
                   const uint32_t* box);
-
-int num_sms();
 
 // Heads per group of the attention kernels' heavy-first block order (heavy_first_decode): as many heads as keep the
 // group's tensors (`bytes_per_head` each) within `budget_bytes` of L2, or the value of the environment variable `env`

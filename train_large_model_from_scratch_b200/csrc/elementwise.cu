@@ -96,6 +96,7 @@ add_rmsnorm_fwd_reg_kernel(const float* x, const __nv_bfloat16* delta,
                            const __nv_bfloat16* w, float* __restrict__ x_new,
                            __nv_bfloat16* __restrict__ h, float* __restrict__ rstd_out, int rows, float eps) {
   griddep_wait();
+  griddep_launch();
   constexpr int D = NV * 256;
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int r = blockIdx.x * warps + warp; r < rows; r += gridDim.x * warps) {
@@ -167,6 +168,7 @@ add_rmsnorm_fwd_wide_kernel(const float* x, const __nv_bfloat16* delta,
                             const __nv_bfloat16* w, float* __restrict__ x_new,
                             __nv_bfloat16* __restrict__ h, float* __restrict__ rstd_out, int rows, int D, float eps) {
   griddep_wait();
+  griddep_launch();
   __shared__ float red[2][RMS_WIDE_MAX_WARPS];
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c0 = (warp * NV * 32 + lane) * 8;
@@ -298,6 +300,7 @@ add_rmsnorm_bwd_reg_kernel(const float* g_xnew, const __nv_bfloat16* g_h,
                            const __nv_bfloat16* w, float* __restrict__ g_x,
                            __nv_bfloat16* __restrict__ g_delta, float* __restrict__ dw_out, int rows) {
   griddep_wait();
+  griddep_launch();
   constexpr int D = NV * 256;
   __shared__ float dw_s[rms_bwd_threads<NV>() / 32][D];                      // block fold
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -382,6 +385,7 @@ add_rmsnorm_bwd_wide_kernel(const float* g_xnew, const __nv_bfloat16* g_h,
                             const __nv_bfloat16* w, float* __restrict__ g_x,
                             __nv_bfloat16* __restrict__ g_delta, float* __restrict__ dw_out, int rows, int D) {
   griddep_wait();
+  griddep_launch();
   __shared__ float red[2][RMS_WIDE_MAX_WARPS];
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c0 = (warp * NV * 32 + lane) * 8;

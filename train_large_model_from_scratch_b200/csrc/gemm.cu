@@ -253,6 +253,24 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     if (PAIR) { tmem_alloc_pair(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish_pair(); }
     else { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
   }
+  if (GROUP == 0 && !A_MN && !GATED && threadIdx.x == 0 && p.M <= p.N && p.pair_k == 0 && p.split_k == 1) {
+    // few rows: this block's weights into L2 while the kernel in front still runs (see gemm_split.cu); one tile per block
+    const int tn = (p.N + TILE_N - 1) / TILE_N, tm = (p.M + TILE_M - 1) / TILE_M;
+    if (tn * tm <= n_workers && worker < tn * tm) {
+      const TileCoord t = plain_tile(p, worker, tm, tn, TILE_N, TILE_M, (int)cta_rank * BM);
+      const int half_n0 = PAIR ? (int)cta_rank * (BN / 2) : 0, cols = PAIR ? BN / 2 : BN;
+      for (int k0 = t.k_lo; k0 < t.k_hi && t.m0 < TILE_M; k0 += BK) {
+        if (B_MN) {
+          for (int j = 0; j < cols / 64; ++j) tma_prefetch_3d(&tmB, t.b_n0 + half_n0 + 64 * j, k0, 0);
+        } else if (EPI == EPI_SWIGLU) {
+          if (!PAIR || leader) tma_prefetch_3d(&tmB, k0, t.n0, 0);
+          if (!PAIR || !leader) tma_prefetch_3d(&tmB, k0, p.N + t.n0, 0);
+        } else {
+          tma_prefetch_3d(&tmB, k0, t.b_n0 + half_n0, 0);
+        }
+      }
+    }
+  }
   griddep_wait();
   if (GROUP == 1 && warp == 2) {
     // exclusive prefix sum of the groups' row-tile counts: lane l owns groups [8 l, 8 l + 8)
@@ -478,6 +496,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       __syncwarp();
       if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
+    if (!GATED) griddep_launch();
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)
     const int q = warp & 3;                        // TMEM lane quarter this warp may read

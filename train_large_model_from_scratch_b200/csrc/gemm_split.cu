@@ -19,6 +19,7 @@ namespace tlm {
 constexpr int SP_BM = 128, SP_BK = 64, SP_THREADS = 192;
 constexpr int SP_A_BYTES = SP_BM * SP_BK * 2;
 constexpr int SP_BOX_MN = 64 * SP_BK * 2;                 // one 64(mn) x 64(k) MN-major box
+constexpr int SP_ALONE = 117 * 1024;                      // shared memory of which an SM has room for one
 
 template <int BN>
 struct SplitCfg {
@@ -73,6 +74,21 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  // Where the weights are the larger operand (few rows) they come out of memory: ask for this block's share while the kernel in
+  // front still runs. Into L2 only, so it does not matter whether that kernel writes them. 333 rows, with the same in gemm.cu:
+  // 12 layers 676 -> 644 us; 3003 rows of 768 (weights in L2 anyway) lost 1 % and stay without.
+  if (!A_MN && threadIdx.x == 0 && tm == 0 && g.M <= g.N) {
+    for (int kb = kb_lo; kb < kb_hi; ++kb) {
+      const int k0 = kb * SP_BK;
+      if (B_MN) {
+#pragma unroll
+        for (int j = 0; j < BN / 64; ++j) tma_prefetch_2d(&tmB, n0 + 64 * j, k0);
+      } else {
+        tma_prefetch_2d(&tmB, k0, n0);
+        if (EPI == SPLIT_SWIGLU) tma_prefetch_2d(&tmB, k0, g.N + n0);
+      }
+    }
+  }
   griddep_wait();
 
   if (warp == 0) {
@@ -121,6 +137,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
     }
     if (ok) umma_commit_w(el, acc_bar);
+    griddep_launch();
   } else {
     // accumulator -> this CTA's partial tile in shared memory (every operand read of the ring has retired by then)
     const int row = (warp & 3) * 32 + lane;
@@ -296,11 +313,15 @@ static int launch_split(const CUtensorMap& ma, const CUtensorMap& mb, const Spli
   auto kern = gemm_split_kernel<A_MN, B_MN, EPI, BN, S>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg<BN>::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SP_ALONE);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  return launch_overlapped(kern, dim3((unsigned)(p.tiles_m * p.tiles_n * S)), dim3(SP_THREADS), SplitCfg<BN>::SMEM, st, S, ma, mb, p);
+  // A grid that starts beside the last blocks of the kernel in front would pair up on the free SMs; with more than half of an
+  // SM's shared memory each block gets its own (333 x 1024 x 4096: 13.8 -> 11 us). Only where whole clusters of it surely fit:
+  // 144 blocks in clusters of four took a second wave.
+  const int smem = p.tiles_m * p.tiles_n * S * 4 <= num_sms() * 3 ? SP_ALONE : SplitCfg<BN>::SMEM;
+  return launch_overlapped(kern, dim3((unsigned)(p.tiles_m * p.tiles_n * S)), dim3(SP_THREADS), smem, st, S, ma, mb, p);
 }
 
 static int split_map(CUtensorMap* m, const void* ptr, long long rows, long long k, long long ld, bool mn, int box_rows) {
