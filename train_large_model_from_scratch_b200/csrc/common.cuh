@@ -223,9 +223,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
 }
 
 // The same by a whole warp that stays together: all lanes get the same answer.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, unsigned int site, volatile int* abort_flag,
                                                unsigned int* status) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, site, abort_flag, status));
+  return __all_sync(0xffffffffu, mbar_wait<CLUSTER>(bar, parity, site, abort_flag, status));
 }
 
 // ---- TMA (tiled, no multicast) ------------------------------------------------------
@@ -278,33 +279,16 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// D[tmem] (+)= A[smem] * B[smem], bf16 inputs, fp32 accumulate.
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // One lane of a converged warp, the same one every time (nonzero on that lane).
 __device__ __forceinline__ uint32_t elect_one() {
   uint32_t r;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
   return r;
 }
-// The same two and the commit for a whole converged warp, issued by the lane whose `elected` is nonzero. The operands of an
-// MMA live in uniform registers: where the loop around it is the warp's and not one lane's, they are computed there instead
-// of being moved there one by one.
+// MMA and commit of a whole converged warp, issued by the lane whose `elected` is nonzero. The operands of an MMA live in
+// uniform registers: where the loop around it is the warp's and not one lane's, they are computed there instead of being moved
+// there one by one, which took 76 cycles for each MMA.
+// D[tmem] (+)= A[smem] * B[smem], bf16 inputs, fp32 accumulate.
 __device__ __forceinline__ void umma_bf16_w(uint32_t elected, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                             uint32_t accumulate) {
   asm volatile(
@@ -313,6 +297,7 @@ __device__ __forceinline__ void umma_bf16_w(uint32_t elected, uint32_t tmem_d, u
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elected)
       : "memory");
 }
+// D[tmem] (+)= A[tmem] * B[smem]
 __device__ __forceinline__ void umma_bf16_ts_w(uint32_t elected, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
                                                uint32_t accumulate) {
   asm volatile(
@@ -321,15 +306,12 @@ __device__ __forceinline__ void umma_bf16_ts_w(uint32_t elected, uint32_t tmem_d
       ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elected)
       : "memory");
 }
+// Arrive on an mbarrier once all previously issued MMAs of the elected lane retire.
 __device__ __forceinline__ void umma_commit_w(uint32_t elected, uint32_t bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
       "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
       ::"r"(bar), "r"(elected) : "memory");
-}
-// Arrive on an mbarrier once all previously issued MMAs of this thread retire.
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -435,14 +417,6 @@ constexpr uint32_t attn_mn_step() { return HD == 32 ? 1024 : 2048; }      // byt
 __device__ __forceinline__ uint64_t umma_desc_advance(uint64_t desc, uint32_t byte_off) {
   return desc + (uint64_t)(byte_off >> 4);
 }
-// D[tmem] += A[smem] * B[smem] (accumulate always on: no predicate set-up)
-__device__ __forceinline__ void umma_bf16_acc(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc)
-      : "memory");
-}
 // ---- CTA pairs (cta_group::2) --------------------------------------------------------------------
 // Two CTAs of one cluster (ranks 0 and 1, neighbouring SMs) run one M = 256 MMA: each CTA stages its own 128 rows of A
 // and its own half of B's N rows in its own shared memory at the same offsets, the MMA is issued by one thread of
@@ -500,19 +474,21 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                               uint32_t accumulate) {
+// by a converged warp, as umma_bf16_w
+__device__ __forceinline__ void umma_bf16_pair_w(uint32_t elected, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                                 uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elected)
       : "memory");
 }
-// Arrive on the mbarrier at offset `bar` in BOTH CTAs of the pair once all MMAs issued so far by this thread retire.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+// Arrive on the mbarrier at offset `bar` in BOTH CTAs of the pair once all MMAs issued so far by the elected lane retire.
+__device__ __forceinline__ void umma_commit_pair_w(uint32_t elected, uint32_t bar) {
   asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-      ::"r"(bar), "h"((uint16_t)3)
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+      ::"r"(bar), "h"((uint16_t)3), "r"(elected)
       : "memory");
 }
 

@@ -199,8 +199,8 @@ __device__ __forceinline__ TileCoord plain_tile(const GemmParams& p, int tile_in
 // epilogue warps.
 //
 // GROUP 1 (rows grouped): the row tiles of all groups form one dense list. A warp turns row_start into the number of row
-// tiles before each group (shared memory) when the kernel starts, and every role walks its share of the list, finding
-// the group by moving forward from the previous tile's. The host only knows an upper bound of a group's rows (all of
+// tiles before each group (shared memory) when the kernel starts, and every role walks its share of the list, 32 tiles
+// looked up at a time (see get_tile). The host only knows an upper bound of a group's rows (all of
 // them): enumerating that many tiles per group and skipping the missing ones took most of the time. Gate|up + SwiGLU of
 // 65536 rows: 128 groups x 512 rows, 2 x 256 columns, K 1024: 317 -> 77 us; 8 groups, 32768 rows, 2 x 2048 columns: 255
 // -> 202 us.
@@ -236,7 +236,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
 
   constexpr int TILE_N = EPI == EPI_SWIGLU ? 128 : BN;      // output columns per tile (SwiGLU: 128 gate + 128 up)
   constexpr int TILE_M = PAIR ? 2 * BM : BM;                // rows per tile walker
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   // The SwiGLU-backward epilogue reads gate / up from global memory and is as long as the main loop of its
   // K = hidden-size tiles, so it runs on 8 warps: warps 2-5 take the left 128 columns, warps 6-9 the right.
   constexpr int EPI_WARPS = EPI == EPI_SWIGLU_BWD ? 8 : 4;
@@ -301,20 +301,23 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
   if (PAIR) cluster_sync_all();          // the peer's barriers are initialised before anything signals them
   else __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   const int tiles_n = (p.N + TILE_N - 1) / TILE_N;
   const int tiles_m = (p.M + TILE_M - 1) / TILE_M;          // GROUP 1: per group instead, see get_tile
   const int total_tiles = GROUP == 1 ? tiles_before[p.groups] * tiles_n
                                      : tiles_m * tiles_n * (GROUP == 2 ? p.groups : p.split_k);
 
-  // `grp`: the caller's group cursor (GROUP 1), 0 before its first tile; tiles are asked for in ascending order
-  auto get_tile = [&](int tile, int& grp) -> TileCoord {
+  auto coord = [&](int tile) -> TileCoord {
     if (GROUP == 0) return plain_tile(p, tile, tiles_m, tiles_n, TILE_N, TILE_M, (int)cta_rank * BM);
     TileCoord t;
     if (GROUP == 1) {                   // rows grouped: A rows [lo,hi), B = weight[g]
-      while (tile >= tiles_before[grp + 1] * tiles_n) ++grp;
-      const int g = grp, first = tiles_before[g], g_tiles = tiles_before[g + 1] - first;
+      int g = 0, end = p.groups;        // the last group that starts at or before this tile
+      while (end - g > 1) {
+        const int mid = (g + end) >> 1;
+        if (tiles_before[mid] * tiles_n <= tile) g = mid; else end = mid;
+      }
+      const int first = tiles_before[g], g_tiles = tiles_before[g + 1] - first;
       const int r = tile - first * tiles_n, tn = r / g_tiles, tm = r - tn * g_tiles;
       const int lo = p.row_start[g], hi = p.row_start[g + 1];
       // PAIR: a second half that starts past the group's end runs with every row masked
@@ -336,6 +339,32 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     }
     return t;
   };
+  // This worker's i-th tile; grouped: by a whole warp, i ascending from 0. Finding a grouped tile takes divisions and loads that
+  // wait for memory, 2300 cycles (rows grouped) and more in each role and for every tile, while the products of a 256 x 256 tile
+  // with K 256 take 2048. So the lanes find the next 32 tiles at once, one each, and a tile is fetched by shuffles. With the
+  // products issued by the whole warp, 65536 rows, 128 groups, us: K 256 to 1024 columns 69.3 -> 63.6, K 512 to 1024 columns
+  // 87.3 -> 82.5, gate | up 77.5 -> 74.7; weight gradients of 8 groups, 2048 x 1024 each, 157 -> 149.
+  auto get_tile = [&](int i, TileCoord& cache) -> TileCoord {
+    const int tile = worker + i * n_workers;
+    if (GROUP == 0) return coord(tile);
+    if ((i & 31) == 0) {
+      const int mine = tile + lane * n_workers;
+      if (mine < total_tiles) cache = coord(mine);
+    }
+    __syncwarp();
+    auto from = [&](int v) { return __shfl_sync(0xffffffffu, v, i & 31); };
+    TileCoord t;
+    t.m0 = from(cache.m0); t.n0 = from(cache.n0);
+    if (GROUP == 1) {
+      t.a_row0 = t.m0; t.b_grp = from(cache.b_grp); t.b_n0 = from(cache.b_n0); t.m_end = from(cache.m_end);
+      t.k_lo = 0; t.k_hi = p.K; t.c_grp = 0; t.valid = true;
+    } else {
+      t.a_row0 = from(cache.a_row0); t.b_grp = 0; t.b_n0 = t.n0; t.m_end = p.pair_m > 0 ? p.pair_m : p.M;
+      t.k_lo = from(cache.k_lo); t.k_hi = from(cache.k_hi); t.c_grp = from(cache.c_grp); t.valid = t.k_hi > t.k_lo;
+    }
+    return t;
+  };
+  const int n_mine = worker < total_tiles ? (total_tiles - worker + n_workers - 1) / n_workers : 0;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -349,14 +378,21 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       if (!gate_ok) *abort_flag = 1;
       asm volatile("fence.proxy.async;" ::: "memory");      // the peers' (generic-proxy) stores before this warp's TMA reads
     }
-    if (lane == 0 && (!GATED || gate_ok)) {
-      int stage = 0, grp = 0; uint32_t phase = 0;
+    if ((GROUP != 0 || lane == 0) && (!GATED || gate_ok)) {       // grouped: the warp walks the list together, lane 0 loads
+      int stage = 0; uint32_t phase = 0;
       bool ok = true;
-      for (int tile = worker; tile < total_tiles && ok; tile += n_workers) {
-        TileCoord t = get_tile(tile, grp);
+      TileCoord cache{};
+      for (int i = 0; i < n_mine && ok; ++i) {
+        const TileCoord t = get_tile(i, cache);
         if (!t.valid) continue;
         for (int k0 = t.k_lo; k0 < t.k_hi; k0 += BK) {
-          if (!mbar_wait(empty_bar(stage), phase ^ 1u, 1, abort_flag, p.status)) { ok = false; break; }
+          if (GROUP != 0) {
+            if (!mbar_wait_warp(empty_bar(stage), phase ^ 1u, 1, abort_flag, p.status)) { ok = false; break; }
+            if (lane != 0) {
+              if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+              continue;
+            }
+          } else if (!mbar_wait(empty_bar(stage), phase ^ 1u, 1, abort_flag, p.status)) { ok = false; break; }
           const uint32_t sa = smem_base + stage * STAGE_BYTES, sb = sa + A_BYTES;
           if (PAIR) {
             // both CTAs' loads of this stage complete on the leader's barrier
@@ -414,11 +450,14 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    // The whole warp walks the loop (so it can clean a ragged reduction tail in
-    // shared memory); lane 0 alone issues the MMAs and commits.
+    // The whole warp walks the loop (it cleans a ragged reduction tail in shared memory, and operands stay in uniform
+    // registers, see umma_bf16_w); one lane issues the MMAs and commits. By lane 0's own code, us: 32768 x 8192 x 1024 344 -> 334,
+    // its weight gradient 349 -> 334, gate | up + SwiGLU of 32768 x 4096 412 -> 404.
+    const uint32_t el = elect_one();
     constexpr uint32_t idesc = umma_idesc_bf16(TILE_M, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
     int stage = 0; uint32_t phase = 0;
-    int acc = 0, grp = 0; uint32_t acc_phase = 0;
+    int acc = 0; uint32_t acc_phase = 0;
+    TileCoord cache{};
     bool ok = !PAIR || leader;                      // the follower's MMA warp only allocates and frees tensor memory
     // GROUP 2, last k-block of a group: rows past this group's end belong to the next group. Clear them in the A and B
     // tiles (each k index is one 128-byte row per 64-wide box, so whole-row clearing is independent of the swizzle; the
@@ -435,14 +474,14 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     uint32_t tail_phase = 0;                        // bit s: parity of tail_bar(s)'s current phase
     if (TAIL_PAIR && !leader) {                     // ... except that it clears the tail of its own operand tiles
       bool alive = true;
-      for (int tile = worker; tile < total_tiles && alive; tile += n_workers) {
-        const TileCoord t = get_tile(tile, grp);
+      for (int i = 0; i < n_mine && alive; ++i) {
+        const TileCoord t = get_tile(i, cache);
         if (!t.valid) continue;
         const int blocks = (t.k_hi - t.k_lo + BK - 1) / BK;
         stage = (stage + blocks - 1) % STAGES;
         const int valid = t.k_hi - t.k_lo - (blocks - 1) * BK;
         if (valid < BK) {
-          if (!mbar_wait(tail_bar(stage), (tail_phase >> stage) & 1u, 5, abort_flag, p.status)) { alive = false; break; }
+          if (!mbar_wait_warp(tail_bar(stage), (tail_phase >> stage) & 1u, 5, abort_flag, p.status)) { alive = false; break; }
           tail_phase ^= 1u << stage;
           clear_tail(stage, valid);
           if (lane == 0) mbar_arrive_cluster(mapa_shared(full_bar(stage), 0));
@@ -450,49 +489,42 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
         stage = (stage + 1) % STAGES;
       }
     }
-    for (int tile = worker; tile < total_tiles && ok; tile += n_workers) {
-      TileCoord t = get_tile(tile, grp);
+    for (int i = 0; i < n_mine && ok; ++i) {
+      const TileCoord t = get_tile(i, cache);
       if (!t.valid) continue;
-      if (!mbar_wait(acce_bar(acc), acc_phase ^ 1u, 2, abort_flag, p.status)) { ok = false; break; }
+      if (!mbar_wait_warp(acce_bar(acc), acc_phase ^ 1u, 2, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       const uint32_t tmem_d = tmem_base + (uint32_t)(acc * BN);
       uint32_t accumulate = 0;
       for (int k0 = t.k_lo; k0 < t.k_hi; k0 += BK) {
         if (TAIL_PAIR && t.k_hi - k0 < BK) {
-          if (!mbar_wait(tail_bar(stage), (tail_phase >> stage) & 1u, 5, abort_flag, p.status)) { ok = false; break; }
+          if (!mbar_wait_warp(tail_bar(stage), (tail_phase >> stage) & 1u, 5, abort_flag, p.status)) { ok = false; break; }
           tail_phase ^= 1u << stage;
           clear_tail(stage, t.k_hi - k0);
-          if (!mbar_wait<true>(full_bar(stage), phase, 3, abort_flag, p.status)) { ok = false; break; }
-        } else if (!mbar_wait(full_bar(stage), phase, 3, abort_flag, p.status)) { ok = false; break; }
+          if (!mbar_wait_warp<true>(full_bar(stage), phase, 3, abort_flag, p.status)) { ok = false; break; }
+        } else if (!mbar_wait_warp(full_bar(stage), phase, 3, abort_flag, p.status)) { ok = false; break; }
         tc_fence_after();
         const uint32_t sa = smem_base + stage * STAGE_BYTES, sb = sa + A_BYTES;
         if (GROUP == 2 && !PAIR && t.k_hi - k0 < BK) clear_tail(stage, t.k_hi - k0);
         __syncwarp();
-        if (lane == 0) {
-          // K-major: 16 bf16 = 32 B further along the 128 B row;
-          // MN-major: 16 k-rows = two 8-row groups = 2048 B further.
-          const uint64_t ad0 = A_MN ? umma_smem_desc(sa, BOX_MN_BYTES, 1024) : umma_smem_desc(sa, 16, 1024);
-          const uint64_t bd0 = B_MN ? umma_smem_desc(sb, BOX_MN_BYTES, 1024) : umma_smem_desc(sb, 16, 1024);
-          if (PAIR) {
-            umma_bf16_pair(tmem_d, ad0, bd0, idesc, accumulate);
+        // K-major: 16 bf16 = 32 B further along the 128 B row;
+        // MN-major: 16 k-rows = two 8-row groups = 2048 B further.
+        const uint64_t ad0 = A_MN ? umma_smem_desc(sa, BOX_MN_BYTES, 1024) : umma_smem_desc(sa, 16, 1024);
+        const uint64_t bd0 = B_MN ? umma_smem_desc(sb, BOX_MN_BYTES, 1024) : umma_smem_desc(sb, 16, 1024);
 #pragma unroll
-            for (int kk = 1; kk < BK / UMMA_K; ++kk)
-              umma_bf16_pair(tmem_d, umma_desc_advance(ad0, kk * (A_MN ? 2048 : 32)), umma_desc_advance(bd0, kk * (B_MN ? 2048 : 32)), idesc, 1u);
-            umma_commit_pair(empty_bar(stage));   // both CTAs' producers may refill the stage
-          } else {
-          umma_bf16(tmem_d, ad0, bd0, idesc, accumulate);
-#pragma unroll
-          for (int kk = 1; kk < BK / UMMA_K; ++kk)
-            umma_bf16_acc(tmem_d, umma_desc_advance(ad0, kk * (A_MN ? 2048 : 32)), umma_desc_advance(bd0, kk * (B_MN ? 2048 : 32)), idesc);
-          umma_commit(empty_bar(stage));          // stage reusable once these MMAs retire
-          }
-          accumulate = 1;
+        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+          const uint64_t ad = umma_desc_advance(ad0, kk * (A_MN ? 2048 : 32)), bd = umma_desc_advance(bd0, kk * (B_MN ? 2048 : 32));
+          if (PAIR) umma_bf16_pair_w(el, tmem_d, ad, bd, idesc, accumulate | (kk > 0));
+          else umma_bf16_w(el, tmem_d, ad, bd, idesc, accumulate | (kk > 0));
         }
+        if (PAIR) umma_commit_pair_w(el, empty_bar(stage));   // both CTAs' producers may refill the stage
+        else umma_commit_w(el, empty_bar(stage));             // stage reusable once these MMAs retire
+        accumulate = 1;
         __syncwarp();
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
       if (!ok) break;
-      if (lane == 0) { if (PAIR) umma_commit_pair(accf_bar(acc)); else umma_commit(accf_bar(acc)); }  // accumulator complete
+      if (PAIR) umma_commit_pair_w(el, accf_bar(acc)); else umma_commit_w(el, accf_bar(acc));  // accumulator complete
       __syncwarp();
       if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
@@ -500,10 +532,11 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)
     const int q = warp & 3;                        // TMEM lane quarter this warp may read
-    int acc = 0, grp = 0; uint32_t acc_phase = 0;
+    int acc = 0; uint32_t acc_phase = 0;
     bool ok = true;
-    for (int tile = worker; tile < total_tiles && ok; tile += n_workers) {
-      TileCoord t = get_tile(tile, grp);
+    TileCoord cache{}, next_cache{};
+    for (int i = 0; i < n_mine && ok; ++i) {
+      const TileCoord t = get_tile(i, cache);
       if (!t.valid) continue;
       // EPI_HEADS_ANY: this lane's own batch entry and position, and its row of the fp32 tables: 32 (cos, sin) of the lower and
       // of the upper half-head columns [c, c + n). Requested before the accumulator is waited for and kept for all heads of
@@ -553,12 +586,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
             }
           }
         };
-        if (tile == worker) prefetch_aux(t);
-        const int nxt = tile + n_workers;
-        int ngrp = grp;
-        if (nxt < total_tiles) { const TileCoord tn = get_tile(nxt, ngrp); if (tn.valid) prefetch_aux(tn); }
+        if (i == 0) {
+          prefetch_aux(t);
+          next_cache = cache;
+        }
+        if (i + 1 < n_mine) { const TileCoord tn = get_tile(i + 1, next_cache); if (tn.valid) prefetch_aux(tn); }
       }
-      if (!mbar_wait(accf_bar(acc), acc_phase, 4, abort_flag, p.status)) { ok = false; break; }
+      if (!mbar_wait_warp(accf_bar(acc), acc_phase, 4, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       const int row = t.m0 + q * 32 + lane;
       const bool row_ok = row < t.m_end;
