@@ -23,17 +23,18 @@ constexpr int SP_ALONE = 117 * 1024;                      // shared memory of wh
 
 template <int BN>
 struct SplitCfg {
-  static constexpr int STAGES = BN == 64 ? 4 : 3;         // 96 KB ring either way: two CTAs per SM (192 KB measured the same)
+  // 96 KB ring: two CTAs per SM. A CTA that has an SM to itself takes as deep a one as it has k-blocks for (see launch_split).
+  static constexpr int STAGES = BN == 64 ? 4 : 3, MAX_STAGES = BN == 64 ? 9 : 6;
   static constexpr int STAGE_BYTES = SP_A_BYTES + BN * SP_BK * 2;
   static constexpr int PITCH = BN + 4;                    // floats per row of the partial tile (reuses the ring)
-  static constexpr int RING = STAGES * STAGE_BYTES;
-  static constexpr int SMEM = RING + 1024 /*align slack*/ + 256 /*barriers*/;
-  static_assert(SP_BM * PITCH * 4 <= RING, "the partial tile reuses the operand ring");
+  static constexpr int REST = 1024 /*align slack*/ + 256 /*barriers*/;
+  static_assert(SP_BM * PITCH * 4 <= STAGES * STAGE_BYTES, "the partial tile reuses the operand ring");
+  static_assert(MAX_STAGES * STAGE_BYTES + REST <= 227 * 1024, "shared memory of one block");
 };
 
 struct SplitParams {
   SplitGemm g;
-  int tiles_m, tiles_n;
+  int tiles_m, tiles_n, stages;
   unsigned int* status;
 };
 
@@ -44,12 +45,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   extern __shared__ uint8_t smem_raw[];
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sal = smem_raw + (sbase - smem_u32(smem_raw));
-  // barriers: full[0..STAGES), empty[STAGES..2 STAGES), accumulator full
-  const uint32_t bar0 = sbase + C::RING;
+  // barriers: full[MAX_STAGES], empty[MAX_STAGES], accumulator full
+  const int ring = p.stages * C::STAGE_BYTES;
+  const uint32_t bar0 = sbase + ring;
   auto full_bar = [&](int s) { return bar0 + 8u * s; };
-  auto empty_bar = [&](int s) { return bar0 + 8u * (C::STAGES + s); };
-  const uint32_t acc_bar = bar0 + 8u * (2 * C::STAGES);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sal + C::RING + 8 * (2 * C::STAGES + 1));
+  auto empty_bar = [&](int s) { return bar0 + 8u * (C::MAX_STAGES + s); };
+  const uint32_t acc_bar = bar0 + 8u * (2 * C::MAX_STAGES);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sal + ring + 8 * (2 * C::MAX_STAGES + 1));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const SplitGemm& g = p.g;
@@ -63,7 +65,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int kb_lo = (int)((long long)kblocks * rank / S), kb_hi = (int)((long long)kblocks * (rank + 1) / S);
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 2 * C::STAGES + 1; ++i) mbar_init(bar0 + 8u * i, 1);
+    for (int i = 0; i < 2 * C::MAX_STAGES + 1; ++i) mbar_init(bar0 + 8u * i, 1);
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmA);
@@ -114,7 +116,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         } else {
           tma_load_2d(sb, &tmB, fb, k0, n0);
         }
-        if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
+        if (++stage == p.stages) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
@@ -134,7 +136,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       for (int kk = 0; kk < SP_BK / 16; ++kk)
         umma_bf16_w(el, tmem, umma_desc_advance(ad, kk * (A_MN ? 2048 : 32)), umma_desc_advance(bd, kk * (B_MN ? 2048 : 32)), idesc, (kb > kb_lo) | (kk > 0));
       umma_commit_w(el, empty_bar(stage));
-      if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
+      if (++stage == p.stages) { stage = 0; phase ^= 1u; }
     }
     if (ok) umma_commit_w(el, acc_bar);
     griddep_launch();
@@ -308,20 +310,30 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 }
 
 // ---- host side ----------------------------------------------------------------------------------
+// Has every CTA of a plan an SM to itself? Always up to one CTA per SM without a cluster; with one only where whole clusters of
+// them surely fit (144 CTAs in clusters of four took a second wave).
+static bool one_per_sm(long long ctas, int split) { return split == 1 ? ctas <= num_sms() : ctas * 4 <= num_sms() * 3; }
+
 template <bool A_MN, bool B_MN, int EPI, int BN, int S>
-static int launch_split(const CUtensorMap& ma, const CUtensorMap& mb, const SplitParams& p, cudaStream_t st) {
+static int launch_split(const CUtensorMap& ma, const CUtensorMap& mb, SplitParams p, cudaStream_t st) {
   auto kern = gemm_split_kernel<A_MN, B_MN, EPI, BN, S>;
+  using C = SplitCfg<BN>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SP_ALONE);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::MAX_STAGES * C::STAGE_BYTES + C::REST);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
+  const int ctas = p.tiles_m * p.tiles_n * S, per_cta = ((p.g.K + SP_BK - 1) / SP_BK + S - 1) / S;
   // A grid that starts beside the last blocks of the kernel in front would pair up on the free SMs; with more than half of an
-  // SM's shared memory each block gets its own (333 x 1024 x 4096: 13.8 -> 11 us). Only where whole clusters of it surely fit:
-  // 144 blocks in clusters of four took a second wave.
-  const int smem = p.tiles_m * p.tiles_n * S * 4 <= num_sms() * 3 ? SP_ALONE : SplitCfg<BN>::SMEM;
-  return launch_overlapped(kern, dim3((unsigned)(p.tiles_m * p.tiles_n * S)), dim3(SP_THREADS), smem, st, S, ma, mb, p);
+  // SM's shared memory each block gets its own (333 x 1024 x 4096: 13.8 -> 11 us). And a ring as deep as there are k-blocks or
+  // room for: 96 KB in flight do not cover the latency of memory. Same product 10.1 -> 9.0 us, 512 x 256 x 50304 40.1 -> 31.0,
+  // 1000 x 768 x 50304 141 -> 112.
+  const bool alone = one_per_sm(ctas, S);
+  p.stages = !alone || per_cta <= C::STAGES ? C::STAGES : per_cta < C::MAX_STAGES ? per_cta : C::MAX_STAGES;
+  int smem = p.stages * C::STAGE_BYTES + C::REST;
+  if (alone && smem < SP_ALONE) smem = SP_ALONE;
+  return launch_overlapped(kern, dim3((unsigned)ctas), dim3(SP_THREADS), smem, st, S, ma, mb, p);
 }
 
 static int split_map(CUtensorMap* m, const void* ptr, long long rows, long long k, long long ld, bool mn, int box_rows) {
@@ -346,7 +358,7 @@ int split_run(const SplitGemm& g, const SplitPlan& plan, cudaStream_t st) {
   if (e) return e;
   e = split_map(&mb, g.B, g.epi == SPLIT_SWIGLU ? 2LL * g.N : g.N, g.K, g.ldb, g.b_mn, tile_n);
   if (e) return e;
-  SplitParams p{g, (g.M + SP_BM - 1) / SP_BM, (g.N + tile_n - 1) / tile_n, status_word()};
+  SplitParams p{g, (g.M + SP_BM - 1) / SP_BM, (g.N + tile_n - 1) / tile_n, 0, status_word()};
 #define TLM_SPLIT_S(A, B, E, BN)                                   \
   switch (plan.split) {                                            \
     case 1: return launch_split<A, B, E, BN, 1>(ma, mb, p, st);    \
@@ -366,28 +378,27 @@ int split_run(const SplitGemm& g, const SplitPlan& plan, cudaStream_t st) {
   return -2;
 }
 
-// Estimated time in us, fitted to 380 products (M 1 - 8192, N 256 - 50304, K 8 - 8000; every plan and the wide tiles timed with
-// operands in L2 and with weights and gradients out of memory). A k-block takes 0.24 us (64 columns, four stages) or 0.33 us
-// (128 columns: 0.27 out of L2, 0.36 where three stages are not enough for the latency of memory: 966 x 1536, K 6784 took 41.5 us
-// on 128 columns, 33.7 on 64, 35.9 on wide tiles) of a CTA, and no less than all CTAs' blocks take at 17.6 TB/s out of the whole
-// L2 (7.5 TB/s when the operands do not stay in it: 2560 x 512, K 50304 on 80 CTAs took 273 us against 224 us on wide tiles),
-// 1.3 times as long when the rows of a K-major operand do not start on 128-byte lines (2436 x 512, K 1384: 16.4 us, wide tiles
-// 14.5); plus what surrounds the main loop and the exchange of the partial tiles. Few rows: when all of A is less than 128 KB, its
-// lines come from too few places in L2, and the CTAs wait for each other there, 3.5 ns each per k-block (6000 gate | up columns,
-// K 2048, on 188 CTAs: 28 us at 24 rows, 12.3 us at 32; wide tiles 14.8). A weight gradient's C is read and written by the
-// reductions, 4 bytes at 6.5 TB/s (1024 x 3872, K 80: 9.1 us, wide tiles 7.7), and has to win clearly: the wide tiles add
-// whole TMA boxes. Of the 380 products none is more than 4 % slower than on wide tiles (28 were without the last three terms).
+// Estimated time in us, fitted to 840 products (M 16 - 8192, N 256 - 50304, K 8 - 13000; every plan and the wide tiles timed with
+// operands in L2 and with weights and gradients out of memory). A k-block of 64 / 128 columns takes 0.21 / 0.30 us of a CTA with
+// an SM and a deep ring to itself, else 0.29 / 0.31, and no less than all CTAs' blocks take at 11.7 TB/s out of the whole L2,
+// 5 % longer when the rows of a K-major operand do not start on 128-byte lines; plus what surrounds the main loop and the
+// exchange of the partial tiles. Few rows: when all of A is less than 128 KB, its lines come from too few places in L2, and the
+// CTAs wait for each other there, 5 ns each per k-block (6000 gate | up columns, K 2048, 16 rows: 19.3 us on 128-wide tiles, 18.7
+// on the wide ones). A weight gradient's C is read and written by the reductions, 4 bytes at 6.5 TB/s. Single 128-wide tiles of
+// more than 100 k-blocks count 0.42 us a block, as before deep rings, and stay where they were. A plan has to beat the wide
+// tiles by 9 %. Of 1260 products (420 of them others) the picks are 1.5 % slower than the fastest plan in the geometric mean
+// (4.5 % by the figures from before deep rings and whole-warp issue) and take 0.618 of the wide tiles' time (0.636); 8 are more
+// than 4 % slower than these (22).
 SplitPlan split_plan(const SplitGemm& g, double wide_us) {
   SplitPlan best{0, 0};
   if (!aligned_ok(g)) return best;
   const long long kblocks = (g.K + SP_BK - 1) / SP_BK, slots = 2LL * num_sms();
-  const double operand_bytes = 2.0 * g.K * ((double)g.M + (g.epi == SPLIT_SWIGLU ? 2.0 : 1.0) * g.N);
-  const double lines = (!g.a_mn && g.lda % 64 != 0) || (!g.b_mn && g.ldb % 64 != 0) ? 1.3 : 1.0;
-  const double l2_rate = operand_bytes > 64e6 ? 7.5e6 : 17.6e6;        // bytes per us
-  const double per_cta = !g.a_mn && 2.0 * g.M * g.K < 131072.0 ? 0.0035 : 0.0;
+  const double lines = (!g.a_mn && g.lda % 64 != 0) || (!g.b_mn && g.ldb % 64 != 0) ? 1.05 : 1.0;
+  const double l2_rate = 11.7e6;        // bytes per us
+  const double per_cta = !g.a_mn && 2.0 * g.M * g.K < 131072.0 ? 0.005 : 0.0;
   const double c_us = g.epi == SPLIT_F32_ACC ? 4.0 * g.M * g.N / 6.5e6 : 0.0;
-  static const double exchange[2][4] = {{0.0, 1.5, 1.3, 2.8}, {0.0, 2.2, 2.0, 2.3}};       // S = 1, 2, 4, 8
-  double best_us = (g.epi == SPLIT_F32_ACC ? 0.85 : 0.95) * wide_us;
+  static const double exchange[2][4] = {{0.0, 1.8, 1.45, 2.6}, {0.0, 3.3, 2.15, 2.7}};       // S = 1, 2, 4, 8
+  double best_us = 0.91 * wide_us;
   for (int bn = 64; bn <= 128; bn *= 2) {
     if (g.epi == SPLIT_HEADS && (g.hd > bn || bn % g.hd != 0)) continue;
     const int tile_n = g.epi == SPLIT_SWIGLU ? bn / 2 : bn;
@@ -395,11 +406,13 @@ SplitPlan split_plan(const SplitGemm& g, double wide_us) {
     for (int i = 0, s = 1; s <= 8 && s <= kblocks; ++i, s *= 2) {
       const long long ctas = tiles * s, resident = ctas < slots ? ctas : slots;
       if (ctas > (s > 1 ? num_sms() : slots)) continue;          // a second wave of clusters costs more than it saves
-      double block = bn == 64 ? 0.24 : 0.33;
+      if (s == 1 && kblocks > 100 && g.epi == SPLIT_F32_ACC) continue;      // 1800 x 768, 6416 tokens: 50 us, wide tiles 35
+      const bool alone = one_per_sm(ctas, s);
+      double block = bn == 64 ? (alone ? 0.21 : 0.29) : s == 1 && kblocks > 100 ? 0.42 : (alone ? 0.30 : 0.31);
       const double shared = (double)resident * (bn == 64 ? 24576.0 : 32768.0) / l2_rate, queue = (double)resident * per_cta;
       if (shared > block) block = shared;
       if (queue > block) block = queue;
-      const double us = (bn == 64 ? 3.4 : 3.8) + (g.a_mn ? 1.0 : 0.0) + exchange[bn / 128][i] + c_us +
+      const double us = (bn == 64 ? 3.8 : 3.9) + (g.a_mn ? 1.1 : 0.0) + exchange[bn / 128][i] + c_us +
                         (double)((kblocks + s - 1) / s) * lines * block;
       if (us < best_us) { best_us = us; best = {bn, s}; }
     }
