@@ -737,10 +737,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
 }
 
 // CTAs per KV tile. One CTA per KV tile walks over all its query heads and tiles, so the tile with the most steps bounds the
-// launch from below however idle the chip is. A cluster divides that, but every CTA of a cluster costs about 5.4 steps (12 us:
-// start-up and the exchange of dV and dK while its SM has no other CTA). The estimate is the longer of a CTA's own time and the
-// work per SM; it picked the fastest of 1, 2, 4, 8 on eleven of twelve measured shapes. With delta and conversion passes, in us:
-// 1 x 8192, 8 / 1 heads of 64 961 -> 274; 4 x 777, 16 / 2 126 -> 60; 3 x 1001, 12 / 4 66 -> 49; 2 x 256, 8 / 2 of 32 26 -> 17.
+// launch from below however idle the chip is. A cluster divides that, but every CTA of a cluster costs about 5.4 steps
+// (start-up and the exchange of dV and dK while its SM has no other CTA). The estimate is the longer of a CTA's own time and the
+// work per SM; its pick is within 1 % of the fastest of 1, 2, 4, 8 on seventeen measured shapes of all head dims. With delta and
+// conversion passes, in us, unsplit -> picked: 1 x 8192, 8 / 1 heads of 64 680 -> 194; 4 x 777, 16 / 2 94 -> 51; 3 x 1001, 12 / 4
+// 50 -> 40; 1 x 1074, 8 / 2 of 128 108 -> 41; 2 x 256, 8 / 2 of 32 20 -> 14.
 static int split_for(int n_tiles, int heads_kv, int rep) {
   const char* v = getenv("TLM_ATTN_BWD_SPLIT");          // 1, 2, 4 or 8: for tests and measurements
   const int forced = v != nullptr ? atoi(v) : 0;
