@@ -1237,13 +1237,9 @@ static int for_group_chunks(GemmParams p, int groups, const int* row_start, int 
   }
   return 0;
 }
-// Estimated time (us) of a product on this file's tiles of `tile_n` output columns, for the choice against gemm_split.cu:
-// 4.6 us around the main loops (fp32 accumulation 7.3), 0.445 us per k-block of a tile, one wave of tiles after another; fitted
-// together with the figures of split_plan.
+// Estimated time (us) of a product on this file's tiles of `tile_n` output columns, for the choice against gemm_split.cu
 static double wide_cost(int M, int N, int tile_n, int K, bool pair, int splits = 0) {
-  const int tile_m = pair ? 2 * BM : BM, walkers = pair ? num_sms() / 2 : num_sms();
-  const long long items = (long long)((M + tile_m - 1) / tile_m) * ((N + tile_n - 1) / tile_n) * (splits > 0 ? splits : 1);
-  return (splits > 0 ? 7.3 : 4.6) + (double)((items + walkers - 1) / walkers) * ((K + BK - 1) / BK) * 0.445;
+  return wide_rule(M, N, pair ? 2 * BM : BM, tile_n, K, pair ? num_sms() / 2 : num_sms(), splits);
 }
 // Operand description: `ptr` points at element (0,0); K-major operands are
 // [rows, K] with leading dimension `ld`; MN-major operands are [K, rows] with

@@ -378,46 +378,9 @@ int split_run(const SplitGemm& g, const SplitPlan& plan, cudaStream_t st) {
   return -2;
 }
 
-// Estimated time in us, fitted to 840 products (M 16 - 8192, N 256 - 50304, K 8 - 13000; every plan and the wide tiles timed with
-// operands in L2 and with weights and gradients out of memory). A k-block of 64 / 128 columns takes 0.21 / 0.30 us of a CTA with
-// an SM and a deep ring to itself, else 0.29 / 0.31, and no less than all CTAs' blocks take at 11.7 TB/s out of the whole L2,
-// 5 % longer when the rows of a K-major operand do not start on 128-byte lines; plus what surrounds the main loop and the
-// exchange of the partial tiles. Few rows: when all of A is less than 128 KB, its lines come from too few places in L2, and the
-// CTAs wait for each other there, 5 ns each per k-block (6000 gate | up columns, K 2048, 16 rows: 19.3 us on 128-wide tiles, 18.7
-// on the wide ones). A weight gradient's C is read and written by the reductions, 4 bytes at 6.5 TB/s. Single 128-wide tiles of
-// more than 100 k-blocks count 0.42 us a block, as before deep rings, and stay where they were. A plan has to beat the wide
-// tiles by 9 %. Of 1260 products (420 of them others) the picks are 1.5 % slower than the fastest plan in the geometric mean
-// (4.5 % by the figures from before deep rings and whole-warp issue) and take 0.618 of the wide tiles' time (0.636); 8 are more
-// than 4 % slower than these (22).
 SplitPlan split_plan(const SplitGemm& g, double wide_us) {
-  SplitPlan best{0, 0};
-  if (!aligned_ok(g)) return best;
-  const long long kblocks = (g.K + SP_BK - 1) / SP_BK, slots = 2LL * num_sms();
-  const double lines = (!g.a_mn && g.lda % 64 != 0) || (!g.b_mn && g.ldb % 64 != 0) ? 1.05 : 1.0;
-  const double l2_rate = 11.7e6;        // bytes per us
-  const double per_cta = !g.a_mn && 2.0 * g.M * g.K < 131072.0 ? 0.005 : 0.0;
-  const double c_us = g.epi == SPLIT_F32_ACC ? 4.0 * g.M * g.N / 6.5e6 : 0.0;
-  static const double exchange[2][4] = {{0.0, 1.8, 1.45, 2.6}, {0.0, 3.3, 2.15, 2.7}};       // S = 1, 2, 4, 8
-  double best_us = 0.91 * wide_us;
-  for (int bn = 64; bn <= 128; bn *= 2) {
-    if (g.epi == SPLIT_HEADS && (g.hd > bn || bn % g.hd != 0)) continue;
-    const int tile_n = g.epi == SPLIT_SWIGLU ? bn / 2 : bn;
-    const long long tiles = (long long)((g.M + SP_BM - 1) / SP_BM) * ((g.N + tile_n - 1) / tile_n);
-    for (int i = 0, s = 1; s <= 8 && s <= kblocks; ++i, s *= 2) {
-      const long long ctas = tiles * s, resident = ctas < slots ? ctas : slots;
-      if (ctas > (s > 1 ? num_sms() : slots)) continue;          // a second wave of clusters costs more than it saves
-      if (s == 1 && kblocks > 100 && g.epi == SPLIT_F32_ACC) continue;      // 1800 x 768, 6416 tokens: 50 us, wide tiles 35
-      const bool alone = one_per_sm(ctas, s);
-      double block = bn == 64 ? (alone ? 0.21 : 0.29) : s == 1 && kblocks > 100 ? 0.42 : (alone ? 0.30 : 0.31);
-      const double shared = (double)resident * (bn == 64 ? 24576.0 : 32768.0) / l2_rate, queue = (double)resident * per_cta;
-      if (shared > block) block = shared;
-      if (queue > block) block = queue;
-      const double us = (bn == 64 ? 3.8 : 3.9) + (g.a_mn ? 1.1 : 0.0) + exchange[bn / 128][i] + c_us +
-                        (double)((kblocks + s - 1) / s) * lines * block;
-      if (us < best_us) { best_us = us; best = {bn, s}; }
-    }
-  }
-  return best;
+  if (!aligned_ok(g)) return SplitPlan{0, 0};
+  return split_rule(g, wide_us, num_sms());
 }
 
 }  // namespace tlm
