@@ -62,3 +62,24 @@ def test_a_width_without_a_kernel_is_an_error():
     switches = [m.end() for m in re.finditer(r"switch \((?:D / 256|sp\.nv)\) \{[^\n]*\}\n#undef TLM_RMS_CASE\n", text)]
     assert len(switches) == 4
     assert all(text[at:].lstrip().startswith("return -4;") for at in switches)
+
+
+def test_waits_of_single_lanes_stay_in_single_lane_code():
+    """A wait that gives up answers lane by lane (one lane may see the phase complete, another the abort flag). In front of
+    warp-wide instructions a warp would split there for good, so `mbar_wait` is for the code of one lane, and everything that a
+    warp runs together asks `mbar_wait_warp`, whose answer is a vote."""
+    common = _source("common.cuh")
+    assert "__all_sync(0xffffffffu, mbar_wait<CLUSTER>(" in _body(common, common.index("bool mbar_wait_warp("))
+    calls = 0
+    for path in sorted(glob.glob(os.path.join(SRC, "*.cu"))):
+        text = _source(os.path.basename(path))
+        for m in re.finditer(r"\bmbar_wait(?:<\w+>)?\(", text):
+            calls += 1
+            depth, headers = 0, []
+            for i in range(m.start() - 1, -1, -1):
+                depth += {"}": 1, "{": -1}.get(text[i], 0)
+                if depth < 0:
+                    depth = 0
+                    headers.append(text[text.rindex("\n", 0, i) + 1:i])
+            assert any("lane == 0" in h for h in headers), (os.path.basename(path), text[m.start():text.index("\n", m.start())])
+    assert calls >= 4

@@ -529,10 +529,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
       const int st = it % C::STAGES, qi = j + (it0 + it) % per_head;
       const float* rows = reinterpret_cast<const float*>(sal + C::OFF_ROW) + st * 2 * AB_TILE + s * 64 + col0;
       uint8_t* drow = sal + C::OFF_DS + (C::WIDE ? 0 : it & 1) * C::DS_BYTES + s * 16384 + row * 128;
-      if (!mbar_wait(bar(RING_FULL + st), (uint32_t)(it / C::STAGES) & 1u, 28, abort_flag, p.status)) { ok = false; break; }
+      if (!mbar_wait_warp(bar(RING_FULL + st), (uint32_t)(it / C::STAGES) & 1u, 28, abort_flag, p.status)) { ok = false; break; }
       const int h = 2 * it + s, sb = C::WIDE ? 0 : h % C::NS;
       const uint32_t t_s = t_lane + C::S_COL + (C::WIDE ? s : sb) * 64 + col0, t_dp = t_lane + C::DP_COL + s * 64 + col0;
-      if (!mbar_wait(bar(S_FULL + sb), (uint32_t)(C::WIDE ? it : h / C::NS) & 1u, 29, abort_flag, p.status)) { ok = false; break; }
+      if (!mbar_wait_warp(bar(S_FULL + sb), (uint32_t)(C::WIDE ? it : h / C::NS) & 1u, 29, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       float2 pr[16];
       // two copies: the compare and select of the diagonal tiles doubled the instructions of a pair in all the others
@@ -544,7 +544,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
         for (int i = 0; i < 16; ++i) pp[i] = pack_bf16(pr[i].x, pr[i].y);
         tmem_st16(t_s, pp);
       }
-      if (!mbar_wait(bar(DP_FULL + (C::WIDE ? 0 : s)), (uint32_t)it & 1u, 33, abort_flag, p.status)) { ok = false; break; }
+      if (!mbar_wait_warp(bar(DP_FULL + (C::WIDE ? 0 : s)), (uint32_t)it & 1u, 33, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       uint32_t dd[16];
 #pragma unroll
@@ -563,7 +563,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
         }
       }
       tmem_st16(t_s + 16, dd);
-      if (!C::WIDE && it > 1 && !mbar_wait(bar(DQ_FULL + (it & 1)), ((uint32_t)(it >> 1) & 1u) ^ 1u, 30, abort_flag, p.status)) { ok = false; break; }
+      if (!C::WIDE && it > 1 && !mbar_wait_warp(bar(DQ_FULL + (it & 1)), ((uint32_t)(it >> 1) & 1u) ^ 1u, 30, abort_flag, p.status)) { ok = false; break; }
 #pragma unroll
       for (int ch = 0; ch < 4; ++ch)
         *reinterpret_cast<uint4*>(drow + ((((col0 >> 3) + ch) ^ (row & 7)) << 4)) = make_uint4(dd[4 * ch], dd[4 * ch + 1], dd[4 * ch + 2], dd[4 * ch + 3]);
@@ -573,7 +573,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(PDS + s));
     }
-    if (ok && n_it > 0) ok = mbar_wait(bar(ALL_DONE), 0, 31, abort_flag, p.status);
+    if (ok && n_it > 0) ok = mbar_wait_warp(bar(ALL_DONE), 0, 31, abort_flag, p.status);
     tc_fence_after();
     constexpr int W = C::OUT_COLS;
     const int out0 = g * W;                                    // first of this warp's columns of dV and dK
@@ -652,7 +652,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
     for (int it = 0; it < n_it; ++it) {
       const int hq = kvh * rep + (it0 + it) / per_head, qi = j + (it0 + it) % per_head;
       const int y0 = qi * AB_TILE + q4 * 32;                  // first of this warp's 32 query rows
-      if (!mbar_wait(bar(DQ_FULL + (C::WIDE ? 0 : it & 1)), (uint32_t)(C::WIDE ? it : it >> 1) & 1u, 32, abort_flag, p.status)) break;
+      if (!mbar_wait_warp(bar(DQ_FULL + (C::WIDE ? 0 : it & 1)), (uint32_t)(C::WIDE ? it : it >> 1) & 1u, 32, abort_flag, p.status)) break;
       tc_fence_after();
       constexpr int COLS = HD < 64 ? HD : 64;                 // in registers at a time
 #pragma unroll

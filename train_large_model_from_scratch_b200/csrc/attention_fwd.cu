@@ -186,7 +186,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const AttnFwdParams 
     bool ok = true;
     for (int j = 0; j < n_kv; ++j) {
       const uint32_t par = (uint32_t)j & 1u;
-      if (!mbar_wait(bar(7), par, 16, abort_flag, p.status)) { ok = false; break; }
+      if (!mbar_wait_warp(bar(7), par, 16, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       const bool diag = (j == qt);
       // ---- the whole S row (128 fp32) moves to registers in one go; S may then be overwritten by the next
@@ -232,7 +232,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const AttnFwdParams 
       // ---- only now is the previous tile's P V needed to be complete (P is overwritten, O may be rescaled):
       // by this time it is, so the wait costs nothing
       if (j > 0) {
-        if (!mbar_wait(bar(9), par ^ 1u, 17, abort_flag, p.status)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(9), par ^ 1u, 17, abort_flag, p.status)) { ok = false; break; }
         tc_fence_after();
         if (__any_sync(0xffffffffu, grow)) {
 #pragma unroll
@@ -255,7 +255,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const AttnFwdParams 
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(8));
     }
-    if (ok) ok = mbar_wait(bar(9), (uint32_t)(n_kv - 1) & 1u, 19, abort_flag, p.status);
+    if (ok) ok = mbar_wait_warp(bar(9), (uint32_t)(n_kv - 1) & 1u, 19, abort_flag, p.status);
     const int t_row = q0 + row;
     if (ok) {
       tc_fence_after();

@@ -143,7 +143,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   } else {
     // accumulator -> this CTA's partial tile in shared memory (every operand read of the ring has retired by then)
     const int row = (warp & 3) * 32 + lane;
-    if (mbar_wait(acc_bar, 0, 83, abort_flag, p.status)) {
+    if (mbar_wait_warp(acc_bar, 0, 83, abort_flag, p.status)) {
       tc_fence_after();
       const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
       float* dst = reinterpret_cast<float*>(sal) + row * C::PITCH;
