@@ -1,5 +1,6 @@
 """The choice between the GEMM's small-tile plans and its wide tiles (csrc/gemm_cost.h), as a host program."""
 import os
+import re
 import shutil
 import subprocess
 
@@ -18,6 +19,8 @@ static SplitPlan pick(int M, int N, int K, int epi) {           // 148 SMs, cont
   const bool pair = M >= 256;
   return split_rule(g, wide_rule(M, N, pair ? 256 : 128, epi == SPLIT_SWIGLU ? 128 : 256, K, pair ? 74 : 148, epi == SPLIT_F32_ACC ? 1 : 0), 148);
 }
+static_assert(weights_ahead_end(0, 50304) == 384 && weights_ahead_end(128, 512) == 512 && weights_ahead_end(64, 65) == 65 && weights_ahead_end(0, 0) == 0, "");
+static_assert(148 * (weights_ahead_end(0, 1 << 30) / 64) * 32768 <= (126 << 20) / 4, "a full chip of 256-wide blocks stays in a quarter of L2");
 int main() {
   int M, N, K, epi;
   while (std::scanf("%d %d %d %d", &M, &N, &K, &epi) == 4) { const SplitPlan p = pick(M, N, K, epi); std::printf("%d %d\n", p.bn, p.split); }
@@ -61,3 +64,16 @@ def test_no_plan_changes_at_a_line_in_the_reduction(picks, epi):
         for N in (256, 512, 768, 1024, 1536, 2048, 3072):
             got = picks([(M, N, 64 * b, epi) for b in blocks])
             assert len(set(got)) == 1, (M, N, list(zip(blocks, got)))
+
+
+@pytest.mark.parametrize("name", ["gemm.cu", "gemm_split.cu"])
+def test_weights_are_asked_for_ahead_only_so_far(name):
+    """A block's requests ahead of its turn end at `weights_ahead_end` (bounds: the program above) and do not come from thread 0,
+    whose own loads would queue behind them."""
+    with open(os.path.join(CSRC, name)) as f:
+        text = f.read()
+    first = text.index("tma_prefetch_2d(&tmB") if name == "gemm_split.cu" else text.index("tma_prefetch_3d(&tmB")
+    block = text[text.rindex("if (", 0, text.rindex("M <= ", 0, first)):text.index("griddep_wait();", first)]
+    assert "threadIdx.x == 64" in block and len(re.findall(r"tma_prefetch_\dd", block)) == len(re.findall(r"tma_prefetch_\dd", text))
+    loops = re.findall(r"for \(int k[b0][^;]*; ([^;]*);", block)
+    assert loops == ["k0 < end"] and "weights_ahead_end(" in block

@@ -253,13 +253,14 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
     if (PAIR) { tmem_alloc_pair(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish_pair(); }
     else { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
   }
-  if (GROUP == 0 && !A_MN && !GATED && threadIdx.x == 0 && p.M <= p.N && p.pair_k == 0 && p.split_k == 1) {
-    // few rows: this block's weights into L2 while the kernel in front still runs (see gemm_split.cu); one tile per block
+  if (GROUP == 0 && !A_MN && !GATED && threadIdx.x == 64 && p.M <= p.N && p.pair_k == 0 && p.split_k == 1) {
+    // few rows: this block's first weights into L2 while the kernel in front still runs (see weights_ahead_end); one tile per block
     const int tn = (p.N + TILE_N - 1) / TILE_N, tm = (p.M + TILE_M - 1) / TILE_M;
     if (tn * tm <= n_workers && worker < tn * tm) {
       const TileCoord t = plain_tile(p, worker, tm, tn, TILE_N, TILE_M, (int)cta_rank * BM);
       const int half_n0 = PAIR ? (int)cta_rank * (BN / 2) : 0, cols = PAIR ? BN / 2 : BN;
-      for (int k0 = t.k_lo; k0 < t.k_hi && t.m0 < TILE_M; k0 += BK) {
+      const int end = t.m0 < TILE_M ? weights_ahead_end(t.k_lo, t.k_hi) : t.k_lo;
+      for (int k0 = t.k_lo; k0 < end; k0 += BK) {
         if (B_MN) {
           for (int j = 0; j < cols / 64; ++j) tma_prefetch_3d(&tmB, t.b_n0 + half_n0 + 64 * j, k0, 0);
         } else if (EPI == EPI_SWIGLU) {

@@ -1,6 +1,12 @@
-// Which products run on the small tiles of gemm_split.cu and on which plan: estimated times, without device code so that a host
-// test can walk over sizes (tests/test_gemm_cost_cpu.py).
+// Which products run on the small tiles of gemm_split.cu and on which plan (estimated times), and how far a GEMM reads ahead:
+// without device code, so that a host test can walk over sizes (tests/test_gemm_cost_cpu.py).
 #pragma once
+
+#ifdef __CUDACC__
+#define TLM_COST_HD __host__ __device__ __forceinline__
+#else
+#define TLM_COST_HD inline
+#endif
 
 namespace tlm {
 
@@ -25,6 +31,16 @@ struct SplitGemm {
 };
 
 struct SplitPlan { int bn, split; };          // tile width (64 / 128), CTAs that share one tile's reduction; bn == 0: not this path
+
+// End of the part of a block's reduction [lo, hi) whose weights are asked for while the kernel in front still runs (few rows: the
+// weights are the larger operand and come out of memory). What the ring takes first, six k-blocks of 64; over the whole chip that
+// is 28 MB, which L2 keeps until it is read. The whole reduction instead (786 k-blocks of an LM head's data gradient, up to 309 MB)
+// put the first loads behind thousands of requests and read lines twice: 1024 x 1024, K 50304 291 us, 235 this way and without;
+// 333 x 1024 82, 64 and 64; 333 x 3072 300, 234 and 234. Logits of prompts whose weights do not stay in L2, without -> six
+// k-blocks (twelve gave the same): 10 layers of 2048, 32 rows 716 -> 696 us; 16 of 768, 329 rows 790 -> 780; 8 of 2048, 200 rows
+// 656 -> 644; 12 of 1024, 333 rows 672 -> 669.
+constexpr int WEIGHTS_AHEAD = 6 * 64;
+TLM_COST_HD constexpr int weights_ahead_end(int lo, int hi) { return hi - lo > WEIGHTS_AHEAD ? lo + WEIGHTS_AHEAD : hi; }
 
 // Estimated time (us) of a product on the wide tiles of gemm.cu, `tile_m` x `tile_n` outputs each, taken by `walkers`:
 // 5.4 us around the main loops (fp32 accumulation 7.2), 0.28 us per k-block of a tile, one wave of tiles after another.

@@ -76,12 +76,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-  // Where the weights are the larger operand (few rows) they come out of memory: ask for this block's share while the kernel in
-  // front still runs. Into L2 only, so it does not matter whether that kernel writes them. 333 rows, with the same in gemm.cu:
-  // 12 layers 676 -> 644 us; 3003 rows of 768 (weights in L2 anyway) lost 1 % and stay without.
-  if (!A_MN && threadIdx.x == 0 && tm == 0 && g.M <= g.N) {
-    for (int kb = kb_lo; kb < kb_hi; ++kb) {
-      const int k0 = kb * SP_BK;
+  // Few rows: the first of this block's weights into L2 while the kernel in front still runs (see weights_ahead_end), asked for by
+  // a warp that is idle until the accumulator is there. Into L2 only, so it does not matter whether that kernel writes them.
+  // 3003 rows of 768 (weights in L2 anyway) lost 1 % and stay without.
+  if (!A_MN && threadIdx.x == 64 && tm == 0 && g.M <= g.N) {
+    const int end = weights_ahead_end(kb_lo * SP_BK, kb_hi * SP_BK);
+    for (int k0 = kb_lo * SP_BK; k0 < end; k0 += SP_BK) {
       if (B_MN) {
 #pragma unroll
         for (int j = 0; j < BN / 64; ++j) tma_prefetch_2d(&tmB, n0 + 64 * j, k0);
