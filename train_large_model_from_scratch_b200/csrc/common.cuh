@@ -37,8 +37,13 @@ unsigned int* status_word();
 // and attention kernels call it when their last MMA has been issued, so that launch, barriers, tensor memory and descriptor
 // fetch of the next kernel run beside the epilogue; norms at their start. Called at the start by all of them (the next kernel's
 // blocks then sit on the few SMs that are free, two on one SM) a 333-token prompt took 703 us, not called 686, so 668.
-// A grid of more than one block per SM is launched without all this (and costs what it did): its early blocks pile up on the
-// SMs that happen to be free, eight norm blocks or two of the heaviest attention tiles on each; 3003-row norms 5.0 -> 6.3 us.
+// Early blocks pile up on the SMs that happen to be free, so a grid of more blocks than starts_early allows is launched as an
+// ordinary kernel, which also gives up the launch hidden behind the end of the kernel in front. Both sides, us: norms of 3003 rows
+// 5.7 (6.2 early), norm and GEMM of 32768 x 1024 107.6 (119.9), of 8192 x 1024 32.9 (35.5); norms of 1500 rows alone 5.4 (5.1), but
+// with the GEMM behind them 12.3 (13.1). Small-tile GEMMs run two blocks per SM by design and pile up no further: 1000 x 2048,
+// K 256 5.8 ordinary, 4.9 early; eleven such products 0.92 of the time, a step of 13 layers of 512 2529 -> 2478. Clusters start
+// early whatever their grid: split attention backward 51.3 (ordinary 52.7) for 4 x 777, 16 / 2 heads of 64, 65.0 (66.3) for
+// 2 x 1699, 8 / 4 of 128, 193 (194) for 1 x 8192, 8 / 1 of 64.
 // Steps of 512 tokens (tiny model) 1163 -> 1064 us, of 6006 tokens (8 layers of 768) 6930 -> 6580 us.
 // The kernel lives from before that wait, so what other kernels write is not read-only for its whole life: such kernels take
 // their inputs as plain pointers (no const __restrict__, from which the compiler may make read-only loads that need not stay
@@ -47,7 +52,8 @@ int num_sms();
 #ifdef __CUDACC__
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-template <typename... P, typename... A>
+// PER_SM: see starts_early
+template <int PER_SM = 1, typename... P, typename... A>
 inline int launch_overlapped(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, A&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
@@ -57,7 +63,7 @@ inline int launch_overlapped(void (*kern)(P...), dim3 grid, dim3 block, size_t s
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 2 : (int)grid.x > num_sms() ? 0 : 1;
+  cfg.numAttrs = !starts_early(grid.x, cluster, PER_SM, num_sms()) ? 0 : cluster > 1 ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, P(args)...);
   count_launch();
   return (int)(e != cudaSuccess ? e : cudaPeekAtLastError());

@@ -333,7 +333,7 @@ static int launch_split(const CUtensorMap& ma, const CUtensorMap& mb, SplitParam
   p.stages = !alone || per_cta <= C::STAGES ? C::STAGES : per_cta < C::MAX_STAGES ? per_cta : C::MAX_STAGES;
   int smem = p.stages * C::STAGE_BYTES + C::REST;
   if (alone && smem < SP_ALONE) smem = SP_ALONE;
-  return launch_overlapped(kern, dim3((unsigned)ctas), dim3(SP_THREADS), smem, st, S, ma, mb, p);
+  return launch_overlapped<2>(kern, dim3((unsigned)ctas), dim3(SP_THREADS), smem, st, S, ma, mb, p);
 }
 
 static int split_map(CUtensorMap* m, const void* ptr, long long rows, long long k, long long ld, bool mn, int box_rows) {

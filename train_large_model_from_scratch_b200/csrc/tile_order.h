@@ -1,5 +1,5 @@
-// Block order of the causal attention grids, written once for the device and for a host test
-// (tests/tile_order_host_test.cpp).
+// Block order of the causal attention grids and the choice of grids that start early, written once for the device and for
+// host tests (tests/tile_order_host_test.cpp, tests/test_tile_order_cpu.py).
 #pragma once
 
 #ifdef __CUDACC__
@@ -32,5 +32,9 @@ TLM_TILE_HD int even_group(int n_heads, int most) {
   const int groups = (n_heads + most - 1) / most;
   return (n_heads + groups - 1) / groups;
 }
+
+// May a grid start beside the last blocks of the kernel in front (see launch_overlapped)? `per_sm`: blocks of it that share an SM
+// without loss.
+TLM_TILE_HD constexpr bool starts_early(long long blocks, int cluster, int per_sm, int sms) { return cluster > 1 || blocks <= (long long)per_sm * sms; }
 
 }  // namespace tlm
