@@ -55,6 +55,22 @@ def test_kernels_that_start_early_read_through_plain_loads():
     assert "griddep_wait();" in body and "__ldg" not in body and "ld.global.nc" not in body
 
 
+def test_no_block_leaves_before_the_wait():
+    """`griddep_wait` promises that the kernel in front has ended, and with it those before, because it waited itself. A block that
+    leaves early, on an error too, breaks that for its successor."""
+    kernels = 0
+    for path in glob.glob(os.path.join(SRC, "*.cu")):
+        text = _source(os.path.basename(path))
+        for m in re.finditer(r"__global__|void gemm_body\(", text):
+            body = _body(text, m.start())
+            at = body.find("griddep_wait();")
+            if at >= 0:
+                kernels += 1
+                for r in re.finditer(r"\breturn;", body):
+                    assert "griddep_wait();" in body[:r.start()], (os.path.basename(path), body[:120])
+    assert kernels >= 9
+
+
 def test_a_width_without_a_kernel_is_an_error():
     """The norms pick their kernel with a `switch` whose every case launches and returns; should a width ever get there
     without a case, the call has to fail instead of reporting a launch that did not happen."""
