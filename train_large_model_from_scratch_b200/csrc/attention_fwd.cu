@@ -75,6 +75,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const AttnFwdParams 
   const uint32_t sbase = smem_u32(smem_raw);
   uint8_t* sal = smem_raw;
   if (sbase & 1023u) {                                // swizzled tiles need a 1024-byte aligned base
+    griddep_wait();
     if (threadIdx.x == 0) report_status(p.status, (10u << 8) | 2u);
     return;
   }
