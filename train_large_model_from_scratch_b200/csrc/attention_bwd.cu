@@ -508,17 +508,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
     const uint32_t t_lane = tmem + ((uint32_t)(q4 * 32) << 16);
     bool ok = true;
     if constexpr (C::KV_TMEM) {   // K (warps of half 0) and V (half 1) rows become tensor-memory operands, half a row per warp
-      const int c0 = (g & 1) * (HD / 2);
-      const __nv_bfloat16* src = p.qkv + (((long long)b * p.T + t_row) * heads_total + p.Hq + s * p.Hkv + kvh) * p.hd + c0;
-      uint32_t w[HD / 4];
+      static_assert(HD == 32, "half a row is 16 columns, 8 words; p.hd is HD (the scatter form has wider tiles)");
+      const int c0 = (g & 1) * 16;
+      const __nv_bfloat16* src = p.qkv + (((long long)b * p.T + t_row) * heads_total + p.Hq + s * p.Hkv + kvh) * HD + c0;
+      uint32_t w[8];
 #pragma unroll
-      for (int c = 0; c < HD / 16; ++c) {
-        const uint4 v = t_row < p.T && c0 + c * 8 < p.hd ? reinterpret_cast<const uint4*>(src)[c] : make_uint4(0, 0, 0, 0);
+      for (int c = 0; c < 2; ++c) {
+        const uint4 v = t_row < p.T ? reinterpret_cast<const uint4*>(src)[c] : make_uint4(0, 0, 0, 0);
         w[4 * c] = v.x; w[4 * c + 1] = v.y; w[4 * c + 2] = v.z; w[4 * c + 3] = v.w;
       }
-      const uint32_t col = (s == 0 ? C::K_COL : C::V_COL) + c0 / 2;
-      if constexpr (HD == 32) tmem_st8(t_lane + col, w);
-      else tmem_st16(t_lane + col, w);
+      tmem_st8(t_lane + (s == 0 ? C::K_COL : C::V_COL) + c0 / 2, w);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
