@@ -230,12 +230,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
 
 // The same by a whole warp that stays together: all lanes get the same answer. In front of warp-wide instructions (tcgen05.ld / st,
 // MMAs by an elected lane, __syncwarp, named barriers) it has to be this one: while an abort is under way one lane may see the
-// phase complete and another the flag, and a warp that splits there never meets again. The vote on the first poll costs the
-// attention kernels' softmax warps -1 to +1 %.
+// phase complete and another the flag, and a warp that splits there never meets again. The vote costs the attention kernels'
+// softmax warps -1 to +1 %; voting on the first poll already changes nothing beyond the noise.
 template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, unsigned int site, volatile int* abort_flag,
                                                unsigned int* status) {
-  if (__all_sync(0xffffffffu, mbar_try_wait<CLUSTER>(bar, parity))) return true;
   return __all_sync(0xffffffffu, mbar_wait<CLUSTER>(bar, parity, site, abort_flag, status));
 }
 
