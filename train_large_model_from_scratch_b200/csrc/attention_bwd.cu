@@ -197,15 +197,17 @@ __global__ void attn_dq_convert_kernel(const float* dq_acc, __nv_bfloat16* __res
 // P^T and dS^T, and its warps come to it only after their exponentials. Head dim 128 (WIDE) has 256 tensor-memory columns
 // beside dV and dK: scores of both halves, and dP^T in turns with dQ; a step's chain is dQ -> its way out, beside dV, dK and
 // the next scores -> dP^T -> dS, and the exponentials of the next step run beside the last link.
-// Cycles per 128 x 128 step, head dim 64 / 32: products 1664 / 832, exponentials 1024 (16 a cycle), shared memory 300 KB /
-// 184 KB at 128 B a cycle; measured 2640 / 2460, head dim 128 about 4700. Long runs are under the power cap at 1.5 - 1.7 GHz,
-// so what counts is energy: without the dQ reductions to L2 head dim 64 would take 8 % less, without any other part 2 - 4 %.
+// Cycles per 128 x 128 step, head dim 64 / 32 / 128: products 1664 / 832 / 2560, exponentials 1024 (16 a cycle); shared memory
+// moves 300 / 184 KB at head dim 64 / 32, 128 B a cycle. By ncu (B 8, T 4096, 16 / 8 heads: 457 steps and 14 blocks an SM) 2750 / 2630 / 5190, what
+// surrounds a block's steps included, about five steps each; tensor pipe 48 / 25 / 51 %, exponential unit 45 / 46 / 23 %, shared
+// memory 47 / 26 / 39 % of its cycles. Long runs are under the power cap at 1.5 - 1.7 GHz, so what counts is energy: without the dQ
+// reductions to L2 head dim 64 would take 8 % less, without any other part 2 - 4 %.
 // In us with the delta and conversion passes, in sequence, against the form before (scores [q][kv], P and dS through shared
-// memory, eight softmax warps that also flushed dQ, products issued by one lane's own code):
-//   B 8, T 4096, 16 / 8 heads of 64: 1115 -> 974     B 1, T 32768, the same: 7440 -> 6270
-//   B 8, T 4096, 32 / 4 heads of 32: 2083 -> 1520    B 2, T 4096, 24 / 8 heads of 128: 941 -> 774
-// The one lane was the largest part: every MMA operand then goes from an ordinary to a uniform register on its own, and a
-// step's products took 76 cycles each to issue, whatever their size (see umma_bf16_w).
+// memory, eight softmax warps that also flushed dQ, products issued by one lane's own code, a smaller last group of heads):
+//   B 8, T 4096, 16 / 8 heads of 64: 1098 -> 930     B 1, T 32768, the same: 7400 -> 6040
+//   B 8, T 4096, 32 / 4 heads of 32: 2055 -> 1350    B 2, T 4096, 24 / 8 heads of 128: 929 -> 667
+// The parts were not timed one by one. What was measured is that a step's products, issued by one lane's own code, took 76 cycles
+// each whatever their size (see umma_bf16_w), more than those of 64 columns run.
 template <int HD>
 struct AttnBwdCfg {
   static constexpr bool WIDE = HD == 128;
@@ -739,7 +741,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
 // CTAs per KV tile. One CTA per KV tile walks over all its query heads and tiles, so the tile with the most steps bounds the
 // launch from below however idle the chip is. A cluster divides that, but every CTA of a cluster costs about 5.4 steps
 // (start-up and the exchange of dV and dK while its SM has no other CTA). The estimate is the longer of a CTA's own time and the
-// work per SM; its pick is within 1 % of the fastest of 1, 2, 4, 8 on seventeen measured shapes of all head dims. With delta and
+// work per SM; its pick was within 1 % of the fastest of 1, 2, 4, 8 on seventeen measured shapes of all head dims. With delta and
 // conversion passes, in us, unsplit -> picked: 1 x 8192, 8 / 1 heads of 64 680 -> 194; 4 x 777, 16 / 2 94 -> 51; 3 x 1001, 12 / 4
 // 50 -> 40; 1 x 1074, 8 / 2 of 128 108 -> 41; 2 x 256, 8 / 2 of 32 20 -> 14.
 static int split_for(int n_tiles, int heads_kv, int rep) {
@@ -811,9 +813,9 @@ static int attn_bwd_impl(const void* qkv, const void* o, const void* dout, const
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status_word(); p.hd = hd; p.cosT = cosT; p.sinT = sinT;
   p.n_dst = n_dst; p.dst_rows = dst_rows; p.dst_heads = dst_heads; p.dst_q0 = dst_q0; p.dst_k0 = dst_k0; p.dst_v0 = dst_v0;
   // per (batch, KV head): Q, dO, dQ (fp32 accumulator + bf16 result) of its query heads, K, V, dK, dV. In us with the delta and
-  // conversion passes: B 8, T 4096, 16 / 8 heads of 64: 930 with groups of 8 - 16, 957 with 32, 1040 with all 64.
-  // Groups of one size (even_group): 24 / 8 heads of 128, B 2, T 4096, in 4 x 4 instead of 5 + 5 + 5 + 1: 740 -> 652;
-  // 32 / 4 heads of 32, B 8, in 4 x 8 instead of 10 + 10 + 10 + 2: 1494 -> 1287
+  // conversion passes: B 8, T 4096, 16 / 8 heads of 64: 910 - 925 with groups of 4 - 16, 957 with 32, 1055 with all 64.
+  // What is left for the last group counts (even_group): 24 / 8 heads of 128, B 2, T 4096, 4 x 4 650, 5 + 5 + 5 + 1 730, 6 + 6 + 4 720,
+  // 2 x 8 650; 32 / 4 heads of 32, B 8, 4 x 8 1345, 10 + 10 + 10 + 2 1515, 5 x 6 + 2 1478, 2 x 16 1367
   p.head_group = attn_head_group("TLM_ATTN_BWD_GROUP", (long long)T * hd * (10LL * (Hq / Hkv) + 8), 112LL << 20, B * Hkv);
   AttnBwdDst dd{};
   dd.n = n_dst; dd.rows = dst_rows; dd.heads = dst_heads;

@@ -136,9 +136,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const AttnFwdParams 
       }
     }
   } else if (warp == 1) {
-    // The warp stays together and one lane issues, so that the operands are computed in uniform registers (see umma_bf16_w): as
-    // one lane's own code a tile's 12 MMAs took 76 cycles each, longer than they run. Long runs, in us: B 8, T 4096, 16 heads of
-    // 64 467 -> 432, 32 heads of 32 833 -> 765; B 2, 24 heads of 128 275 -> 264.
+    // The warp stays together and one lane issues (see umma_bf16_w): as one lane's own code a tile's 12 MMAs took 76 cycles each
+    // to issue, longer than they run. Long runs, in us: B 8, T 4096, 16 heads of 64 452 -> 424, 32 heads of 32 832 -> 780; B 2, 24
+    // heads of 128 269 -> 268. By ncu (B 8, 16 / 8 heads) the exponential unit is busy 65 / 68 / 43 % of the cycles at head dim
+    // 64 / 32 / 128, the tensor pipe 32 / 17 / 42 %.
     // Descriptors are built once per tile and advanced with one add per MMA.
     const uint32_t el = elect_one();
     constexpr uint32_t idesc_s = umma_idesc_bf16(AT_BQ, AT_BKV, 0, 0);
@@ -333,9 +334,11 @@ static int attn_fwd_impl(const void* qkv, void* o, float* lse, int B, int T, int
   p.scale_log2 = scale * 1.4426950408889634f; p.scale = scale; p.status = status_word();
   p.n_dst = n_dst; p.dst_rows = dst_rows; p.dst_heads = dst_heads; p.dst_head0 = dst_head0; p.hd = hd;
   for (int i = 0; i < n_dst; ++i) p.o_dst[i] = (__nv_bfloat16*)o_dst[i];
-  // a head's Q, K, V and O rows; at B 8, T 4096, 16 heads of 64 groups of 16 - 32 heads are best (0.45 ms against 0.49 ms with
-  // each head's tiles adjacent), all 128 heads at once are no better alone and lose to L2 misses in a step. 64 MB (48 MB before):
-  // 16 heads of 64, T 32768, in four groups of 4 instead of five of 3 and one of 1: 3270 -> 3160 us
+  // a head's Q, K, V and O rows, groups within 64 MB of them. B 8, T 4096, 16 heads of 64: 435 us with groups of 22 - 43, 459 with
+  // each head's tiles adjacent; all 128 heads at once are no better alone and lose to L2 misses in a step. Against 48 MB, 16 heads
+  // of 64: T 28000 2224 us (groups of 4) and 2327 (3), T 30000 2550 and 2662, T 32768 3031 and 3137; but T 36000 3762 (3) and 3687
+  // (2), T 40000 4635 and 4410; T 24000 1653 either way (4; 6: 1646, 8: 1632). 16 of 128: T 16384 1166 (4) and 1201 (3), T 18000 1446
+  // (3) and 1406 (2). So it is groups of three that lose, five and a rest of one, wherever the budget puts them (see even_group).
   p.head_group = attn_head_group("TLM_ATTN_FWD_GROUP", 8LL * T * hd, 64LL << 20, B * Hq);
   return hd == 128 ? launch_fwd<128>(map, p, st) : hd == 64 ? launch_fwd<64>(map, p, st) : launch_fwd<32>(map, p, st);
 }

@@ -43,7 +43,10 @@ unsigned int* status_word();
 // with the GEMM behind them 12.3 (13.1). Small-tile GEMMs run two blocks per SM by design and pile up no further: 1000 x 2048,
 // K 256 5.8 ordinary, 4.9 early; eleven such products 0.92 of the time, a step of 13 layers of 512 2529 -> 2478. Clusters start
 // early whatever their grid: split attention backward 51.3 (ordinary 52.7) for 4 x 777, 16 / 2 heads of 64, 65.0 (66.3) for
-// 2 x 1699, 8 / 4 of 128, 193 (194) for 1 x 8192, 8 / 1 of 64.
+// 2 x 1699, 8 / 4 of 128, 193 (194) for 1 x 8192, 8 / 1 of 64. Attention forward of 149 - 296 blocks is ordinary: in a row with itself
+// it loses 1 us (3 x 1001, 12 heads of 64 16.4, early 15.2), between its GEMMs and a norm it does not (36.3, early 37.3; 1 x 3000
+// 55.6, early 61.2). So are the delta and conversion passes of its backward: 1 us in a row, 172.8 (early 188.7) for 4 x 2048 behind
+// a GEMM.
 // Steps of 512 tokens (tiny model) 1163 -> 1064 us, of 6006 tokens (8 layers of 768) 6930 -> 6580 us.
 // The kernel lives from before that wait, so what other kernels write is not read-only for its whole life: such kernels take
 // their inputs as plain pointers (no const __restrict__, from which the compiler may make read-only loads that need not stay
@@ -294,9 +297,9 @@ __device__ __forceinline__ uint32_t elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
   return r;
 }
-// MMA and commit of a whole converged warp, issued by the lane whose `elected` is nonzero. The operands of an MMA live in
-// uniform registers: where the loop around it is the warp's and not one lane's, they are computed there instead of being moved
-// there one by one, which took 76 cycles for each MMA.
+// MMA and commit of a whole converged warp, issued by the lane whose `elected` is nonzero. Issued by one lane's own code, MMAs of any
+// size took 76 cycles each (clock reads around a step's issue); issued like this they take what they run. The likely reason:
+// an MMA's operands live in uniform registers, and are computed there only where the code around it is the warp's.
 // D[tmem] (+)= A[smem] * B[smem], bf16 inputs, fp32 accumulate.
 __device__ __forceinline__ void umma_bf16_w(uint32_t elected, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                             uint32_t accumulate) {

@@ -25,9 +25,10 @@ TLM_TILE_HD void heavy_first_decode(int linear, int n_tiles, int n_heads, int gr
   head = g * group + (r - tile_rank * g_heads);
 }
 
-// Group size for at most `most` heads a group: the same number of groups, all of about one size. The chip runs dry at the end of
-// the last group, from the heaviest of its tiles on, and a small rest of heads has too few tiles to fill it beside those: 32
-// heads of 8 x 32 steps in groups of 10 + 10 + 10 + 2 took 1104 steps' time on 148 SMs, in four of 8 949 (total / 148 is 913).
+// Group size for at most `most` heads a group: the smallest that needs no more groups, so that the last group, which takes what is
+// left, is as large as that allows. The chip runs dry at the end of the last group, from the heaviest of its tiles on, and a
+// small rest of heads has too few tiles to fill it beside those: 32 heads of 8 x 32 steps in groups of 10 + 10 + 10 + 2 took 1104
+// steps' time on 148 SMs, in four of 8 949 (total / 148 is 913). A small rest can remain: 16 heads of at most 3 are 5 x 3 + 1.
 TLM_TILE_HD int even_group(int n_heads, int most) {
   const int groups = (n_heads + most - 1) / most;
   return (n_heads + groups - 1) / groups;
