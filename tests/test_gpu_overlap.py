@@ -45,7 +45,7 @@ def test_a_chain_of_kernels_is_the_same_with_and_without_waiting(T, D, n_q, n_kv
 # ---------------------------------------------------------------------- backward kernels, against a process that launches one by one
 # B, T, query / KV heads, head dim, MLP width, CTAs that share a KV tile (0: the rule's choice). T <= 128 has one KV tile, and dQ
 # is one sum; 40 x 128 and 5 x 1000 rows have more than 148 blocks in the pass that also zeroes the dQ accumulator, the others a
-# memset; 160 rows of 256 with 2048-wide products run small tiles two blocks to an SM.
+# memset. Those two, 1 x 777 and 2 x 500 have small-tile products of 160 to 256 blocks, two to an SM.
 BACKWARD = [(3, 100, 8, 2, 32, 520, 0), (2, 128, 4, 4, 64, 512, 0), (40, 128, 4, 2, 64, 1024, 0), (1, 65, 4, 2, 128, 264, 0),
             (1, 777, 8, 2, 64, 1032, 1), (1, 777, 8, 2, 64, 1032, 4), (2, 500, 4, 2, 128, 2048, 2), (5, 1000, 8, 2, 32, 512, 0)]
 
